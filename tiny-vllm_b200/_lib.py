@@ -124,6 +124,7 @@ SIGNATURES = {
 
 _lock = threading.Lock()
 _lib = None
+_native = None
 
 
 class B200QError(RuntimeError):
@@ -167,6 +168,26 @@ def lib() -> ctypes.CDLL:
                     f"{ABI_VERSION}: rebuild with `python tiny-vllm_b200/build.py`")
             _lib = handle
     return _lib
+
+
+def native():
+    """The CPython binding of the hot calls (``csrc/torch_binding.cpp``), over the same library."""
+    global _native
+    if _native is not None:
+        return _native
+    lib()   # loads libb200q.so and checks that the build is current
+    with _lock:
+        if _native is None:
+            import importlib.util
+
+            import torch  # noqa: F401  (its shared libraries must be loaded first)
+            path = LIB_PATH.parent / "_b200q_torch.so"
+            spec = importlib.util.spec_from_file_location("_b200q_torch", path)
+            module = importlib.util.module_from_spec(spec)
+            spec.loader.exec_module(module)
+            module.set_error_handler(check)
+            _native = module
+    return _native
 
 
 def check_device(where: str = "device status") -> None:

@@ -1,4 +1,5 @@
-"""Builds libb200q.so (the C-ABI CUDA library) in-tree with nvcc for sm_100a.
+"""Builds libb200q.so (the C-ABI CUDA library) in-tree with nvcc for sm_100a, and beside it
+``_b200q_torch.so``, the CPython binding of the hot calls (tensors in, tensors out).
 
 Run as ``python tiny-vllm_b200/build.py`` or call :func:`build`.  The library is
 written to ``tiny-vllm_b200/lib/libb200q.so``; a hash of the sources and flags is
@@ -12,6 +13,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
@@ -19,6 +21,8 @@ PKG_DIR = Path(__file__).resolve().parent
 CSRC = PKG_DIR / "csrc"
 LIB_DIR = PKG_DIR / "lib"
 LIB_PATH = LIB_DIR / "libb200q.so"
+BINDING_SRC = CSRC / "torch_binding.cpp"
+BINDING_PATH = LIB_DIR / "_b200q_torch.so"
 HEADER = PKG_DIR.parent / "include" / "b200q.h"
 
 SOURCES = ["api.cu", "act_quant.cu", "act_quant_fused.cu", "gemm_simt.cu", "gemm_umma.cu", "gemm_umma_w8a16.cu", "gemm_umma_w8a16_ts.cu",
@@ -39,9 +43,38 @@ def _nvcc() -> str:
     return cand
 
 
+def _torch_version() -> str:
+    import torch
+    return torch.__version__
+
+
+def _binding_flags() -> list[str]:
+    import torch
+    return ["-O2", "-std=c++17", "-fPIC", "-shared",
+            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+
+
+def _build_binding() -> None:
+    """The CPython extension over libb200q.so and torch's own libraries (no GPU needed)."""
+    import torch
+    site = Path(torch.__file__).resolve().parent
+    cuda = Path(_nvcc()).resolve().parent.parent
+    cmd = [os.environ.get("CXX", "g++"), *_binding_flags(), str(BINDING_SRC), "-o", str(BINDING_PATH),
+           f"-I{site / 'include'}", f"-I{site / 'include' / 'torch' / 'csrc' / 'api' / 'include'}",
+           f"-I{sysconfig.get_path('include')}", f"-I{cuda / 'include'}",
+           f"-L{LIB_DIR}", "-l:libb200q.so", "-Wl,-rpath,$ORIGIN",
+           f"-L{site / 'lib'}", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python", "-lc10",
+           "-lc10_cuda"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        sys.stderr.write(r.stdout + r.stderr)
+        raise RuntimeError("compiling the CPython binding failed")
+
+
 def _source_hash() -> str:
     h = hashlib.sha256()
-    h.update(" ".join(NVCC_FLAGS).encode())
+    h.update(" ".join(NVCC_FLAGS + _binding_flags()).encode())
+    h.update(f"{sys.version_info[:2]} {_torch_version()}".encode())   # the binding's ABI
     files = sorted(CSRC.glob("*")) + [HEADER]
     for f in files:
         if f.is_file():
@@ -52,11 +85,12 @@ def _source_hash() -> str:
 
 def is_current() -> bool:
     stamp = LIB_DIR / ".build_hash"
-    return LIB_PATH.exists() and stamp.exists() and stamp.read_text().strip() == _source_hash()
+    return LIB_PATH.exists() and BINDING_PATH.exists() and stamp.exists() and stamp.read_text().strip() == _source_hash()
 
 
 def build(force: bool = False, verbose: bool = False) -> Path:
-    """Compiles every .cu of csrc/ and links the shared library.  Returns its path."""
+    """Compiles every .cu of csrc/, links the shared library and builds the CPython binding.
+    Returns the library's path."""
     if not force and is_current():
         return LIB_PATH
     nvcc = _nvcc()
@@ -84,6 +118,7 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     if r.returncode != 0:
         sys.stderr.write(r.stdout + r.stderr)
         raise RuntimeError("link of libb200q.so failed")
+    _build_binding()
     (LIB_DIR / ".build_hash").write_text(_source_hash())
     return LIB_PATH
 

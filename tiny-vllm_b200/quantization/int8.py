@@ -9,7 +9,7 @@ from __future__ import annotations
 import torch
 from torch import nn
 
-from .base import QuantMethod, frozen
+from .base import QuantMethod, frozen, linear_params
 from .cuda import apply_int8_weight_only_linear
 
 
@@ -24,8 +24,8 @@ class Int8WeightOnlyQuantMethod(QuantMethod):
 
     def apply(self, x: torch.Tensor, layer: nn.Module,
               bias: torch.Tensor | None = None) -> torch.Tensor:
-        chosen_bias = bias if bias is not None else layer.bias
-        return apply_int8_weight_only_linear(x, layer.qweight, layer.scales, chosen_bias)
+        qweight, scales, own_bias = linear_params(layer, "qweight", "scales", "bias")
+        return apply_int8_weight_only_linear(x, qweight, scales, own_bias if bias is None else bias)
 
     def apply_row_parallel(self, x: torch.Tensor, layer: nn.Module, bias, comm):
         """Multiply and sum over the tensor-parallel ranks in one GEMM kernel (decode-sized

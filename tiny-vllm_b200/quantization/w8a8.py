@@ -10,8 +10,8 @@ from __future__ import annotations
 import torch
 from torch import nn
 
-from .base import QuantMethod, frozen
-from .cuda import apply_w8a8_linear, quantize_activation_int8
+from .base import QuantMethod, frozen, linear_params
+from .cuda import apply_w8a8_linear, quantize_activation_int8, w8a8_linear_dynamic
 
 
 class W8A8QuantMethod(QuantMethod):
@@ -26,14 +26,16 @@ class W8A8QuantMethod(QuantMethod):
 
     def apply(self, x: torch.Tensor, layer: nn.Module,
               bias: torch.Tensor | None = None) -> torch.Tensor:
+        qweight, w_scales, own_bias = linear_params(layer, "qweight", "w_scales", "bias")
+        bias = own_bias if bias is None else bias
+        if x.is_cuda:
+            y = w8a8_linear_dynamic(x, qweight, w_scales, bias)
+            if y is not None:
+                return y
+        # inputs the one-call form does not take: strided, of a wrong type, not on the GPU
         x_q, a_scales = self.quantize_activation(x)
-        n_out = layer.qweight.shape[0]
-        return apply_w8a8_linear(
-            x_q, a_scales, layer.qweight, layer.w_scales,
-            bias=layer.bias if bias is None else bias,
-            out_dtype=x.dtype,
-            out_shape=(*x.shape[:-1], n_out),
-        )
+        return apply_w8a8_linear(x_q, a_scales, qweight, w_scales, bias=bias, out_dtype=x.dtype,
+                                 out_shape=(*x.shape[:-1], qweight.shape[0]))
 
     def apply_quantized(self, x_q: torch.Tensor, a_scales: torch.Tensor, layer: nn.Module,
                         out_dtype: torch.dtype, bias: torch.Tensor | None = None,
@@ -45,8 +47,9 @@ class W8A8QuantMethod(QuantMethod):
         always quantises itself: ``nanovllm/quantization/w8a8.py:25-40``.)  ``out``: a
         contiguous ``[tokens, out_features]`` tensor to write into, e.g. ``comm.buffer(...)`` of
         the tensor-parallel communicator when ``comm.reduce_rmsnorm_quant`` consumes the result."""
-        return apply_w8a8_linear(x_q, a_scales, layer.qweight, layer.w_scales,
-                                 bias=layer.bias if bias is None else bias,
+        qweight, w_scales, own_bias = linear_params(layer, "qweight", "w_scales", "bias")
+        return apply_w8a8_linear(x_q, a_scales, qweight, w_scales,
+                                 bias=own_bias if bias is None else bias,
                                  out_dtype=out_dtype, out_shape=out_shape, out=out)
 
     def apply_row_parallel(self, x: torch.Tensor, layer: nn.Module, bias, comm):
