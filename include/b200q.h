@@ -203,7 +203,7 @@ enum {
   B200Q_KNOB_FLAGS = 1,            /* tcgen05 kernels: 1 skip epilogue arithmetic, 2 skip MMAs, 4 skip output stores */
   B200Q_KNOB_BN = 2,               /* single-CTA kernels: UMMA N */
   B200Q_KNOB_SPLITS = 3,           /* single-CTA kernels: split-K factor */
-  B200Q_KNOB_CLUSTER = 4,          /* single-CTA kernels: cluster split-K size */
+  B200Q_KNOB_CLUSTER = 4,          /* single-CTA kernels: cluster split-K size (1, 2, 4, 8) */
   B200Q_KNOB_NO_PAIR = 5,          /* 1: never take the CTA-pair kernels */
   B200Q_KNOB_NO_TS = 6,            /* 1: never take the W8A16 kernel with weights in tensor memory */
   B200Q_KNOB_TS_MIN_K = 7,         /* smallest K for that kernel */
@@ -217,6 +217,7 @@ enum {
   B200Q_KNOB_BULK_DECODE = 15,  /* persistent ring-fed decode kernels: 1 never, 2 wherever they can run */
   B200Q_KNOB_BULK_SLOTS = 16,   /* ring depth per consumer warp of those kernels (>= 2; default: what fits) */
   B200Q_KNOB_BULK_WPP = 17,     /* consumer warps per ring of the W8A8 one-token-tile kernel: 1 or 2 (default 2) */
+  B200Q_KNOB_NO_MID = 18,       /* 1: never take the two-CTAs-per-SM tcgen05 kernel (M <= 512) */
   B200Q_KNOB_COUNT = 20
 };
 int b200q_debug_set(int knob, int value);

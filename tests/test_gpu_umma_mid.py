@@ -1,0 +1,45 @@
+"""The tcgen05 kernel for tens to hundreds of tokens (two CTAs per SM, K split over a cluster whose
+CTAs share the reduction): edges of its tiles, K tails, every tile width, cluster and ring shape."""
+import pytest
+import torch
+
+from oracle import quant_linear_oracle as O
+from tests.gpu_util import bits, device_status_ok, forced_path, knobs
+import tiny_vllm_b200  # noqa: F401
+from tiny_vllm_b200 import _lib
+from tiny_vllm_b200.quantization.cuda import (apply_int8_weight_only_linear, apply_w8a8_linear,
+                                              select_path, w8a8_int32_accumulators)
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = [  # (M, N, K): one row of a tile, ragged everything, several token tiles, long and short K
+    (1, 8, 1024), (17, 72, 1040), (33, 264, 1616), (77, 4096, 1024), (128, 768, 4096),
+    (129, 1000, 528), (300, 1024, 3072), (512, 264, 2112), (40, 136, 96), (1500, 640, 1184), (20, 128, 16),
+]
+
+
+@pytest.mark.parametrize("cluster,bn", [(None, None), (1, 32), (2, 64), (4, 128), (8, 64), (1, 256)])
+@pytest.mark.parametrize("M,N,K", SHAPES)
+def test_both_schemes(M, N, K, cluster, bn, oracle_c_lib):
+    dtype = torch.bfloat16 if M % 2 else torch.float16
+    q, s = O.make_weight(N, K, seed=N + K)
+    x = O.make_activation(M, K, seed=M, dtype=dtype)
+    xq, a_s = O.quantize_per_row_dynamic(x)
+    b = (torch.randn(N, generator=torch.Generator().manual_seed(M)) * 0.1).to(dtype)
+    args = {k: v for k, v in (("CLUSTER", cluster), ("BN", bn)) if v is not None}
+    with forced_path("umma"), knobs(**args):
+        mid = [select_path(op, M, N, K).startswith("umma_mid") for op in (_lib.OP_W8A8, _lib.OP_W8A16)]
+        if cluster is None:
+            assert all(mid)
+        if mid[0]:
+            ref = O.w8a8_int32_accumulators(xq, q)
+            assert torch.equal(w8a8_int32_accumulators(xq.cuda(), q.cuda()).cpu(), ref)
+            y = apply_w8a8_linear(xq.cuda(), a_s.cuda(), q.cuda(), s.cuda(), b.cuda(), out_dtype=dtype)
+            assert torch.equal(bits(y.cpu()), bits(O.w8a8_native_epilogue(ref, a_s, s, b, dtype)))
+        if mid[1]:
+            y = apply_int8_weight_only_linear(x.cuda(), q.cuda(), s.cuda(), b.cuda())
+            m = O.tensor_metrics(O.w8a16_native_reference(x, q, s, b), y)
+            assert m["relative_l2"] <= 4e-3 and m["cosine_similarity"] >= 0.9999, m
+            again = apply_int8_weight_only_linear(x.cuda(), q.cuda(), s.cuda(), b.cuda())
+            assert torch.equal(bits(y), bits(again))     # sums in a fixed order
+    assert device_status_ok()

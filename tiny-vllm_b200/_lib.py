@@ -59,6 +59,7 @@ KNOB_PAIR_MIN_TILES = 14
 KNOB_BULK_DECODE = 15
 KNOB_BULK_SLOTS = 16
 KNOB_BULK_WPP = 17
+KNOB_NO_MID = 18
 
 # B200Q_VERSION of include/b200q.h this binding was written for
 ABI_VERSION = 2

@@ -67,34 +67,24 @@ int check_dims(int M, int N, int K) {
   return B200Q_OK;
 }
 
-// Kernel family for a W8A8 problem when nothing is forced.
-// The weight-streaming mma.sync kernel re-reads the activations once per 8 output channels,
-// so its range shrinks as N grows; thresholds from graph-replayed launches of the
-// Qwen3-0.6B projections at M = 32, 48, 64 (e.g. M = 48: 4.6 vs 7.6 us for 2048 -> 1024,
-// 7.3 vs 6.4 us for 1024 -> 6144).
-// Matrices of 8 MB and more (the 8B model): the ring-fed persistent kernels take M <= 32
-// (M <= 16 for the widest projections: 24576 channels at M = 32 run 29.9 us there against
-// 24.1 us on the tcgen05 kernel), the tcgen05 kernels the rest; the register-streaming kernel's
-// activation re-reads, N / 8 x M x K bytes from L2, rule it out (M = 64: 35-101 us against 13-24).
+// Kernel family when nothing is forced; figures from graph-replayed chains of launches.
+// Up to 16 tokens the weight-streaming mma.sync kernels: the ring-fed persistent ones for matrices of 8 MB
+// and more, the register-streaming ones below.  Both re-read the activations (the latter once per 8
+// channels), so from 17 tokens on the tcgen05 kernels are ahead — 32 tokens: 6144 x 1024 3.7 against
+// 5.4 us, 24576 x 4096 20.4 against 28.5 — except on matrices below 4 MB, whose few K blocks
+// the register-streaming kernel has in flight at once (1536 x 1088 at 32 tokens: 2.4 against
+// 3.8 us, at 48 already 4.0 against 3.6).
 int auto_path_w8a8(int M, int N, int K) {
   if (M <= debug_knob(B200Q_KNOB_SIMT_MAX_M, 0)) return B200Q_PATH_SIMT_STREAM;
-  if (static_cast<long long>(N) * K >= (8ll << 20))
-    return (M <= 16 || (M <= 32 && N < 16384)) ? B200Q_PATH_MMA_STREAM : B200Q_PATH_UMMA;
-  if (M <= 32 || (M <= 48 && N <= 4096) || (M <= 64 && N <= 2048)) return B200Q_PATH_MMA_STREAM;
+  if (M <= 16 || (M <= 32 && static_cast<long long>(N) * K < (4ll << 20))) return B200Q_PATH_MMA_STREAM;
   return B200Q_PATH_UMMA;
 }
 
-// Kernel family for a W8A16 problem when nothing is forced.
-// Same for W8A16, where the tcgen05 kernel's expansion stage costs more at small M
-// (M = 64: 7.2 vs 17.7 us for 2048 -> 1024, 12.4 vs 11.0 us for 1024 -> 6144).
-// Matrices of 8 MB and more: the ring-fed kernel takes one token tile (M <= 16); beyond it the
-// register-streaming kernel re-reads N / 8 x M x 2 K bytes of activations from L2 (M = 32 on
-// 24576 x 4096: 79 us against 52 us for the tcgen05 kernel at M = 64).
+// W8A16: the activations are twice as wide, so the lines lie lower (32 tokens: 1024 x 2048 4.2
+// against 6.2 us, 1536 x 1088 4.2 against 4.0).
 int auto_path_w8a16(int M, int N, int K) {
   if (M <= debug_knob(B200Q_KNOB_SIMT_MAX_M, 0)) return B200Q_PATH_SIMT_STREAM;
-  if (static_cast<long long>(N) * K >= (8ll << 20))
-    return M <= 16 ? B200Q_PATH_MMA_STREAM : B200Q_PATH_UMMA;
-  if (M <= 48 || (M <= 64 && N <= 4096)) return B200Q_PATH_MMA_STREAM;
+  if (M <= 16 || (M <= 32 && static_cast<long long>(N) * K < (2ll << 20))) return B200Q_PATH_MMA_STREAM;
   return B200Q_PATH_UMMA;
 }
 
@@ -130,6 +120,8 @@ int run_w8a8(GemmArgs& a) {
   }
   if (path == B200Q_PATH_UMMA && umma_pair_applicable(a.M, a.N, a.K, a.acc_out != nullptr))
     return launch_w8a8_umma_pair(a);
+  if (path == B200Q_PATH_UMMA && umma_mid_applicable(a.M, a.N, a.K, false))
+    return launch_umma_mid(a, false);
   if (path == B200Q_PATH_UMMA || path == B200Q_PATH_UMMA_SWAP) {
     UmmaPlan plan;
     if (!umma_make_plan(B200Q_OP_W8A8, a.M, a.N, a.K, path == B200Q_PATH_UMMA_SWAP, &plan))
@@ -404,6 +396,7 @@ int b200q_w8a16_gemm(const void* x, const int8_t* qweight, const float* scales, 
     return B200Q_OK;
   }
   if (path == B200Q_PATH_UMMA && umma16_pair_applicable(M, N, K)) return launch_w8a16_umma_pair(a);
+  if (path == B200Q_PATH_UMMA && umma_mid_applicable(M, N, K, true)) return launch_umma_mid(a, true);
   if (path == B200Q_PATH_UMMA && umma16_ts_applicable(M, N, K)) return launch_w8a16_umma_ts(a);
   if (path == B200Q_PATH_UMMA || path == B200Q_PATH_UMMA_SWAP) {
     UmmaPlan plan;
@@ -418,12 +411,13 @@ size_t b200q_workspace_bytes(int op, int M, int N, int K) {
   if (op == B200Q_OP_W8A16 && check_dims(M, N, K) == B200Q_OK &&
       resolve_path(op, M, N, K) == B200Q_PATH_UMMA) {
     if (umma16_pair_applicable(M, N, K)) return umma16_pair_workspace_bytes(N, K);
-    if (umma16_ts_applicable(M, N, K)) return 0;
   }
   if (op != B200Q_OP_W8A8 && op != B200Q_OP_W8A16) return 0;
   if (check_dims(M, N, K) != B200Q_OK) return 0;
   const int path = resolve_path(op, M, N, K);
   if (path != B200Q_PATH_UMMA && path != B200Q_PATH_UMMA_SWAP) return 0;
+  if (path == B200Q_PATH_UMMA && umma_mid_applicable(M, N, K, op == B200Q_OP_W8A16)) return 0;
+  if (path == B200Q_PATH_UMMA && op == B200Q_OP_W8A16 && umma16_ts_applicable(M, N, K)) return 0;
   UmmaPlan plan;
   const bool ok = op == B200Q_OP_W8A8
                       ? umma_make_plan(op, M, N, K, path == B200Q_PATH_UMMA_SWAP, &plan)
@@ -447,6 +441,8 @@ const char* b200q_select_path(int op, int M, int N, int K) {
     case B200Q_PATH_UMMA:
       if (!a16 && umma_pair_applicable(M, N, K, false)) return "umma_i8_pair_tokens256";
       if (a16 && umma16_pair_applicable(M, N, K)) return "umma_f16_pair_expand_once_tokens256";
+      if (umma_mid_applicable(M, N, K, a16))
+        return a16 ? "umma_mid_f16_expand_cluster_splitk" : "umma_mid_i8_cluster_splitk";
       if (a16 && umma16_ts_applicable(M, N, K)) return "umma_f16_tmem_weights_channels256";
       return a16 ? "umma_f16_expand_tokens128" : "umma_i8_tokens128";
     case B200Q_PATH_UMMA_SWAP:

@@ -88,13 +88,15 @@ int launch_w8a8_umma(const GemmArgs& a, const UmmaPlan& plan);
 
 // gemm_umma.cu: TMA descriptor of a dense row-major matrix viewed as bytes [rows, row_bytes],
 // box = box_bytes (128: 128-byte swizzle, 64: 64-byte swizzle) x box_rows, zero fill outside.
+// box_blocks > 0: a 3-D view [row_bytes / box_bytes][rows][box_bytes] of the whole blocks of a row,
+// whose box holds that many blocks of box_bytes x box_rows.
 // make_tensor_map encodes on every call (activations and outputs: their addresses change from
 // call to call); get_tensor_map keeps the result in a per-process cache (weights: same
 // address for the life of the model).
 bool make_tensor_map(const void* base, uint64_t rows, uint64_t row_bytes, uint32_t box_rows,
-                     uint32_t box_bytes, CUtensorMap* out);
+                     uint32_t box_bytes, CUtensorMap* out, uint32_t box_blocks = 0);
 bool get_tensor_map(const void* base, uint64_t rows, uint64_t row_bytes, uint32_t box_rows,
-                    uint32_t box_bytes, CUtensorMap* out);
+                    uint32_t box_bytes, CUtensorMap* out, uint32_t box_blocks = 0);
 
 // Test and tuning hooks (B200Q_KNOB_* of b200q.h).  Every knob is unset (the built-in
 // behaviour) until the CALLING THREAD sets it through b200q_debug_set(); nothing is read from
@@ -122,6 +124,10 @@ int launch_tp_reduce_gather(const void* stage, void* const* peer_y,
 bool umma16_pair_applicable(int M, int N, int K);
 size_t umma16_pair_workspace_bytes(int N, int K);
 int launch_w8a16_umma_pair(const GemmArgs& a);
+
+// gemm_umma_mid.cu: both schemes at up to 512 tokens, two CTAs per SM, cluster split-K
+bool umma_mid_applicable(int M, int N, int K, bool a16);
+int launch_umma_mid(const GemmArgs& a, bool a16);
 
 // gemm_umma_w8a16.cu
 bool umma16_make_plan(int M, int N, int K, int swap, UmmaPlan* plan);

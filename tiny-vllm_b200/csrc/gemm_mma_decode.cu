@@ -27,6 +27,7 @@
 #include <type_traits>
 
 #include "common.h"
+#include "expand_device.cuh"
 #include "peer_sync.cuh"
 #include "ptx_sm100.cuh"
 
@@ -189,36 +190,6 @@ __device__ __forceinline__ void mma_16<__half>(float (&c)[4], uint32_t a0, uint3
       "{%8,%9}, {%0,%1,%2,%3};"
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
-// Four int8 (one word) -> four 16-bit values (two words), exact for all 256 codes.
-template <typename T>
-__device__ __forceinline__ uint2 expand4(uint32_t w);
-template <>
-__device__ __forceinline__ uint2 expand4<__half>(uint32_t w) {
-  // 0x6400 | u is the half 1024 + u with u = q + 128; subtract 1152
-  const uint32_t t = w ^ 0x80808080u;
-  uint32_t lo = __byte_perm(t, 0x64646464u, 0x4140);
-  uint32_t hi = __byte_perm(t, 0x64646464u, 0x4342);
-  const __half2 bias = __floats2half2_rn(1152.f, 1152.f);
-  const __half2 l = __hsub2(*reinterpret_cast<__half2*>(&lo), bias);
-  const __half2 h = __hsub2(*reinterpret_cast<__half2*>(&hi), bias);
-  return make_uint2(*reinterpret_cast<const uint32_t*>(&l), *reinterpret_cast<const uint32_t*>(&h));
-}
-template <>
-__device__ __forceinline__ uint2 expand4<__nv_bfloat16>(uint32_t w) {
-  // 0x4B000000 | u is the float 2^23 + u; subtract 2^23 + 128; at most 8 significant bits
-  const uint32_t t = w ^ 0x80808080u;
-  // packed fp32 adds (each half rounds like the scalar instruction; the sums are exact anyway)
-  const float2 m = make_float2(-8388736.f, -8388736.f);
-  const float2 f01 = __fadd2_rn(make_float2(__uint_as_float(__byte_perm(t, 0x4B000000u, 0x7540)),
-                                            __uint_as_float(__byte_perm(t, 0x4B000000u, 0x7541))), m);
-  const float2 f23 = __fadd2_rn(make_float2(__uint_as_float(__byte_perm(t, 0x4B000000u, 0x7542)),
-                                            __uint_as_float(__byte_perm(t, 0x4B000000u, 0x7543))), m);
-  // the sums are integers of at most 8 significant bits: their bf16 form is the upper half of
-  // the fp32 word, taken with a byte permute (the packing conversion runs on a slower pipe)
-  return make_uint2(__byte_perm(__float_as_uint(f01.x), __float_as_uint(f01.y), 0x7632),
-                    __byte_perm(__float_as_uint(f23.x), __float_as_uint(f23.y), 0x7632));
 }
 
 // ------------------------------------------------------------------------- W8A8

@@ -377,11 +377,11 @@ EncodeTiledFn encode_fn() {
 struct MapKey {
   const void* base;
   uint64_t rows, row_bytes;
-  uint32_t box_rows, box_bytes;
+  uint32_t box_rows, box_bytes, box_blocks;
   int device;
   bool operator==(const MapKey& o) const {
     return base == o.base && rows == o.rows && row_bytes == o.row_bytes &&
-           box_rows == o.box_rows && box_bytes == o.box_bytes && device == o.device;
+           box_rows == o.box_rows && box_bytes == o.box_bytes && box_blocks == o.box_blocks && device == o.device;
   }
 };
 struct MapKeyHash {
@@ -389,7 +389,7 @@ struct MapKeyHash {
     size_t h = reinterpret_cast<size_t>(k.base);
     h ^= k.rows * 0x9E3779B97F4A7C15ull + (h << 6) + (h >> 2);
     h ^= k.row_bytes * 0xC2B2AE3D27D4EB4Full + (h << 6) + (h >> 2);
-    h ^= (static_cast<size_t>(k.box_rows) << 8) ^ static_cast<size_t>(k.device) ^
+    h ^= (static_cast<size_t>(k.box_rows) << 8) ^ (static_cast<size_t>(k.box_blocks) << 32) ^ static_cast<size_t>(k.device) ^
          (static_cast<size_t>(k.box_bytes) << 20);
     return h;
   }
@@ -398,15 +398,17 @@ struct MapKeyHash {
 }  // namespace
 
 bool make_tensor_map(const void* base, uint64_t rows, uint64_t row_bytes, uint32_t box_rows,
-                     uint32_t box_bytes, CUtensorMap* out) {
+                     uint32_t box_bytes, CUtensorMap* out, uint32_t box_blocks) {
   EncodeTiledFn fn = encode_fn();
   if (fn == nullptr) return false;
-  cuuint64_t dims[2] = {row_bytes, rows};
-  cuuint64_t strides[1] = {row_bytes};
-  cuuint32_t box[2] = {box_bytes, box_rows};
-  cuuint32_t estr[2] = {1, 1};
-  CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box,
-                  estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+  const bool blocked = box_blocks != 0;
+  if (blocked && row_bytes < box_bytes) return false;
+  cuuint64_t dims[3] = {blocked ? box_bytes : row_bytes, rows, blocked ? row_bytes / box_bytes : 1};
+  cuuint64_t strides[2] = {row_bytes, box_bytes};
+  cuuint32_t box[3] = {box_bytes, box_rows, box_blocks};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_UINT8, blocked ? 3 : 2, const_cast<void*>(base), dims,
+                  strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                   box_bytes == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {
@@ -419,12 +421,12 @@ bool make_tensor_map(const void* base, uint64_t rows, uint64_t row_bytes, uint32
 // Cached variant for matrices that keep their address (weights): encoding costs about a
 // microsecond of host time.
 bool get_tensor_map(const void* base, uint64_t rows, uint64_t row_bytes, uint32_t box_rows,
-                    uint32_t box_bytes, CUtensorMap* out) {
+                    uint32_t box_bytes, CUtensorMap* out, uint32_t box_blocks) {
   static std::mutex mu;
   static std::unordered_map<MapKey, CUtensorMap, MapKeyHash> cache;
   int dev = 0;
   cudaGetDevice(&dev);
-  MapKey key{base, rows, row_bytes, box_rows, box_bytes, dev};
+  MapKey key{base, rows, row_bytes, box_rows, box_bytes, box_blocks, dev};
   {
     std::lock_guard<std::mutex> g(mu);
     auto it = cache.find(key);
@@ -434,7 +436,7 @@ bool get_tensor_map(const void* base, uint64_t rows, uint64_t row_bytes, uint32_
     }
   }
   CUtensorMap m;
-  if (!make_tensor_map(base, rows, row_bytes, box_rows, box_bytes, &m)) return false;
+  if (!make_tensor_map(base, rows, row_bytes, box_rows, box_bytes, &m, box_blocks)) return false;
   {
     std::lock_guard<std::mutex> g(mu);
     if (cache.size() > 8192) cache.clear();
@@ -575,8 +577,8 @@ int launch_w8a8_umma(const GemmArgs& a, const UmmaPlan& plan) {
   // the weight map is cached (fixed address), the activation map is encoded per call
   const auto map_a = plan.swap ? get_tensor_map : make_tensor_map;
   const auto map_b = plan.swap ? make_tensor_map : get_tensor_map;
-  if (!map_a(base_a, plan.rows_a, a.K, kTileA, kBlockK, &ta)) return B200Q_ERR_LAUNCH;
-  if (!map_b(base_b, plan.rows_b, a.K, plan.bn, kBlockK, &tb)) return B200Q_ERR_LAUNCH;
+  if (!map_a(base_a, plan.rows_a, a.K, kTileA, kBlockK, &ta, 0)) return B200Q_ERR_LAUNCH;
+  if (!map_b(base_b, plan.rows_b, a.K, plan.bn, kBlockK, &tb, 0)) return B200Q_ERR_LAUNCH;
   // Prefill orientation, 16-bit output, no split-K: outputs are transposed through shared
   // memory so that every store instruction writes complete 128-byte lines.
   const bool fast_store = !plan.swap && a.acc_out == nullptr &&

@@ -8,6 +8,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "expand_device.cuh"
+
 namespace b200q {
 namespace {
 
@@ -36,8 +38,6 @@ struct KernelParams {
   int k_blocks, splits, kb_per_split;
   int stages;
   int conv_bufs;
-  int cluster;        // CTAs per cluster splitting K (1 = off); split index = cluster rank
-  int partial_bytes;  // shared memory the cluster leader receives partial tiles in
   int tmem_cols;
   int swap;
   int n_channels;
@@ -86,37 +86,6 @@ __device__ __forceinline__ uint32_t pack2_rn<__half>(float2 v) {
 }
 
 // ------------------------------------------------------------ int8 -> 16-bit expansion
-// Four int8 (one 32-bit word) -> four values of type T, exact.
-//   fp16: 0x6400 | u is the half 1024 + u (u = q + 128 in 0..255); subtract 1152.
-//   bf16: 0x4B000000 | u is the float 2^23 + u; subtract 2^23 + 128; the result has at
-//         most 8 significant bits, so the conversion to bf16 is exact.
-template <typename T>
-__device__ __forceinline__ uint2 expand4(uint32_t w);
-template <>
-__device__ __forceinline__ uint2 expand4<__half>(uint32_t w) {
-  const uint32_t t = w ^ 0x80808080u;
-  uint32_t lo = __byte_perm(t, 0x64646464u, 0x4140);
-  uint32_t hi = __byte_perm(t, 0x64646464u, 0x4342);
-  const __half2 bias = __floats2half2_rn(1152.f, 1152.f);
-  const __half2 l = __hsub2(*reinterpret_cast<__half2*>(&lo), bias);
-  const __half2 h = __hsub2(*reinterpret_cast<__half2*>(&hi), bias);
-  return make_uint2(*reinterpret_cast<const uint32_t*>(&l), *reinterpret_cast<const uint32_t*>(&h));
-}
-template <>
-__device__ __forceinline__ uint2 expand4<__nv_bfloat16>(uint32_t w) {
-  const uint32_t t = w ^ 0x80808080u;
-  const float2 magic = make_float2(-8388736.f, -8388736.f);  // -(2^23 + 128)
-  const float2 f01 = __fadd2_rn(make_float2(__uint_as_float(__byte_perm(t, 0x4B000000u, 0x7540)),
-                                            __uint_as_float(__byte_perm(t, 0x4B000000u, 0x7541))),
-                                magic);
-  const float2 f23 = __fadd2_rn(make_float2(__uint_as_float(__byte_perm(t, 0x4B000000u, 0x7542)),
-                                            __uint_as_float(__byte_perm(t, 0x4B000000u, 0x7543))),
-                                magic);
-  // the sums are integers of at most 8 significant bits: their bf16 form is the upper half of
-  // the fp32 word, taken with a byte permute (the packing conversion runs on a slower pipe)
-  return make_uint2(__byte_perm(__float_as_uint(f01.x), __float_as_uint(f01.y), 0x7632),
-                    __byte_perm(__float_as_uint(f23.x), __float_as_uint(f23.y), 0x7632));
-}
 
 // One row (64 int8) of the raw tile -> one row (128 bytes) of the 16-bit tile.
 //   raw tile : rows of 64 bytes, 64-byte swizzle  (chunk c of row r at c ^ ((r >> 1) & 3))
