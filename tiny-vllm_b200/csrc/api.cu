@@ -416,7 +416,8 @@ size_t b200q_workspace_bytes(int op, int M, int N, int K) {
   if (check_dims(M, N, K) != B200Q_OK) return 0;
   const int path = resolve_path(op, M, N, K);
   if (path != B200Q_PATH_UMMA && path != B200Q_PATH_UMMA_SWAP) return 0;
-  if (path == B200Q_PATH_UMMA && umma_mid_applicable(M, N, K, op == B200Q_OP_W8A16)) return 0;
+  // (an upper bound at sizes where gemm_umma_mid.cu, which needs none, takes over the W8A8 problem)
+  if (path == B200Q_PATH_UMMA && op == B200Q_OP_W8A16 && umma_mid_applicable(M, N, K, true)) return 0;
   if (path == B200Q_PATH_UMMA && op == B200Q_OP_W8A16 && umma16_ts_applicable(M, N, K)) return 0;
   UmmaPlan plan;
   const bool ok = op == B200Q_OP_W8A8
@@ -441,9 +442,8 @@ const char* b200q_select_path(int op, int M, int N, int K) {
     case B200Q_PATH_UMMA:
       if (!a16 && umma_pair_applicable(M, N, K, false)) return "umma_i8_pair_tokens256";
       if (a16 && umma16_pair_applicable(M, N, K)) return "umma_f16_pair_expand_once_tokens256";
-      if (umma_mid_applicable(M, N, K, a16))
-        return a16 ? "umma_mid_f16_expand_cluster_splitk" : "umma_mid_i8_cluster_splitk";
-      if (a16 && umma16_ts_applicable(M, N, K)) return "umma_f16_tmem_weights_channels256";
+      // the two single-CTA kernels (gemm_umma_mid.cu and gemm_umma.cu / gemm_umma_w8a16.cu) are one family
+      if (a16 && !umma_mid_applicable(M, N, K, true) && umma16_ts_applicable(M, N, K)) return "umma_f16_tmem_weights_channels256";
       return a16 ? "umma_f16_expand_tokens128" : "umma_i8_tokens128";
     case B200Q_PATH_UMMA_SWAP:
       return a16 ? "umma_f16_expand_channels128_splitk" : "umma_i8_channels128_splitk";
