@@ -28,11 +28,11 @@ namespace {
 // Requires K <= G * 8 * CHUNKS.
 template <typename T, int G, int CHUNKS>
 __global__ void __launch_bounds__(256)
-act_quant_rows_kernel(const T* __restrict__ x, int64_t ldx, int8_t* __restrict__ xq,
-                      float* __restrict__ a_scales, int M, int K) {
+act_quant_rows_kernel(const T* x, int64_t ldx, int8_t* xq, float* a_scales, int M, int K) {
   constexpr int kRowsPerBlock = 256 / G;
-  ptx::grid_dependency_wait();     // x may be the previous kernel's output
-  ptx::grid_launch_dependents();
+  ptx::grid_launch_dependents();   // the successor's weights do not depend on this kernel
+  ptx::grid_dependency_wait();     // x may be the previous kernel's output (neither __ldg nor __restrict__,
+                                   // which makes a non-coherent load of it too: such a load may move ahead)
   const int g = threadIdx.x / G;  // row group inside the block
   const int t = threadIdx.x % G;  // thread inside the group
   const int row = blockIdx.x * kRowsPerBlock + g;
@@ -47,7 +47,7 @@ act_quant_rows_kernel(const T* __restrict__ x, int64_t ldx, int8_t* __restrict__
 #pragma unroll
     for (int c = 0; c < CHUNKS; ++c) {
       const int idx = c * G + t;
-      raw[c] = idx < nchunk ? __ldg(src + idx) : make_uint4(0u, 0u, 0u, 0u);
+      raw[c] = idx < nchunk ? src[idx] : make_uint4(0u, 0u, 0u, 0u);
     }
 #pragma unroll
     for (int c = 0; c < CHUNKS; ++c) {
@@ -83,17 +83,16 @@ act_quant_rows_kernel(const T* __restrict__ x, int64_t ldx, int8_t* __restrict__
 // Any K: one 256-thread CTA per row, the row is read twice (the second read hits L2).
 template <typename T>
 __global__ void __launch_bounds__(256)
-act_quant_long_rows_kernel(const T* __restrict__ x, int64_t ldx, int8_t* __restrict__ xq,
-                           float* __restrict__ a_scales, int M, int K) {
-  ptx::grid_dependency_wait();
+act_quant_long_rows_kernel(const T* x, int64_t ldx, int8_t* xq, float* a_scales, int M, int K) {
   ptx::grid_launch_dependents();
+  ptx::grid_dependency_wait();
   const int row = blockIdx.x;
   __shared__ float red[8];
   const int nchunk = K >> 3;
   const uint4* src = reinterpret_cast<const uint4*>(x + static_cast<size_t>(row) * ldx);
   AbsMax2<T> running;
   for (int idx = threadIdx.x; idx < nchunk; idx += 256) {
-    const uint4 r = __ldg(src + idx);
+    const uint4 r = src[idx];
     running.add(r.x);
     running.add(r.y);
     running.add(r.z);
@@ -110,7 +109,7 @@ act_quant_long_rows_kernel(const T* __restrict__ x, int64_t ldx, int8_t* __restr
   if (threadIdx.x == 0) a_scales[row] = scale;
   uint2* dst = reinterpret_cast<uint2*>(xq + static_cast<size_t>(row) * K);
   for (int idx = threadIdx.x; idx < nchunk; idx += 256)
-    dst[idx] = quant8<T>(__ldg(src + idx), scale, inv_scale);
+    dst[idx] = quant8<T>(src[idx], scale, inv_scale);
 }
 
 template <typename T>
@@ -119,6 +118,17 @@ cudaError_t launch_typed(const T* x, int64_t ldx, int8_t* xq, float* a_scales, i
   // Four 16-byte chunks per thread keep the register count low (high occupancy); longer
   // rows are spread over more threads instead of more chunks.
   auto blocks = [&](int g) { return (M + (256 / g) - 1) / (256 / g); };
+  // Few rows: the chain of one thread counts, not the occupancy, so every thread gets one chunk.
+  if (M <= 512 && K > 32 * 8) {
+    if (K <= 64 * 8)
+      return launch_overlapped(act_quant_rows_kernel<T, 64, 1>, blocks(64), 256, 0, s, x, ldx, xq, a_scales, M, K);
+    if (K <= 128 * 8)
+      return launch_overlapped(act_quant_rows_kernel<T, 128, 1>, blocks(128), 256, 0, s, x, ldx, xq, a_scales, M, K);
+    if (K <= 256 * 8)
+      return launch_overlapped(act_quant_rows_kernel<T, 256, 1>, blocks(256), 256, 0, s, x, ldx, xq, a_scales, M, K);
+    if (K <= 256 * 8 * 2)
+      return launch_overlapped(act_quant_rows_kernel<T, 256, 2>, blocks(256), 256, 0, s, x, ldx, xq, a_scales, M, K);
+  }
   if (K <= 32 * 8 * 2) {
     return launch_overlapped(act_quant_rows_kernel<T, 32, 2>, blocks(32), 256, 0, s, x, ldx, xq, a_scales, M, K);
   } else if (K <= 32 * 8 * 4) {

@@ -76,8 +76,8 @@ __device__ __noinline__ uint2 quant8_exact(const uint4 raw, float scale) {
 // Fast path: the exact product p = v * (1/scale) is within 1.3e-5 of the rounded quotient
 // fl(v / scale) (|p| <= 127; one rounding in the reciprocal, one in the quotient), hence
 // rint(p) can differ from rint(fl(v / scale)) only when p lies that close to a rounding tie
-// k + 0.5.  A chunk that has such an element (|p - rint(p)| > 0.4999, about one chunk in
-// 600 for random data) is redone with exact divisions.  Rounding uses the 1.5 * 2^23
+// k + 0.5.  A chunk that has such an element (|p - rint(p)| > 0.49998, about one chunk in
+// 3000 for random data) is redone with exact divisions.  Rounding uses the 1.5 * 2^23
 // trick: u = fma(v, 1/scale, 1.5 * 2^23) rounds p half-to-even to an integer and leaves
 // that integer in the low mantissa bits (two's complement), i.e. the low byte of u is the
 // int8 code; r = u - 1.5 * 2^23 is that integer exactly (its negative is formed by one fused
@@ -101,7 +101,7 @@ __device__ __forceinline__ uint2 quant8(const uint4 raw, float scale, float inv_
     ub[2 * i] = __float_as_uint(u.x);
     ub[2 * i + 1] = __float_as_uint(u.y);
   }
-  if (!(worst <= 0.4999f)) return quant8_exact<T>(raw, scale);  // also taken for NaN
+  if (!(worst <= 0.49998f)) return quant8_exact<T>(raw, scale);  // also taken for NaN
   uint2 o;
   o.x = __byte_perm(__byte_perm(ub[0], ub[1], 0x0040), __byte_perm(ub[2], ub[3], 0x0040), 0x5410);
   o.y = __byte_perm(__byte_perm(ub[4], ub[5], 0x0040), __byte_perm(ub[6], ub[7], 0x0040), 0x5410);

@@ -34,12 +34,11 @@ namespace {
 
 template <typename T, int G, int CHUNKS>
 __global__ void __launch_bounds__(256)
-add_rmsnorm_quant_kernel(const T* __restrict__ x, const T* residual_in, const T* __restrict__ weight,
-                         float eps, T* residual_out, T* __restrict__ y_out, int8_t* __restrict__ xq,
-                         float* __restrict__ a_scales, int M, int K) {
+add_rmsnorm_quant_kernel(const T* x, const T* residual_in, const T* __restrict__ weight, float eps,
+                         T* residual_out, T* y_out, int8_t* xq, float* a_scales, int M, int K) {
   constexpr int kRowsPerBlock = 256 / G;
-  ptx::grid_dependency_wait();
-  ptx::grid_launch_dependents();
+  ptx::grid_launch_dependents();   // the successor's weights do not depend on this kernel
+  ptx::grid_dependency_wait();     // ordinary loads from here on: a non-coherent one may move ahead
   const int g = threadIdx.x / G, t = threadIdx.x % G;
   const int row = blockIdx.x * kRowsPerBlock + g;
   __shared__ float red[8];
@@ -54,7 +53,7 @@ add_rmsnorm_quant_kernel(const T* __restrict__ x, const T* residual_in, const T*
     const bool live = active && idx < nchunk;
     uint4 xv = make_uint4(0u, 0u, 0u, 0u), rv = xv;
     if (live) {
-      xv = __ldg(reinterpret_cast<const uint4*>(x + static_cast<size_t>(row) * K) + idx);
+      xv = *(reinterpret_cast<const uint4*>(x + static_cast<size_t>(row) * K) + idx);
       if (residual_in != nullptr)
         rv = *(reinterpret_cast<const uint4*>(residual_in + static_cast<size_t>(row) * K) + idx);
     }
@@ -106,11 +105,11 @@ __device__ __forceinline__ float silu(float v) { return __fdividef(v, 1.0f + __e
 // gate_up: [M, ld] with the gate in columns [0, I) and the up projection in [I, 2 I).
 template <typename T, int G, int CHUNKS>
 __global__ void __launch_bounds__(256)
-silu_mul_quant_kernel(const T* __restrict__ gate_up, int64_t ld, T* __restrict__ y_out,
-                      int8_t* __restrict__ xq, float* __restrict__ a_scales, int M, int I) {
+silu_mul_quant_kernel(const T* gate_up, int64_t ld, T* y_out, int8_t* xq, float* a_scales, int M,
+                      int I) {
   constexpr int kRowsPerBlock = 256 / G;
-  ptx::grid_dependency_wait();
-  ptx::grid_launch_dependents();
+  ptx::grid_launch_dependents();   // the successor's weights do not depend on this kernel
+  ptx::grid_dependency_wait();     // ordinary loads from here on: a non-coherent one may move ahead
   const int g = threadIdx.x / G, t = threadIdx.x % G;
   const int row = blockIdx.x * kRowsPerBlock + g;
   __shared__ float red[8];
@@ -124,8 +123,8 @@ silu_mul_quant_kernel(const T* __restrict__ gate_up, int64_t ld, T* __restrict__
     uint4 gv = make_uint4(0u, 0u, 0u, 0u), uv = gv;
     if (active && idx < nchunk) {
       const uint4* base = reinterpret_cast<const uint4*>(gate_up + static_cast<size_t>(row) * ld);
-      gv = __ldg(base + idx);
-      uv = __ldg(base + nchunk + idx);
+      gv = base[idx];
+      uv = base[nchunk + idx];
     }
     const uint32_t gw[4] = {gv.x, gv.y, gv.z, gv.w}, uw[4] = {uv.x, uv.y, uv.z, uv.w};
     uint32_t out[4];
