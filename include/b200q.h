@@ -145,6 +145,19 @@ int b200q_w8a16_gemm(const void* x, const int8_t* qweight, const float* scales, 
                      size_t workspace_bytes, void* stream);
 
 /*
+ * The W8A8 linear on 16-bit activations x [M, K] (x_dtype, also the type of y and bias): per-token
+ * quantisation exactly as b200q_act_quant_i8 followed by b200q_w8a8_gemm — the whole of
+ * nanovllm/quantization/w8a8.py:25-40.  For decode-sized problems one kernel does both; otherwise the
+ * codes and scales pass through `scratch`, 16-byte aligned, of at least
+ * b200q_w8a8_dynamic_scratch_bytes() bytes (0: scratch may be NULL).
+ */
+int b200q_w8a8_dynamic_gemm(const void* x, const int8_t* qweight, const float* w_scales,
+                            const void* bias, void* y, int M, int N, int K, int x_dtype,
+                            void* scratch, size_t scratch_bytes, void* workspace,
+                            size_t workspace_bytes, void* stream);
+size_t b200q_w8a8_dynamic_scratch_bytes(int M, int N, int K);
+
+/*
  * Scratch bytes the given op needs for the given problem (0 when none).  The
  * first use of a workspace must find it zero-filled; every successful call
  * leaves it zero-filled where that matters, so one zeroed buffer of the maximum
@@ -218,6 +231,7 @@ enum {
   B200Q_KNOB_BULK_SLOTS = 16,   /* ring depth per consumer warp of those kernels (>= 2; default: what fits) */
   B200Q_KNOB_BULK_WPP = 17,     /* consumer warps per ring of the W8A8 one-token-tile kernel: 1 or 2 (default 2) */
   B200Q_KNOB_NO_MID = 18,       /* 1: never take the two-CTAs-per-SM tcgen05 kernel (M <= 512) */
+  B200Q_KNOB_NO_REG = 19,       /* 1: never take the decode kernels that hold the weights in registers */
   B200Q_KNOB_COUNT = 20
 };
 int b200q_debug_set(int knob, int value);

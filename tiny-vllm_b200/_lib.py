@@ -60,6 +60,7 @@ KNOB_BULK_DECODE = 15
 KNOB_BULK_SLOTS = 16
 KNOB_BULK_WPP = 17
 KNOB_NO_MID = 18
+KNOB_NO_REG = 19
 
 # B200Q_VERSION of include/b200q.h this binding was written for
 ABI_VERSION = 2
@@ -77,6 +78,10 @@ SIGNATURES = {
     "b200q_w8a16_gemm": (_c.c_int, [_c.c_void_p, _c.c_void_p, _c.c_void_p, _c.c_void_p, _c.c_void_p,
                                     _c.c_int, _c.c_int, _c.c_int, _c.c_int, _c.c_void_p,
                                     _c.c_size_t, _c.c_void_p]),
+    "b200q_w8a8_dynamic_gemm": (_c.c_int, [_c.c_void_p, _c.c_void_p, _c.c_void_p, _c.c_void_p, _c.c_void_p,
+                                           _c.c_int, _c.c_int, _c.c_int, _c.c_int, _c.c_void_p,
+                                           _c.c_size_t, _c.c_void_p, _c.c_size_t, _c.c_void_p]),
+    "b200q_w8a8_dynamic_scratch_bytes": (_c.c_size_t, [_c.c_int, _c.c_int, _c.c_int]),
     "b200q_workspace_bytes": (_c.c_size_t, [_c.c_int, _c.c_int, _c.c_int, _c.c_int]),
     "b200q_select_path": (_c.c_char_p, [_c.c_int, _c.c_int, _c.c_int, _c.c_int]),
     "b200q_strerror": (_c.c_char_p, [_c.c_int]),

@@ -68,30 +68,26 @@ int check_dims(int M, int N, int K) {
 }
 
 // Kernel family when nothing is forced; figures from graph-replayed chains of launches.
-// Up to 16 tokens the weight-streaming mma.sync kernels: the ring-fed persistent ones for matrices of 8 MB
-// and more, the register-streaming ones below.  Both re-read the activations (the latter once per 8
-// channels), so from 17 tokens on the tcgen05 kernels are ahead — 32 tokens: 6144 x 1024 3.7 against
-// 5.4 us, 24576 x 4096 20.4 against 28.5 — except on matrices below 4 MB, whose few K blocks
-// the register-streaming kernel has in flight at once (1536 x 1088 at 32 tokens: 2.4 against
-// 3.8 us, at 48 already 4.0 against 3.6).
-int auto_path_w8a8(int M, int N, int K) {
+// * Few tokens: the weight-streaming mma.sync family — the kernels that hold the weights in registers where
+//   they are the fastest, the ring-fed persistent ones for larger matrices (gemm_bulk_decode.cu).
+// * Long rows of a narrow matrix (K > 4096, too few channels for the rings): tcgen05 with K split over clusters
+//   (128 x 8192 at 16 tokens: 3.4 against 5.7 us W8A8, 4.4 against 7.1 W8A16).
+// * Everything else: tcgen05.  Its single-CTA kernel for mid sizes wants 16-byte output pieces; with an odd
+//   channel count up to 32 tokens stay on the streaming kernels.
+int auto_path(int M, int N, int K, bool a16) {
   if (M <= debug_knob(B200Q_KNOB_SIMT_MAX_M, 0)) return B200Q_PATH_SIMT_STREAM;
-  if (M <= 16 || (M <= 32 && static_cast<long long>(N) * K < (4ll << 20))) return B200Q_PATH_MMA_STREAM;
-  return B200Q_PATH_UMMA;
-}
-
-// W8A16: the activations are twice as wide, so the lines lie lower (32 tokens: 1024 x 2048 4.2
-// against 6.2 us, 1536 x 1088 4.2 against 4.0).
-int auto_path_w8a16(int M, int N, int K) {
-  if (M <= debug_knob(B200Q_KNOB_SIMT_MAX_M, 0)) return B200Q_PATH_SIMT_STREAM;
-  if (M <= 16 || (M <= 32 && static_cast<long long>(N) * K < (2ll << 20))) return B200Q_PATH_MMA_STREAM;
-  return B200Q_PATH_UMMA;
+  if (reg_decode_preferred(M, N, K, a16)) return B200Q_PATH_MMA_STREAM;
+  if (M <= 16) {
+    if (bulk_decode_applicable(M, N, K, a16)) return B200Q_PATH_MMA_STREAM;
+    return K > 4096 && (N % 8) == 0 ? B200Q_PATH_UMMA : B200Q_PATH_MMA_STREAM;
+  }
+  return M <= 32 && (N % 8) != 0 ? B200Q_PATH_MMA_STREAM : B200Q_PATH_UMMA;
 }
 
 int resolve_path(int op, int M, int N, int K) {
   const int forced = debug_knob(B200Q_KNOB_FORCE_PATH, B200Q_PATH_AUTO);
   if (forced != B200Q_PATH_AUTO) return forced;
-  return op == B200Q_OP_W8A16 ? auto_path_w8a16(M, N, K) : auto_path_w8a8(M, N, K);
+  return auto_path(M, N, K, op == B200Q_OP_W8A16);
 }
 
 int run_w8a8(GemmArgs& a) {
@@ -111,7 +107,8 @@ int run_w8a8(GemmArgs& a) {
   if (path == B200Q_PATH_MMA_STREAM) {
     if (!mma_decode_applicable(a.M)) return B200Q_ERR_UNSUPPORTED_SHAPE;
     cudaError_t e = bulk_decode_applicable(a.M, a.N, a.K, false) ? launch_w8a8_bulk_decode(a)
-                                                          : launch_w8a8_mma_decode(a);
+                    : reg_decode_applicable(a.M, a.N, a.K)     ? launch_w8a8_reg_decode(a, false)
+                                                               : launch_w8a8_mma_decode(a);
     if (e != cudaSuccess) {
       note_cuda_error(e);
       return B200Q_ERR_LAUNCH;
@@ -130,6 +127,14 @@ int run_w8a8(GemmArgs& a) {
   }
   return B200Q_ERR_BAD_ARGUMENT;
 }
+
+// One kernel for quantisation and GEMM, where each CTA can afford to read all tokens' rows.
+bool dynamic_is_fused(int M, int N, int K) {
+  return resolve_path(B200Q_OP_W8A8, M, N, K) == B200Q_PATH_MMA_STREAM &&
+         !bulk_decode_applicable(M, N, K, false) && reg_decode_dynamic_applicable(M, N, K);
+}
+
+size_t dynamic_code_offset(int M) { return (static_cast<size_t>(M) * 4 + 255) / 256 * 256; }
 
 }  // namespace
 
@@ -388,7 +393,8 @@ int b200q_w8a16_gemm(const void* x, const int8_t* qweight, const float* scales, 
   if (path == B200Q_PATH_MMA_STREAM) {
     if (!mma_decode_applicable(M)) return B200Q_ERR_UNSUPPORTED_SHAPE;
     cudaError_t e = bulk_decode_applicable(M, N, K, true) ? launch_w8a16_bulk_decode(a)
-                                                    : launch_w8a16_mma_decode(a);
+                    : reg_decode_applicable(M, N, K)    ? launch_w8a16_reg_decode(a)
+                                                        : launch_w8a16_mma_decode(a);
     if (e != cudaSuccess) {
       note_cuda_error(e);
       return B200Q_ERR_LAUNCH;
@@ -405,6 +411,54 @@ int b200q_w8a16_gemm(const void* x, const int8_t* qweight, const float* scales, 
     return launch_w8a16_umma(a, plan);
   }
   return B200Q_ERR_BAD_ARGUMENT;
+}
+
+size_t b200q_w8a8_dynamic_scratch_bytes(int M, int N, int K) {
+  if (check_dims(M, N, K) != B200Q_OK || dynamic_is_fused(M, N, K)) return 0;
+  return dynamic_code_offset(M) + static_cast<size_t>(M) * K;
+}
+
+int b200q_w8a8_dynamic_gemm(const void* x, const int8_t* qweight, const float* w_scales,
+                            const void* bias, void* y, int M, int N, int K, int x_dtype,
+                            void* scratch, size_t scratch_bytes, void* workspace,
+                            size_t workspace_bytes, void* stream) {
+  if (x == nullptr || qweight == nullptr || w_scales == nullptr || y == nullptr)
+    return B200Q_ERR_NULL_POINTER;
+  if (int rc = check_dims(M, N, K)) return rc;
+  if (x_dtype != B200Q_DTYPE_F16 && x_dtype != B200Q_DTYPE_BF16) return B200Q_ERR_BAD_ARGUMENT;
+  if (!dynamic_is_fused(M, N, K)) {
+    // scales first, codes behind them
+    if (scratch == nullptr || scratch_bytes < b200q_w8a8_dynamic_scratch_bytes(M, N, K))
+      return B200Q_ERR_WORKSPACE;
+    float* a_s = static_cast<float*>(scratch);
+    int8_t* xq = static_cast<int8_t*>(scratch) + dynamic_code_offset(M);
+    if (int rc = b200q_act_quant_i8(x, K, x_dtype, xq, a_s, M, K, stream)) return rc;
+    return b200q_w8a8_gemm(xq, a_s, qweight, w_scales, bias, y, M, N, K, x_dtype, workspace,
+                           workspace_bytes, stream);
+  }
+  if (!aligned16(x) || !aligned16(qweight) || !aligned16(y) || !aligned16(w_scales) ||
+      (bias != nullptr && (reinterpret_cast<uintptr_t>(bias) & 1u) != 0))
+    return B200Q_ERR_MISALIGNED;
+  DeviceInfo* d = device_info();
+  if (d == nullptr) return B200Q_ERR_LAUNCH;
+  if (d->cc_major != 10) return B200Q_ERR_UNSUPPORTED_ARCH;
+  GemmArgs a{};
+  a.x = x;
+  a.w = qweight;
+  a.w_scales = w_scales;
+  a.bias = bias;
+  a.y = y;
+  a.M = M;
+  a.N = N;
+  a.K = K;
+  a.dtype = x_dtype;
+  a.stream = static_cast<cudaStream_t>(stream);
+  const cudaError_t e = launch_w8a8_reg_decode(a, true);
+  if (e != cudaSuccess) {
+    note_cuda_error(e);
+    return B200Q_ERR_LAUNCH;
+  }
+  return B200Q_OK;
 }
 
 size_t b200q_workspace_bytes(int op, int M, int N, int K) {

@@ -75,6 +75,14 @@ int launch_w8a8_mma_decode_fused(const GemmArgs& a, void* const* peer_recv,
 int launch_w8a16_mma_decode_fused(const GemmArgs& a, void* const* peer_recv,
                                   void* const* peer_flags, size_t recv_bytes, int rank, int world);
 
+// gemm_reg_decode.cu: few tokens, the weights in registers before the activations exist;
+// applicable = can run, preferred = is the fastest; `dynamic`: a.x holds 16-bit activations that the kernel quantises itself
+bool reg_decode_applicable(int M, int N, int K);
+bool reg_decode_preferred(int M, int N, int K, bool a16);
+bool reg_decode_dynamic_applicable(int M, int N, int K);
+cudaError_t launch_w8a8_reg_decode(const GemmArgs& a, bool dynamic);
+cudaError_t launch_w8a16_reg_decode(const GemmArgs& a);
+
 // gemm_bulk_decode.cu: persistent decode kernels for large matrices; a producer warp streams
 // weights and activations through a shared-memory ring of bulk asynchronous copies
 bool bulk_decode_applicable(int M, int N, int K, bool a16);

@@ -45,6 +45,7 @@
 
 #include "common.h"
 #include "expand_device.cuh"
+#include "mma_device.cuh"
 #include "ptx_sm100.cuh"
 
 namespace b200q {
@@ -61,60 +62,6 @@ constexpr int kMaxMT = 2;  // token tiles: more would not fit the register file 
 constexpr int kRedBytes = kPipes * 16 * kUnitRows * 4;
 constexpr int kBarBytes = 2 * kPipes * kMaxSlots * 8;
 constexpr int kSmemLimit = 227 * 1024;
-
-template <typename T>
-__device__ __forceinline__ T from_float(float v);
-template <>
-__device__ __forceinline__ __half from_float<__half>(float v) {
-  return __float2half_rn(v);
-}
-template <>
-__device__ __forceinline__ __nv_bfloat16 from_float<__nv_bfloat16>(float v) {
-  return __float2bfloat16_rn(v);
-}
-template <typename T>
-__device__ __forceinline__ float to_float(T v);
-template <>
-__device__ __forceinline__ float to_float<__half>(__half v) {
-  return __half2float(v);
-}
-template <>
-__device__ __forceinline__ float to_float<__nv_bfloat16>(__nv_bfloat16 v) {
-  return __bfloat162float(v);
-}
-
-__device__ __forceinline__ void mma_s8(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2,
-                                       uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-      "{%0,%1,%2,%3};"
-      : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
-template <typename T>
-__device__ __forceinline__ void mma_16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2,
-                                       uint32_t a3, uint32_t b0, uint32_t b1);
-template <>
-__device__ __forceinline__ void mma_16<__nv_bfloat16>(float (&c)[4], uint32_t a0, uint32_t a1,
-                                                      uint32_t a2, uint32_t a3, uint32_t b0,
-                                                      uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, "
-      "{%8,%9}, {%0,%1,%2,%3};"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-template <>
-__device__ __forceinline__ void mma_16<__half>(float (&c)[4], uint32_t a0, uint32_t a1,
-                                               uint32_t a2, uint32_t a3, uint32_t b0,
-                                               uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, "
-      "{%8,%9}, {%0,%1,%2,%3};"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
 
 // Host-made description of the rings.  Shared memory of a CTA (1 KB aligned):
 // [8 rings x slots x weight tile][partial tiles of the consumer warps][full barriers]
@@ -666,10 +613,9 @@ cudaError_t launch_stream(int grid, int threads, size_t smem, cudaStream_t strea
 
 }  // namespace
 
-// Decode-sized batches over matrices large enough that every SM gets a share worth a ring.
-// Thresholds from graph-replayed launches of the Qwen3-0.6B and -8B projections and the 8B
-// model's 8-way shards: below 6-8 MB the register-streaming kernels (one short CTA per 8
-// channels) are as fast or faster.  Knob BULK_DECODE: 1 = never, 2 = wherever the kernel can run.
+// One token tile over matrices large enough that every SM gets a share worth a ring, unless the whole matrix
+// is better held in registers (reg_decode_preferred).  Beyond 16 tokens the tcgen05 kernels are ahead (W8A8 at 32:
+// 24576 x 4096 20.4 against 28.5 us).  Knob BULK_DECODE: 1 = never, 2 = wherever the kernel can run.
 bool bulk_decode_applicable(int M, int N, int K, bool a16) {
   const int knob = debug_knob(B200Q_KNOB_BULK_DECODE, 0);
   if (knob == 1) return false;
@@ -678,7 +624,8 @@ bool bulk_decode_applicable(int M, int N, int K, bool a16) {
   StreamPlan p;
   if (!make_plan(M, N, K, a16, p)) return false;
   if (knob == 2) return true;
-  return static_cast<long long>(N) * K >= ((a16 ? 6ll : 8ll) << 20) && N >= 8 * sm_count();
+  return M <= 16 && static_cast<long long>(N) * K >= (8ll << 20) && N >= 8 * sm_count() &&
+         !reg_decode_preferred(M, N, K, a16);
 }
 
 cudaError_t launch_w8a8_bulk_decode(const GemmArgs& a) {

@@ -314,7 +314,7 @@ umma_mid_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
     const bool live = grow < p.M;
     float a_s = 1.f;
     if (KIND == MID_I8) {
-      a_s = live ? __ldg(p.a_scales + grow) : 0.f;             // while the main loop runs
+      a_s = live ? p.a_scales[grow] : 0.f;   // while the main loop runs (not __ldg: it must stay behind the wait)
       if (cw < 4) s_as[row] = a_s;
     }
     const T* bias = reinterpret_cast<const T*>(p.bias);

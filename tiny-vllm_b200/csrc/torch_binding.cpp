@@ -164,20 +164,6 @@ PyObject* w8a16(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   END_HANDLE_TH_ERRORS
 }
 
-int run_w8a8(const at::Device& device, const int8_t* xq, const float* a_s, const Weights& p, void* y,
-             int m, int out_dt) {
-  const int n = static_cast<int>(p.N), k = static_cast<int>(p.K);
-  at::Tensor ws;
-  const size_t need = b200q_workspace_bytes(B200Q_OP_W8A8, m, n, k);
-  if (need > 0) ws = workspace(device, static_cast<int64_t>(need));
-  return unlocked([&] {
-    return b200q_w8a8_gemm(xq, a_s, static_cast<const int8_t*>(ptr(p.w)),
-                           static_cast<const float*>(ptr(p.s)), ptr(p.b), y, m, n, k, out_dt,
-                           need > 0 ? ws.data_ptr() : nullptr, need > 0 ? ws.numel() : 0,
-                           stream_of(device));
-  });
-}
-
 // w8a8_dynamic(x, qweight, w_scales, bias | None) -> y: per-token quantisation and the GEMM
 PyObject* w8a8_dynamic(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   HANDLE_TH_ERRORS
@@ -195,20 +181,37 @@ PyObject* w8a8_dynamic(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   c10::cuda::CUDAGuard guard(device);
   const int m = static_cast<int>(M);
   at::Tensor y = empty_on(out_shape(*x, p.N), x->scalar_type(), device);
-  // the scales first, the codes behind them on a 256-byte boundary
-  const int64_t code_off = (M * 4 + 255) / 256 * 256;
-  at::Tensor quant = empty_on({code_off + M * p.K}, at::kByte, device);
-  float* a_s = reinterpret_cast<float*>(quant.data_ptr());
-  int8_t* xq = static_cast<int8_t*>(quant.data_ptr()) + code_off;
-  int rc = unlocked([&] {
-    return b200q_act_quant_i8(x->data_ptr(), p.K, dt, xq, a_s, m, static_cast<int>(p.K),
-                              stream_of(device));
+  const int n = static_cast<int>(p.N), k = static_cast<int>(p.K);
+  at::Tensor quant, ws;
+  const size_t scratch = b200q_w8a8_dynamic_scratch_bytes(m, n, k);
+  if (scratch > 0) {
+    quant = empty_on({static_cast<int64_t>(scratch)}, at::kByte, device);
+    const size_t need = b200q_workspace_bytes(B200Q_OP_W8A8, m, n, k);
+    if (need > 0) ws = workspace(device, static_cast<int64_t>(need));
+  }
+  const int rc = unlocked([&] {
+    return b200q_w8a8_dynamic_gemm(
+        x->data_ptr(), static_cast<const int8_t*>(ptr(p.w)), static_cast<const float*>(ptr(p.s)),
+        ptr(p.b), y.data_ptr(), m, n, k, dt, scratch > 0 ? quant.data_ptr() : nullptr, scratch,
+        ws.defined() ? ws.data_ptr() : nullptr, ws.defined() ? ws.numel() : 0, stream_of(device));
   });
-  if (rc != B200Q_OK) return fail(rc, "b200q_act_quant_i8", M, p.N, p.K);
-  rc = run_w8a8(device, xq, a_s, p, y.data_ptr(), m, dt);
-  if (rc != B200Q_OK) return fail(rc, "b200q_w8a8_gemm", M, p.N, p.K);
+  if (rc != B200Q_OK) return fail(rc, "b200q_w8a8_dynamic_gemm", M, p.N, p.K);
   return THPVariable_Wrap(std::move(y));
   END_HANDLE_TH_ERRORS
+}
+
+int run_w8a8(const at::Device& device, const int8_t* xq, const float* a_s, const Weights& p, void* y,
+             int m, int out_dt) {
+  const int n = static_cast<int>(p.N), k = static_cast<int>(p.K);
+  at::Tensor ws;
+  const size_t need = b200q_workspace_bytes(B200Q_OP_W8A8, m, n, k);
+  if (need > 0) ws = workspace(device, static_cast<int64_t>(need));
+  return unlocked([&] {
+    return b200q_w8a8_gemm(xq, a_s, static_cast<const int8_t*>(ptr(p.w)),
+                           static_cast<const float*>(ptr(p.s)), ptr(p.b), y, m, n, k, out_dt,
+                           need > 0 ? ws.data_ptr() : nullptr, need > 0 ? ws.numel() : 0,
+                           stream_of(device));
+  });
 }
 
 // w8a8(x_q, a_scales, qweight, w_scales, bias | None, dtype id, shape | None, out | None) -> y
