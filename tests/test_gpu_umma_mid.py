@@ -40,3 +40,17 @@ def test_both_schemes(M, N, K, cluster, bn, oracle_c_lib):
         again = apply_int8_weight_only_linear(x.cuda(), q.cuda(), s.cuda(), b.cuda())
         assert torch.equal(bits(y), bits(again))     # sums in a fixed order
     assert device_status_ok()
+
+
+@pytest.mark.parametrize("M,N,K,bn", [(1100, 4104, 272, None), (12, 16384, 2064, None), (2048, 1032, 1040, 192),
+                                      (50, 264, 1616, 16), (97, 1000, 528, 48), (200, 136, 2112, 96)])
+def test_w8a16_more_than_one_wave_and_every_token_tile(M, N, K, bn):
+    # several waves of tiles, matrices too large for the ring kernel from 9 tokens on, the other tile widths
+    q, s = O.make_weight(N, K, seed=N + K)
+    x = O.make_activation(M, K, seed=M, dtype=torch.bfloat16)
+    with knobs(**({} if bn is None else {"BN": bn})):
+        assert select_path(_lib.OP_W8A16, M, N, K) == "umma_f16_expand_tokens128"
+        y = apply_int8_weight_only_linear(x.cuda(), q.cuda(), s.cuda())
+    m = O.tensor_metrics(O.w8a16_native_reference(x, q, s, None), y)
+    assert m["relative_l2"] <= 4e-3 and m["cosine_similarity"] >= 0.9999, m
+    assert device_status_ok()

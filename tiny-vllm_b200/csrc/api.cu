@@ -79,7 +79,8 @@ int auto_path(int M, int N, int K, bool a16) {
   if (reg_decode_preferred(M, N, K, a16)) return B200Q_PATH_MMA_STREAM;
   if (M <= 16) {
     if (bulk_decode_applicable(M, N, K, a16)) return B200Q_PATH_MMA_STREAM;
-    return K > 4096 && (N % 8) == 0 ? B200Q_PATH_UMMA : B200Q_PATH_MMA_STREAM;
+    // long K, or a matrix that the ring leaves to them: the tcgen05 kernels
+    return (K > 4096 || (a16 && bulk_decode_too_large(M, N, K))) && (N % 8) == 0 ? B200Q_PATH_UMMA : B200Q_PATH_MMA_STREAM;
   }
   return M <= 32 && (N % 8) != 0 ? B200Q_PATH_MMA_STREAM : B200Q_PATH_UMMA;
 }
@@ -117,8 +118,8 @@ int run_w8a8(GemmArgs& a) {
   }
   if (path == B200Q_PATH_UMMA && umma_pair_applicable(a.M, a.N, a.K, a.acc_out != nullptr))
     return launch_w8a8_umma_pair(a);
-  if (path == B200Q_PATH_UMMA && umma_mid_applicable(a.M, a.N, a.K, false))
-    return launch_umma_mid(a, false);
+  if (path == B200Q_PATH_UMMA && umma_mid_applicable(a.M, a.N, a.K))
+    return launch_umma_mid(a);
   if (path == B200Q_PATH_UMMA || path == B200Q_PATH_UMMA_SWAP) {
     UmmaPlan plan;
     if (!umma_make_plan(B200Q_OP_W8A8, a.M, a.N, a.K, path == B200Q_PATH_UMMA_SWAP, &plan))
@@ -401,8 +402,8 @@ int b200q_w8a16_gemm(const void* x, const int8_t* qweight, const float* scales, 
     }
     return B200Q_OK;
   }
+  if (path == B200Q_PATH_UMMA && umma16_mid_applicable(M, N, K)) return launch_umma16_mid(a);
   if (path == B200Q_PATH_UMMA && umma16_pair_applicable(M, N, K)) return launch_w8a16_umma_pair(a);
-  if (path == B200Q_PATH_UMMA && umma_mid_applicable(M, N, K, true)) return launch_umma_mid(a, true);
   if (path == B200Q_PATH_UMMA && umma16_ts_applicable(M, N, K)) return launch_w8a16_umma_ts(a);
   if (path == B200Q_PATH_UMMA || path == B200Q_PATH_UMMA_SWAP) {
     UmmaPlan plan;
@@ -464,14 +465,14 @@ int b200q_w8a8_dynamic_gemm(const void* x, const int8_t* qweight, const float* w
 size_t b200q_workspace_bytes(int op, int M, int N, int K) {
   if (op == B200Q_OP_W8A16 && check_dims(M, N, K) == B200Q_OK &&
       resolve_path(op, M, N, K) == B200Q_PATH_UMMA) {
-    if (umma16_pair_applicable(M, N, K)) return umma16_pair_workspace_bytes(N, K);
+    if (!umma16_mid_applicable(M, N, K) && umma16_pair_applicable(M, N, K)) return umma16_pair_workspace_bytes(N, K);
   }
   if (op != B200Q_OP_W8A8 && op != B200Q_OP_W8A16) return 0;
   if (check_dims(M, N, K) != B200Q_OK) return 0;
   const int path = resolve_path(op, M, N, K);
   if (path != B200Q_PATH_UMMA && path != B200Q_PATH_UMMA_SWAP) return 0;
   // (an upper bound at sizes where gemm_umma_mid.cu, which needs none, takes over the W8A8 problem)
-  if (path == B200Q_PATH_UMMA && op == B200Q_OP_W8A16 && umma_mid_applicable(M, N, K, true)) return 0;
+  if (path == B200Q_PATH_UMMA && op == B200Q_OP_W8A16 && umma16_mid_applicable(M, N, K)) return 0;
   if (path == B200Q_PATH_UMMA && op == B200Q_OP_W8A16 && umma16_ts_applicable(M, N, K)) return 0;
   UmmaPlan plan;
   const bool ok = op == B200Q_OP_W8A8
@@ -495,9 +496,12 @@ const char* b200q_select_path(int op, int M, int N, int K) {
       return a16 ? "mma_stream_w8a16_splitk" : "mma_stream_s8_splitk";
     case B200Q_PATH_UMMA:
       if (!a16 && umma_pair_applicable(M, N, K, false)) return "umma_i8_pair_tokens256";
-      if (a16 && umma16_pair_applicable(M, N, K)) return "umma_f16_pair_expand_once_tokens256";
-      // the two single-CTA kernels (gemm_umma_mid.cu and gemm_umma.cu / gemm_umma_w8a16.cu) are one family
-      if (a16 && !umma_mid_applicable(M, N, K, true) && umma16_ts_applicable(M, N, K)) return "umma_f16_tmem_weights_channels256";
+      // the single-CTA kernels of a scheme (gemm_umma_mid.cu and gemm_umma.cu; gemm_umma_mid_w8a16.cu and
+      // gemm_umma_w8a16.cu) are one family
+      if (a16 && !umma16_mid_applicable(M, N, K)) {
+        if (umma16_pair_applicable(M, N, K)) return "umma_f16_pair_expand_once_tokens256";
+        if (umma16_ts_applicable(M, N, K)) return "umma_f16_tmem_weights_channels256";
+      }
       return a16 ? "umma_f16_expand_tokens128" : "umma_i8_tokens128";
     case B200Q_PATH_UMMA_SWAP:
       return a16 ? "umma_f16_expand_channels128_splitk" : "umma_i8_channels128_splitk";

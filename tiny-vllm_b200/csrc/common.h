@@ -86,6 +86,7 @@ cudaError_t launch_w8a16_reg_decode(const GemmArgs& a);
 // gemm_bulk_decode.cu: persistent decode kernels for large matrices; a producer warp streams
 // weights and activations through a shared-memory ring of bulk asynchronous copies
 bool bulk_decode_applicable(int M, int N, int K, bool a16);
+bool bulk_decode_too_large(int M, int N, int K);
 cudaError_t launch_w8a8_bulk_decode(const GemmArgs& a);
 cudaError_t launch_w8a16_bulk_decode(const GemmArgs& a);
 
@@ -133,9 +134,11 @@ bool umma16_pair_applicable(int M, int N, int K);
 size_t umma16_pair_workspace_bytes(int N, int K);
 int launch_w8a16_umma_pair(const GemmArgs& a);
 
-// gemm_umma_mid.cu: both schemes at up to 512 tokens, two CTAs per SM, cluster split-K
-bool umma_mid_applicable(int M, int N, int K, bool a16);
-int launch_umma_mid(const GemmArgs& a, bool a16);
+// gemm_umma_mid.cu, gemm_umma_mid_w8a16.cu: W8A8 and W8A16 at up to 512 tokens, two CTAs per SM, cluster split-K
+bool umma_mid_applicable(int M, int N, int K);
+int launch_umma_mid(const GemmArgs& a);
+bool umma16_mid_applicable(int M, int N, int K);
+int launch_umma16_mid(const GemmArgs& a);
 
 // gemm_umma_w8a16.cu
 bool umma16_make_plan(int M, int N, int K, int swap, UmmaPlan* plan);

@@ -625,7 +625,14 @@ bool bulk_decode_applicable(int M, int N, int K, bool a16) {
   if (!make_plan(M, N, K, a16, p)) return false;
   if (knob == 2) return true;
   return M <= 16 && static_cast<long long>(N) * K >= (8ll << 20) && N >= 8 * sm_count() &&
-         !reg_decode_preferred(M, N, K, a16);
+         !(a16 && bulk_decode_too_large(M, N, K)) && !reg_decode_preferred(M, N, K, a16);
+}
+
+// W8A16 from 9 tokens on: the MMAs of a second token half and the expansion bound this kernel (36 us for 24576 x
+// 4096 at 12 tokens, 27 at 8), so matrices of 32 MB and more go to tcgen05 (32 us; 4096 x 12288 at
+// 12 tokens 16.3 against 19.4).
+bool bulk_decode_too_large(int M, int N, int K) {
+  return M > 8 && static_cast<long long>(N) * K >= (32ll << 20) && (N % 8) == 0;
 }
 
 cudaError_t launch_w8a8_bulk_decode(const GemmArgs& a) {

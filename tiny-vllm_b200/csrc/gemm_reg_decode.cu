@@ -315,15 +315,16 @@ bool reg_decode_applicable(int M, int N, int K) {
 //   weights: 3.5 / 4.2), 12288 x 2048 6.7 / 9.6 (ring: 7.7 / 12.8).  Longer rows leave one MMA tile per
 //   activation fragment, so only while the matrix is one wave of CTAs: 2048 x 4096 3.1 / 4.4 (4.8 / 6.1), but
 //   4096 x 4096 5.9 / 8.8 (5.3 / 8.9) and 5120 x 2560 5.7 / 8.5 (4.6 / 7.4).
-// * 17 to 32 tokens take a second pass over the activations; the tcgen05 kernel is the rival: at 32
-//   1024 x 2048 2.7 / 3.4 (3.4 / 4.1), 4096 x 1536 3.1 / 4.3 (4.5 / 6.1), 6144 x 1024 3.8 / 4.5 (3.6 / 5.8).
-// * Up to 48 only W8A16 with short rows: 4096 x 1536 5.7 (7.5), 2304 x 1088 4.5 (4.7), 1024 x 2048 4.6 (4.3).
+// * 17 to 32 tokens take a second pass over the activations; the tcgen05 kernels are the rivals.  W8A8 at 32:
+//   1024 x 2048 2.7 (3.4), 4096 x 1536 3.1 (4.5), but 6144 x 1024 3.8 (3.6).  W8A16: 4096 x 1024 at 32 3.6
+//   (3.9), 1024 x 3072 at 24 4.1 (4.3) but at 32 4.7 (4.4), 1024 x 4096 at 17 5.0 (4.5), 4096 x 1024 at 40 4.5 (4.2).
 bool reg_decode_preferred(int M, int N, int K, bool a16) {
   if (!reg_decode_applicable(M, N, K)) return false;
   const bool one_wave = static_cast<long long>(N) * K <= (17ll << 19);   // 8.5 MB
   if (M <= 16) return K <= 2048 || one_wave;
-  if (M <= 32) return one_wave && (a16 || N <= 5120);
-  return M <= 48 && a16 && one_wave && K <= 1536;
+  if (!a16) return M <= 32 && one_wave && N <= 5120;
+  // W8A16: until the tcgen05 kernel is ahead (that one needs whole groups of 8 channels)
+  return one_wave && (M <= 24 ? K <= 3072 : M <= 32 ? K <= 2048 : M <= 48 && K <= 1536 && (N % 8) != 0);
 }
 
 // Every CTA quantises all tokens, so only few values: 8 tokens of 1024 3.6 us in all against 4.4 in two kernels, 16

@@ -1,0 +1,510 @@
+// W8A16 at tens to hundreds of tokens on tcgen05: weights expanded int8 -> 16 bit on the way (exact) into
+// TENSOR memory, kind::f16, fp32 sums, then acc * s[n] + b[n]
+// (nanovllm/quantization/csrc/int8_weight_only_gemm.cu:258-292, 397-412).
+//
+// The W8A16 counterpart of gemm_umma_mid.cu, whose reasons hold here too: the next kernel of the stream is resident
+// while this one runs, weights are loaded AND expanded before the wait for the activations, several K
+// blocks per TMA instruction and turn of the issue loop, K split over a cluster whose CTAs share the
+// reduction.  What differs is where the expanded weights go.  In shared memory (as operand B beside the
+// activations) they took a third of the ring, and their write, proxy fence and second read made the
+// expansion the slowest stage.  Here
+//   * the channels are the 128 rows of the UMMA tile and the tokens its columns (16 to 256): a converter thread
+//     reads one row of int8 from shared memory and writes it expanded to its TMEM lane (tcgen05.st);
+//     the MMA takes its A operand from there;
+//   * an MMA of 64 columns takes 51 cycles and one of 128 68, whatever part of the 128 rows is used, so
+//     it is the tokens, the operand with fewer rows, that are cut finely.
+// Chains of launches, us per linear (expanded weights in shared memory; persistent kernels before that): 768 x
+// 4096 at 64 tokens 4.4 (5.9; 16.0), 4096 x 1024 at 512 9.0 (11.6; 13.7), 6144 x 4096 at 256 21.4 (35.4; 39.6).
+//
+// Warp roles (352 threads): warp 0 TMA of the activations, warp 1 UMMA, warps 2-9 expansion (two groups of
+// four that take the chunks in turn: a warp reaches one TMEM lane quarter), then epilogue, warp 10
+// TMA of the weights.
+// Every mbarrier wait is bounded; the cluster barrier is reached by every thread on every path.
+#include <cuda.h>
+#include <cuda_bf16.h>
+#include <cuda_fp16.h>
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cmath>
+
+#include "common.h"
+#include "ptx_sm100.cuh"
+#include "umma_mid_common.cuh"
+#include "w8a16_device.cuh"
+
+namespace b200q {
+namespace {
+
+constexpr int kMidCh = 128;                      // UMMA M: channels of a tile
+constexpr int kMidWeightWarp = kMidThreads / 32 - 1;
+constexpr int kMidACols = 32;                    // TMEM columns of one K block of expanded weights
+
+struct MidParams {
+  int M, N;
+  int bt;                  // tokens per tile (UMMA N)
+  int tiles_t;
+  int kc;                  // K blocks (64 elements) per chunk
+  int chunks, chunks_per_split;
+  int chunks_3d;           // chunks below this one come through the 3-D maps: one TMA instruction
+  int splits;              // cluster size
+  int stages;              // ring of chunks of activations and of int8 weights: an even number, or one in all
+  int stage_bytes, raw_bytes;
+  int a_stages;            // ring of chunks of expanded weights in TMEM (likewise)
+  int a_col0;              // its first TMEM column
+  int tmem_cols;
+  int is_bf16;
+  const float* w_scales;   // per channel
+  const void* bias;        // per channel or nullptr
+  void* out;
+  int* status;
+};
+
+template <typename T>
+__device__ __forceinline__ uint16_t bits16(T v) {
+  return *reinterpret_cast<const uint16_t*>(&v);
+}
+
+// One sum -> one scaled value.
+template <typename T>
+__device__ __forceinline__ T finish(uint32_t acc, float w_s, const T* bias, int n) {
+  float v = __fmul_rn(__uint_as_float(acc), w_s);
+  if (bias != nullptr) v = __fadd_rn(v, to_float<T>(bias[n]));
+  return from_float<T>(v);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kMidThreads, 2)
+w8a16_mid_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
+                 const __grid_constant__ CUtensorMap tmap_x3, const __grid_constant__ CUtensorMap tmap_w3,
+                 const MidParams p) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  const int rows_own = (p.bt + p.splits - 1) / p.splits;       // tokens a CTA owns
+  const uint32_t raw_base = static_cast<uint32_t>(p.stages * p.stage_bytes);
+  uint8_t* red = smem + raw_base + p.stages * p.raw_bytes; // [S][rows_own][128] 32-bit sums (S > 1)
+  float* s_ws = reinterpret_cast<float*>(red + (p.splits > 1 ? p.splits * rows_own * kMidCh * 4 : 0));   // [128]
+  uint8_t* ctrl = reinterpret_cast<uint8_t*>(s_ws + kMidCh);
+  uint64_t* xfull = reinterpret_cast<uint64_t*>(ctrl);         // activations of a stage have landed
+  uint64_t* empty = xfull + kMidMaxStages;                     // the MMAs that read a stage are done
+  uint64_t* wfull = empty + kMidMaxStages;                     // int8 weights have landed
+  uint64_t* rempty = wfull + kMidMaxStages;                    // ... and are read
+  uint64_t* cfull = rempty + kMidMaxStages;                    // [4] expanded weights are in TMEM
+  uint64_t* aempty = cfull + 4;                                // [4] the MMAs that read them are done
+  uint64_t* tfull = aempty + 4;                                // accumulator complete
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tfull + 1);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = static_cast<int>(p.splits > 1 ? ptx::cluster_ctarank() : 0);
+  const int tile = static_cast<int>(blockIdx.x) / p.splits;
+  const int tile_t = tile % p.tiles_t, tile_c = tile / p.tiles_t;  // neighbours share the weights
+  const int c0 = rank * p.chunks_per_split;
+  const int n_ch = min(p.chunks, c0 + p.chunks_per_split) - c0;    // >= 1 by construction
+  const uint32_t smem_base = ptx::smem_u32(smem);
+  const bool aligned = (smem_base & 1023u) == 0u;
+  const int x_blk = p.bt * 128;                                // one K block of activations
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < p.stages; ++s) {
+      ptx::mbar_init(ptx::smem_u32(xfull + s), 1);
+      ptx::mbar_init(ptx::smem_u32(empty + s), 1);
+      ptx::mbar_init(ptx::smem_u32(wfull + s), 1);
+      ptx::mbar_init(ptx::smem_u32(rempty + s), 4);
+    }
+    for (int s = 0; s < 4; ++s) {
+      ptx::mbar_init(ptx::smem_u32(cfull + s), 4);
+      ptx::mbar_init(ptx::smem_u32(aempty + s), 1);
+    }
+    ptx::mbar_init(ptx::smem_u32(tfull), 1);
+    *abort_flag = aligned ? 0 : 2;
+    ptx::fence_mbar_init();
+  }
+  if (warp == 1) {
+    ptx::tmem_alloc(ptx::smem_u32(tmem_slot), static_cast<uint32_t>(p.tmem_cols));
+    ptx::tmem_relinquish();
+  }
+  ptx::tc_fence_before_sync();
+  __syncthreads();
+  ptx::tc_fence_after_sync();
+  const uint32_t tmem_base = *tmem_slot;
+  if (p.splits > 1) cluster_arrive();   // "this CTA runs": awaited before the first remote store
+  ptx::grid_launch_dependents();        // the successor does not touch our results before it waits
+  const bool run = aligned;             // a misaligned shared window (never seen) skips all work
+
+  if (warp == 0 || warp == kMidWeightWarp) {
+    if (run) {
+      // -------------------------------------------------------------- TMA producers
+      const bool weights = warp != 0;
+      const MidStream s{weights ? &tmap_w : &tmap_x, weights ? &tmap_w3 : &tmap_x3,
+                        weights ? tile_c * kMidCh : tile_t * p.bt, weights ? kRow8 : 128,
+                        weights ? kMidCh * kRow8 : x_blk, p.kc, smem_base + (weights ? raw_base : 0u),
+                        static_cast<uint32_t>(weights ? p.raw_bytes : p.stage_bytes), p.stages,
+                        weights ? wfull : xfull, weights ? rempty : empty, c0, n_ch, p.chunks_3d};
+      if (weights) {
+        if (ptx::elect_one())
+          for (int i = p.stages; i < n_ch && i < p.stages + 8 && c0 + i < p.chunks_3d; ++i)
+            ptx::tma_prefetch_l2_3d(s.map3, 0, s.row0, (c0 + i) * p.kc);
+      } else {
+        ptx::grid_dependency_wait();
+      }
+      mid_produce(s, abort_flag);
+    }
+  } else if (warp == 1) {
+    if (run) {
+      // ----------------------------------------------------------------- UMMA issuer
+      const uint32_t idesc = ptx::umma_idesc(1u, p.is_bf16 ? 1u : 0u, kMidCh, static_cast<uint32_t>(p.bt));
+      int stage = 0, as = 0;
+      uint32_t phase = 0, aphase = 0;
+      bool ok = true;
+      for (int i = 0; i < n_ch; ++i) {
+        if (!ptx::mbar_wait(ptx::smem_u32(cfull + as), aphase, abort_flag) ||
+            !ptx::mbar_wait(ptx::smem_u32(xfull + stage), phase, abort_flag)) {
+          ok = false;
+          break;
+        }
+        ptx::tc_fence_after_sync();
+        if (ptx::elect_one()) {
+          uint64_t b_desc = ptx::umma_desc_k_sw128(smem_base + stage * p.stage_bytes);
+          uint32_t a_tmem = tmem_base + static_cast<uint32_t>(p.a_col0 + as * p.kc * kMidACols);
+          for (int b = 0; b < p.kc; ++b) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {   // 32 bytes of K per instruction
+              const uint32_t acc = (i > 0 || b > 0 || k > 0) ? 1u : 0u;
+              ptx::umma_f16_ts(tmem_base, a_tmem + 8u * k, b_desc + 2u * k, idesc, acc);
+            }
+            b_desc += static_cast<uint32_t>(x_blk >> 4);
+            a_tmem += kMidACols;
+          }
+          ptx::umma_commit(ptx::smem_u32(empty + stage));
+          ptx::umma_commit(ptx::smem_u32(aempty + as));
+        }
+        __syncwarp();
+        if (++stage == p.stages) {
+          stage = 0;
+          phase ^= 1u;
+        }
+        if (++as == p.a_stages) {
+          as = 0;
+          aphase ^= 1u;
+        }
+      }
+      if (ok && ptx::elect_one()) ptx::umma_commit(ptx::smem_u32(tfull));
+    }
+  } else {
+    const int cw = warp - 2, tid = threadIdx.x - 64;
+    const int quarter = warp & 3;                              // the TMEM lanes this warp may access
+    const int ch = quarter * 32 + lane;                        // channel of the tile = TMEM lane
+    const uint32_t lanes = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
+    // channel scales: constants, fetched ahead of the wait
+    if (tid < kMidCh) {
+      const int col = tile_c * kMidCh + tid;
+      s_ws[tid] = col < p.N ? __ldg(p.w_scales + col) : 0.f;
+    }
+    if (run) {
+      // -------------------------------------------------------------- expansion
+      // Both rings have an even number of slots, so a slot always belongs to the same group: a group that has not
+      // seen the previous use of a slot complete could not tell its barrier's phases apart.
+      const int group = cw >> 2;
+      const int sw8 = (ch >> 1) & 3;
+      int rs = group, as = group;
+      uint32_t rphase = 0, aphase = 1;
+      for (int i = group; i < n_ch; i += 2) {
+        if (!ptx::mbar_wait(ptx::smem_u32(wfull + rs), rphase, abort_flag)) break;
+        if (i >= p.a_stages && !ptx::mbar_wait(ptx::smem_u32(aempty + as), aphase, abort_flag)) break;
+        ptx::tc_fence_after_sync();
+        const uint8_t* src = smem + raw_base + rs * p.raw_bytes + ch * kRow8;
+        for (int b = 0; b < p.kc; ++b, src += kMidCh * kRow8) {
+          uint32_t v[32];
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            const uint4 w = *reinterpret_cast<const uint4*>(src + ((c ^ sw8) << 4));
+            const uint2 e0 = expand4<T>(w.x), e1 = expand4<T>(w.y), e2 = expand4<T>(w.z), e3 = expand4<T>(w.w);
+            v[8 * c + 0] = e0.x;
+            v[8 * c + 1] = e0.y;
+            v[8 * c + 2] = e1.x;
+            v[8 * c + 3] = e1.y;
+            v[8 * c + 4] = e2.x;
+            v[8 * c + 5] = e2.y;
+            v[8 * c + 6] = e3.x;
+            v[8 * c + 7] = e3.y;
+          }
+          ptx::tmem_st_32x32b_x32(lanes + static_cast<uint32_t>(p.a_col0 + (as * p.kc + b) * kMidACols), v);
+        }
+        ptx::tmem_st_wait();
+        ptx::tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) {
+          ptx::mbar_arrive(ptx::smem_u32(cfull + as));
+          ptx::mbar_arrive(ptx::smem_u32(rempty + rs));
+        }
+        if ((rs += 2) >= p.stages) {
+          rs = group;
+          rphase ^= 1u;
+        }
+        if ((as += 2) >= p.a_stages) {
+          as = group;
+          aphase ^= 1u;
+        }
+      }
+    }
+    __syncwarp();
+    ptx::grid_dependency_wait();         // y may be in use by the previous kernel
+    // every CTA of the cluster runs: its memory may be written / scales of this CTA complete
+    if (p.splits > 1) cluster_wait();
+    else ptx::named_bar_sync(1, 256);
+    bool done = run && ptx::mbar_wait(ptx::smem_u32(tfull), 0u, abort_flag);
+    done = __all_sync(0xFFFFFFFFu, done);
+    if (done) {
+      ptx::tc_fence_after_sync();
+      const T* bias = reinterpret_cast<const T*>(p.bias);
+      const int n = tile_c * kMidCh + ch;
+      const int shift = __ffs(p.splits) - 1;
+      const uint32_t mine = ptx::smem_u32(red) + static_cast<uint32_t>(rank * rows_own * kMidCh + ch) * 4u;
+      const int live = min(p.bt, p.M - tile_t * p.bt);         // tokens of this tile
+      for (int c = (cw >> 2) * 32; c < live; c += 64) {
+        uint32_t v[32];
+        ptx::tmem_ld_32x32b_x32(lanes + static_cast<uint32_t>(c), v);
+        ptx::tmem_ld_wait();
+        if (p.splits > 1) {
+          // ------------------------------------------ partial sums -> the tokens' owners
+#pragma unroll
+          for (int j = 0; j < 32; ++j) {
+            const int tok = c + j;
+            if (tok < live)
+              ptx::st_shared_cluster_u32(
+                  ptx::map_to_cta(mine + static_cast<uint32_t>((tok >> shift) * kMidCh) * 4u,
+                                  static_cast<uint32_t>(tok & (p.splits - 1))),
+                  v[j]);
+          }
+        } else {
+          // no split: straight from the registers.  Neighbouring lanes exchange halves, so that each
+          // stores two channels of one token: even lanes token j, odd lanes token j + 1.
+          const float w_s = s_ws[ch];
+          const bool odd = (lane & 1) != 0;
+          T* out = static_cast<T*>(p.out) + static_cast<size_t>(tile_t * p.bt + c + (odd ? 1 : 0)) * p.N + (odd ? n - 1 : n);
+#pragma unroll
+          for (int j = 0; j < 32; j += 2) {
+            const T* b = n < p.N ? bias : nullptr;
+            const uint32_t lo = bits16(finish<T>(v[j], w_s, b, n));
+            const uint32_t hi = bits16(finish<T>(v[j + 1], w_s, b, n));
+            const uint32_t got = __shfl_xor_sync(0xFFFFFFFFu, odd ? lo : hi, 1);
+            const uint32_t word = odd ? (got | (hi << 16)) : (lo | (got << 16));
+            if (c + j + (odd ? 1 : 0) < live && n < p.N) *reinterpret_cast<uint32_t*>(out) = word;   // N is even
+            out += 2 * static_cast<size_t>(p.N);
+          }
+        }
+      }
+    }
+  }
+  if (p.splits > 1 && (warp < 2 || warp == kMidWeightWarp)) {
+    __syncwarp();
+    cluster_wait();      // the arrival at the start
+  }
+  __syncwarp();
+  ptx::tc_fence_before_sync();
+  if (p.splits > 1) {
+    cluster_arrive();    // release: this CTA's stores; after the wait nothing is written remotely
+    cluster_wait();
+  } else {
+    __syncthreads();
+  }
+  if (warp == 1) {
+    ptx::tc_fence_after_sync();
+    ptx::tmem_dealloc(tmem_base, static_cast<uint32_t>(p.tmem_cols));
+  }
+
+  // ------------------------------------------------------ own tokens: add, scale, round, store
+  if (p.splits > 1) {
+    const T* bias = reinterpret_cast<const T*>(p.bias);
+    for (int u = threadIdx.x; u < rows_own * (kMidCh / 8); u += kMidThreads) {
+      const int tl = u / (kMidCh / 8), cg = u % (kMidCh / 8);  // 8 channels: one 16-byte store
+      const int tok = tl * p.splits + rank;
+      const int row = tile_t * p.bt + tok, col = tile_c * kMidCh + cg * 8;
+      if (tok >= p.bt || row >= p.M || col >= p.N) continue;   // N % 8 == 0
+      uint32_t w[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
+      for (int s = 0; s < p.splits; ++s) {       // rank order: results do not depend on the run
+        const uint4* src = reinterpret_cast<const uint4*>(red) + ((s * rows_own + tl) * kMidCh + cg * 8) / 4;
+        const uint4 a = src[0], b = src[1];
+        const uint32_t in[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          w[j] = s == 0 ? in[j] : __float_as_uint(__fadd_rn(__uint_as_float(w[j]), __uint_as_float(in[j])));
+      }
+      uint32_t packed[4];
+#pragma unroll
+      for (int j = 0; j < 8; j += 2)
+        packed[j / 2] =
+            bits16(finish<T>(w[j], s_ws[cg * 8 + j], bias, col + j)) |
+            (static_cast<uint32_t>(bits16(finish<T>(w[j + 1], s_ws[cg * 8 + j + 1], bias, col + j + 1))) << 16);
+      *reinterpret_cast<uint4*>(static_cast<T*>(p.out) + static_cast<size_t>(row) * p.N + col) =
+          make_uint4(packed[0], packed[1], packed[2], packed[3]);
+    }
+  }
+  if (threadIdx.x == 0 && *abort_flag != 0)
+    atomicCAS(p.status, 0, 0xB00 | (*abort_flag << 4) | (static_cast<int>(blockIdx.x) << 12));
+}
+
+}  // namespace
+
+// ------------------------------------------------------------------------------ host
+namespace {
+
+struct MidPlan {
+  int bt, splits, kc, chunks, chunks_per_split, tiles_t, tiles_c;
+  int stages, stage_bytes, raw_bytes, a_stages, a_col0, tmem_cols;
+  size_t smem;
+};
+
+bool mid_plan_for(int M, int N, int k_blocks, int bt, int splits, int kc, int smem_cap, MidPlan* pl) {
+  pl->bt = bt;
+  pl->kc = kc;
+  pl->splits = splits;
+  pl->chunks = (k_blocks + kc - 1) / kc;
+  pl->chunks_per_split = (pl->chunks + splits - 1) / splits;
+  if (pl->chunks_per_split * (splits - 1) >= pl->chunks) return false;   // a CTA without work
+  pl->tiles_t = (M + bt - 1) / bt;
+  pl->tiles_c = (N + kMidCh - 1) / kMidCh;
+  pl->stage_bytes = kc * bt * 128;
+  pl->raw_bytes = kc * kMidCh * kRow8;
+  const int rows_own = (bt + splits - 1) / splits;
+  const int fixed = (splits > 1 ? splits * rows_own * kMidCh * 4 : 0) + kMidCh * 4 + kMidCtrlBytes;
+  const int ring_bytes = pl->stage_bytes + pl->raw_bytes;
+  int stages = std::min({(smem_cap - fixed) / ring_bytes, kMidMaxStages, pl->chunks_per_split});
+  if (stages < 1 || (stages < 2 && pl->chunks_per_split > 1)) return false;
+  // the converter groups take the chunks in turn: an even number of slots, or a single chunk
+  if (pl->chunks_per_split > 1) stages &= ~1;
+  int cols = (bt + 31) / 32 * 32;
+  pl->a_col0 = cols;
+  // at most 256 columns leave room for the next CTA; a wide tile takes them all
+  const int chunk_cols = kc * kMidACols, room = (cols + 2 * chunk_cols <= 256 ? 256 : 512) - cols;
+  pl->a_stages = std::min({room / chunk_cols, 4, pl->chunks_per_split});
+  if (pl->chunks_per_split > 1) pl->a_stages &= ~1;
+  if (pl->a_stages < 1) return false;
+  cols += pl->a_stages * chunk_cols;
+  pl->stages = stages;
+  pl->tmem_cols = 32;
+  while (pl->tmem_cols < cols) pl->tmem_cols *= 2;
+  pl->smem = static_cast<size_t>(stages) * ring_bytes + fixed;
+  return true;
+}
+
+// Predicted time of one call in a stream of such calls, in microseconds.  The form follows what the
+// kernel does (MMAs, expansion and HBM overlap, hence the root of cubes); the coefficients are
+// fitted to 8,400 measured configurations (17 shapes from 2 to 100 MB of weights, 24 to 3000 tokens): the
+// one with the smallest prediction is on average 3 %, at worst 20 %, slower than the best measured one.
+double mid_cost(const MidPlan& pl, int M, double matrix_bytes) {
+  const double clk = 1850.0;   // cycles per microsecond
+  const int ctas = pl.tiles_t * pl.tiles_c * pl.splits;
+  const int per_sm = pl.smem <= kMidSmemTwo && pl.tmem_cols <= 256 ? 2 : 1;
+  // clusters of 4 and 8 do not fill every SM (a cluster lives inside one group of SMs)
+  const int sms = sm_count() - (pl.splits == 8 ? 28 : pl.splits == 4 ? 12 : 0);
+  const double passes = (ctas + sms - 1) / sms, waves = (ctas + sms * per_sm - 1) / (sms * per_sm);
+  const double kb = pl.chunks_per_split * pl.kc;
+  const double per_mma = pl.bt <= 32 ? 43 : pl.bt <= 64 ? 51 : pl.bt <= 128 ? 68 : 130 * pl.bt / 256.0;   // cycles
+  const double mma = 0.825 * kb * 4 * per_mma * passes, expand = 140.5 * kb * passes;
+  const double hbm = matrix_bytes / sm_count() / 20.4;
+  double us = 2.07 + std::cbrt(mma * mma * mma + expand * expand * expand + hbm * hbm * hbm) / clk;
+  // a ring shorter than the K loop goes round at the latency of a load
+  us += 0.467 * waves * std::max(0, pl.chunks_per_split - pl.stages) / pl.stages;
+  us += 0.231 * waves * pl.chunks_per_split;
+  if (pl.splits > 1) us += 0.0153 * std::min(M, pl.bt) * passes;
+  // start-up (1 us, and the first weights from HBM) hides under the previous kernel only as far as
+  // both fit the GPU; alone on its SM a tile's start and end hide under nothing
+  const double slots = static_cast<double>(sm_count()) * per_sm;
+  us += 2.42 * std::min(1.0, std::max(0.0, (2.0 * ctas - slots) / slots));
+  if (per_sm == 1) us += 5.12 * (waves - 1);
+  return us;
+}
+
+bool search_plan(int M, int N, int K, MidPlan* best) {
+  const int k_blocks = (K + kBlockK - 1) / kBlockK;
+  const int want_bt = debug_knob(B200Q_KNOB_BN, 0), want_s = debug_knob(B200Q_KNOB_CLUSTER, 0);
+  double best_cost = 1e30;
+  for (int bt : {16, 32, 48, 64, 96, 128, 192, 256}) {
+    if (want_bt != 0 ? bt != want_bt : bt >= M + 32 && bt > 32) continue;
+    for (int s : {1, 2, 4, 8}) {
+      if (want_s != 0 && s != want_s) continue;
+      for (int kc : {4, 2, 1}) {
+        for (int cap : {kMidSmemOne, kMidSmemTwo}) {
+          MidPlan pl;
+          if (!mid_plan_for(M, N, k_blocks, bt, s, kc, cap, &pl)) continue;
+          const double cost = mid_cost(pl, M, static_cast<double>(N) * K);
+          if (cost < best_cost) {
+            best_cost = cost;
+            *best = pl;
+          }
+        }
+      }
+    }
+  }
+  return best_cost < 1e30;
+}
+
+}  // namespace
+
+// Up to 2.6 waves of 128 x 128 outputs.  There this kernel beats the persistent ones (gemm_umma_w8a16_ts.cu,
+// and from 1024 tokens gemm_umma_pair.cu on weights expanded beforehand) at every measured shape: 24576 x 4096 at 24 tokens 28 against 49 us, at 256 61 against 106; 4096 x 4096 at 1200
+// tokens 42 against 59; 6144 x 1024 at 800 15.0 against 24.4; 1024 x 2048 at 1500 12.7 against
+// 21.6.  Beyond, an overlapped epilogue and an expansion done once win (6144 x 1024 at 1200 tokens, 3.2 waves:
+// 23.1 against 22.1; 4096 x 1024 at 2000, 3.5 waves: 23.9 against 20.5), and above 2048 tokens little is left
+// to gain on few tiles either (1024 x 2048 at 3000: 16.6 against 18.2).
+bool umma16_mid_applicable(int M, int N, int K) {
+  if (debug_knob(B200Q_KNOB_NO_MID, 0) != 0) return false;
+  if ((K % 16) != 0 || (N % 8) != 0 || M < 1) return false;
+  const long long tiles = static_cast<long long>((M + 127) / 128) * ((N + 127) / 128);
+  if (M > 2048 || 5 * tiles > 13 * sm_count()) return false;
+  if (debug_knob(B200Q_KNOB_BN, 0) == 0 && debug_knob(B200Q_KNOB_CLUSTER, 0) == 0) return true;
+  MidPlan pl;   // a forced tile or cluster may not fit
+  return mid_plan<MidPlan, search_plan>(M, N, K, &pl);
+}
+
+int launch_umma16_mid(const GemmArgs& a) {
+  MidPlan pl;
+  if (!mid_plan<MidPlan, search_plan>(a.M, a.N, a.K, &pl)) return B200Q_ERR_UNSUPPORTED_SHAPE;
+  CUtensorMap tx, tw;
+  const uint64_t x_row = static_cast<uint64_t>(a.K) * 2;
+  if (!make_tensor_map(a.x, a.M, x_row, static_cast<uint32_t>(pl.bt), 128, &tx) ||
+      !get_tensor_map(a.w, a.N, a.K, static_cast<uint32_t>(kMidCh), kRow8, &tw))
+    return B200Q_ERR_LAUNCH;
+  // K a multiple of a block: everything comes through the 3-D maps (blocks beyond K read as zeros);
+  // otherwise the chunk with the partial block, and what follows it, goes block by block
+  const int chunks_3d = a.K % kBlockK == 0 ? pl.chunks : a.K / kBlockK / pl.kc;
+  CUtensorMap tx3 = tx, tw3 = tw;
+  if (chunks_3d > 0 &&
+      (!make_tensor_map(a.x, a.M, x_row, static_cast<uint32_t>(pl.bt), 128, &tx3, pl.kc) ||
+       !get_tensor_map(a.w, a.N, a.K, static_cast<uint32_t>(kMidCh), kRow8, &tw3, pl.kc)))
+    return B200Q_ERR_LAUNCH;
+  MidParams mp{};
+  mp.M = a.M;
+  mp.N = a.N;
+  mp.bt = pl.bt;
+  mp.tiles_t = pl.tiles_t;
+  mp.kc = pl.kc;
+  mp.chunks = pl.chunks;
+  mp.chunks_per_split = pl.chunks_per_split;
+  mp.chunks_3d = chunks_3d;
+  mp.splits = pl.splits;
+  mp.stages = pl.stages;
+  mp.stage_bytes = pl.stage_bytes;
+  mp.raw_bytes = pl.raw_bytes;
+  mp.a_stages = pl.a_stages;
+  mp.a_col0 = pl.a_col0;
+  mp.tmem_cols = pl.tmem_cols;
+  mp.is_bf16 = a.dtype == B200Q_DTYPE_BF16 ? 1 : 0;
+  mp.w_scales = a.w_scales;
+  mp.bias = a.bias;
+  mp.out = a.y;
+  mp.status = a.status;
+  const int ctas = pl.tiles_t * pl.tiles_c * pl.splits;
+  const cudaError_t e =
+      mp.is_bf16 ? launch_mid_kernel<w8a16_mid_kernel<__nv_bfloat16>>(ctas, pl.splits, pl.smem, a.stream, tx, tw, tx3, tw3, mp)
+                 : launch_mid_kernel<w8a16_mid_kernel<__half>>(ctas, pl.splits, pl.smem, a.stream, tx, tw, tx3, tw3, mp);
+  if (e != cudaSuccess) {
+    note_cuda_error(e);
+    return B200Q_ERR_LAUNCH;
+  }
+  count_launch();
+  return B200Q_OK;
+}
+
+}  // namespace b200q

@@ -1,0 +1,115 @@
+// What the two kernels for tens to hundreds of tokens (gemm_umma_mid.cu, gemm_umma_mid_w8a16.cu) share:
+// cluster operations, the TMA producer warps, the table of plans and the launch.
+#pragma once
+#include <cuda.h>
+#include <cuda_runtime.h>
+
+#include "common.h"
+#include "ptx_sm100.cuh"
+
+namespace b200q {
+
+constexpr int kMidThreads = 352;
+constexpr int kMidMaxStages = 12;
+constexpr int kMidCtrlBytes = 768;
+constexpr int kMidSmemTwo = 112 * 1024;          // two CTAs per SM
+constexpr int kMidSmemOne = 226 * 1024;          // one, with a deep ring
+
+__device__ __forceinline__ void st_cluster_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c,
+                                              uint32_t d) {
+  asm volatile("st.shared::cluster.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b),
+               "r"(c), "r"(d)
+               : "memory");
+}
+__device__ __forceinline__ void cluster_arrive() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() {
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// One operand's way through its ring of chunks of K blocks.
+struct MidStream {
+  const CUtensorMap* map;      // a block at a time: the end of K
+  const CUtensorMap* map3;     // whole chunks of whole blocks: one instruction
+  int row0, k_step;            // first row of the tile; bytes of a row per block
+  int blk, kc;                 // bytes of a block's tile; blocks per chunk
+  uint32_t dst, dst_step;      // shared address of the first slot, distance to the next
+  int ring;                    // slots
+  uint64_t *full, *free_bar;
+  int c0, chunks, chunks_3d;   // first chunk, how many; chunks below chunks_3d come through map3
+};
+
+// One warp per operand: the weights run ahead as far as their ring allows, first of all ahead of
+// the kernel that produces the activations.
+__device__ __forceinline__ void mid_produce(const MidStream& s, volatile int* abort_flag) {
+  int stage = 0, issued = 0;
+  uint32_t phase = 1;                                      // the first round waits for nobody
+  for (; issued < s.chunks; ++issued) {
+    if (issued >= s.ring && !ptx::mbar_wait(ptx::smem_u32(s.free_bar + stage), phase, abort_flag)) break;
+    if (ptx::elect_one()) {
+      const uint32_t bar = ptx::smem_u32(s.full + stage), dst = s.dst + stage * s.dst_step;
+      const int c = (s.c0 + issued) * s.kc;
+      ptx::mbar_arrive_expect_tx(bar, static_cast<uint32_t>(s.kc * s.blk));
+      if (s.c0 + issued < s.chunks_3d) {
+        ptx::tma_load_3d(dst, s.map3, bar, 0, s.row0, c);
+      } else {
+        for (int b = 0; b < s.kc; ++b) ptx::tma_load_2d(dst + b * s.blk, s.map, bar, (c + b) * s.k_step, s.row0);
+      }
+    }
+    __syncwarp();
+    if (++stage == s.ring) {
+      stage = 0;
+      phase ^= 1u;
+    }
+  }
+  if (*abort_flag != 0) {
+    // a wait ran out: give the copies in flight a bounded time to land before the CTA ends
+    for (int j = max(0, issued - s.ring); j < issued; ++j) {
+      const uint32_t parity = static_cast<uint32_t>((j / s.ring) & 1);
+      for (int tries = 0;
+           tries < (1 << 16) && !ptx::mbar_try_wait(ptx::smem_u32(s.full + j % s.ring), parity); ++tries) {
+      }
+    }
+  }
+}
+
+// The search for a plan costs some 10 us of host time, more than the launch: its results are kept per
+// thread, in a table of fixed size where a new shape replaces the one in its slot.
+template <typename Plan, bool (*search)(int, int, int, Plan*)>
+bool mid_plan(int M, int N, int K, Plan* best) {
+  if (debug_knob(B200Q_KNOB_BN, 0) != 0 || debug_knob(B200Q_KNOB_CLUSTER, 0) != 0) return search(M, N, K, best);
+  struct Entry {
+    int M, N, K;   // M = 0: empty
+    Plan plan;
+  };
+  constexpr unsigned kSlots = 1024;
+  thread_local Entry table[kSlots];
+  const unsigned h = static_cast<unsigned>(M) * 0x9E3779B1u ^ static_cast<unsigned>(N) * 0x85EBCA77u ^
+                     static_cast<unsigned>(K) * 0xC2B2AE3Du;
+  Entry& e = table[(h >> 16) % kSlots];
+  if (e.M != M || e.N != N || e.K != K) {
+    Entry fresh{M, N, K, {}};
+    if (!search(M, N, K, &fresh.plan)) return false;
+    e = fresh;
+  }
+  *best = e.plan;
+  return true;
+}
+
+template <auto kernel, typename Params>
+cudaError_t launch_mid_kernel(int ctas, int splits, size_t smem, cudaStream_t stream, const CUtensorMap& tx,
+                              const CUtensorMap& tw, const CUtensorMap& tx3, const CUtensorMap& tw3,
+                              const Params& mp) {
+  static bool attr_set[64] = {false};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 64 || !attr_set[dev]) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMidSmemOne);
+    if (e != cudaSuccess) return e;
+    if (dev < 64) attr_set[dev] = true;
+  }
+  return launch_clustered(splits, true, kernel, dim3(ctas), dim3(kMidThreads), smem, stream, tx, tw, tx3, tw3, mp);
+}
+
+}  // namespace b200q
