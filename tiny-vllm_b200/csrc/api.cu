@@ -80,7 +80,7 @@ int auto_path(int M, int N, int K, bool a16) {
   if (M <= 16) {
     if (bulk_decode_applicable(M, N, K, a16)) return B200Q_PATH_MMA_STREAM;
     // long K, or a matrix that the ring leaves to them: the tcgen05 kernels
-    return (K > 4096 || (a16 && bulk_decode_too_large(M, N, K))) && (N % 8) == 0 ? B200Q_PATH_UMMA : B200Q_PATH_MMA_STREAM;
+    return (K > 4096 || (a16 && bulk_decode_yields(M, N, K))) && (N % 8) == 0 ? B200Q_PATH_UMMA : B200Q_PATH_MMA_STREAM;
   }
   return M <= 32 && (N % 8) != 0 ? B200Q_PATH_MMA_STREAM : B200Q_PATH_UMMA;
 }

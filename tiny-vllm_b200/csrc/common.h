@@ -86,7 +86,7 @@ cudaError_t launch_w8a16_reg_decode(const GemmArgs& a);
 // gemm_bulk_decode.cu: persistent decode kernels for large matrices; a producer warp streams
 // weights and activations through a shared-memory ring of bulk asynchronous copies
 bool bulk_decode_applicable(int M, int N, int K, bool a16);
-bool bulk_decode_too_large(int M, int N, int K);
+bool bulk_decode_yields(int M, int N, int K);
 cudaError_t launch_w8a8_bulk_decode(const GemmArgs& a);
 cudaError_t launch_w8a16_bulk_decode(const GemmArgs& a);
 

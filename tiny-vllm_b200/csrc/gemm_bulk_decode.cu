@@ -157,6 +157,14 @@ __device__ __forceinline__ void init_barriers(const CtaSmem& c, const StreamPlan
 }
 
 // ------------------------------------------------------------------------- W8A8
+// 16 bytes of activations: a plain load (the read-only path may move it above the wait for the kernel that
+// writes them).
+__device__ __forceinline__ uint4 ld_act(const void* p) {
+  uint4 v;
+  asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+  return v;
+}
+
 // Activations come straight from global memory (they are small and stay in L2): the lane's
 // 32 bytes of token rows g and g + 8 of the NEXT segment are requested before the wait for
 // the current weight tile, so their latency is covered by a whole segment of work.  (Keeping a
@@ -164,8 +172,8 @@ __device__ __forceinline__ void init_barriers(const CtaSmem& c, const StreamPlan
 // K <= 4096, measured 1-2 us SLOWER: every CTA then asks for the same few lines at once.)
 template <typename OutT, int MT, bool RAW_I32, int WPP>
 __global__ void __launch_bounds__(kPipes * WPP * 32 + 32, 1)
-w8a8_stream_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const int8_t* __restrict__ xq,
-                          const float* __restrict__ a_s, const float* __restrict__ w_s,
+w8a8_stream_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const int8_t* xq,
+                          const float* a_s, const float* __restrict__ w_s,
                           const OutT* __restrict__ bias, void* __restrict__ out, int M, int N, int K,
                           const StreamPlan p, int* status) {
   constexpr int kCW = kPipes * WPP, kCT = kCW * 32;  // consumer warps / threads
@@ -204,10 +212,10 @@ w8a8_stream_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const int8_t
       const int r0 = m * 16 + g, r1 = r0 + 8;
       const int8_t* p0 = xq + static_cast<size_t>(r0) * K + k;
       const int8_t* p1 = xq + static_cast<size_t>(r1) * K + k;
-      x[m][0] = (r0 < M && k < K) ? __ldg(reinterpret_cast<const uint4*>(p0)) : zero;
-      x[m][1] = (r0 < M && k + 16 < K) ? __ldg(reinterpret_cast<const uint4*>(p0 + 16)) : zero;
-      x[m][2] = (r1 < M && k < K) ? __ldg(reinterpret_cast<const uint4*>(p1)) : zero;
-      x[m][3] = (r1 < M && k + 16 < K) ? __ldg(reinterpret_cast<const uint4*>(p1 + 16)) : zero;
+      x[m][0] = (r0 < M && k < K) ? ld_act(p0) : zero;
+      x[m][1] = (r0 < M && k + 16 < K) ? ld_act(p0 + 16) : zero;
+      x[m][2] = (r1 < M && k < K) ? ld_act(p1) : zero;
+      x[m][3] = (r1 < M && k + 16 < K) ? ld_act(p1 + 16) : zero;
     }
   };
 
@@ -304,7 +312,7 @@ w8a8_stream_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const int8_t
 // of the lane (4 codes) meets activation words 2 i and 2 i + 1 (2 values each) in one k16 step.
 template <typename T, int MT, int WPP>
 __global__ void __launch_bounds__(kPipes * WPP * 32 + 32, 1)
-w8a16_stream_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const T* __restrict__ x,
+w8a16_stream_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const T* x,
                            const float* __restrict__ sc, const T* __restrict__ bias,
                            T* __restrict__ y, int M, int N, int K, const StreamPlan p, int* status) {
   constexpr int kCW = kPipes * WPP, kCT = kCW * 32;  // consumer warps / threads
@@ -345,8 +353,8 @@ w8a16_stream_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const T* __
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const bool k_ok = k + 8 * j < K;  // K is a multiple of 16: a piece is inside or outside
-        xa[m][j] = (r0 < M && k_ok) ? __ldg(reinterpret_cast<const uint4*>(p0) + j) : zero;
-        xb[m][j] = (r1 < M && k_ok) ? __ldg(reinterpret_cast<const uint4*>(p1) + j) : zero;
+        xa[m][j] = (r0 < M && k_ok) ? ld_act(p0 + 8 * j) : zero;
+        xb[m][j] = (r1 < M && k_ok) ? ld_act(p1 + 8 * j) : zero;
       }
     }
   };
@@ -380,9 +388,9 @@ w8a16_stream_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const T* __
           if (jj * 8 < rows) {
             const uint4 w0 = *reinterpret_cast<const uint4*>(ws + jj * 1024 + o0);
             const uint4 w1 = *reinterpret_cast<const uint4*>(ws + jj * 1024 + o1);
-            const uint2 e0 = expand4<T>(w0.x), e1 = expand4<T>(w0.y), e2 = expand4<T>(w0.z),
-                        e3 = expand4<T>(w0.w), e4 = expand4<T>(w1.x), e5 = expand4<T>(w1.y),
-                        e6 = expand4<T>(w1.z), e7 = expand4<T>(w1.w);
+            const uint2 e0 = expand4_scaled<T>(w0.x), e1 = expand4_scaled<T>(w0.y), e2 = expand4_scaled<T>(w0.z),
+                        e3 = expand4_scaled<T>(w0.w), e4 = expand4_scaled<T>(w1.x), e5 = expand4_scaled<T>(w1.y),
+                        e6 = expand4_scaled<T>(w1.z), e7 = expand4_scaled<T>(w1.w);
 #pragma unroll
             for (int m = 0; m < MT; ++m) {
               mma_16<T>(acc[m][j], ca[m][0].x, cb[m][0].x, ca[m][0].y, cb[m][0].y, e0.x, e0.y);
@@ -428,7 +436,7 @@ w8a16_stream_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const T* __
           sum = __fadd_rn(sum, red[wi * (16 * kUnitRows) + o]);  // fixed order
         const int n = ulo + ch;
         const float b = bias != nullptr ? to_float<T>(bias[n]) : 0.f;
-        y[static_cast<size_t>(tok) * N + n] = from_float<T>(__fadd_rn(__fmul_rn(sum, sc[n]), b));
+        y[static_cast<size_t>(tok) * N + n] = from_float<T>(__fadd_rn(__fmul_rn(sum, sc[n] * kCodeUnit<T>), b));
       }
       consumer_barrier<kCT>();
     }
@@ -447,7 +455,7 @@ w8a16_stream_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const T* __
 // fixed-order reduction — is as above.
 template <typename T, int WPP>
 __global__ void __launch_bounds__(kPipes * WPP * 32 + 32, 1)
-w8a16_stream_decode_m8_kernel(const __grid_constant__ CUtensorMap tm_w, const T* __restrict__ x,
+w8a16_stream_decode_m8_kernel(const __grid_constant__ CUtensorMap tm_w, const T* x,
                               const float* __restrict__ sc, const T* __restrict__ bias,
                               T* __restrict__ y, int M, int N, int K, const StreamPlan p,
                               int* status) {
@@ -489,7 +497,7 @@ w8a16_stream_decode_m8_kernel(const __grid_constant__ CUtensorMap tm_w, const T*
     const T* p0 = x + static_cast<size_t>(g) * K + k;
 #pragma unroll
     for (int j = 0; j < 2 * kHalves; ++j)
-      xv[j] = (g < M && k + 8 * j < K) ? __ldg(reinterpret_cast<const uint4*>(p0) + j) : zero;
+      xv[j] = (g < M && k + 8 * j < K) ? ld_act(p0 + 8 * j) : zero;
   };
 
   uint4 xc[2 * kHalves], xn[2 * kHalves];
@@ -524,13 +532,13 @@ w8a16_stream_decode_m8_kernel(const __grid_constant__ CUtensorMap tm_w, const T*
               const uint4 x0 = xc[2 * h], x1 = xc[2 * h + 1];
               uint2 ea, eb;
               // weight word i of the piece meets activation words 2 i and 2 i + 1
-              ea = expand4<T>(a.x); eb = expand4<T>(b.x);
+              ea = expand4_scaled<T>(a.x); eb = expand4_scaled<T>(b.x);
               mma_16<T>(acc[q], ea.x, eb.x, ea.y, eb.y, x0.x, x0.y);
-              ea = expand4<T>(a.y); eb = expand4<T>(b.y);
+              ea = expand4_scaled<T>(a.y); eb = expand4_scaled<T>(b.y);
               mma_16<T>(acc[q], ea.x, eb.x, ea.y, eb.y, x0.z, x0.w);
-              ea = expand4<T>(a.z); eb = expand4<T>(b.z);
+              ea = expand4_scaled<T>(a.z); eb = expand4_scaled<T>(b.z);
               mma_16<T>(acc[q], ea.x, eb.x, ea.y, eb.y, x1.x, x1.y);
-              ea = expand4<T>(a.w); eb = expand4<T>(b.w);
+              ea = expand4_scaled<T>(a.w); eb = expand4_scaled<T>(b.w);
               mma_16<T>(acc[q], ea.x, eb.x, ea.y, eb.y, x1.z, x1.w);
             }
           }
@@ -562,7 +570,7 @@ w8a16_stream_decode_m8_kernel(const __grid_constant__ CUtensorMap tm_w, const T*
         sum = __fadd_rn(sum, red[wi * (8 * kUnitRows) + o]);  // fixed order
       const int n = ulo + ch;
       const float b = bias != nullptr ? to_float<T>(bias[n]) : 0.f;
-      y[static_cast<size_t>(tok) * N + n] = from_float<T>(__fadd_rn(__fmul_rn(sum, sc[n]), b));
+      y[static_cast<size_t>(tok) * N + n] = from_float<T>(__fadd_rn(__fmul_rn(sum, sc[n] * kCodeUnit<T>), b));
     }
     consumer_barrier<kCT>();
   }
@@ -625,14 +633,16 @@ bool bulk_decode_applicable(int M, int N, int K, bool a16) {
   if (!make_plan(M, N, K, a16, p)) return false;
   if (knob == 2) return true;
   return M <= 16 && static_cast<long long>(N) * K >= (8ll << 20) && N >= 8 * sm_count() &&
-         !(a16 && bulk_decode_too_large(M, N, K)) && !reg_decode_preferred(M, N, K, a16);
+         !(a16 && bulk_decode_yields(M, N, K)) && !reg_decode_preferred(M, N, K, a16);
 }
 
-// W8A16 from 9 tokens on: the MMAs of a second token half and the expansion bound this kernel (36 us for 24576 x
-// 4096 at 12 tokens, 27 at 8), so matrices of 32 MB and more go to tcgen05 (32 us; 4096 x 12288 at
-// 12 tokens 16.3 against 19.4).
-bool bulk_decode_too_large(int M, int N, int K) {
-  return M > 8 && static_cast<long long>(N) * K >= (32ll << 20) && (N % 8) == 0;
+// W8A16 from 9 tokens on: this kernel then needs twice the MMAs, and the tcgen05 kernel is ahead (us at 16 tokens, this
+// kernel first): 24576 x 4096 34.4 and 22.9, 4096 x 12288 18.6 and 14.3, 9728 x 2560 12.6 and 9.4, 2560 x 9728 13.6
+// and 10.1, 4096 x 4096 8.4 and 6.6.  It stays where a CTA's share is one well-filled unit of 40 to 48
+// channels and the matrix is not large (6144 x 4096), the case it is laid out for.
+bool bulk_decode_yields(int M, int N, int K) {
+  const bool one_unit = N >= 40 * sm_count() && N <= kUnitRows * sm_count();
+  return M > 8 && (N % 8) == 0 && !(one_unit && static_cast<long long>(N) * K < (32ll << 20));
 }
 
 cudaError_t launch_w8a8_bulk_decode(const GemmArgs& a) {

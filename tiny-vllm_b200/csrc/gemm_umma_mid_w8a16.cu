@@ -11,6 +11,8 @@
 //   * the channels are the 128 rows of the UMMA tile and the tokens its columns (16 to 256): a converter thread
 //     reads one row of int8 from shared memory and writes it expanded to its TMEM lane (tcgen05.st);
 //     the MMA takes its A operand from there;
+//   * a tile may have fewer than 128 channels: as many as give every CTA that the GPU holds one tile
+//     (24576 x 4096 at 64 tokens: 280 tiles of 88 channels 26.3 us, 192 of 128 30.4);
 //   * an MMA of 64 columns takes 51 cycles and one of 128 68, whatever part of the 128 rows is used, so
 //     it is the tokens, the operand with fewer rows, that are cut finely.
 // Chains of launches, us per linear (expanded weights in shared memory; persistent kernels before that): 768 x
@@ -43,6 +45,7 @@ constexpr int kMidACols = 32;                    // TMEM columns of one K block 
 struct MidParams {
   int M, N;
   int bt;                  // tokens per tile (UMMA N)
+  int rows;                // channels per tile: 128, or fewer where that spreads the matrix better
   int tiles_t;
   int kc;                  // K blocks (64 elements) per chunk
   int chunks, chunks_per_split;
@@ -136,8 +139,8 @@ w8a16_mid_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
       // -------------------------------------------------------------- TMA producers
       const bool weights = warp != 0;
       const MidStream s{weights ? &tmap_w : &tmap_x, weights ? &tmap_w3 : &tmap_x3,
-                        weights ? tile_c * kMidCh : tile_t * p.bt, weights ? kRow8 : 128,
-                        weights ? kMidCh * kRow8 : x_blk, p.kc, smem_base + (weights ? raw_base : 0u),
+                        weights ? tile_c * p.rows : tile_t * p.bt, weights ? kRow8 : 128,
+                        weights ? p.rows * kRow8 : x_blk, p.kc, smem_base + (weights ? raw_base : 0u),
                         static_cast<uint32_t>(weights ? p.raw_bytes : p.stage_bytes), p.stages,
                         weights ? wfull : xfull, weights ? rempty : empty, c0, n_ch, p.chunks_3d};
       if (weights) {
@@ -197,28 +200,29 @@ w8a16_mid_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
     const uint32_t lanes = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
     // channel scales: constants, fetched ahead of the wait
     if (tid < kMidCh) {
-      const int col = tile_c * kMidCh + tid;
-      s_ws[tid] = col < p.N ? __ldg(p.w_scales + col) : 0.f;
+      const int col = tile_c * p.rows + tid;
+      s_ws[tid] = tid < p.rows && col < p.N ? __ldg(p.w_scales + col) * kCodeUnit<T> : 0.f;
     }
     if (run) {
       // -------------------------------------------------------------- expansion
       // Both rings have an even number of slots, so a slot always belongs to the same group: a group that has not
       // seen the previous use of a slot complete could not tell its barrier's phases apart.
       const int group = cw >> 2;
-      const int sw8 = (ch >> 1) & 3;
+      const int sw8 = (min(ch, p.rows - 1) >> 1) & 3;          // rows % 8 == 0: the same in every block
       int rs = group, as = group;
       uint32_t rphase = 0, aphase = 1;
       for (int i = group; i < n_ch; i += 2) {
         if (!ptx::mbar_wait(ptx::smem_u32(wfull + rs), rphase, abort_flag)) break;
         if (i >= p.a_stages && !ptx::mbar_wait(ptx::smem_u32(aempty + as), aphase, abort_flag)) break;
         ptx::tc_fence_after_sync();
-        const uint8_t* src = smem + raw_base + rs * p.raw_bytes + ch * kRow8;
-        for (int b = 0; b < p.kc; ++b, src += kMidCh * kRow8) {
+        // rows beyond the tile's last: what they hold only reaches accumulator lanes nobody reads
+        const uint8_t* src = smem + raw_base + rs * p.raw_bytes + min(ch, p.rows - 1) * kRow8;
+        for (int b = quarter * 32 < p.rows ? 0 : p.kc; b < p.kc; ++b, src += p.rows * kRow8) {
           uint32_t v[32];
 #pragma unroll
           for (int c = 0; c < 4; ++c) {
             const uint4 w = *reinterpret_cast<const uint4*>(src + ((c ^ sw8) << 4));
-            const uint2 e0 = expand4<T>(w.x), e1 = expand4<T>(w.y), e2 = expand4<T>(w.z), e3 = expand4<T>(w.w);
+            const uint2 e0 = expand4_scaled<T>(w.x), e1 = expand4_scaled<T>(w.y), e2 = expand4_scaled<T>(w.z), e3 = expand4_scaled<T>(w.w);
             v[8 * c + 0] = e0.x;
             v[8 * c + 1] = e0.y;
             v[8 * c + 2] = e1.x;
@@ -257,7 +261,8 @@ w8a16_mid_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
     if (done) {
       ptx::tc_fence_after_sync();
       const T* bias = reinterpret_cast<const T*>(p.bias);
-      const int n = tile_c * kMidCh + ch;
+      const int n = tile_c * p.rows + ch;
+      const bool mine_n = ch < p.rows && n < p.N;
       const int shift = __ffs(p.splits) - 1;
       const uint32_t mine = ptx::smem_u32(red) + static_cast<uint32_t>(rank * rows_own * kMidCh + ch) * 4u;
       const int live = min(p.bt, p.M - tile_t * p.bt);         // tokens of this tile
@@ -270,7 +275,7 @@ w8a16_mid_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
 #pragma unroll
           for (int j = 0; j < 32; ++j) {
             const int tok = c + j;
-            if (tok < live)
+            if (tok < live && ch < p.rows)
               ptx::st_shared_cluster_u32(
                   ptx::map_to_cta(mine + static_cast<uint32_t>((tok >> shift) * kMidCh) * 4u,
                                   static_cast<uint32_t>(tok & (p.splits - 1))),
@@ -284,12 +289,12 @@ w8a16_mid_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
           T* out = static_cast<T*>(p.out) + static_cast<size_t>(tile_t * p.bt + c + (odd ? 1 : 0)) * p.N + (odd ? n - 1 : n);
 #pragma unroll
           for (int j = 0; j < 32; j += 2) {
-            const T* b = n < p.N ? bias : nullptr;
+            const T* b = mine_n ? bias : nullptr;
             const uint32_t lo = bits16(finish<T>(v[j], w_s, b, n));
             const uint32_t hi = bits16(finish<T>(v[j + 1], w_s, b, n));
             const uint32_t got = __shfl_xor_sync(0xFFFFFFFFu, odd ? lo : hi, 1);
             const uint32_t word = odd ? (got | (hi << 16)) : (lo | (got << 16));
-            if (c + j + (odd ? 1 : 0) < live && n < p.N) *reinterpret_cast<uint32_t*>(out) = word;   // N is even
+            if (c + j + (odd ? 1 : 0) < live && mine_n) *reinterpret_cast<uint32_t*>(out) = word;   // N is even
             out += 2 * static_cast<size_t>(p.N);
           }
         }
@@ -319,8 +324,8 @@ w8a16_mid_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
     for (int u = threadIdx.x; u < rows_own * (kMidCh / 8); u += kMidThreads) {
       const int tl = u / (kMidCh / 8), cg = u % (kMidCh / 8);  // 8 channels: one 16-byte store
       const int tok = tl * p.splits + rank;
-      const int row = tile_t * p.bt + tok, col = tile_c * kMidCh + cg * 8;
-      if (tok >= p.bt || row >= p.M || col >= p.N) continue;   // N % 8 == 0
+      const int row = tile_t * p.bt + tok, col = tile_c * p.rows + cg * 8;
+      if (tok >= p.bt || cg * 8 >= p.rows || row >= p.M || col >= p.N) continue;   // N % 8 == 0
       uint32_t w[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
       for (int s = 0; s < p.splits; ++s) {       // rank order: results do not depend on the run
         const uint4* src = reinterpret_cast<const uint4*>(red) + ((s * rows_own + tl) * kMidCh + cg * 8) / 4;
@@ -350,22 +355,23 @@ w8a16_mid_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
 namespace {
 
 struct MidPlan {
-  int bt, splits, kc, chunks, chunks_per_split, tiles_t, tiles_c;
+  int bt, rows, splits, kc, chunks, chunks_per_split, tiles_t, tiles_c;
   int stages, stage_bytes, raw_bytes, a_stages, a_col0, tmem_cols;
   size_t smem;
 };
 
-bool mid_plan_for(int M, int N, int k_blocks, int bt, int splits, int kc, int smem_cap, MidPlan* pl) {
+bool mid_plan_for(int M, int N, int k_blocks, int bt, int rows, int splits, int kc, int smem_cap, MidPlan* pl) {
   pl->bt = bt;
+  pl->rows = rows;
   pl->kc = kc;
   pl->splits = splits;
   pl->chunks = (k_blocks + kc - 1) / kc;
   pl->chunks_per_split = (pl->chunks + splits - 1) / splits;
   if (pl->chunks_per_split * (splits - 1) >= pl->chunks) return false;   // a CTA without work
   pl->tiles_t = (M + bt - 1) / bt;
-  pl->tiles_c = (N + kMidCh - 1) / kMidCh;
+  pl->tiles_c = (N + rows - 1) / rows;
   pl->stage_bytes = kc * bt * 128;
-  pl->raw_bytes = kc * kMidCh * kRow8;
+  pl->raw_bytes = (kc * rows * kRow8 + 1023) / 1024 * 1024;
   const int rows_own = (bt + splits - 1) / splits;
   const int fixed = (splits > 1 ? splits * rows_own * kMidCh * 4 : 0) + kMidCh * 4 + kMidCtrlBytes;
   const int ring_bytes = pl->stage_bytes + pl->raw_bytes;
@@ -422,16 +428,28 @@ bool search_plan(int M, int N, int K, MidPlan* best) {
   double best_cost = 1e30;
   for (int bt : {16, 32, 48, 64, 96, 128, 192, 256}) {
     if (want_bt != 0 ? bt != want_bt : bt >= M + 32 && bt > 32) continue;
+    const int tiles_t = (M + bt - 1) / bt;
     for (int s : {1, 2, 4, 8}) {
       if (want_s != 0 && s != want_s) continue;
-      for (int kc : {4, 2, 1}) {
-        for (int cap : {kMidSmemOne, kMidSmemTwo}) {
-          MidPlan pl;
-          if (!mid_plan_for(M, N, k_blocks, bt, s, kc, cap, &pl)) continue;
-          const double cost = mid_cost(pl, M, static_cast<double>(N) * K);
-          if (cost < best_cost) {
-            best_cost = cost;
-            *best = pl;
+      // channels per tile: all 128, or as many as make one tile for every CTA that the GPU holds
+      for (int ctas : {0, 1, 2}) {
+        int rows = kMidCh;
+        if (ctas > 0) {
+          const int tiles_c = ctas * sm_count() / (s * tiles_t);
+          if (tiles_c < 1) continue;
+          rows = ((N + tiles_c - 1) / tiles_c + 7) / 8 * 8;
+          if (rows < 64 || rows >= kMidCh) continue;
+        }
+        for (int kc : {4, 2, 1}) {
+          for (int cap : {kMidSmemOne, kMidSmemTwo}) {
+            MidPlan pl;
+            if (!mid_plan_for(M, N, k_blocks, bt, rows, s, kc, cap, &pl)) continue;
+            if (s > 1 && pl.tiles_t * pl.tiles_c * s > 2 * sm_count()) continue;   // beyond what was measured
+            const double cost = mid_cost(pl, M, static_cast<double>(N) * K);
+            if (cost < best_cost) {
+              best_cost = cost;
+              *best = pl;
+            }
           }
         }
       }
@@ -464,7 +482,7 @@ int launch_umma16_mid(const GemmArgs& a) {
   CUtensorMap tx, tw;
   const uint64_t x_row = static_cast<uint64_t>(a.K) * 2;
   if (!make_tensor_map(a.x, a.M, x_row, static_cast<uint32_t>(pl.bt), 128, &tx) ||
-      !get_tensor_map(a.w, a.N, a.K, static_cast<uint32_t>(kMidCh), kRow8, &tw))
+      !get_tensor_map(a.w, a.N, a.K, static_cast<uint32_t>(pl.rows), kRow8, &tw))
     return B200Q_ERR_LAUNCH;
   // K a multiple of a block: everything comes through the 3-D maps (blocks beyond K read as zeros);
   // otherwise the chunk with the partial block, and what follows it, goes block by block
@@ -472,12 +490,13 @@ int launch_umma16_mid(const GemmArgs& a) {
   CUtensorMap tx3 = tx, tw3 = tw;
   if (chunks_3d > 0 &&
       (!make_tensor_map(a.x, a.M, x_row, static_cast<uint32_t>(pl.bt), 128, &tx3, pl.kc) ||
-       !get_tensor_map(a.w, a.N, a.K, static_cast<uint32_t>(kMidCh), kRow8, &tw3, pl.kc)))
+       !get_tensor_map(a.w, a.N, a.K, static_cast<uint32_t>(pl.rows), kRow8, &tw3, pl.kc)))
     return B200Q_ERR_LAUNCH;
   MidParams mp{};
   mp.M = a.M;
   mp.N = a.N;
   mp.bt = pl.bt;
+  mp.rows = pl.rows;
   mp.tiles_t = pl.tiles_t;
   mp.kc = pl.kc;
   mp.chunks = pl.chunks;

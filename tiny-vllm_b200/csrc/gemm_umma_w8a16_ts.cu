@@ -222,8 +222,8 @@ w8a16_umma_ts_kernel(const __grid_constant__ CUtensorMap tmap_x,
         for (int c = 0; c < 4; ++c) {
           uint4 w = make_uint4(0u, 0u, 0u, 0u);
           if (!(p.debug_flags & 8)) w = *reinterpret_cast<const uint4*>(src_row + ((c ^ sw8) << 4));
-          const uint2 e0 = expand4<T>(w.x), e1 = expand4<T>(w.y), e2 = expand4<T>(w.z),
-                      e3 = expand4<T>(w.w);
+          const uint2 e0 = expand4_scaled<T>(w.x), e1 = expand4_scaled<T>(w.y), e2 = expand4_scaled<T>(w.z),
+                      e3 = expand4_scaled<T>(w.w);
           v[8 * c + 0] = e0.x;
           v[8 * c + 1] = e0.y;
           v[8 * c + 2] = e1.x;
@@ -261,7 +261,7 @@ w8a16_umma_ts_kernel(const __grid_constant__ CUtensorMap tmap_x,
       const int ch0 = tile_ch * kTsChannels + t * kTileA;       // first channel of this A tile
       const int ch = ch0 + quarter * 32 + lane;
       const bool ch_ok = ch < p.N;
-      const float s = ch_ok ? __ldg(p.w_scales + ch) : 0.f;
+      const float s = ch_ok ? __ldg(p.w_scales + ch) * kCodeUnit<T> : 0.f;
       const float b = (ch_ok && bias != nullptr) ? to_float<T>(bias[ch]) : 0.f;
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) +
                              static_cast<uint32_t>(t * kTsTokens);
