@@ -114,36 +114,12 @@ act_quant_long_rows_kernel(const T* x, int64_t ldx, int8_t* xq, float* a_scales,
 
 template <typename T>
 cudaError_t launch_typed(const T* x, int64_t ldx, int8_t* xq, float* a_scales, int M, int K,
-                         cudaStream_t s) {
-  // Four 16-byte chunks per thread keep the register count low (high occupancy); longer
-  // rows are spread over more threads instead of more chunks.
-  auto blocks = [&](int g) { return (M + (256 / g) - 1) / (256 / g); };
-  // Few rows: the chain of one thread counts, not the occupancy, so every thread gets one chunk.
-  if (M <= 512 && K > 32 * 8) {
-    if (K <= 64 * 8)
-      return launch_overlapped(act_quant_rows_kernel<T, 64, 1>, blocks(64), 256, 0, s, x, ldx, xq, a_scales, M, K);
-    if (K <= 128 * 8)
-      return launch_overlapped(act_quant_rows_kernel<T, 128, 1>, blocks(128), 256, 0, s, x, ldx, xq, a_scales, M, K);
-    if (K <= 256 * 8)
-      return launch_overlapped(act_quant_rows_kernel<T, 256, 1>, blocks(256), 256, 0, s, x, ldx, xq, a_scales, M, K);
-    if (K <= 256 * 8 * 2)
-      return launch_overlapped(act_quant_rows_kernel<T, 256, 2>, blocks(256), 256, 0, s, x, ldx, xq, a_scales, M, K);
-  }
-  if (K <= 32 * 8 * 2) {
-    return launch_overlapped(act_quant_rows_kernel<T, 32, 2>, blocks(32), 256, 0, s, x, ldx, xq, a_scales, M, K);
-  } else if (K <= 32 * 8 * 4) {
-    return launch_overlapped(act_quant_rows_kernel<T, 32, 4>, blocks(32), 256, 0, s, x, ldx, xq, a_scales, M, K);
-  } else if (K <= 64 * 8 * 4) {
-    return launch_overlapped(act_quant_rows_kernel<T, 64, 4>, blocks(64), 256, 0, s, x, ldx, xq, a_scales, M, K);
-  } else if (K <= 128 * 8 * 4) {
-    return launch_overlapped(act_quant_rows_kernel<T, 128, 4>, blocks(128), 256, 0, s, x, ldx, xq, a_scales, M, K);
-  } else if (K <= 256 * 8 * 4) {
-    return launch_overlapped(act_quant_rows_kernel<T, 256, 4>, blocks(256), 256, 0, s, x, ldx, xq, a_scales, M, K);
-  } else if (K <= 256 * 8 * 8) {
-    return launch_overlapped(act_quant_rows_kernel<T, 256, 8>, blocks(256), 256, 0, s, x, ldx, xq, a_scales, M, K);
-  } else {
-    return launch_overlapped(act_quant_long_rows_kernel<T>, M, 256, 0, s, x, ldx, xq, a_scales, M, K);
-  }
+                         cudaStream_t st) {
+  cudaError_t e;
+  if (K > 256 * 8 * 8)
+    return launch_overlapped(act_quant_long_rows_kernel<T>, M, 256, 0, st, x, ldx, xq, a_scales, M, K);
+  B200Q_ROWS_DISPATCH(act_quant_rows_kernel, K >> 3, x, ldx, xq, a_scales, M, K);
+  return e;
 }
 
 }  // namespace

@@ -151,10 +151,10 @@ __device__ __forceinline__ float warp_sum(float v) {
   return v;
 }
 
-// Reduction over the G threads of a row group (warps of a group are neighbours in the CTA).
-template <int G, bool IS_MAX>
-__device__ __forceinline__ float group_reduce(float v, float* red, int g) {
-  v = IS_MAX ? warp_max(v) : warp_sum(v);
+// Maximum over the G threads of a row group (warps of a group are neighbours in the CTA).
+template <int G>
+__device__ __forceinline__ float group_max(float v, float* red, int g) {
+  v = warp_max(v);
   if (G > 32) {
     constexpr int kWarpsPerRow = G / 32;
     __syncthreads();  // red may still be read from the previous reduction
@@ -163,10 +163,38 @@ __device__ __forceinline__ float group_reduce(float v, float* red, int g) {
     float m = red[g * kWarpsPerRow];
 #pragma unroll
     for (int i = 1; i < kWarpsPerRow; ++i)
-      m = IS_MAX ? fmaxf(m, red[g * kWarpsPerRow + i]) : m + red[g * kWarpsPerRow + i];
+      m = fmaxf(m, red[g * kWarpsPerRow + i]);
     v = m;
   }
   return v;
+}
+
+// Sum over a row from one partial sum per 16-byte chunk (chunk c * G + t belongs to thread t), in an order that
+// depends on the chunks alone: 32 neighbouring chunks by butterfly, then these sums in ascending order.
+// So the kernels that sum squares agree bit for bit however many threads they give a row.  red: 8 * CHUNKS.
+template <int G, int CHUNKS>
+__device__ __forceinline__ float row_sum(float (&part)[CHUNKS], float* red, int g) {
+#pragma unroll
+  for (int c = 0; c < CHUNKS; ++c) part[c] = warp_sum(part[c]);
+  float total;
+  if (G == 32) {
+    total = part[0];
+#pragma unroll
+    for (int c = 1; c < CHUNKS; ++c) total += part[c];
+  } else {
+    constexpr int kWarpsPerRow = G / 32, kSums = kWarpsPerRow * CHUNKS;
+    __syncthreads();  // red may still be read from the previous reduction
+    if ((threadIdx.x & 31) == 0) {
+#pragma unroll
+      for (int c = 0; c < CHUNKS; ++c)
+        red[g * kSums + c * kWarpsPerRow + ((threadIdx.x % G) >> 5)] = part[c];
+    }
+    __syncthreads();
+    total = red[g * kSums];
+#pragma unroll
+    for (int i = 1; i < kSums; ++i) total += red[g * kSums + i];
+  }
+  return total;
 }
 
 // Common tail: y (CHUNKS chunks of 8 values per thread) -> optional store, absmax, int8 codes.
@@ -183,7 +211,7 @@ __device__ __forceinline__ void quantise_row(const uint4 (&y)[CHUNKS], bool acti
     running.add(y[c].z);
     running.add(y[c].w);
   }
-  const float amax = group_reduce<G, true>(running.value(), red, g);
+  const float amax = group_max<G>(running.value(), red, g);
   if (!active) return;
   const float scale = fmaxf(__fdiv_rn(amax, 127.0f), 1e-8f);
   const float inv_scale = __frcp_rn(scale);
@@ -200,6 +228,26 @@ __device__ __forceinline__ void quantise_row(const uint4 (&y)[CHUNKS], bool acti
   }
 }
 
+// Launches KERNEL<T, threads per row, chunks per thread> (`e = launch_overlapped(...)` on stream st) for M rows of
+// NCHUNK 16-byte chunks (at most 2048).
+#define B200Q_ROWS(KERNEL, G, C, ...) \
+  e = launch_overlapped(KERNEL<T, G, C>, (M + 256 / G - 1) / (256 / G), 256, 0, st, __VA_ARGS__)
+#define B200Q_ROWS_C(KERNEL, G, C_, ...)                        \
+  do {                                                          \
+    if ((C_) == 1) B200Q_ROWS(KERNEL, G, 1, __VA_ARGS__);       \
+    else if ((C_) == 2) B200Q_ROWS(KERNEL, G, 2, __VA_ARGS__);  \
+    else if ((C_) == 3) B200Q_ROWS(KERNEL, G, 3, __VA_ARGS__);  \
+    else B200Q_ROWS(KERNEL, G, 4, __VA_ARGS__);                 \
+  } while (0)
+#define B200Q_ROWS_DISPATCH(KERNEL, NCHUNK, ...)                          \
+  do {                                                                    \
+    const RowShape rs_ = row_shape(M, NCHUNK);                            \
+    if (rs_.g == 32) B200Q_ROWS_C(KERNEL, 32, rs_.c, __VA_ARGS__);        \
+    else if (rs_.g == 64) B200Q_ROWS_C(KERNEL, 64, rs_.c, __VA_ARGS__);   \
+    else if (rs_.g == 128) B200Q_ROWS_C(KERNEL, 128, rs_.c, __VA_ARGS__); \
+    else if (rs_.c <= 4) B200Q_ROWS_C(KERNEL, 256, rs_.c, __VA_ARGS__);   \
+    else B200Q_ROWS(KERNEL, 256, 8, __VA_ARGS__);                         \
+  } while (0)
 
 }  // namespace
 }  // namespace b200q

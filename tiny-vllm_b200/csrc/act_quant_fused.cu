@@ -41,23 +41,34 @@ add_rmsnorm_quant_kernel(const T* x, const T* residual_in, const T* __restrict__
   ptx::grid_dependency_wait();     // ordinary loads from here on: a non-coherent one may move ahead
   const int g = threadIdx.x / G, t = threadIdx.x % G;
   const int row = blockIdx.x * kRowsPerBlock + g;
-  __shared__ float red[8];
+  __shared__ float red[8 * CHUNKS];
   const bool active = row < M;
   const int nchunk = K >> 3;
 
-  float s[CHUNKS][8];
-  float sumsq = 0.f;
+  // The norm weight is loaded with the row, which takes it out of the chain behind the reduction's barriers (512 x 1024
+  // 3.2 -> 3.0 us, 8192 x 4096 45 -> 42), except by a warp with a long row of its own: no barriers, and the
+  // registers count for more (8192 x 1024 12.1 -> 11.4).
+  constexpr bool kEarlyWeight = G > 32 || CHUNKS <= 2;
+  // all loads first: the store of the new residual may not be moved ahead of a later load
+  // (8192 x 4096 52.9 -> 42 us, 1999 x 1024 6.6 -> 4.8)
+  uint4 xv[CHUNKS], rv[CHUNKS], wv[CHUNKS];
 #pragma unroll
   for (int c = 0; c < CHUNKS; ++c) {
     const int idx = c * G + t;
     const bool live = active && idx < nchunk;
-    uint4 xv = make_uint4(0u, 0u, 0u, 0u), rv = xv;
-    if (live) {
-      xv = *(reinterpret_cast<const uint4*>(x + static_cast<size_t>(row) * K) + idx);
-      if (residual_in != nullptr)
-        rv = *(reinterpret_cast<const uint4*>(residual_in + static_cast<size_t>(row) * K) + idx);
-    }
-    const uint32_t xw[4] = {xv.x, xv.y, xv.z, xv.w}, rw[4] = {rv.x, rv.y, rv.z, rv.w};
+    xv[c] = rv[c] = wv[c] = make_uint4(0u, 0u, 0u, 0u);
+    if (kEarlyWeight && idx < nchunk) wv[c] = __ldg(reinterpret_cast<const uint4*>(weight) + idx);
+    if (live) xv[c] = *(reinterpret_cast<const uint4*>(x + static_cast<size_t>(row) * K) + idx);
+    if (live && residual_in != nullptr)
+      rv[c] = *(reinterpret_cast<const uint4*>(residual_in + static_cast<size_t>(row) * K) + idx);
+  }
+  float s[CHUNKS][8];
+  float sumsq[CHUNKS];
+#pragma unroll
+  for (int c = 0; c < CHUNKS; ++c) {
+    const int idx = c * G + t;
+    sumsq[c] = 0.f;
+    const uint32_t xw[4] = {xv[c].x, xv[c].y, xv[c].z, xv[c].w}, rw[4] = {rv[c].x, rv[c].y, rv[c].z, rv[c].w};
     uint32_t out[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -66,24 +77,23 @@ add_rmsnorm_quant_kernel(const T* x, const T* residual_in, const T* __restrict__
       const float s1 = residual_in != nullptr ? __fadd_rn(a.y, b.y) : a.y;
       s[c][2 * i] = s0;
       s[c][2 * i + 1] = s1;
-      sumsq = __fmaf_rn(s0, s0, sumsq);
-      sumsq = __fmaf_rn(s1, s1, sumsq);
+      sumsq[c] = __fmaf_rn(s0, s0, sumsq[c]);
+      sumsq[c] = __fmaf_rn(s1, s1, sumsq[c]);
       out[i] = pack2<T>(s0, s1);
     }
-    if (live && residual_out != nullptr)
+    if (active && idx < nchunk && residual_out != nullptr)
       *(reinterpret_cast<uint4*>(residual_out + static_cast<size_t>(row) * K) + idx) =
           make_uint4(out[0], out[1], out[2], out[3]);
   }
-  const float total = group_reduce<G, false>(sumsq, red, g);
+  const float total = row_sum<G, CHUNKS>(sumsq, red, g);
   const float inv_rms = __frsqrt_rn(__fadd_rn(__fdiv_rn(total, static_cast<float>(K)), eps));
 
   uint4 y[CHUNKS];
 #pragma unroll
   for (int c = 0; c < CHUNKS; ++c) {
     const int idx = c * G + t;
-    uint4 wv = make_uint4(0u, 0u, 0u, 0u);
-    if (idx < nchunk) wv = __ldg(reinterpret_cast<const uint4*>(weight) + idx);
-    const uint32_t ww[4] = {wv.x, wv.y, wv.z, wv.w};
+    if (!kEarlyWeight && idx < nchunk) wv[c] = __ldg(reinterpret_cast<const uint4*>(weight) + idx);
+    const uint32_t ww[4] = {wv[c].x, wv[c].y, wv[c].z, wv[c].w};
     uint32_t out[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -116,17 +126,20 @@ silu_mul_quant_kernel(const T* gate_up, int64_t ld, T* y_out, int8_t* xq, float*
   const bool active = row < M;
   const int nchunk = I >> 3;
 
-  uint4 y[CHUNKS];
+  uint4 gv[CHUNKS], uv[CHUNKS], y[CHUNKS];
 #pragma unroll
   for (int c = 0; c < CHUNKS; ++c) {
     const int idx = c * G + t;
-    uint4 gv = make_uint4(0u, 0u, 0u, 0u), uv = gv;
+    gv[c] = uv[c] = make_uint4(0u, 0u, 0u, 0u);
     if (active && idx < nchunk) {
       const uint4* base = reinterpret_cast<const uint4*>(gate_up + static_cast<size_t>(row) * ld);
-      gv = base[idx];
-      uv = base[nchunk + idx];
+      gv[c] = base[idx];
+      uv[c] = base[nchunk + idx];
     }
-    const uint32_t gw[4] = {gv.x, gv.y, gv.z, gv.w}, uw[4] = {uv.x, uv.y, uv.z, uv.w};
+  }
+#pragma unroll
+  for (int c = 0; c < CHUNKS; ++c) {
+    const uint32_t gw[4] = {gv[c].x, gv[c].y, gv[c].z, gv[c].w}, uw[4] = {uv[c].x, uv[c].y, uv[c].z, uv[c].w};
     uint32_t out[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -138,28 +151,12 @@ silu_mul_quant_kernel(const T* gate_up, int64_t ld, T* y_out, int8_t* xq, float*
   quantise_row<T, G, CHUNKS>(y, active, row, t, g, nchunk, I, y_out, xq, a_scales, red);
 }
 
-// Picks the row-group width for a row of K elements and launches; false = row too long.
-#define B200Q_FUSED_DISPATCH(KERNEL, KLEN, ...)                                              \
-  do {                                                                                       \
-    auto blocks = [&](int g) { return (M + (256 / g) - 1) / (256 / g); };                     \
-    if ((KLEN) <= 32 * 8 * 4)                                                                \
-      e = launch_overlapped(KERNEL<T, 32, 4>, blocks(32), 256, 0, st, __VA_ARGS__);          \
-    else if ((KLEN) <= 64 * 8 * 4)                                                           \
-      e = launch_overlapped(KERNEL<T, 64, 4>, blocks(64), 256, 0, st, __VA_ARGS__);          \
-    else if ((KLEN) <= 128 * 8 * 4)                                                          \
-      e = launch_overlapped(KERNEL<T, 128, 4>, blocks(128), 256, 0, st, __VA_ARGS__);        \
-    else if ((KLEN) <= 256 * 8 * 4)                                                          \
-      e = launch_overlapped(KERNEL<T, 256, 4>, blocks(256), 256, 0, st, __VA_ARGS__);        \
-    else                                                                                     \
-      e = launch_overlapped(KERNEL<T, 256, 8>, blocks(256), 256, 0, st, __VA_ARGS__);        \
-  } while (0)
-
 template <typename T>
 cudaError_t launch_rmsnorm(const void* x, const void* res_in, const void* weight, float eps,
                            void* res_out, void* y, int8_t* xq, float* a_s, int M, int K,
                            cudaStream_t st) {
   cudaError_t e;
-  B200Q_FUSED_DISPATCH(add_rmsnorm_quant_kernel, K, static_cast<const T*>(x),
+  B200Q_ROWS_DISPATCH(add_rmsnorm_quant_kernel, K >> 3, static_cast<const T*>(x),
                        static_cast<const T*>(res_in), static_cast<const T*>(weight), eps,
                        static_cast<T*>(res_out), static_cast<T*>(y), xq, a_s, M, K);
   return e;
@@ -169,7 +166,7 @@ template <typename T>
 cudaError_t launch_silu(const void* gate_up, int64_t ld, void* y, int8_t* xq, float* a_s, int M,
                         int I, cudaStream_t st) {
   cudaError_t e;
-  B200Q_FUSED_DISPATCH(silu_mul_quant_kernel, I, static_cast<const T*>(gate_up), ld,
+  B200Q_ROWS_DISPATCH(silu_mul_quant_kernel, I >> 3, static_cast<const T*>(gate_up), ld,
                        static_cast<T*>(y), xq, a_s, M, I);
   return e;
 }

@@ -52,6 +52,24 @@ constexpr size_t kCounterBytes = 16384;  // zero-initialised tile counters at wo
 
 // Number of SMs of the current device (cached).
 int sm_count();
+
+// Row-wise kernels: threads per row (32 to 256) and 16-byte chunks per thread.  While all rows fit the GPU at
+// once, what counts is the chain of one thread: as few chunks as one wave of threads allows.  Beyond, four
+// chunks keep enough bytes in flight at a moderate register count.  (us, one chunk / this rule / always four:
+// quantiser, K = 1024, 512 tokens 2.2 / 2.2 / 2.9, 1999 3.1 / 3.2 / 4.5, 8192 7.9 / 6.8 / 6.8; RMSNorm, K = 2048,
+// 256 tokens 3.4 / 3.4 / 4.1, 8192 28.6 / 22.5 / 22.5.)
+struct RowShape {
+  int g, c;
+};
+inline RowShape row_shape(int M, int nchunk) {
+  const long long wave = static_cast<long long>(sm_count()) * 2048;
+  int c = 1;
+  while (c < 4 && static_cast<long long>(M) * nchunk > c * wave) ++c;
+  int g = 32;
+  while (g < 256 && g * c < nchunk) g *= 2;
+  return {g, (nchunk + g - 1) / g};
+}
+
 // Compute-capability major of the current device (0 on error) and the device address of
 // its status word (nullptr on error); both cached per device.
 int device_cc_major();

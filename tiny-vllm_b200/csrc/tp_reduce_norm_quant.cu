@@ -71,7 +71,7 @@ tp_reduce_norm_quant_kernel(const ExchangeParams p) {
   constexpr int kRowsPerBlock = 256 / G;
   __shared__ unsigned int s_epoch;
   __shared__ int s_flag;  // 0 ok, 1 = a wait gave up, 2 / 3 = this CTA is the rank's last (ok / failed)
-  __shared__ float red[8];
+  __shared__ float red[8 * CHUNKS];
   unsigned int* my_pad = p.pad[p.rank];
   if (threadIdx.x == 0) s_flag = 0;
   // launch and set-up overlap the tail of the producing kernel; its output is needed from here
@@ -124,13 +124,14 @@ tp_reduce_norm_quant_kernel(const ExchangeParams p) {
     }
 
     float s[CHUNKS][8];
-    float sumsq = 0.f;
+    float sumsq[CHUNKS];
 #pragma unroll
     for (int c = 0; c < CHUNKS; ++c) {
       const int idx = c * G + t;
       const bool live = active && idx < nchunk;
       const uint4 resv = resv_all[c];
       // the all-reduce: fp32 sum in rank order, one rounding to the 16-bit type
+      sumsq[c] = 0.f;
       float acc[8];
 #pragma unroll
       for (int k = 0; k < 8; ++k) acc[k] = 0.f;
@@ -148,15 +149,15 @@ tp_reduce_norm_quant_kernel(const ExchangeParams p) {
         const float s1 = p.residual_in != nullptr ? __fadd_rn(a.y, b.y) : a.y;
         s[c][2 * i] = s0;
         s[c][2 * i + 1] = s1;
-        sumsq = __fmaf_rn(s0, s0, sumsq);
-        sumsq = __fmaf_rn(s1, s1, sumsq);
+        sumsq[c] = __fmaf_rn(s0, s0, sumsq[c]);
+        sumsq[c] = __fmaf_rn(s1, s1, sumsq[c]);
         out[i] = pack2<T>(s0, s1);
       }
       if (live && p.residual_out != nullptr)
         *(reinterpret_cast<uint4*>(static_cast<T*>(p.residual_out) + static_cast<size_t>(local_row) * p.K) + idx) =
             make_uint4(out[0], out[1], out[2], out[3]);
     }
-    const float total = group_reduce<G, false>(sumsq, red, g);
+    const float total = row_sum<G, CHUNKS>(sumsq, red, g);
     const float inv_rms = __frsqrt_rn(__fadd_rn(__fdiv_rn(total, static_cast<float>(p.K)), p.eps));
 
     uint4 y[CHUNKS];
@@ -176,7 +177,7 @@ tp_reduce_norm_quant_kernel(const ExchangeParams p) {
       }
       y[c] = make_uint4(out[0], out[1], out[2], out[3]);
     }
-    const float amax = group_reduce<G, true>(running.value(), red, g);
+    const float amax = group_max<G>(running.value(), red, g);
     if (active) {
       const float scale = fmaxf(__fdiv_rn(amax, 127.0f), 1e-8f);
       const float inv_scale = __frcp_rn(scale);
