@@ -24,11 +24,14 @@
 // Every mbarrier wait is bounded; the two cluster-wide hardware barriers (after set-up,
 // before tear-down) are reached by every thread on every path.
 //
-// Output routes of the epilogue (eight warps, two per TMEM lane quarter):
+// The epilogue: sixteen warps, each 32 rows x 64 columns of a tile.  A warp takes its share of the accumulators
+// into registers at once and hands the TMEM buffer back before it converts anything, so the
+// MMAs of the tile after next never wait for stores (eight warps with two column groups each:
+// 4096 -> 4096 at 8192 tokens 90.0 us, now 88.6; 1024 -> 4096 33.0, now 31.9).  Its output routes:
 //   EPI_TMA     convert -> swizzled shared-memory slab -> one thread issues a TMA tensor store
 //               of the 32 x 64 box (this GPU's memory only); the epilogue warps never read the
-//               slab back and never issue a global store, and the stores drain while the next
-//               64 columns are converted (two slabs per warp).
+//               slab back and never issue a global store, and the stores drain while the warp waits for
+//               its next accumulators.
 //   EPI_LSU     convert -> slab -> the warp reads it back row-wise and stores full 128-byte
 //               lines with st.global (the only route that may write to a peer GPU: SCATTER).
 //   EPI_DIRECT  raw int32 accumulators only: each thread writes its 128-byte row pieces from
@@ -54,7 +57,7 @@ constexpr int kBlockBytes = 128;              // bytes of K per pipeline stage =
 constexpr int kUmmaBytes = 32;                // bytes of K per tcgen05.mma (32 int8 / 16 halves)
 constexpr int kPairBN = 256;                  // N of the pair's UMMA
 constexpr int kStageBytes = 2 * kTileRows * kBlockBytes;  // 32 KB per CTA
-constexpr int kEpiWarps = 8;
+constexpr int kEpiWarps = 16;
 constexpr int kEpiThreads = kEpiWarps * 32;
 constexpr int kThreads = 64 + kEpiThreads;    // + warp 0 (TMA) + warp 1 (UMMA)
 constexpr int kSlabBytes = 32 * 128;          // 32 rows x 64 columns x 2 bytes
@@ -68,8 +71,8 @@ enum { EPI_LSU = 0, EPI_TMA = 1, EPI_DIRECT = 2 };
 
 template <int EPI>
 struct Shape {
-  static constexpr int kSlabs = EPI == EPI_TMA ? 2 : (EPI == EPI_LSU ? 1 : 0);  // per warp
-  static constexpr int kStages = EPI == EPI_TMA ? 5 : (EPI == EPI_LSU ? 6 : 7);
+  static constexpr int kSlabs = EPI == EPI_DIRECT ? 0 : 1;  // per warp
+  static constexpr int kStages = EPI == EPI_DIRECT ? 7 : 5;
   static constexpr int kStagingBytes = kEpiWarps * kSlabs * kSlabBytes;
   static constexpr int kSmem = kStages * kStageBytes + kStagingBytes + kScaleBytes + kCtrlBytes;
   static_assert(kSmem <= 227 * 1024, "shared memory budget");
@@ -132,6 +135,13 @@ __device__ __forceinline__ void item_to_tile(int item, const PairParams& pp, con
     *tile_n = item % pp.tiles_n;
     *tile_m2 = row_tile_of<SCATTER>(item / pp.tiles_n, pp.tiles_m2, sp);
   }
+}
+
+// an ordinary load: the read-only path may move it above the wait for the kernel that writes the value
+__device__ __forceinline__ float ld_plain(const float* p) {
+  float v;
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+  return v;
 }
 
 template <typename T>
@@ -297,23 +307,27 @@ umma_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
   const int pair = blockIdx.x >> 1;
   const int num_pairs = gridDim.x >> 1;
   const int total_items = pp.tiles_m2 * pp.tiles_n;
-  // Weights do not depend on the previous kernel: ask L2 for this CTA's first weight rows while
-  // that kernel is still running (a prefetch is only a hint, so it is safe even if they did).
-  if (KIND != KIND_F16 && threadIdx.x == 0 && aligned && pair < total_items) {
-    const int first_n = pp.m_fastest ? pair / pp.tiles_m2 : pair % pp.tiles_n;
-    const int row_b = first_n * kPairBN + static_cast<int>(rank) * kTileRows;
-    const int n = pp.k_blocks < 8 ? pp.k_blocks : 8;
-    for (int kb = 0; kb < n; ++kb) ptx::tma_prefetch_l2_2d(&tmap_b, kb * kBlockBytes, row_b);
-  }
-  // everything above overlapped the previous kernel's tail; its results are needed from here
-  ptx::grid_dependency_wait();
-  ptx::grid_launch_dependents();
-
+  ptx::grid_launch_dependents();   // the successor waits for our results itself
   const bool run = aligned;  // a misaligned shared window (never seen) skips all work
 
   if (warp == 0) {
     if (lane == 0 && run) {
       // ------------------------------------------------------ TMA producer (both CTAs)
+      // W8A8: weights do not depend on the previous kernel, so the first ring-full of them is on its way
+      // before this kernel waits for it.
+      int ahead = 0;
+      if (KIND != KIND_F16 && pair < total_items) {
+        int tile_n, tile_m2;
+        item_to_tile<SCATTER>(pair, pp, sp, &tile_n, &tile_m2);
+        const int row_b = tile_n * kPairBN + static_cast<int>(rank) * kTileRows;
+        for (; ahead < kStages && ahead < pp.k_blocks; ++ahead) {
+          const uint32_t own_bar = ptx::smem_u32(full_bar + ahead);
+          if (rank == 0) ptx::mbar_arrive_expect_tx(own_bar, 2 * kStageBytes);
+          ptx::tma_load_2d_pair(smem_base + ahead * kStageBytes + kTileRows * kBlockBytes, &tmap_b,
+                                ptx::map_to_cta(own_bar, 0), ahead * kBlockBytes, row_b);
+        }
+      }
+      ptx::grid_dependency_wait();
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -331,10 +345,14 @@ umma_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
           const uint32_t leader_bar = ptx::map_to_cta(own_bar, 0);
           const uint32_t sa = smem_base + stage * kStageBytes;
           const uint32_t sb = sa + kTileRows * kBlockBytes;
-          // the leader expects the bytes of both CTAs on its barrier
-          if (rank == 0) ptx::mbar_arrive_expect_tx(own_bar, 2 * kStageBytes);
+          if (ahead > 0) {
+            --ahead;                     // its weights are on their way
+          } else {
+            // the leader expects the bytes of both CTAs on its barrier
+            if (rank == 0) ptx::mbar_arrive_expect_tx(own_bar, 2 * kStageBytes);
+            ptx::tma_load_2d_pair(sb, &tmap_b, leader_bar, kb * kBlockBytes, row_b);
+          }
           ptx::tma_load_2d_pair(sa, &tmap_a, leader_bar, kb * kBlockBytes, row_a);
-          ptx::tma_load_2d_pair(sb, &tmap_b, leader_bar, kb * kBlockBytes, row_b);
           if (++stage == kStages) {
             stage = 0;
             phase ^= 1u;
@@ -388,12 +406,13 @@ umma_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
     // ------------------------------------------------------------ epilogue (both CTAs)
     const int epi_warp = warp - 2;
     const int quarter = warp & 3;      // the TMEM lane quarter this warp may read
-    const int half = epi_warp >> 2;    // this warp's 64-column groups: half, half + 2
+    const int c0 = (epi_warp >> 2) * 64;   // this warp's 64 columns of the tile
     const int row_in_tile = quarter * 32 + lane;
     const int epi_tid = threadIdx.x - 64;
-    uint8_t* slabs = staging + epi_warp * (S::kSlabs * kSlabBytes);
+    uint8_t* slab = staging + epi_warp * (S::kSlabs * kSlabBytes);
     const uint32_t leader_tempty0 = ptx::map_to_cta(ptx::smem_u32(tempty_bar), 0);
     const OutT* bias = reinterpret_cast<const OutT*>(pp.bias);
+    ptx::grid_dependency_wait();       // a_scales come from the previous kernel, out may be in use by it
     int it = 0;
     for (int item = pair; item < total_items; item += num_pairs, ++it) {
       int tile_n, tile_m2;
@@ -402,12 +421,12 @@ umma_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
       const int buf = it & 1;
       const uint32_t tphase = static_cast<uint32_t>(it >> 1) & 1u;
       float* ws_tile = s_ws + buf * 256;
-      if (KIND != KIND_I8_RAW) {
+      if (KIND != KIND_I8_RAW && epi_tid < kPairBN) {
         const int col = tile_n * kPairBN + epi_tid;
         ws_tile[epi_tid] = col < pp.N ? __ldg(pp.w_scales + col) : 0.f;
       }
       const int row = tile_m * kTileRows + row_in_tile;
-      const float a_s = (KIND == KIND_I8 && row < pp.M) ? __ldg(pp.a_scales + row) : 0.f;
+      const float a_s = (KIND == KIND_I8 && row < pp.M) ? ld_plain(pp.a_scales + row) : 0.f;
       OutT* out = reinterpret_cast<OutT*>(pp.out);
       if (SCATTER) {
         // this tile's rows belong to one owner: redirect the output there
@@ -421,73 +440,51 @@ umma_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) +
                              static_cast<uint32_t>(buf * kPairBN);
       uint32_t va[32], vb[32];
-      ptx::tmem_ld_32x32b_x32(taddr + half * 64, va);
-      ptx::tmem_ld_32x32b_x32(taddr + half * 64 + 32, vb);
-#pragma unroll 1
-      for (int g = 0; g < 2; ++g) {
-        const int c0 = (half + 2 * g) * 64;
-        const int row0 = tile_m * kTileRows + quarter * 32;
-        const int col0 = tile_n * kPairBN + c0;
-        ptx::tmem_ld_wait();
-        if (KIND == KIND_I8_RAW) {
-          if (!(pp.debug_flags & 4)) {
-            store_row_i32(reinterpret_cast<int32_t*>(pp.out), pp.M, pp.N, row, col0, va);
-            store_row_i32(reinterpret_cast<int32_t*>(pp.out), pp.M, pp.N, row, col0 + 32, vb);
-          }
-          if (g == 0) {
-            ptx::tmem_ld_32x32b_x32(taddr + (half + 2) * 64, va);
-            ptx::tmem_ld_32x32b_x32(taddr + (half + 2) * 64 + 32, vb);
-          }
-          continue;
-        }
-        if (pp.debug_flags & 1) {
-          if (g == 0) {
-            ptx::tmem_ld_32x32b_x32(taddr + (half + 2) * 64, va);
-            ptx::tmem_ld_32x32b_x32(taddr + (half + 2) * 64 + 32, vb);
-          }
-          continue;
-        }
-        uint32_t pa[16], pb[16];
-        if (bias != nullptr) {
-          convert32<KIND, OutT, true>(ws_tile + c0, a_s, bias, col0, pp.N, va, pa);
-          convert32<KIND, OutT, true>(ws_tile + c0 + 32, a_s, bias, col0 + 32, pp.N, vb, pb);
-        } else {
-          convert32<KIND, OutT, false>(ws_tile + c0, a_s, bias, col0, pp.N, va, pa);
-          convert32<KIND, OutT, false>(ws_tile + c0 + 32, a_s, bias, col0 + 32, pp.N, vb, pb);
-        }
-        if (g == 0) {
-          ptx::tmem_ld_32x32b_x32(taddr + (half + 2) * 64, va);
-          ptx::tmem_ld_32x32b_x32(taddr + (half + 2) * 64 + 32, vb);
-        }
-        if (EPI == EPI_DIRECT) {
-          // raw accumulators only (handled above)
-        } else if (EPI == EPI_TMA) {
-          uint8_t* slab = slabs + g * kSlabBytes;
-          // the store issued from this slab one tile ago must have finished reading it;
-          // the one issued since (other slab) may still be running
-          if (lane == 0) ptx::bulk_wait_group_read<1>();
-          __syncwarp();
-          park32(slab, lane, 0, pa);
-          park32(slab, lane, 1, pb);
-          ptx::fence_proxy_async_smem();
-          __syncwarp();
-          if (lane == 0) {
-            if (!(pp.debug_flags & 4) && row0 < pp.M && col0 < pp.N)
-              ptx::tma_store_2d(&tmap_y, ptx::smem_u32(slab), col0 * 2, row0);
-            ptx::bulk_commit_group();  // always: the wait above counts groups
-          }
-        } else {
-          uint8_t* slab = slabs;
-          park32(slab, lane, 0, pa);
-          park32(slab, lane, 1, pb);
-          __syncwarp();
-          if (!(pp.debug_flags & 4)) store_slab_rows<OutT>(out, pp.M, pp.N, slab, lane, row0, col0);
-          __syncwarp();
-        }
-      }
-      // accumulator drained: tell the leader's UMMA issuer (local or remote arrive)
+      ptx::tmem_ld_32x32b_x32(taddr + c0, va);
+      ptx::tmem_ld_32x32b_x32(taddr + c0 + 32, vb);
+      ptx::tmem_ld_wait();
+      // the accumulators are in registers: tell the leader's UMMA issuer (local or remote arrive)
       ptx::tc_fence_before_sync();
       ptx::mbar_arrive_cluster(leader_tempty0 + static_cast<uint32_t>(buf) * 8u);
+      const int row0 = tile_m * kTileRows + quarter * 32;
+      const int col0 = tile_n * kPairBN + c0;
+      if (KIND == KIND_I8_RAW) {
+        if (!(pp.debug_flags & 4)) {
+          store_row_i32(reinterpret_cast<int32_t*>(pp.out), pp.M, pp.N, row, col0, va);
+          store_row_i32(reinterpret_cast<int32_t*>(pp.out), pp.M, pp.N, row, col0 + 32, vb);
+        }
+        continue;
+      }
+      if (pp.debug_flags & 1) continue;
+      uint32_t packed[16];
+      if (bias != nullptr)
+        convert32<KIND, OutT, true>(ws_tile + c0, a_s, bias, col0, pp.N, va, packed);
+      else
+        convert32<KIND, OutT, false>(ws_tile + c0, a_s, bias, col0, pp.N, va, packed);
+      if (EPI == EPI_TMA) {
+        // the store issued from the slab one tile ago must have finished reading it
+        if (lane == 0) ptx::bulk_wait_group_read<0>();
+        __syncwarp();
+      }
+      park32(slab, lane, 0, packed);
+      if (bias != nullptr)
+        convert32<KIND, OutT, true>(ws_tile + c0 + 32, a_s, bias, col0 + 32, pp.N, vb, packed);
+      else
+        convert32<KIND, OutT, false>(ws_tile + c0 + 32, a_s, bias, col0 + 32, pp.N, vb, packed);
+      park32(slab, lane, 1, packed);
+      if (EPI == EPI_TMA) {
+        ptx::fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+          if (!(pp.debug_flags & 4) && row0 < pp.M && col0 < pp.N)
+            ptx::tma_store_2d(&tmap_y, ptx::smem_u32(slab), col0 * 2, row0);
+          ptx::bulk_commit_group();
+        }
+      } else {
+        __syncwarp();
+        if (!(pp.debug_flags & 4)) store_slab_rows<OutT>(out, pp.M, pp.N, slab, lane, row0, col0);
+        __syncwarp();
+      }
     }
     // shared memory must stay valid until the last TMA store has read it, and the output
     // must be complete when the kernel ends
