@@ -395,30 +395,28 @@ bool mid_plan_for(int M, int N, int k_blocks, int bt, int rows, int splits, int 
 }
 
 // Predicted time of one call in a stream of such calls, in microseconds.  The form follows what the
-// kernel does (MMAs, expansion and HBM overlap, hence the root of cubes); the coefficients are
-// fitted to 8,400 measured configurations (17 shapes from 2 to 100 MB of weights, 24 to 3000 tokens): the
-// one with the smallest prediction is on average 3 %, at worst 20 %, slower than the best measured one.
-double mid_cost(const MidPlan& pl, int M, double matrix_bytes) {
-  const double clk = 1850.0;   // cycles per microsecond
+// kernel does; the coefficients are fitted to 3,700 measured configurations (17 shapes from 2 to 100 MB of weights, 16
+// to 1500 tokens) so that the one with the smallest prediction is close to the best: on average 1.5 %, at worst
+// 12 % slower than it (a model with the expansion and HBM as further pipes: 3.6 and 30 %).
+double mid_cost(const MidPlan& pl, int M) {
   const int ctas = pl.tiles_t * pl.tiles_c * pl.splits;
   const int per_sm = pl.smem <= kMidSmemTwo && pl.tmem_cols <= 256 ? 2 : 1;
   // clusters of 4 and 8 do not fill every SM (a cluster lives inside one group of SMs)
   const int sms = sm_count() - (pl.splits == 8 ? 28 : pl.splits == 4 ? 12 : 0);
-  const double passes = (ctas + sms - 1) / sms, waves = (ctas + sms * per_sm - 1) / (sms * per_sm);
-  const double kb = pl.chunks_per_split * pl.kc;
-  const double per_mma = pl.bt <= 32 ? 43 : pl.bt <= 64 ? 51 : pl.bt <= 128 ? 68 : 130 * pl.bt / 256.0;   // cycles
-  const double mma = 0.825 * kb * 4 * per_mma * passes, expand = 140.5 * kb * passes;
-  const double hbm = matrix_bytes / sm_count() / 20.4;
-  double us = 2.07 + std::cbrt(mma * mma * mma + expand * expand * expand + hbm * hbm * hbm) / clk;
+  const int passes = (ctas + sms - 1) / sms, waves = (ctas + sms * per_sm - 1) / (sms * per_sm);
+  // two CTAs on an SM wait on different things most of the time: the second costs 18 % of the first
+  const double work = per_sm == 1 ? passes : waves * (1 + 0.182 * ((passes + waves - 1) / waves - 1));
+  const double live = std::min(M, pl.bt);
+  double us = 0.804 + pl.chunks_per_split * pl.kc * 4 * (39.1 + 0.0706 * pl.bt) * work / 1850.0;   // MMAs, at 1850 MHz
   // a ring shorter than the K loop goes round at the latency of a load
-  us += 0.467 * waves * std::max(0, pl.chunks_per_split - pl.stages) / pl.stages;
-  us += 0.231 * waves * pl.chunks_per_split;
-  if (pl.splits > 1) us += 0.0153 * std::min(M, pl.bt) * passes;
+  us += 0.294 * waves * std::max(0, pl.chunks_per_split - pl.stages) / pl.stages;
+  us += 0.319 * waves * pl.chunks_per_split;
+  us += pl.splits > 1 ? 0.0165 * live * passes + 0.882 * std::log2(pl.splits) : 0.0144 * live * work;
   // start-up (1 us, and the first weights from HBM) hides under the previous kernel only as far as
   // both fit the GPU; alone on its SM a tile's start and end hide under nothing
   const double slots = static_cast<double>(sm_count()) * per_sm;
-  us += 2.42 * std::min(1.0, std::max(0.0, (2.0 * ctas - slots) / slots));
-  if (per_sm == 1) us += 5.12 * (waves - 1);
+  us += (per_sm == 1 ? 2.38 : 2.8) * std::min(1.0, std::max(0.0, (2.0 * ctas - slots) / slots));
+  if (per_sm == 1) us += 2.42 * (waves - 1);
   return us;
 }
 
@@ -445,7 +443,7 @@ bool search_plan(int M, int N, int K, MidPlan* best) {
             MidPlan pl;
             if (!mid_plan_for(M, N, k_blocks, bt, rows, s, kc, cap, &pl)) continue;
             if (s > 1 && pl.tiles_t * pl.tiles_c * s > 2 * sm_count()) continue;   // beyond what was measured
-            const double cost = mid_cost(pl, M, static_cast<double>(N) * K);
+            const double cost = mid_cost(pl, M);
             if (cost < best_cost) {
               best_cost = cost;
               *best = pl;
