@@ -324,33 +324,33 @@ bool mid_plan_for(int M, int N, int k_blocks, int bn, int splits, int kc,
 }
 
 // Predicted time of one call in a stream of such calls, in microseconds.  The form follows what the
-// kernel does (the three pipes overlap, hence the root of cubes); the coefficients are fitted to
-// 2,800 measured configurations (13 shapes from 2 to 100 MB of weights, 24 to 512 tokens): the configuration with the smallest prediction is on average 4 % slower than the
-// best measured one.
-double mid_cost(const MidPlan& pl, int M, double matrix_bytes) {
+// kernel does (MMAs, the issue loop's overhead per K block and the loads overlap, hence the root of cubes); the
+// coefficients are fitted to 2,000 measured configurations (18 shapes from 2 to 100 MB of weights, 24 to 2000 tokens) so that
+// the one with the smallest prediction is close to the best: on average 1.6 %, at worst 17 % slower than it (4.3
+// and 34 % for a model that counted two CTAs of an SM as twice the work).
+double mid_cost(const MidPlan& pl, int M) {
   const double clk = 1850.0;   // cycles per microsecond
   const int ctas = pl.tiles_m * pl.tiles_n * pl.splits;
   const int per_sm = pl.smem <= kMidSmemTwo ? 2 : 1;
   // clusters of 4 and 8 do not fill every SM (a cluster lives inside one group of SMs)
   const int sms = sm_count() - (pl.splits == 8 ? 28 : pl.splits == 4 ? 12 : 0);
-  const double passes = (ctas + sms - 1) / sms, waves = (ctas + sms * per_sm - 1) / (sms * per_sm);
+  const int passes = (ctas + sms - 1) / sms, waves = (ctas + sms * per_sm - 1) / (sms * per_sm);
+  // two CTAs on an SM share its load bandwidth, but wait on different things most of the time
+  const double work = per_sm == 1 ? passes : waves;
   const double kb = pl.chunks_per_split * pl.kc;
-  const double per_mma = pl.bn == 256 ? 130 : pl.bn == 128 ? 68 : pl.bn == 64 ? 51 : 43;   // cycles
-  const double mma = 0.68 * kb * 4 * per_mma * passes;
-  const double weights = kb * pl.bn * 128 / 134.0 * passes;
-  const double hbm = matrix_bytes / sm_count() / 26.6;
-  double us = 2.34 + std::cbrt(mma * mma * mma + weights * weights * weights + hbm * hbm * hbm) / clk;
+  const double mma = kb * 4 * 0.637 * pl.bn * work, issue = 211.0 * kb * work;
+  const double load = kb * 128 * (pl.x_rows + pl.bn) * passes / 296.0;
+  double us = 1.93 + std::cbrt(mma * mma * mma + issue * issue * issue + load * load * load) / clk;
   // a ring shorter than the K loop goes round at the latency of a load
-  us += 0.534 * waves * std::max(0, pl.chunks_per_split - pl.stages) / pl.stages;
-  us += 0.135 * waves * pl.chunks_per_split;
-  const double rows = std::min(M, kMidTok);
-  if (pl.splits > 1) us += 0.416 + 0.04 * rows * pl.bn * 4 * passes / clk;
-  us += 0.061 * rows * pl.bn * 2 * passes / clk;
+  us += 1.08 * waves * std::max(0, pl.chunks_per_split - pl.stages) / pl.stages;
+  us += 0.0757 * waves * pl.chunks_per_split;
+  const double values = std::min(M, kMidTok) * pl.bn / 64.0;
+  us += pl.splits > 1 ? 0.00746 * values * passes + 0.746 * std::log2(pl.splits) : 0.00185 * values * work;
   // start-up (1 us, and the first weights from HBM) hides under the previous kernel only as far as
   // both fit the GPU
   const double slots = static_cast<double>(sm_count()) * per_sm;
-  us += 1.345 * std::min(1.0, std::max(0.0, (2.0 * ctas - slots) / slots)) + 1.676 * (waves - 1);
-  return us;
+  us += 1.4 * std::min(1.0, std::max(0.0, (2.0 * ctas - slots) / slots));
+  return us + (per_sm == 1 ? 2.6 : 2.15) * (waves - 1);
 }
 
 bool search_plan(int M, int N, int K, MidPlan* best) {
@@ -365,7 +365,7 @@ bool search_plan(int M, int N, int K, MidPlan* best) {
         for (int cap : {kMidSmemOne, kMidSmemTwo}) {
           MidPlan pl;
           if (!mid_plan_for(M, N, k_blocks, bn, s, kc, cap, &pl)) continue;
-          const double cost = mid_cost(pl, M, static_cast<double>(N) * K);
+          const double cost = mid_cost(pl, M);
           if (cost < best_cost) {
             best_cost = cost;
             *best = pl;
