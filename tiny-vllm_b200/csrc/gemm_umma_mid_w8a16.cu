@@ -413,9 +413,11 @@ double mid_cost(const MidPlan& pl, int M) {
   us += 0.319 * waves * pl.chunks_per_split;
   us += pl.splits > 1 ? 0.0165 * live * passes + 0.882 * std::log2(pl.splits) : 0.0144 * live * work;
   // start-up (1 us, and the first weights from HBM) hides under the previous kernel only as far as
-  // both fit the GPU; alone on its SM a tile's start and end hide under nothing
+  // both fit the GPU; alone on its SM a tile's start and end hide under nothing.  The neighbours in a layer
+  // have other shapes: they are taken to hold 128 SMs at least (64 tokens through one eighth of the 8B model 21.5 us a
+  // layer; planned for neighbours like itself 25.0)
   const double slots = static_cast<double>(sm_count()) * per_sm;
-  us += (per_sm == 1 ? 2.38 : 2.8) * std::min(1.0, std::max(0.0, (2.0 * ctas - slots) / slots));
+  us += (per_sm == 1 ? 2.38 : 2.8) * std::min(1.0, std::max(0.0, (ctas + std::max<double>(ctas, 128.0 * per_sm) - slots) / slots));
   if (per_sm == 1) us += 2.42 * (waves - 1);
   return us;
 }
