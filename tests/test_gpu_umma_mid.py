@@ -55,3 +55,17 @@ def test_w8a16_more_than_one_wave_and_every_token_tile(M, N, K, bn):
     m = O.tensor_metrics(O.w8a16_native_reference(x, q, s, None), y)
     assert m["relative_l2"] <= 4e-3 and m["cosine_similarity"] >= 0.9999, m
     assert device_status_ok()
+
+
+@pytest.mark.parametrize("M,N,K,path", [(200, 24584, 528, "umma_i8_pair_tokens256"), (300, 24584, 528, "umma_i8_tokens128"),
+                                        (450, 12288, 2064, "umma_i8_pair_tokens256"), (129, 9728, 2048, "umma_i8_pair_tokens256"),
+                                        (450, 6144, 1024, "umma_i8_tokens128")])
+def test_w8a8_beyond_one_wave_takes_the_pair_kernel_where_rounding_tokens_up_costs_no_wave(M, N, K, path, oracle_c_lib):
+    assert select_path(_lib.OP_W8A8, M, N, K) == path
+    q, s = O.make_weight(N, K, seed=N + K)
+    xq, a_s = O.quantize_per_row_dynamic(O.make_activation(M, K, seed=M, dtype=torch.bfloat16))
+    ref = O.w8a8_int32_accumulators(xq, q)
+    y = apply_w8a8_linear(xq.cuda(), a_s.cuda(), q.cuda(), s.cuda(), None, out_dtype=torch.bfloat16)
+    assert torch.equal(bits(y.cpu()), bits(O.w8a8_native_epilogue(ref, a_s, s, None, torch.bfloat16)))
+    assert torch.equal(w8a8_int32_accumulators(xq.cuda(), q.cuda()).cpu(), ref)
+    assert device_status_ok()

@@ -600,9 +600,20 @@ int finish(cudaError_t e, int launches = 1) {
 // 10.8 us the other way).
 bool umma_pair_applicable(int M, int N, int K, bool raw_int32_out) {
   if (debug_knob(B200Q_KNOB_NO_PAIR, 0) != 0) return false;
-  if ((K % 16) != 0 || M < 512) return false;
+  if ((K % 16) != 0 || M <= 128) return false;
   if (!raw_int32_out && (N % 8) != 0) return false;
   const int pairs = sm_count() / 2;
+  if (M < 512) {
+    // More 128 x 128 tiles than the kernel for tens to hundreds of tokens takes: the rival is the persistent single-CTA
+    // kernel, whose 128 x 256 tiles cost an SM what a pair's 256 x 256 tile costs its two.  The pair kernel wins where
+    // rounding M up to 256 takes it no more waves (24576 x 4096 at 200 tokens 30.8 against 34.9 us, at 300 38.9 against
+    // 35.1, at 450 41.0 against 46.5; 12288 x 2048 at 450 17.0 against 20.4), on few short tiles it does
+    // not (6144 x 1024 at 450 8.6 against 8.3).
+    const long long cols = (N + kPairBN - 1) / kPairBN, rows = (M + 127) / 128, rows2 = (M + 255) / 256;
+    if (rows * ((N + 127) / 128) <= sm_count() || (K < 2048 && rows2 * cols < 64)) return false;
+    if (debug_knob(B200Q_KNOB_PAIR_MIN_TILES, 0) > rows2 * cols) return false;
+    return (rows2 * cols + pairs - 1) / pairs <= (rows * cols + sm_count() - 1) / sm_count();
+  }
   return enough_pair_tiles(M, N, K >= 4096 ? (pairs * 2) / 3 : pairs);
 }
 
