@@ -596,7 +596,7 @@ int finish(cudaError_t e, int launches = 1) {
 // the Qwen3-0.6B / 8B projections and their tensor-parallel shards at 512-8192 tokens: with one
 // tile per CTA pair or more the pair kernel wins (1024 -> 6144 at 1024 tokens, 96 tiles: 11.6
 // against 13.1 us); with fewer it wins only where the K loop is long (12288 -> 4096 at 1024
-// tokens, 64 tiles: 37.0 against 40.4 us; 2048 -> 1024 at 4096 tokens, 64 tiles: 11.4 against
+// tokens, 64 tiles: 37.0 against 40.4 us; 4096 -> 4096 at 700, 48 tiles: 16.2 against 17.7; 2048 -> 1024 at 4096 tokens, 64 tiles: 11.4 against
 // 10.8 us the other way).
 bool umma_pair_applicable(int M, int N, int K, bool raw_int32_out) {
   if (debug_knob(B200Q_KNOB_NO_PAIR, 0) != 0) return false;
@@ -614,7 +614,7 @@ bool umma_pair_applicable(int M, int N, int K, bool raw_int32_out) {
     if (debug_knob(B200Q_KNOB_PAIR_MIN_TILES, 0) > rows2 * cols) return false;
     return (rows2 * cols + pairs - 1) / pairs <= (rows * cols + sm_count() - 1) / sm_count();
   }
-  return enough_pair_tiles(M, N, K >= 4096 ? (pairs * 2) / 3 : pairs);
+  return enough_pair_tiles(M, N, K >= 4096 ? (pairs * 3) / 5 : pairs);
 }
 
 // Scatter variant for row-parallel layers: partial tiles go to the owners' staging areas.
