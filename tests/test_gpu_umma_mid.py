@@ -69,3 +69,14 @@ def test_w8a8_beyond_one_wave_takes_the_pair_kernel_where_rounding_tokens_up_cos
     assert torch.equal(bits(y.cpu()), bits(O.w8a8_native_epilogue(ref, a_s, s, None, torch.bfloat16)))
     assert torch.equal(w8a8_int32_accumulators(xq.cuda(), q.cuda()).cpu(), ref)
     assert device_status_ok()
+
+
+@pytest.mark.parametrize("M,N,K", [(257, 24584, 1040), (385, 16384, 1024)])
+def test_w8a16_beyond_the_mid_sizes_takes_the_tensor_memory_kernel(M, N, K):
+    assert select_path(_lib.OP_W8A16, M, N, K) == "umma_f16_tmem_weights_channels256"
+    q, s = O.make_weight(N, K, seed=N + K)
+    x = O.make_activation(M, K, seed=M, dtype=torch.bfloat16)
+    y = apply_int8_weight_only_linear(x.cuda(), q.cuda(), s.cuda())
+    m = O.tensor_metrics(O.w8a16_native_reference(x, q, s, None), y)
+    assert m["relative_l2"] <= 4e-3 and m["cosine_similarity"] >= 0.9999, m
+    assert device_status_ok()

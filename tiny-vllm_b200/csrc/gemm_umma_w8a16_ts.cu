@@ -328,14 +328,15 @@ cudaError_t launch_ts(const CUtensorMap& tx, const CUtensorMap& tw, const TsPara
 // the epilogue of a tile is not overlapped here (all of tensor memory is in use), so very short
 // K loops stay on the shared-memory kernel.  M = 8192, this kernel vs that one: 1024 -> 4096
 // 84.3 vs 87.1 us, 2048 -> 1024 44.8 vs 49.9 us, 1024 -> 6144 128.4 vs 131.5 us, 3072 -> 1024
-// 61.6 vs 71.3 us.
+// 61.6 vs 71.3 us.  From 257 tokens on (below, gemm_umma_mid_w8a16.cu takes all that has fewer tiles): 4096 -> 24576 at 300
+// tokens 76.5 vs 89.9 us, 4096 -> 22016 at 400 111 vs 171, 1024 -> 16384 at 450 26.4 vs 29.5.
 bool umma16_ts_applicable(int M, int N, int K) {
   if (debug_knob(B200Q_KNOB_NO_TS, 0) != 0) return false;
   if (K < debug_knob(B200Q_KNOB_TS_MIN_K, 1024)) return false;
   if ((K % 16) != 0 || (N % 8) != 0) return false;   // 16-byte output pieces
   const long long tiles = static_cast<long long>((N + kTsChannels - 1) / kTsChannels) *
                           ((M + kTsTokens - 1) / kTsTokens);
-  return M >= 512 && tiles >= sm_count();
+  return M > 256 && tiles >= sm_count();
 }
 
 int launch_w8a16_umma_ts(const GemmArgs& a) {
