@@ -247,6 +247,13 @@ void b200q_debug_reset(void);
  */
 int b200q_check_status(int* status_word);
 
+/*
+ * Test hook: how the single-CTA tcgen05 kernels for tens to hundreds of tokens would cut this problem.  Returns 1 and
+ * fills plan[6] = {tokens per tile, channels per tile, CTAs per cluster (each with its share of K), tensor-memory
+ * columns and dynamic shared-memory bytes per CTA, CTAs in all}, or returns 0 when another kernel takes it.
+ */
+int b200q_debug_mid_plan(int op, int M, int N, int K, int* plan);
+
 /* Test hook: number of kernels this library has launched in this process. */
 uint64_t b200q_launch_count(void);
 

@@ -582,6 +582,18 @@ int b200q_debug_set(int knob, int value) {
 
 void b200q_debug_reset(void) { t_knobs = Knobs{}; }
 
+int b200q_debug_mid_plan(int op, int M, int N, int K, int* plan) {
+  if (plan == nullptr || (op != B200Q_OP_W8A8 && op != B200Q_OP_W8A16) || check_dims(M, N, K) != B200Q_OK) return 0;
+  if (resolve_path(op, M, N, K) != B200Q_PATH_UMMA) return 0;
+  MidShape s;
+  if (op == B200Q_OP_W8A8 ? umma_pair_applicable(M, N, K, false) || !umma_mid_shape(M, N, K, &s)
+                          : !umma16_mid_shape(M, N, K, &s))
+    return 0;
+  const int v[6] = {s.tokens, s.channels, s.cluster, s.tmem_cols, s.smem_bytes, s.ctas};
+  for (int i = 0; i < 6; ++i) plan[i] = v[i];
+  return 1;
+}
+
 uint64_t b200q_launch_count(void) { return g_launches.load(); }
 
 }  // extern "C"

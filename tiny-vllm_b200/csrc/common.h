@@ -157,6 +157,13 @@ bool umma_mid_applicable(int M, int N, int K);
 int launch_umma_mid(const GemmArgs& a);
 bool umma16_mid_applicable(int M, int N, int K);
 int launch_umma16_mid(const GemmArgs& a);
+// How these kernels would cut a problem (tests); false where they cannot.
+struct MidShape {
+  int tokens, channels;   // of a tile
+  int cluster, tmem_cols, smem_bytes, ctas;
+};
+bool umma_mid_shape(int M, int N, int K, MidShape* s);
+bool umma16_mid_shape(int M, int N, int K, MidShape* s);
 
 // gemm_umma_w8a16.cu
 bool umma16_make_plan(int M, int N, int K, int swap, UmmaPlan* plan);

@@ -21,7 +21,8 @@
 //
 // Warp roles (352 threads): warp 0 TMA of the activations, warp 1 UMMA, warps 2-9 epilogue,
 // warp 10 TMA of the weights.
-// Every mbarrier wait is bounded; the cluster barrier is reached by every thread on every path.
+// Every mbarrier wait is bounded; the cluster barrier is reached by every thread on every path, and no CTA of a
+// cluster waits for tensor memory (the residency rule of umma_mid_common.cuh).
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -391,6 +392,13 @@ bool umma_mid_applicable(int M, int N, int K) {
   if (debug_knob(B200Q_KNOB_BN, 0) == 0 && debug_knob(B200Q_KNOB_CLUSTER, 0) == 0) return true;
   MidPlan pl;   // a forced tile or cluster may not fit
   return mid_plan<MidPlan, search_plan>(M, N, K, &pl);
+}
+
+bool umma_mid_shape(int M, int N, int K, MidShape* s) {
+  MidPlan pl;
+  if (!umma_mid_applicable(M, N, K) || !mid_plan<MidPlan, search_plan>(M, N, K, &pl)) return false;
+  *s = MidShape{kMidTok, pl.bn, pl.splits, pl.bn, static_cast<int>(pl.smem), pl.tiles_m * pl.tiles_n * pl.splits};
+  return true;
 }
 
 int launch_umma_mid(const GemmArgs& a) {

@@ -21,7 +21,8 @@
 // Warp roles (352 threads): warp 0 TMA of the activations, warp 1 UMMA, warps 2-9 expansion (two groups of
 // four that take the chunks in turn: a warp reaches one TMEM lane quarter), then epilogue, warp 10
 // TMA of the weights.
-// Every mbarrier wait is bounded; the cluster barrier is reached by every thread on every path.
+// Every mbarrier wait is bounded; the cluster barrier is reached by every thread on every path, and no CTA of a
+// cluster waits for tensor memory (the residency rule of umma_mid_common.cuh).
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -391,6 +392,8 @@ bool mid_plan_for(int M, int N, int k_blocks, int bt, int rows, int splits, int 
   pl->tmem_cols = 32;
   while (pl->tmem_cols < cols) pl->tmem_cols *= 2;
   pl->smem = static_cast<size_t>(stages) * ring_bytes + fixed;
+  // no other CTA of a cluster fits beside it (see the residency rule in umma_mid_common.cuh)
+  if (splits > 1 && pl->tmem_cols > 256) pl->smem = kMidSmemOne;
   return true;
 }
 
@@ -474,6 +477,13 @@ bool umma16_mid_applicable(int M, int N, int K) {
   if (debug_knob(B200Q_KNOB_BN, 0) == 0 && debug_knob(B200Q_KNOB_CLUSTER, 0) == 0) return true;
   MidPlan pl;   // a forced tile or cluster may not fit
   return mid_plan<MidPlan, search_plan>(M, N, K, &pl);
+}
+
+bool umma16_mid_shape(int M, int N, int K, MidShape* s) {
+  MidPlan pl;
+  if (!umma16_mid_applicable(M, N, K) || !mid_plan<MidPlan, search_plan>(M, N, K, &pl)) return false;
+  *s = MidShape{pl.bt, pl.rows, pl.splits, pl.tmem_cols, static_cast<int>(pl.smem), pl.tiles_t * pl.tiles_c * pl.splits};
+  return true;
 }
 
 int launch_umma16_mid(const GemmArgs& a) {

@@ -9,6 +9,16 @@
 
 namespace b200q {
 
+// Residency rule.  tcgen05.alloc waits, without a limit, until the SM has that many free columns, and a CTA of a
+// cluster keeps its columns until every CTA of the cluster has arrived at the cluster barrier.  Two CTAs of one cluster
+// on one SM, or two clusters that each hold the columns the other one waits for, would therefore never end.  So the
+// CTAs of clusters that can share an SM must not need more than its 512 columns together:
+//   * at most two CTAs of these kernels fit an SM: more would exceed its registers (launch_mid_kernel checks it);
+//   * a CTA of a cluster has at most 256 columns, or it takes the shared memory of a whole SM (kMidSmemOne: beside it there
+//     is room for no kernel with dynamic shared memory).
+// A CTA without a cluster may wait for columns: who holds them ends without it.  The other kernels that allocate
+// tensor memory for clusters are alone on their SM: umma_pair_kernel by its shared memory, the clustered
+// w8a8_umma_kernel by its registers.
 constexpr int kMidThreads = 352;
 constexpr int kMidMaxStages = 12;
 constexpr int kMidCtrlBytes = 768;
@@ -107,6 +117,10 @@ cudaError_t launch_mid_kernel(int ctas, int splits, size_t smem, cudaStream_t st
   if (dev >= 64 || !attr_set[dev]) {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMidSmemOne);
     if (e != cudaSuccess) return e;
+    int per_sm = 0;   // by registers and threads alone: the residency rule
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kMidThreads, 0);
+    if (e != cudaSuccess) return e;
+    if (per_sm > 2) return cudaErrorInvalidConfiguration;
     if (dev < 64) attr_set[dev] = true;
   }
   return launch_clustered(splits, true, kernel, dim3(ctas), dim3(kMidThreads), smem, stream, tx, tw, tx3, tw3, mp);
