@@ -140,15 +140,17 @@ __device__ __forceinline__ void exchange_and_sum(const OutT* part, const FusePar
 }
 
 // ------------------------------------------------------------------------- W8A8
+// Activations and their scales are read with ordinary loads through pointers without __restrict__: a
+// non-coherent load (__ldg, const __restrict__) of what the previous kernel writes may be moved ahead of
+// grid_dependency_wait() and see the old values.
 // MT = number of 16-token tiles.  Lane (g = lane / 4, t = lane % 4): weight row g of the
 // CTA's 8 channels, bytes [16 t, 16 t + 16) of each 64-byte K block; the same byte range
 // of token rows g and g + 8 of every token tile.
 template <typename OutT, int MT, bool RAW_I32, bool FUSED>
 __global__ void __launch_bounds__(kThreads)
-w8a8_mma_decode_kernel(const int8_t* __restrict__ xq, const int8_t* __restrict__ w,
-                       const float* __restrict__ a_s, const float* __restrict__ w_s,
-                       const OutT* __restrict__ bias, void* __restrict__ out, int M, int N, int K,
-                       const FuseParams fp, int* status) {
+w8a8_mma_decode_kernel(const int8_t* xq, const int8_t* __restrict__ w, const float* a_s,
+                       const float* __restrict__ w_s, const OutT* __restrict__ bias, void* out, int M,
+                       int N, int K, const FuseParams fp, int* status) {
   __shared__ int red[kWarps][MT * 16 * kChannels];
   __shared__ __align__(16) OutT part[FUSED ? MT * 16 * kChannels : 8];
   ptx::grid_dependency_wait();
@@ -183,14 +185,10 @@ w8a8_mma_decode_kernel(const int8_t* __restrict__ xq, const int8_t* __restrict__
 #pragma unroll
       for (int m = 0; m < MT; ++m) {
         const int r0 = m * 16 + g, r1 = r0 + 8;
-        const uint4 x0 = (k_ok && r0 < M)
-                             ? __ldg(reinterpret_cast<const uint4*>(
-                                   xq + static_cast<size_t>(r0) * K + blk * kBlock + 16 * t))
-                             : zero;
-        const uint4 x1 = (k_ok && r1 < M)
-                             ? __ldg(reinterpret_cast<const uint4*>(
-                                   xq + static_cast<size_t>(r1) * K + blk * kBlock + 16 * t))
-                             : zero;
+        const int8_t* p0 = xq + static_cast<size_t>(r0) * K + blk * kBlock + 16 * t;
+        const int8_t* p1 = xq + static_cast<size_t>(r1) * K + blk * kBlock + 16 * t;
+        const uint4 x0 = (k_ok && r0 < M) ? *reinterpret_cast<const uint4*>(p0) : zero;
+        const uint4 x1 = (k_ok && r1 < M) ? *reinterpret_cast<const uint4*>(p1) : zero;
         // bytes 0-7 feed the first k32 step (slots 0/1), bytes 8-15 the second
         mma_s8(acc[m], x0.x, x1.x, x0.y, x1.y, wv.x, wv.y);
         mma_s8(acc[m], x0.z, x1.z, x0.w, x1.w, wv.z, wv.w);
@@ -236,9 +234,9 @@ w8a8_mma_decode_kernel(const int8_t* __restrict__ xq, const int8_t* __restrict__
 // k [16 t + 4 j, 16 t + 4 j + 4) to step j (4 weights = one word, 4 activations = 8 bytes).
 template <typename T, int MT, bool FUSED>
 __global__ void __launch_bounds__(kThreads)
-w8a16_mma_decode_kernel(const T* __restrict__ x, const int8_t* __restrict__ w,
-                        const float* __restrict__ s, const T* __restrict__ bias,
-                        T* __restrict__ y, int M, int N, int K, const FuseParams fp, int* status) {
+w8a16_mma_decode_kernel(const T* x, const int8_t* __restrict__ w, const float* __restrict__ s,
+                        const T* __restrict__ bias, T* y, int M, int N, int K, const FuseParams fp,
+                        int* status) {
   __shared__ float red[kWarps][MT * 16 * kChannels];
   __shared__ __align__(16) T part[FUSED ? MT * 16 * kChannels : 8];
   ptx::grid_dependency_wait();
@@ -280,8 +278,8 @@ w8a16_mma_decode_kernel(const T* __restrict__ x, const int8_t* __restrict__ w,
         const uint4* p1 = reinterpret_cast<const uint4*>(x + static_cast<size_t>(r1) * K +
                                                          blk * kBlock + 16 * t);
         const bool v0 = k_ok && r0 < M, v1 = k_ok && r1 < M;
-        const uint4 x0a = v0 ? __ldg(p0) : zero, x0b = v0 ? __ldg(p0 + 1) : zero;
-        const uint4 x1a = v1 ? __ldg(p1) : zero, x1b = v1 ? __ldg(p1 + 1) : zero;
+        const uint4 x0a = v0 ? p0[0] : zero, x0b = v0 ? p0[1] : zero;
+        const uint4 x1a = v1 ? p1[0] : zero, x1b = v1 ? p1[1] : zero;
         mma_16<T>(acc[m], x0a.x, x1a.x, x0a.y, x1a.y, e0.x, e0.y);
         mma_16<T>(acc[m], x0a.z, x1a.z, x0a.w, x1a.w, e1.x, e1.y);
         mma_16<T>(acc[m], x0b.x, x1b.x, x0b.y, x1b.y, e2.x, e2.y);

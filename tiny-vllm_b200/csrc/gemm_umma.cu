@@ -225,7 +225,7 @@ w8a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_a,
         const int col = tile_b * p.bn + epi_tid;
         if (epi_tid < p.bn) ws_tile[epi_tid] = col < p.rows_b ? __ldg(p.w_scales + col) : 0.f;
         const int row = tile_a * kTileA + row_in_tile;
-        if (row < p.rows_a) a_s = __ldg(p.a_scales + row);
+        if (row < p.rows_a) a_s = p.a_scales[row];   // (not __ldg: the previous kernel writes it)
         ptx::named_bar_sync(2, kEpiThreads);
       }
       if (!ptx::mbar_wait(ptx::smem_u32(tfull_bar + buf), tphase, abort_flag)) break;

@@ -107,7 +107,7 @@ __device__ __forceinline__ void emit_chunk(const KernelParams& p, int tile_a, in
           if (col_b0 + j < p.rows_b) dst[j] = static_cast<int32_t>(v[j]);
       }
     } else {
-      const float a_s = __ldg(p.a_scales + row_a);
+      const float a_s = p.a_scales[row_a];   // (not __ldg: the previous kernel writes it)
       const OutT* bias = reinterpret_cast<const OutT*>(p.bias);
       OutT* dst = reinterpret_cast<OutT*>(p.out) + off;
       if (full && (N & 7) == 0) {
@@ -160,7 +160,7 @@ __device__ __forceinline__ void emit_chunk(const KernelParams& p, int tile_a, in
       for (int j = 0; j < 32; ++j) {
         const int tok = col_b0 + j;
         if (tok < p.rows_b) {
-          const float a_s = __ldg(p.a_scales + tok);
+          const float a_s = p.a_scales[tok];
           dst[static_cast<size_t>(tok) * N + row_a] =
               from_float<OutT>(scale_acc(static_cast<int>(v[j]), a_s, w_s, b));
         }
