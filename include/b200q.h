@@ -16,6 +16,13 @@
  *   - No call synchronises the device and no call falls back to another
  *     implementation: a non-zero return code means nothing was launched.
  *   - Matrices are row-major and dense: x[M,K], qweight[N,K], y[M,N].
+ *   - Weights are constants.  A call may read qweight, the channel scales, the bias and a norm's
+ *     weight BEFORE the work ahead of it in the stream has ended.  It does see what copies, ordinary kernels of
+ *     the caller and b200q_act_quant_i8 wrote to them in stream order.  Do not pass it there what
+ *     another entry point of this library (y, codes or scales of the fused producers and of the exchange) or a kernel
+ *     of the caller that lets its successors start early (griddepcontrol.launch_dependents) has written, unless
+ *     an ordinary kernel, a copy or a synchronisation lies between.  Activations, residuals and outputs
+ *     follow stream order without such a rule.
  *   - K must be a multiple of 16 (the row pitch of an int8 [rows,K] matrix must
  *     be 16-byte aligned for TMA); all base pointers must be 16-byte aligned.
  *   - Return value: B200Q_OK (0) or one of the B200Q_ERR_* codes below;

@@ -47,3 +47,17 @@ def test_the_rule_covers_the_kernels():
     names = {p.name for p in sources()}
     assert {"gemm_mma_decode.cu", "gemm_umma.cu", "w8a8_device.cuh", "gemm_umma_pair.cu", "gemm_umma_mid.cu",
             "gemm_umma_mid_w8a16.cu", "gemm_reg_decode.cu", "gemm_bulk_decode.cu", "act_quant.cu"} <= names
+
+
+def test_the_stand_alone_quantiser_holds_its_successors_back():
+    # its rows may be weights, which the GEMM kernels read ahead of their wait; only inside
+    # b200q_w8a8_dynamic_gemm is it known that they are not
+    quantiser = code(CSRC / "act_quant.cu")
+    triggers = re.findall(r"[^;{}]*grid_launch_dependents\(\)", quantiser)
+    assert triggers and all(re.search(r"if \(early\)", t) for t in triggers), triggers
+    api = code(CSRC / "api.cu")
+    body = {name: re.search(rf"\bint {name}\([^)]*\) \{{(.*?)\n\}}", api, re.S).group(1)
+            for name in ("b200q_act_quant_i8", "b200q_w8a8_dynamic_gemm")}
+    early = {name: argument(text, text.index("run_act_quant(") + len("run_act_quant")).split(",")[-2].strip()
+             for name, text in body.items()}
+    assert early == {"b200q_act_quant_i8": "false", "b200q_w8a8_dynamic_gemm": "true"}

@@ -26,11 +26,14 @@ namespace {
 
 // G threads per row (32, 64, 128 or 256), CHUNKS 16-byte chunks per thread held in registers.
 // Requires K <= G * 8 * CHUNKS.
+// early: the successor may start at once.  Only where it is known to take the codes as activations: the GEMM
+// kernels read their weights before they wait for their predecessor, and rows quantised here may well be somebody's
+// weights (with the quantiser of the tokens launched in between, or without).
 template <typename T, int G, int CHUNKS>
 __global__ void __launch_bounds__(256)
-act_quant_rows_kernel(const T* x, int64_t ldx, int8_t* xq, float* a_scales, int M, int K) {
+act_quant_rows_kernel(const T* x, int64_t ldx, int8_t* xq, float* a_scales, int M, int K, bool early) {
   constexpr int kRowsPerBlock = 256 / G;
-  ptx::grid_launch_dependents();   // the successor's weights do not depend on this kernel
+  if (early) ptx::grid_launch_dependents();
   ptx::grid_dependency_wait();     // x may be the previous kernel's output (neither __ldg nor __restrict__,
                                    // which makes a non-coherent load of it too: such a load may move ahead)
   const int g = threadIdx.x / G;  // row group inside the block
@@ -83,8 +86,8 @@ act_quant_rows_kernel(const T* x, int64_t ldx, int8_t* xq, float* a_scales, int 
 // Any K: one 256-thread CTA per row, the row is read twice (the second read hits L2).
 template <typename T>
 __global__ void __launch_bounds__(256)
-act_quant_long_rows_kernel(const T* x, int64_t ldx, int8_t* xq, float* a_scales, int M, int K) {
-  ptx::grid_launch_dependents();
+act_quant_long_rows_kernel(const T* x, int64_t ldx, int8_t* xq, float* a_scales, int M, int K, bool early) {
+  if (early) ptx::grid_launch_dependents();
   ptx::grid_dependency_wait();
   const int row = blockIdx.x;
   __shared__ float red[8];
@@ -114,23 +117,24 @@ act_quant_long_rows_kernel(const T* x, int64_t ldx, int8_t* xq, float* a_scales,
 
 template <typename T>
 cudaError_t launch_typed(const T* x, int64_t ldx, int8_t* xq, float* a_scales, int M, int K,
-                         cudaStream_t st) {
+                         bool early, cudaStream_t st) {
   cudaError_t e;
   if (K > 256 * 8 * 8)
-    return launch_overlapped(act_quant_long_rows_kernel<T>, M, 256, 0, st, x, ldx, xq, a_scales, M, K);
-  B200Q_ROWS_DISPATCH(act_quant_rows_kernel, K >> 3, x, ldx, xq, a_scales, M, K);
+    return launch_overlapped(act_quant_long_rows_kernel<T>, M, 256, 0, st, x, ldx, xq, a_scales, M, K,
+                             early);
+  B200Q_ROWS_DISPATCH(act_quant_rows_kernel, K >> 3, x, ldx, xq, a_scales, M, K, early);
   return e;
 }
 
 }  // namespace
 
 cudaError_t launch_act_quant(const void* x, int64_t ldx, int x_dtype, int8_t* xq, float* a_scales,
-                             int M, int K, cudaStream_t stream) {
+                             int M, int K, bool early, cudaStream_t stream) {
   cudaError_t e;
   if (x_dtype == B200Q_DTYPE_BF16) {
-    e = launch_typed(reinterpret_cast<const __nv_bfloat16*>(x), ldx, xq, a_scales, M, K, stream);
+    e = launch_typed(reinterpret_cast<const __nv_bfloat16*>(x), ldx, xq, a_scales, M, K, early, stream);
   } else {
-    e = launch_typed(reinterpret_cast<const __half*>(x), ldx, xq, a_scales, M, K, stream);
+    e = launch_typed(reinterpret_cast<const __half*>(x), ldx, xq, a_scales, M, K, early, stream);
   }
   if (e == cudaSuccess) count_launch();
   return e;

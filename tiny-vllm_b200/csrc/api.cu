@@ -135,6 +135,27 @@ bool dynamic_is_fused(int M, int N, int K) {
          !bulk_decode_applicable(M, N, K, false) && reg_decode_dynamic_applicable(M, N, K);
 }
 
+// b200q_act_quant_i8 with the choice of `early` (common.h)
+int run_act_quant(const void* x, int64_t ldx, int x_dtype, int8_t* xq, float* a_scales, int M, int K,
+                  bool early, void* stream) {
+  if (x == nullptr || xq == nullptr || a_scales == nullptr) return B200Q_ERR_NULL_POINTER;
+  if (M <= 0 || K <= 0 || static_cast<long long>(M) * K > INT_MAX) return B200Q_ERR_BAD_SHAPE;
+  if (x_dtype != B200Q_DTYPE_F16 && x_dtype != B200Q_DTYPE_BF16) return B200Q_ERR_BAD_ARGUMENT;
+  if ((K % 16) != 0 || ldx < K || (ldx % 8) != 0) return B200Q_ERR_UNSUPPORTED_SHAPE;
+  if (!aligned16(x) || !aligned16(xq) || (reinterpret_cast<uintptr_t>(a_scales) & 3u) != 0)
+    return B200Q_ERR_MISALIGNED;
+  DeviceInfo* d = device_info();
+  if (d == nullptr) return B200Q_ERR_LAUNCH;
+  if (d->cc_major != 10) return B200Q_ERR_UNSUPPORTED_ARCH;
+  cudaError_t e =
+      launch_act_quant(x, ldx, x_dtype, xq, a_scales, M, K, early, static_cast<cudaStream_t>(stream));
+  if (e != cudaSuccess) {
+    note_cuda_error(e);
+    return B200Q_ERR_LAUNCH;
+  }
+  return B200Q_OK;
+}
+
 size_t dynamic_code_offset(int M) { return (static_cast<size_t>(M) * 4 + 255) / 256 * 256; }
 
 }  // namespace
@@ -172,22 +193,7 @@ extern "C" {
 
 int b200q_act_quant_i8(const void* x, int64_t ldx, int x_dtype, int8_t* xq, float* a_scales, int M,
                        int K, void* stream) {
-  if (x == nullptr || xq == nullptr || a_scales == nullptr) return B200Q_ERR_NULL_POINTER;
-  if (M <= 0 || K <= 0 || static_cast<long long>(M) * K > INT_MAX) return B200Q_ERR_BAD_SHAPE;
-  if (x_dtype != B200Q_DTYPE_F16 && x_dtype != B200Q_DTYPE_BF16) return B200Q_ERR_BAD_ARGUMENT;
-  if ((K % 16) != 0 || ldx < K || (ldx % 8) != 0) return B200Q_ERR_UNSUPPORTED_SHAPE;
-  if (!aligned16(x) || !aligned16(xq) || (reinterpret_cast<uintptr_t>(a_scales) & 3u) != 0)
-    return B200Q_ERR_MISALIGNED;
-  DeviceInfo* d = device_info();
-  if (d == nullptr) return B200Q_ERR_LAUNCH;
-  if (d->cc_major != 10) return B200Q_ERR_UNSUPPORTED_ARCH;
-  cudaError_t e =
-      launch_act_quant(x, ldx, x_dtype, xq, a_scales, M, K, static_cast<cudaStream_t>(stream));
-  if (e != cudaSuccess) {
-    note_cuda_error(e);
-    return B200Q_ERR_LAUNCH;
-  }
-  return B200Q_OK;
+  return run_act_quant(x, ldx, x_dtype, xq, a_scales, M, K, false, stream);
 }
 
 int b200q_w8a8_gemm(const int8_t* xq, const float* a_scales, const int8_t* qweight,
@@ -433,7 +439,7 @@ int b200q_w8a8_dynamic_gemm(const void* x, const int8_t* qweight, const float* w
       return B200Q_ERR_WORKSPACE;
     float* a_s = static_cast<float*>(scratch);
     int8_t* xq = static_cast<int8_t*>(scratch) + dynamic_code_offset(M);
-    if (int rc = b200q_act_quant_i8(x, K, x_dtype, xq, a_s, M, K, stream)) return rc;
+    if (int rc = run_act_quant(x, K, x_dtype, xq, a_s, M, K, true, stream)) return rc;
     return b200q_w8a8_gemm(xq, a_s, qweight, w_scales, bias, y, M, N, K, x_dtype, workspace,
                            workspace_bytes, stream);
   }

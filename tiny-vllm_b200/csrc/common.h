@@ -75,9 +75,9 @@ inline RowShape row_shape(int M, int nchunk) {
 int device_cc_major();
 int* device_status_ptr();
 
-// act_quant.cu
+// act_quant.cu; early: the next kernel takes the codes as activations and may start at once
 cudaError_t launch_act_quant(const void* x, int64_t ldx, int x_dtype, int8_t* xq, float* a_scales,
-                             int M, int K, cudaStream_t stream);
+                             int M, int K, bool early, cudaStream_t stream);
 
 // gemm_simt.cu
 cudaError_t launch_w8a8_simt(const GemmArgs& a);
@@ -174,9 +174,13 @@ bool umma16_ts_applicable(int M, int N, int K);
 int launch_w8a16_umma_ts(const GemmArgs& a);
 
 // Launches `kernel` so that it may overlap its start-up (barrier set-up, TMEM allocation,
-// descriptor prefetch, launch latency) with the tail of the previous kernel in the stream
-// (programmatic dependent launch).  Only for kernels that call ptx::grid_dependency_wait()
-// before their first access to global memory.  B200Q_KNOB_NO_PDL turns the overlap off.
+// descriptor prefetch, launch latency, first weights) with the tail of the previous kernel in the
+// stream (programmatic dependent launch).  Only for kernels that call ptx::grid_dependency_wait()
+// before their first access to what that kernel, or one before it, may read or write.  Weights, their scales
+// and the bias count as constants (b200q.h states the caller's side): they may be read before the
+// wait.  A predecessor that does not call ptx::grid_launch_dependents() has then ended, and with it all
+// that was ahead of it; so a kernel whose output may become somebody's weights must not call it
+// (act_quant.cu).  B200Q_KNOB_NO_PDL turns the overlap off.
 bool pdl_enabled();
 template <typename... KArgs, typename... Args>
 cudaError_t launch_clustered(int cluster, bool overlap, void (*kernel)(KArgs...), dim3 grid,

@@ -426,10 +426,11 @@ __device__ __forceinline__ void named_bar_sync(uint32_t id, uint32_t nthreads) {
 }
 
 // ---- programmatic dependent launch.  A kernel launched with the programmatic-serialization
-// attribute may start while its predecessor in the stream is still running; it must not
-// touch memory the predecessor reads or writes before grid_dependency_wait(), which
-// returns once the predecessor grid has completed and its writes are visible.  Both are
-// no-ops for a kernel launched without the attribute.
+// attribute may start while its predecessor in the stream is still running (once all its CTAs have
+// called grid_launch_dependents() or ended); it must not touch memory the predecessor reads or writes
+// before grid_dependency_wait(), which returns once the predecessor grid has completed and its
+// writes are visible.  Weights are read before it (launch_clustered in common.h has the rule).  Both
+// are no-ops for a kernel launched without the attribute.
 __device__ __forceinline__ void grid_dependency_wait() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
