@@ -165,8 +165,9 @@ int b200q_w8a8_dynamic_gemm(const void* x, const int8_t* qweight, const float* w
 size_t b200q_w8a8_dynamic_scratch_bytes(int M, int N, int K);
 
 /*
- * Scratch bytes the given op needs for the given problem (0 when none).  The
- * first use of a workspace must find it zero-filled; every successful call
+ * Scratch bytes that are enough for the given op and problem (0 when none).  An upper bound: a
+ * W8A8 problem that a kernel without scratch takes runs with less, down to NULL; a call that does need
+ * more than it is given returns B200Q_ERR_WORKSPACE and launches nothing.  The first use of a workspace must find it zero-filled; every successful call
  * leaves it zero-filled where that matters, so one zeroed buffer of the maximum
  * size can be shared by all calls that are ordered on one stream.
  */

@@ -143,3 +143,26 @@ def test_python_entry_points_refuse_cpu_tensors():
         quantize_activation_int8(x)
     with pytest.raises(RuntimeError):
         apply_w8a8_linear(q[:4], torch.ones(4), q, s, out_dtype=torch.bfloat16)
+
+
+def test_dynamic_linear_refuses_before_the_quantiser_is_launched(L):
+    # (without a GPU a launch would answer ERR_LAUNCH: the refusal has to come first)
+    buf = ctypes.create_string_buffer(4096 + 64)
+    p = (ctypes.addressof(buf) + 63) & ~63  # never dereferenced
+    big = 1 << 30
+
+    def call(x=p, w=p, s=p, bias=None, y=p, M=300, N=4096, K=1024, scratch=p, nbytes=big, ws=None, ws_bytes=0):
+        return L.b200q_w8a8_dynamic_gemm(x, w, s, bias, y, M, N, K, _lib.DTYPE_BF16, scratch, nbytes, ws, ws_bytes, None)
+
+    assert call(w=p + 8) == _lib.ERR_MISALIGNED
+    assert call(s=p + 4) == _lib.ERR_MISALIGNED
+    assert call(y=p + 2) == _lib.ERR_MISALIGNED
+    assert call(bias=p + 1) == _lib.ERR_MISALIGNED
+    assert call(scratch=None) == _lib.ERR_WORKSPACE
+    prev = L.b200q_debug_force_path(_lib.PATH_UMMA_SWAP)      # K split through the workspace
+    try:
+        need = L.b200q_workspace_bytes(_lib.OP_W8A8, 48, 256, 8192)
+        assert call(M=48, N=256, K=8192) == _lib.ERR_WORKSPACE
+        assert call(M=48, N=256, K=8192, ws=p, ws_bytes=need - 1) == _lib.ERR_WORKSPACE
+    finally:
+        L.b200q_debug_force_path(prev)

@@ -129,6 +129,15 @@ int run_w8a8(GemmArgs& a) {
   return B200Q_ERR_BAD_ARGUMENT;
 }
 
+// Workspace that run_w8a8 insists on: only the persistent single-CTA kernel with its K split through memory.
+size_t w8a8_workspace_needed(int M, int N, int K) {
+  const int path = resolve_path(B200Q_OP_W8A8, M, N, K);
+  if (path != B200Q_PATH_UMMA && path != B200Q_PATH_UMMA_SWAP) return 0;
+  if (path == B200Q_PATH_UMMA && (umma_pair_applicable(M, N, K, false) || umma_mid_applicable(M, N, K))) return 0;
+  UmmaPlan plan;
+  return umma_make_plan(B200Q_OP_W8A8, M, N, K, path == B200Q_PATH_UMMA_SWAP, &plan) ? plan.ws_bytes : 0;
+}
+
 // One kernel for quantisation and GEMM, where each CTA can afford to read all tokens' rows.
 bool dynamic_is_fused(int M, int N, int K) {
   return resolve_path(B200Q_OP_W8A8, M, N, K) == B200Q_PATH_MMA_STREAM &&
@@ -433,19 +442,22 @@ int b200q_w8a8_dynamic_gemm(const void* x, const int8_t* qweight, const float* w
     return B200Q_ERR_NULL_POINTER;
   if (int rc = check_dims(M, N, K)) return rc;
   if (x_dtype != B200Q_DTYPE_F16 && x_dtype != B200Q_DTYPE_BF16) return B200Q_ERR_BAD_ARGUMENT;
+  if (!aligned16(x) || !aligned16(qweight) || !aligned16(y) || !aligned16(w_scales) || !aligned16(scratch) ||
+      !aligned16(workspace) || (bias != nullptr && (reinterpret_cast<uintptr_t>(bias) & 1u) != 0))
+    return B200Q_ERR_MISALIGNED;
   if (!dynamic_is_fused(M, N, K)) {
-    // scales first, codes behind them
-    if (scratch == nullptr || scratch_bytes < b200q_w8a8_dynamic_scratch_bytes(M, N, K))
+    // what could refuse the GEMM refuses the call before the quantiser is launched
+    if (scratch == nullptr || scratch_bytes < dynamic_code_offset(M) + static_cast<size_t>(M) * K)
       return B200Q_ERR_WORKSPACE;
+    const size_t need = w8a8_workspace_needed(M, N, K);
+    if (need > 0 && (workspace == nullptr || workspace_bytes < need)) return B200Q_ERR_WORKSPACE;
+    // scales first, codes behind them
     float* a_s = static_cast<float*>(scratch);
     int8_t* xq = static_cast<int8_t*>(scratch) + dynamic_code_offset(M);
     if (int rc = run_act_quant(x, K, x_dtype, xq, a_s, M, K, true, stream)) return rc;
     return b200q_w8a8_gemm(xq, a_s, qweight, w_scales, bias, y, M, N, K, x_dtype, workspace,
                            workspace_bytes, stream);
   }
-  if (!aligned16(x) || !aligned16(qweight) || !aligned16(y) || !aligned16(w_scales) ||
-      (bias != nullptr && (reinterpret_cast<uintptr_t>(bias) & 1u) != 0))
-    return B200Q_ERR_MISALIGNED;
   DeviceInfo* d = device_info();
   if (d == nullptr) return B200Q_ERR_LAUNCH;
   if (d->cc_major != 10) return B200Q_ERR_UNSUPPORTED_ARCH;

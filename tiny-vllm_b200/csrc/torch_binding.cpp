@@ -101,6 +101,12 @@ std::mutex g_ws_mutex;
 at::Tensor* const g_ws = new at::Tensor[kMaxDevices];  // never destroyed: CUDA may be gone at exit
 int64_t g_ws_floor = 64ll << 20;
 
+// The buffer as it is; undefined before the first call that needed one.
+at::Tensor current_workspace(const at::Device& device) {
+  std::lock_guard<std::mutex> lock(g_ws_mutex);
+  return g_ws[device.index()];
+}
+
 // A reference to the buffer of at least `bytes` bytes; throws std::runtime_error during capture.
 at::Tensor workspace(const at::Device& device, int64_t bytes) {
   std::lock_guard<std::mutex> lock(g_ws_mutex);
@@ -133,6 +139,22 @@ inline int unlocked(F&& call) {
   return rc;
 }
 
+// call(workspace, bytes) -> return code.  Most calls need no workspace: it is allocated only for one that asks for
+// it (and then has launched nothing), so that a capture is refused only for such a call.
+template <typename F>
+inline int with_workspace(const at::Device& device, int op, int m, int n, int k, F&& call) {
+  at::Tensor ws = current_workspace(device);
+  auto once = [&] {
+    return unlocked([&] { return call(ws.defined() ? ws.data_ptr() : nullptr, ws.defined() ? ws.numel() : 0); });
+  };
+  int rc = once();
+  if (rc == B200Q_ERR_WORKSPACE) {
+    ws = workspace(device, static_cast<int64_t>(b200q_workspace_bytes(op, m, n, k)));
+    rc = once();
+  }
+  return rc;
+}
+
 // ------------------------------------------------------------------------- functions
 // w8a16(x, qweight, scales, bias | None) -> y
 PyObject* w8a16(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
@@ -150,13 +172,9 @@ PyObject* w8a16(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   c10::cuda::CUDAGuard guard(device);
   const int m = static_cast<int>(M), n = static_cast<int>(p.N), k = static_cast<int>(p.K);
   at::Tensor y = empty_on(out_shape(*x, p.N), x->scalar_type(), device);
-  at::Tensor ws;
-  const size_t need = b200q_workspace_bytes(B200Q_OP_W8A16, m, n, k);
-  if (need > 0) ws = workspace(device, static_cast<int64_t>(need));
-  const int rc = unlocked([&] {
+  const int rc = with_workspace(device, B200Q_OP_W8A16, m, n, k, [&](void* ws, size_t bytes) {
     return b200q_w8a16_gemm(x->data_ptr(), static_cast<const int8_t*>(ptr(p.w)),
-                            static_cast<const float*>(ptr(p.s)), ptr(p.b), y.data_ptr(), m, n, k, dt,
-                            need > 0 ? ws.data_ptr() : nullptr, need > 0 ? ws.numel() : 0,
+                            static_cast<const float*>(ptr(p.s)), ptr(p.b), y.data_ptr(), m, n, k, dt, ws, bytes,
                             stream_of(device));
   });
   if (rc != B200Q_OK) return fail(rc, "b200q_w8a16_gemm", M, p.N, p.K);
@@ -182,18 +200,14 @@ PyObject* w8a8_dynamic(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   const int m = static_cast<int>(M);
   at::Tensor y = empty_on(out_shape(*x, p.N), x->scalar_type(), device);
   const int n = static_cast<int>(p.N), k = static_cast<int>(p.K);
-  at::Tensor quant, ws;
+  at::Tensor quant;
   const size_t scratch = b200q_w8a8_dynamic_scratch_bytes(m, n, k);
-  if (scratch > 0) {
-    quant = empty_on({static_cast<int64_t>(scratch)}, at::kByte, device);
-    const size_t need = b200q_workspace_bytes(B200Q_OP_W8A8, m, n, k);
-    if (need > 0) ws = workspace(device, static_cast<int64_t>(need));
-  }
-  const int rc = unlocked([&] {
+  if (scratch > 0) quant = empty_on({static_cast<int64_t>(scratch)}, at::kByte, device);
+  const int rc = with_workspace(device, B200Q_OP_W8A8, m, n, k, [&](void* ws, size_t bytes) {
     return b200q_w8a8_dynamic_gemm(
         x->data_ptr(), static_cast<const int8_t*>(ptr(p.w)), static_cast<const float*>(ptr(p.s)),
-        ptr(p.b), y.data_ptr(), m, n, k, dt, scratch > 0 ? quant.data_ptr() : nullptr, scratch,
-        ws.defined() ? ws.data_ptr() : nullptr, ws.defined() ? ws.numel() : 0, stream_of(device));
+        ptr(p.b), y.data_ptr(), m, n, k, dt, scratch > 0 ? quant.data_ptr() : nullptr, scratch, ws, bytes,
+        stream_of(device));
   });
   if (rc != B200Q_OK) return fail(rc, "b200q_w8a8_dynamic_gemm", M, p.N, p.K);
   return THPVariable_Wrap(std::move(y));
@@ -203,14 +217,9 @@ PyObject* w8a8_dynamic(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
 int run_w8a8(const at::Device& device, const int8_t* xq, const float* a_s, const Weights& p, void* y,
              int m, int out_dt) {
   const int n = static_cast<int>(p.N), k = static_cast<int>(p.K);
-  at::Tensor ws;
-  const size_t need = b200q_workspace_bytes(B200Q_OP_W8A8, m, n, k);
-  if (need > 0) ws = workspace(device, static_cast<int64_t>(need));
-  return unlocked([&] {
-    return b200q_w8a8_gemm(xq, a_s, static_cast<const int8_t*>(ptr(p.w)),
-                           static_cast<const float*>(ptr(p.s)), ptr(p.b), y, m, n, k, out_dt,
-                           need > 0 ? ws.data_ptr() : nullptr, need > 0 ? ws.numel() : 0,
-                           stream_of(device));
+  return with_workspace(device, B200Q_OP_W8A8, m, n, k, [&](void* ws, size_t bytes) {
+    return b200q_w8a8_gemm(xq, a_s, static_cast<const int8_t*>(ptr(p.w)), static_cast<const float*>(ptr(p.s)),
+                           ptr(p.b), y, m, n, k, out_dt, ws, bytes, stream_of(device));
   });
 }
 
@@ -285,15 +294,10 @@ PyObject* w8a8_i32(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   const int m = static_cast<int>(xq->size(0)), n = static_cast<int>(w->size(0)),
             k = static_cast<int>(w->size(1));
   at::Tensor acc = empty_on({m, n}, at::kInt, device);
-  at::Tensor ws;
-  const size_t need = b200q_workspace_bytes(B200Q_OP_W8A8, m, n, k);
-  if (need > 0) ws = workspace(device, static_cast<int64_t>(need));
-  const int rc = unlocked([&] {
+  const int rc = with_workspace(device, B200Q_OP_W8A8, m, n, k, [&](void* ws, size_t bytes) {
     return b200q_w8a8_gemm_i32(static_cast<const int8_t*>(xq->data_ptr()),
                                static_cast<const int8_t*>(w->data_ptr()),
-                               static_cast<int32_t*>(acc.data_ptr()), m, n, k,
-                               need > 0 ? ws.data_ptr() : nullptr, need > 0 ? ws.numel() : 0,
-                               stream_of(device));
+                               static_cast<int32_t*>(acc.data_ptr()), m, n, k, ws, bytes, stream_of(device));
   });
   if (rc != B200Q_OK) return fail(rc, "b200q_w8a8_gemm_i32", m, n, k);
   return THPVariable_Wrap(std::move(acc));
