@@ -1,5 +1,5 @@
 """The scratch buffer behind the Python entry points: allocated by the first call that needs one, so a capture is refused
-for such a call and for no other.  Each case is a process of its own: the buffer lives as long as the process."""
+for such a call and for no other, and kept for the graphs that were captured with it.  Each case is a process of its own: the buffer lives as long as the process."""
 import subprocess
 import sys
 from pathlib import Path
@@ -57,7 +57,22 @@ assert torch.equal(y, fn())
 """
 
 
-@pytest.mark.parametrize("body", [NEEDS_NONE, NEEDS_SOME], ids=["needs-none", "needs-some"])
+OUTGROWN = """
+x, q, s = problem(3000, 2048, 2048)
+fn = lambda: apply_int8_weight_only_linear(x, q, s)
+expect = fn()
+graph, y = captured(fn)                    # holds the address of the buffer of that moment
+x2, q2, s2 = problem(3000, 8192, 8192)     # 128 MiB of expanded weights: more than the buffer has
+apply_int8_weight_only_linear(x2, q2, s2)
+others = [torch.full((4 << 20,), 7, dtype=torch.uint8, device="cuda") for _ in range(64)]   # from freed blocks first
+graph.replay()
+torch.cuda.synchronize()
+assert all(bool((t == 7).all()) for t in others), "the graph wrote into another tensor"
+assert torch.equal(y, expect)
+"""
+
+
+@pytest.mark.parametrize("body", [NEEDS_NONE, NEEDS_SOME, OUTGROWN], ids=["needs-none", "needs-some", "outgrown"])
 def test_capture_in_a_fresh_process(body):
     r = subprocess.run([sys.executable, "-c", HEAD + body], cwd=ROOT, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout + r.stderr

@@ -27,6 +27,7 @@
 #include <mutex>
 #include <stdexcept>
 #include <string>
+#include <vector>
 
 #include "../../include/b200q.h"
 
@@ -99,6 +100,9 @@ PyObject* fail(int rc, const char* where, int64_t M, int64_t N, int64_t K) {
 constexpr int kMaxDevices = 64;
 std::mutex g_ws_mutex;
 at::Tensor* const g_ws = new at::Tensor[kMaxDevices];  // never destroyed: CUDA may be gone at exit
+// Outgrown buffers: a captured graph may go on writing to the one that it was captured with.  A buffer grows
+// by half at least, so what is kept here is at most twice the current one.
+std::vector<at::Tensor>* const g_ws_outgrown = new std::vector<at::Tensor>;
 int64_t g_ws_floor = 64ll << 20;
 
 // The buffer as it is; undefined before the first call that needed one.
@@ -119,7 +123,11 @@ at::Tensor workspace(const at::Device& device, int64_t bytes) {
           "reserve_workspace() before capture");
     // a buffer of this process must be an ordinary tensor whatever mode the first caller is in
     c10::InferenceMode normal(false);
-    ws = at::zeros({std::max(bytes, g_ws_floor)}, at::TensorOptions().dtype(at::kByte).device(device));
+    const int64_t least = ws.defined() ? ws.numel() / 2 * 3 : 0;
+    at::Tensor larger =
+        at::zeros({std::max({bytes, g_ws_floor, least})}, at::TensorOptions().dtype(at::kByte).device(device));
+    if (ws.defined()) g_ws_outgrown->push_back(ws);
+    ws = std::move(larger);
   }
   return ws;
 }
