@@ -42,8 +42,14 @@ def reserve_workspace(nbytes: int, device: torch.device | None = None) -> None:
     _native().reserve(int(nbytes), index)
 
 
-def _not_taken(what: str):
-    return RuntimeError(f"{what} does not support the provided tensors (all of them must be on one GPU)")
+def _refuse(what: str, entry: str, dims: dict[str, int], *tensors: torch.Tensor | None) -> None:
+    """Raises for dense tensors of the right types that the native function did not take: they are on
+    different GPUs, or have a shape that the C entry point refuses."""
+    if len({t.device for t in tensors if t is not None}) > 1:
+        raise RuntimeError(f"{what} does not support the provided tensors (all of them must be on one GPU)")
+    too_large = any(d >= 1 << 31 for d in dims.values())
+    _lib.check(_lib.ERR_BAD_SHAPE if too_large else _lib.ERR_UNSUPPORTED_SHAPE, entry,
+               " ".join(f"{name}={d}" for name, d in dims.items()))
 
 
 def _require_cuda(*tensors: torch.Tensor) -> None:
@@ -83,7 +89,7 @@ def quantize_activation_int8(x_2d: torch.Tensor) -> tuple[torch.Tensor, torch.Te
                 torch.empty((0,), dtype=torch.float32, device=x_2d.device))
     out = _native().quantize(_dense(x_2d))
     if out is None:
-        raise _not_taken("activation quantisation")
+        _refuse("activation quantisation", "b200q_act_quant_i8", {"M": M, "K": K}, x_2d)
     return out
 
 
@@ -113,7 +119,9 @@ def add_rmsnorm_quantize_int8(x: torch.Tensor, weight: torch.Tensor, eps: float,
     out = _native().rmsnorm_quant(_dense(x), _dense(weight), eps,
                                   None if residual is None else _dense(residual), return_normed)
     if out is None:
-        raise _not_taken("add_rmsnorm_quantize_int8")
+        K = x.shape[-1]
+        _refuse("add_rmsnorm_quantize_int8", "b200q_add_rmsnorm_quant_i8", {"M": x.numel() // K, "K": K},
+                x, weight, residual)
     return out
 
 
@@ -140,7 +148,9 @@ def silu_mul_quantize_int8(gate_up: torch.Tensor, return_act: bool = False):
         _lib.check(_lib.ERR_BAD_SHAPE, "b200q_silu_mul_quant_i8", f"M=0 I={gate_up.shape[-1] // 2}")
     out = _native().silu_mul_quant(_dense(gate_up), return_act)
     if out is None:
-        raise _not_taken("silu_mul_quantize_int8")
+        two_i = gate_up.shape[-1]
+        _refuse("silu_mul_quantize_int8", "b200q_silu_mul_quant_i8",
+                {"M": gate_up.numel() // two_i, "I": two_i // 2}, gate_up)
     return out
 
 
@@ -178,7 +188,9 @@ def apply_int8_weight_only_linear(
     _check_w8a16(x, qweight, scales, bias)
     y = _native().w8a16(_dense(x), _dense(qweight), _dense(scales), None if bias is None else _dense(bias))
     if y is None:
-        raise _not_taken("CUDA INT8 weight-only backend")
+        N, K = qweight.shape
+        _refuse("CUDA INT8 weight-only backend", "b200q_w8a16_gemm", {"M": x.numel() // K, "N": N, "K": K},
+                x, qweight, scales, bias)
     return y
 
 
@@ -241,7 +253,8 @@ def apply_w8a8_linear(
     y = _native().w8a8(_dense(x_q), _dense(a_scales), _dense(qweight), _dense(w_scales),
                        None if bias is None else _dense(bias), dtype_id, None, out)
     if y is None:
-        raise _not_taken("CUDA W8A8 backend")
+        _refuse("CUDA W8A8 backend", "b200q_w8a8_gemm", {"M": M, "N": N, "K": x_q.shape[1]},
+                x_q, a_scales, qweight, w_scales, bias)
     return y if out_shape is None else y.view(out_shape)
 
 
@@ -257,5 +270,6 @@ def w8a8_int32_accumulators(x_q: torch.Tensor, qweight: torch.Tensor) -> torch.T
         raise RuntimeError("x_q and qweight shapes do not align")
     acc = _native().w8a8_i32(_dense(x_q), _dense(qweight))
     if acc is None:
-        raise _not_taken("w8a8_int32_accumulators")
+        (M, K), N = x_q.shape, qweight.shape[0]
+        _refuse("w8a8_int32_accumulators", "b200q_w8a8_gemm_i32", {"M": M, "N": N, "K": K}, x_q, qweight)
     return acc
