@@ -175,7 +175,8 @@ size_t b200q_workspace_bytes(int op, int M, int N, int K);
 
 /*
  * Name of the kernel family the library would run for this problem, e.g.
- * "umma_i8_128xN" — the counterpart of `select_path(...)` in
+ * "umma_i8_tokens128" (one name for the two single-CTA tcgen05 kernels of a scheme:
+ * b200q_debug_mid_plan() tells them apart) — the counterpart of `select_path(...)` in
  * nanovllm/quantization/csrc/w8a8_gemm.cpp:51-54 and
  * int8_weight_only_gemm.cpp:40-43.  Never NULL.
  */

@@ -1,5 +1,6 @@
 """Helpers of the GPU parity tests."""
 import contextlib
+import ctypes
 
 import torch
 
@@ -36,6 +37,15 @@ def knobs(**settings):
     finally:
         L.b200q_debug_reset()
         L.b200q_debug_force_path(path)
+
+
+def mid_plan(op, M, N, K):
+    """How the tcgen05 kernel for tens to hundreds of tokens would cut a problem, or None where
+    another kernel takes it (host code, needs no GPU)."""
+    out = (ctypes.c_int * 6)()
+    if not _lib.lib().b200q_debug_mid_plan(op, M, N, K, out):
+        return None
+    return dict(zip(("tokens", "channels", "cluster", "columns", "shared", "ctas"), out))
 
 
 def device_status_ok():

@@ -166,3 +166,18 @@ def test_dynamic_linear_refuses_before_the_quantiser_is_launched(L):
         assert call(M=48, N=256, K=8192, ws=p, ws_bytes=need - 1) == _lib.ERR_WORKSPACE
     finally:
         L.b200q_debug_force_path(prev)
+
+
+def test_quantiser_path_names_follow_the_row_split(L):
+    # 16-byte chunks of a row over the threads that hold them: a warp where its 32 x 4 suffice at the row count
+    name = lambda M, K: L.b200q_select_path(_lib.OP_ACT_QUANT, M, 4, K).decode()
+    assert name(1, 256) == "act_quant_warp_per_row"             # 32 chunks
+    assert name(1, 512) == "act_quant_multiwarp_row"            # 64 chunks, one each while one wave holds all rows
+    assert name(1999, 1024) == "act_quant_multiwarp_row"
+    assert name(8192, 1024) == "act_quant_warp_per_row"         # 128 chunks, four each
+    assert name(8192, 1040) == "act_quant_multiwarp_row"
+    assert name(16, 16384) == "act_quant_multiwarp_row"
+    assert name(16, 16400) == "act_quant_long_row"
+    assert name(16, 1000) == "unsupported_shape"
+    # W8A8 and W8A16 single-CTA kernels: one family name each
+    assert L.b200q_select_path(_lib.OP_W8A16, 64, 4096, 1024) == b"umma_f16_expand_tokens128"

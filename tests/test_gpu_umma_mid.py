@@ -4,7 +4,7 @@ import pytest
 import torch
 
 from oracle import quant_linear_oracle as O
-from tests.gpu_util import bits, device_status_ok, forced_path, knobs
+from tests.gpu_util import bits, device_status_ok, forced_path, knobs, mid_plan
 import tiny_vllm_b200  # noqa: F401
 from tiny_vllm_b200 import _lib
 from tiny_vllm_b200.quantization.cuda import (apply_int8_weight_only_linear, apply_w8a8_linear,
@@ -16,6 +16,12 @@ SHAPES = [  # (M, N, K): one row of a tile, ragged everything, several token til
     (1, 8, 1024), (17, 72, 1040), (33, 264, 1616), (77, 4096, 1024), (128, 768, 4096),
     (129, 1000, 528), (300, 1024, 3072), (512, 264, 2112), (40, 136, 96), (1500, 640, 1184), (20, 128, 16),
 ]
+
+
+def splits_over(K, block, cluster):
+    """Every CTA of a cluster gets a chunk of 1, 2 or 4 K blocks."""
+    chunks = [-(-(-(-K // block)) // kc) for kc in (1, 2, 4)]
+    return any(-(-c // cluster) * (cluster - 1) < c for c in chunks)
 
 
 @pytest.mark.parametrize("cluster,bn", [(None, None), (1, 32), (2, 64), (4, 128), (8, 64), (1, 256)])
@@ -30,6 +36,10 @@ def test_both_schemes(M, N, K, cluster, bn, oracle_c_lib):
     # (a tile and cluster that do not fit a shape fall back to the family's persistent kernel)
     with forced_path("umma"), knobs(**args):
         assert select_path(_lib.OP_W8A8, M, N, K) == "umma_i8_tokens128"
+        for op, block, tile in ((_lib.OP_W8A8, 128, "channels"), (_lib.OP_W8A16, 64, "tokens")):
+            plan = mid_plan(op, M, N, K)         # ... and which ones these are is known
+            assert (plan is not None) == (cluster is None or splits_over(K, block, cluster)), (op, plan)
+            assert plan is None or cluster is None or (plan["cluster"], plan[tile]) == (cluster, bn), (op, plan)
         ref = O.w8a8_int32_accumulators(xq, q)
         assert torch.equal(w8a8_int32_accumulators(xq.cuda(), q.cuda()).cpu(), ref)
         y = apply_w8a8_linear(xq.cuda(), a_s.cuda(), q.cuda(), s.cuda(), b.cuda(), out_dtype=dtype)
@@ -51,6 +61,8 @@ def test_w8a16_more_than_one_wave_and_every_token_tile(M, N, K, bn):
     x = O.make_activation(M, K, seed=M, dtype=torch.bfloat16)
     with knobs(**({} if bn is None else {"BN": bn})):
         assert select_path(_lib.OP_W8A16, M, N, K) == "umma_f16_expand_tokens128"
+        plan = mid_plan(_lib.OP_W8A16, M, N, K)
+        assert plan is not None and (bn is None or plan["tokens"] == bn), plan
         y = apply_int8_weight_only_linear(x.cuda(), q.cuda(), s.cuda())
     m = O.tensor_metrics(O.w8a16_native_reference(x, q, s, None), y)
     assert m["relative_l2"] <= 4e-3 and m["cosine_similarity"] >= 0.9999, m
@@ -62,6 +74,7 @@ def test_w8a16_more_than_one_wave_and_every_token_tile(M, N, K, bn):
                                         (450, 6144, 1024, "umma_i8_tokens128")])
 def test_w8a8_beyond_one_wave_takes_the_pair_kernel_where_rounding_tokens_up_costs_no_wave(M, N, K, path, oracle_c_lib):
     assert select_path(_lib.OP_W8A8, M, N, K) == path
+    assert mid_plan(_lib.OP_W8A8, M, N, K) is None    # beyond one wave the name means the persistent kernel
     q, s = O.make_weight(N, K, seed=N + K)
     xq, a_s = O.quantize_per_row_dynamic(O.make_activation(M, K, seed=M, dtype=torch.bfloat16))
     ref = O.w8a8_int32_accumulators(xq, q)

@@ -1,10 +1,8 @@
 """Plans of the tcgen05 kernels for tens to hundreds of tokens (host code, no GPU).  A CTA of a cluster that waits for
 tensor memory held by another such CTA never ends, so the ones that fit an SM together may not need more than it has."""
-import ctypes
-
 import pytest
 
-from tests.gpu_util import knobs
+from tests.gpu_util import knobs, mid_plan
 import tiny_vllm_b200  # noqa: F401
 from tiny_vllm_b200 import _lib, build as b200_build
 
@@ -17,13 +15,6 @@ CHANNELS = [8, 72, 128, 264, 440, 512, 640, 768, 1024, 1536, 2048, 3072, 3968, 4
 INNER = [16, 96, 528, 896, 1024, 1536, 2048, 2112, 2944, 3072, 4096, 8192, 12288]
 
 
-def plan_of(op, M, N, K):
-    out = (ctypes.c_int * 6)()
-    if not _lib.lib().b200q_debug_mid_plan(op, M, N, K, out):
-        return None
-    return dict(zip(("tokens", "channels", "cluster", "columns", "shared", "ctas"), out))
-
-
 @pytest.mark.parametrize("forced", [{}, {"CLUSTER": 2}, {"CLUSTER": 4, "BN": 64}, {"CLUSTER": 8, "BN": 256}],
                          ids=["chosen", "cluster2", "cluster4-bn64", "cluster8-bn256"])
 @pytest.mark.parametrize("op", [_lib.OP_W8A8, _lib.OP_W8A16], ids=["w8a8", "w8a16"])
@@ -34,7 +25,7 @@ def test_clusters_never_wait_for_tensor_memory(op, forced):
         for M in TOKENS:
             for N in CHANNELS:
                 for K in INNER:
-                    p = plan_of(op, M, N, K)
+                    p = mid_plan(op, M, N, K)
                     if p is None or p["cluster"] == 1:
                         continue
                     seen += 1

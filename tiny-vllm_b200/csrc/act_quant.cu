@@ -119,7 +119,7 @@ template <typename T>
 cudaError_t launch_typed(const T* x, int64_t ldx, int8_t* xq, float* a_scales, int M, int K,
                          bool early, cudaStream_t st) {
   cudaError_t e;
-  if (K > 256 * 8 * 8)
+  if (act_quant_long_row(K))
     return launch_overlapped(act_quant_long_rows_kernel<T>, M, 256, 0, st, x, ldx, xq, a_scales, M, K,
                              early);
   B200Q_ROWS_DISPATCH(act_quant_rows_kernel, K >> 3, x, ldx, xq, a_scales, M, K, early);

@@ -75,7 +75,9 @@ inline RowShape row_shape(int M, int nchunk) {
 int device_cc_major();
 int* device_status_ptr();
 
-// act_quant.cu; early: the next kernel takes the codes as activations and may start at once
+// act_quant.cu: rows too long for a thread group's registers are read twice
+inline bool act_quant_long_row(int K) { return K > 256 * 8 * 8; }
+// early: the next kernel takes the codes as activations and may start at once
 cudaError_t launch_act_quant(const void* x, int64_t ldx, int x_dtype, int8_t* xq, float* a_scales,
                              int M, int K, bool early, cudaStream_t stream);
 
