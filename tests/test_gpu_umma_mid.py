@@ -18,9 +18,14 @@ SHAPES = [  # (M, N, K): one row of a tile, ragged everything, several token til
 ]
 
 
-def splits_over(K, block, cluster):
-    """Every CTA of a cluster gets a chunk of 1, 2 or 4 K blocks."""
-    chunks = [-(-(-(-K // block)) // kc) for kc in (1, 2, 4)]
+def takes(op, M, N, K, cluster, bn):
+    """Every CTA of the cluster gets a chunk of 1, 2 or 4 K blocks; W8A16 clusters in two CTAs per SM at most."""
+    if cluster is None or cluster == 1:
+        return True
+    if op == _lib.OP_W8A16 and -(-M // bn) * -(-N // 128) * cluster > 2 * 148:
+        return False
+    blocks = -(-K // (128 if op == _lib.OP_W8A8 else 64))
+    chunks = [-(-blocks // kc) for kc in (1, 2, 4)]
     return any(-(-c // cluster) * (cluster - 1) < c for c in chunks)
 
 
@@ -36,9 +41,9 @@ def test_both_schemes(M, N, K, cluster, bn, oracle_c_lib):
     # (a tile and cluster that do not fit a shape fall back to the family's persistent kernel)
     with forced_path("umma"), knobs(**args):
         assert select_path(_lib.OP_W8A8, M, N, K) == "umma_i8_tokens128"
-        for op, block, tile in ((_lib.OP_W8A8, 128, "channels"), (_lib.OP_W8A16, 64, "tokens")):
+        for op, tile in ((_lib.OP_W8A8, "channels"), (_lib.OP_W8A16, "tokens")):
             plan = mid_plan(op, M, N, K)         # ... and which ones these are is known
-            assert (plan is not None) == (cluster is None or splits_over(K, block, cluster)), (op, plan)
+            assert (plan is not None) == takes(op, M, N, K, cluster, bn), (op, plan)
             assert plan is None or cluster is None or (plan["cluster"], plan[tile]) == (cluster, bn), (op, plan)
         ref = O.w8a8_int32_accumulators(xq, q)
         assert torch.equal(w8a8_int32_accumulators(xq.cuda(), q.cuda()).cpu(), ref)
