@@ -263,6 +263,9 @@ int b200q_check_status(int* status_word);
  */
 int b200q_debug_mid_plan(int op, int M, int N, int K, int* plan);
 
+/* Test hook: number of TMA descriptors this library has encoded in this process. */
+uint64_t b200q_debug_maps_encoded(void);
+
 /* Test hook: number of kernels this library has launched in this process. */
 uint64_t b200q_launch_count(void);
 

@@ -92,6 +92,7 @@ SIGNATURES = {
     "b200q_debug_set": (_c.c_int, [_c.c_int, _c.c_int]),
     "b200q_debug_reset": (None, []),
     "b200q_debug_mid_plan": (_c.c_int, [_c.c_int, _c.c_int, _c.c_int, _c.c_int, _c.POINTER(_c.c_int)]),
+    "b200q_debug_maps_encoded": (_c.c_uint64, []),
     "b200q_check_status": (_c.c_int, [_c.POINTER(_c.c_int)]),
     "b200q_launch_count": (_c.c_uint64, []),
     "b200q_tp_allreduce": (_c.c_int, [_c.c_void_p, _c.c_void_p, _c.c_int, _c.c_int, _c.c_size_t,

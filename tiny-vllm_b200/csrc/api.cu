@@ -616,6 +616,8 @@ int b200q_debug_mid_plan(int op, int M, int N, int K, int* plan) {
   return 1;
 }
 
+uint64_t b200q_debug_maps_encoded(void) { return maps_encoded(); }
+
 uint64_t b200q_launch_count(void) { return g_launches.load(); }
 
 }  // extern "C"

@@ -126,6 +126,7 @@ bool make_tensor_map(const void* base, uint64_t rows, uint64_t row_bytes, uint32
                      uint32_t box_bytes, CUtensorMap* out, uint32_t box_blocks = 0);
 bool get_tensor_map(const void* base, uint64_t rows, uint64_t row_bytes, uint32_t box_rows,
                     uint32_t box_bytes, CUtensorMap* out, uint32_t box_blocks = 0);
+uint64_t maps_encoded();   // how many descriptors this process has encoded
 
 // Test and tuning hooks (B200Q_KNOB_* of b200q.h).  Every knob is unset (the built-in
 // behaviour) until the CALLING THREAD sets it through b200q_debug_set(); nothing is read from

@@ -22,9 +22,11 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstdlib>
 #include <mutex>
 #include <unordered_map>
+#include <vector>
 
 #include "common.h"
 #include "ptx_sm100.cuh"
@@ -361,6 +363,8 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
                                   const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
+std::atomic<uint64_t> g_maps_encoded{0};
+
 EncodeTiledFn encode_fn() {
   static EncodeTiledFn fn = nullptr;
   static std::once_flag once;
@@ -415,15 +419,22 @@ bool make_tensor_map(const void* base, uint64_t rows, uint64_t row_bytes, uint32
     note_cuda_error(cudaErrorInvalidValue);
     return false;
   }
+  g_maps_encoded.fetch_add(1, std::memory_order_relaxed);
   return true;
 }
 
+uint64_t maps_encoded() { return g_maps_encoded.load(std::memory_order_relaxed); }
+
 // Cached variant for matrices that keep their address (weights): encoding costs about a
-// microsecond of host time.
+// microsecond of host time.  The oldest entry makes room for a new one: emptying the whole table would encode
+// a serving process's weights again whenever its token counts have used up the entries.
 bool get_tensor_map(const void* base, uint64_t rows, uint64_t row_bytes, uint32_t box_rows,
                     uint32_t box_bytes, CUtensorMap* out, uint32_t box_blocks) {
   static std::mutex mu;
   static std::unordered_map<MapKey, CUtensorMap, MapKeyHash> cache;
+  constexpr size_t kEntries = 8192;
+  static std::vector<MapKey> age;   // ring of the keys in the order of their arrival
+  static size_t oldest = 0;
   int dev = 0;
   cudaGetDevice(&dev);
   MapKey key{base, rows, row_bytes, box_rows, box_bytes, box_blocks, dev};
@@ -439,8 +450,15 @@ bool get_tensor_map(const void* base, uint64_t rows, uint64_t row_bytes, uint32_
   if (!make_tensor_map(base, rows, row_bytes, box_rows, box_bytes, &m, box_blocks)) return false;
   {
     std::lock_guard<std::mutex> g(mu);
-    if (cache.size() > 8192) cache.clear();
-    cache.emplace(key, m);
+    if (cache.emplace(key, m).second) {   // (another thread may have been first)
+      if (age.size() < kEntries) {
+        age.push_back(key);
+      } else {
+        cache.erase(age[oldest]);
+        age[oldest] = key;
+        oldest = (oldest + 1) % kEntries;
+      }
+    }
   }
   *out = m;
   return true;

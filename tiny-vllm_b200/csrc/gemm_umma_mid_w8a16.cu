@@ -489,18 +489,10 @@ bool umma16_mid_shape(int M, int N, int K, MidShape* s) {
 int launch_umma16_mid(const GemmArgs& a) {
   MidPlan pl;
   if (!mid_plan<MidPlan, search_plan>(a.M, a.N, a.K, &pl)) return B200Q_ERR_UNSUPPORTED_SHAPE;
-  CUtensorMap tx, tw;
-  const uint64_t x_row = static_cast<uint64_t>(a.K) * 2;
-  if (!make_tensor_map(a.x, a.M, x_row, static_cast<uint32_t>(pl.bt), 128, &tx) ||
-      !get_tensor_map(a.w, a.N, a.K, static_cast<uint32_t>(pl.rows), kRow8, &tw))
-    return B200Q_ERR_LAUNCH;
-  // K a multiple of a block: everything comes through the 3-D maps (blocks beyond K read as zeros);
-  // otherwise the chunk with the partial block, and what follows it, goes block by block
-  const int chunks_3d = a.K % kBlockK == 0 ? pl.chunks : a.K / kBlockK / pl.kc;
-  CUtensorMap tx3 = tx, tw3 = tw;
-  if (chunks_3d > 0 &&
-      (!make_tensor_map(a.x, a.M, x_row, static_cast<uint32_t>(pl.bt), 128, &tx3, pl.kc) ||
-       !get_tensor_map(a.w, a.N, a.K, static_cast<uint32_t>(pl.rows), kRow8, &tw3, pl.kc)))
+  MidMaps maps;
+  if (!maps.make({a.x, static_cast<uint64_t>(a.M), static_cast<uint64_t>(a.K) * 2, static_cast<uint32_t>(pl.bt), 128},
+                 {a.w, static_cast<uint64_t>(a.N), static_cast<uint64_t>(a.K), static_cast<uint32_t>(pl.rows), kRow8},
+                 a.K, kBlockK, pl.kc, pl.chunks))
     return B200Q_ERR_LAUNCH;
   MidParams mp{};
   mp.M = a.M;
@@ -511,7 +503,7 @@ int launch_umma16_mid(const GemmArgs& a) {
   mp.kc = pl.kc;
   mp.chunks = pl.chunks;
   mp.chunks_per_split = pl.chunks_per_split;
-  mp.chunks_3d = chunks_3d;
+  mp.chunks_3d = maps.chunks_3d;
   mp.splits = pl.splits;
   mp.stages = pl.stages;
   mp.stage_bytes = pl.stage_bytes;
@@ -526,8 +518,8 @@ int launch_umma16_mid(const GemmArgs& a) {
   mp.status = a.status;
   const int ctas = pl.tiles_t * pl.tiles_c * pl.splits;
   const cudaError_t e =
-      mp.is_bf16 ? launch_mid_kernel<w8a16_mid_kernel<__nv_bfloat16>>(ctas, pl.splits, pl.smem, a.stream, tx, tw, tx3, tw3, mp)
-                 : launch_mid_kernel<w8a16_mid_kernel<__half>>(ctas, pl.splits, pl.smem, a.stream, tx, tw, tx3, tw3, mp);
+      mp.is_bf16 ? launch_mid_kernel<w8a16_mid_kernel<__nv_bfloat16>>(ctas, pl.splits, pl.smem, a.stream, maps, mp)
+                 : launch_mid_kernel<w8a16_mid_kernel<__half>>(ctas, pl.splits, pl.smem, a.stream, maps, mp);
   if (e != cudaSuccess) {
     note_cuda_error(e);
     return B200Q_ERR_LAUNCH;

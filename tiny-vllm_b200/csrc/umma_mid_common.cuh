@@ -107,9 +107,35 @@ bool mid_plan(int M, int N, int K, Plan* best) {
   return true;
 }
 
+// Descriptors of a call's two operands.  Chunks of whole K blocks come through the 3-D maps, one instruction each; the
+// chunk with a partial block, and what follows it, goes block by block through the 2-D ones (blocks beyond K
+// read as zeros either way).  Only those that the kernel reads are made: an encoding costs a microsecond of
+// host time, and the weights' are all made again on the first pass over a model and over a new box.
+struct MidMaps {
+  struct Matrix {
+    const void* base;
+    uint64_t rows, row_bytes;
+    uint32_t box_rows, box_bytes;
+  };
+  CUtensorMap x, w, x3, w3;
+  int chunks_3d;   // chunks below this one come through the 3-D maps
+  bool make(const Matrix& mx, const Matrix& mw, int K, int block, int kc, int chunks) {
+    chunks_3d = K % block == 0 ? chunks : K / block / kc;
+    const uint32_t box = static_cast<uint32_t>(kc);
+    if (chunks_3d < chunks && (!make_tensor_map(mx.base, mx.rows, mx.row_bytes, mx.box_rows, mx.box_bytes, &x) ||
+                               !get_tensor_map(mw.base, mw.rows, mw.row_bytes, mw.box_rows, mw.box_bytes, &w)))
+      return false;
+    if (chunks_3d > 0 && (!make_tensor_map(mx.base, mx.rows, mx.row_bytes, mx.box_rows, mx.box_bytes, &x3, box) ||
+                          !get_tensor_map(mw.base, mw.rows, mw.row_bytes, mw.box_rows, mw.box_bytes, &w3, box)))
+      return false;
+    if (chunks_3d == chunks) x = x3, w = w3;   // never read
+    if (chunks_3d == 0) x3 = x, w3 = w;
+    return true;
+  }
+};
+
 template <auto kernel, typename Params>
-cudaError_t launch_mid_kernel(int ctas, int splits, size_t smem, cudaStream_t stream, const CUtensorMap& tx,
-                              const CUtensorMap& tw, const CUtensorMap& tx3, const CUtensorMap& tw3,
+cudaError_t launch_mid_kernel(int ctas, int splits, size_t smem, cudaStream_t stream, const MidMaps& maps,
                               const Params& mp) {
   static bool attr_set[64] = {false};
   int dev = 0;
@@ -123,7 +149,8 @@ cudaError_t launch_mid_kernel(int ctas, int splits, size_t smem, cudaStream_t st
     if (per_sm > 2) return cudaErrorInvalidConfiguration;
     if (dev < 64) attr_set[dev] = true;
   }
-  return launch_clustered(splits, true, kernel, dim3(ctas), dim3(kMidThreads), smem, stream, tx, tw, tx3, tw3, mp);
+  return launch_clustered(splits, true, kernel, dim3(ctas), dim3(kMidThreads), smem, stream, maps.x, maps.w,
+                          maps.x3, maps.w3, mp);
 }
 
 }  // namespace b200q
