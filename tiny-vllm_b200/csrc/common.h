@@ -155,7 +155,8 @@ bool umma16_pair_applicable(int M, int N, int K);
 size_t umma16_pair_workspace_bytes(int N, int K);
 int launch_w8a16_umma_pair(const GemmArgs& a);
 
-// gemm_umma_mid.cu, gemm_umma_mid_w8a16.cu: W8A8 and W8A16 at up to 512 tokens, two CTAs per SM, cluster split-K
+// gemm_umma_mid.cu, gemm_umma_mid_w8a16.cu: tens to hundreds of tokens (W8A8: up to a wave of 128 x 128 tiles; W8A16: 2.6
+// waves, at most 2048 tokens), one tile per CTA, K split over a cluster
 bool umma_mid_applicable(int M, int N, int K);
 int launch_umma_mid(const GemmArgs& a);
 bool umma16_mid_applicable(int M, int N, int K);

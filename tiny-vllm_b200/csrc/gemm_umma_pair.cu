@@ -26,8 +26,11 @@
 //
 // The epilogue: sixteen warps, each 32 rows x 64 columns of a tile.  A warp takes its share of the accumulators
 // into registers at once and hands the TMEM buffer back before it converts anything, so the
-// MMAs of the tile after next never wait for stores (eight warps with two column groups each:
-// 4096 -> 4096 at 8192 tokens 90.0 us, now 88.6; 1024 -> 4096 33.0, now 31.9).  Its output routes:
+// MMAs of the tile after next never wait for stores.  Against eight warps with two column groups each
+// this gains where a pair has many short tiles and loses where it has two (8192 tokens, us before / now: 1024 -> 4096
+// 34.0 / 32.9, 1024 -> 6144 48.1 / 48.0, 4096 -> 4096 90.2 / 89.7, 4096 -> 6144 136.5 / 134.7, but 2048 -> 1024 17.9 / 18.4,
+// 3072 -> 1024 22.8 / 23.2): level over the projections of a layer.  Eighteen warps leave 96 registers a thread, and the
+// int8 instances spill (40 bytes stored, 68 loaded per thread with EPI_TMA).  Its output routes:
 //   EPI_TMA     convert -> swizzled shared-memory slab -> one thread issues a TMA tensor store
 //               of the 32 x 64 box (this GPU's memory only); the epilogue warps never read the
 //               slab back and never issue a global store, and the stores drain while the warp waits for

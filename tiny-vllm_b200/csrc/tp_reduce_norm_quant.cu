@@ -255,7 +255,8 @@ cudaError_t launch_exchange_g(const ExchangeParams& p, cudaStream_t st) {
 template <typename T, int W>
 cudaError_t launch_exchange(const ExchangeParams& p, cudaStream_t st) {
   const int K = p.K;
-  // same row-group widths as the stand-alone add-RMSNorm quantiser (bit-identical sums)
+  // (row_sum adds in an order that depends on the chunks alone: the same bits as the stand-alone add-RMSNorm
+  // quantiser, whatever widths that one takes)
   if (K <= 32 * 8 * 4) return launch_exchange_g<T, 32, 4, W>(p, st);
   if (K <= 64 * 8 * 4) return launch_exchange_g<T, 64, 4, W>(p, st);
   if (K <= 128 * 8 * 4) return launch_exchange_g<T, 128, 4, W>(p, st);
