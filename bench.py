@@ -25,8 +25,8 @@ GEMM, decode batches, the Qwen3-8B shapes, the reference's own CUDA kernels).
 
 ``--impl reference`` times the reference's own CPU implementation of the path — its
 ``quantize_int8_per_row_dynamic`` and ``w8a8_linear_fallback`` from the mirror that
-``oracle/build_ref.py`` keeps in ``oracle/_ref`` (kind "reference"), or the oracle's port of
-them when no mirror was built (kind "port") — on all host cores, same workload, same steps.
+``oracle/build_ref.py`` keeps in ``oracle/_ref`` — on all host cores, same workload, same steps.
+Without a mirror it says so in an ``unavailable`` line: a port is not the reference.
 """
 from __future__ import annotations
 
@@ -142,6 +142,10 @@ def run_reference_arm(args):
         return
     threads = use_all_host_threads()
     quantise, linear, kind = cpu_path()
+    if kind != "reference":
+        print(json.dumps({"impl": "reference", "unavailable": "oracle/_ref holds no mirror of the reference (no checkout "
+                          "of it was at hand when the tree was built)"}))
+        return
     problems = cpu_problems(TOKENS)          # inputs are made once, outside the timed steps
     for _ in range(max(0, args.warmup)):
         cpu_sweep_once(problems, quantise, linear)
