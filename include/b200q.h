@@ -238,7 +238,7 @@ enum {
   B200Q_KNOB_PAIR_MIN_TILES = 14,  /* CTA-pair kernels: fewest 256 x 256 tiles a problem must have */
   B200Q_KNOB_BULK_DECODE = 15,  /* persistent ring-fed decode kernels: 1 never, 2 wherever they can run */
   B200Q_KNOB_BULK_SLOTS = 16,   /* ring depth per consumer warp of those kernels (>= 2; default: what fits) */
-  B200Q_KNOB_BULK_WPP = 17,     /* consumer warps per ring of the W8A8 one-token-tile kernel: 1 or 2 (default 2) */
+  B200Q_KNOB_BULK_WPP = 17,     /* 1: the 16-token ring kernels for at most 8 tokens too, W8A8 with one consumer warp per ring */
   B200Q_KNOB_NO_MID = 18,       /* 1: never take the one-tile-per-CTA tcgen05 kernels (tens to hundreds of tokens) */
   B200Q_KNOB_NO_REG = 19,       /* 1: never take the decode kernels that hold the weights in registers */
   B200Q_KNOB_COUNT = 20

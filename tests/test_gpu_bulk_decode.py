@@ -23,6 +23,8 @@ SHAPES = [  # (M, N, K)
     (1, 1024, 2048), (7, 1029, 2064), (16, 512, 3072), (17, 260, 4096), (33, 1000, 5136),
     (48, 384, 8192), (64, 264, 12288), (5, 96, 17408), (64, 72, 25600), (3, 100, 48), (16, 20000, 528),
     (16, 6144, 4096), (2, 14800, 1024), (32, 520, 4224), (20, 300, 8192), (9, 4096, 12288),
+    # at most 8 tokens: units of 16, 32 and 48 channels, activations staged (tokens <= units) or not, ragged K
+    (1, 4100, 2064), (4, 4100, 1040), (3, 20000, 528), (2, 14801, 1040), (8, 7105, 1168), (1, 24576, 400), (1, 148, 16),
 ]
 
 
