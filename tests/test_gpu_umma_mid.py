@@ -59,7 +59,8 @@ def test_both_schemes(M, N, K, cluster, bn, oracle_c_lib):
 
 @pytest.mark.parametrize("M,N,K,bn", [(1100, 4104, 272, None), (12, 16384, 2064, None), (2048, 1032, 1040, 192),
                                       (50, 264, 1616, 16), (97, 1000, 528, 48), (200, 136, 2112, 96),
-                                      (64, 9728, 2560, None), (33, 12296, 1040, None)])
+                                      (64, 9728, 2560, None), (33, 12296, 1040, None),
+                                      (33, 16384, 528, None), (255, 1000, 208, 256)])
 def test_w8a16_more_than_one_wave_and_every_token_tile(M, N, K, bn):
     # several waves of tiles, matrices too large for the ring kernel from 9 tokens on, the other tile widths
     q, s = O.make_weight(N, K, seed=N + K)

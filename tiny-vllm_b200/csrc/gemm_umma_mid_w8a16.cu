@@ -15,8 +15,12 @@
 //     (24576 x 4096 at 64 tokens: 280 tiles of 88 channels 26.3 us, 192 of 128 30.4);
 //   * an MMA of 64 columns takes 51 cycles and one of 128 68, whatever part of the 128 rows is used, so
 //     it is the tokens, the operand with fewer rows, that are cut finely.
-// Chains of launches, us per linear (expanded weights in shared memory; persistent kernels before that): 768 x
-// 4096 at 64 tokens 4.4 (5.9; 16.0), 4096 x 1024 at 512 9.0 (11.6; 13.7), 6144 x 4096 at 256 21.4 (35.4; 39.6).
+// The output tile leaves through shared memory, two tokens to a word as the accumulators lie in a thread, then whole
+// rows, 16 bytes a thread.  (4-byte stores from the registers, which neighbouring lanes had paired, took 2.2 us of a 128 x 128
+// tile, this 1.2.)  With K split the owner's sums, scales and conversions work on vectors: 1.0 -> 0.7 us.
+// Chains of launches, us per linear (without the two; expanded weights in shared memory; persistent kernels before
+// that): 4096 x 1024 at 512 tokens 7.7 (8.6; 11.6; 13.7), 6144 x 1024 at 512 10.0 (10.7), 4096 x 1024 at 77 4.2 (4.7), 4096 x
+// 512 at 64 3.3 (3.7), 4096 x 1536 at 64 4.8 (5.1), 768 x 4096 at 64 4.4 (4.4; 5.9; 16.0), 6144 x 4096 at 256 18.3 (19.3; 35.4; 39.6).
 //
 // Warp roles (352 threads): warp 0 TMA of the activations, warp 1 UMMA, warps 2-9 expansion (two groups of
 // four that take the chunks in turn: a warp reaches one TMEM lane quarter), then epilogue, warp 10
@@ -42,6 +46,7 @@ namespace {
 constexpr int kMidCh = 128;                      // UMMA M: channels of a tile
 constexpr int kMidWeightWarp = kMidThreads / 32 - 1;
 constexpr int kMidACols = 32;                    // TMEM columns of one K block of expanded weights
+constexpr int kOutPitch = kMidCh * 4;            // bytes of two tokens' rows of the output tile in shared memory
 
 struct MidParams {
   int M, N;
@@ -54,6 +59,7 @@ struct MidParams {
   int splits;              // cluster size
   int stages;              // ring of chunks of activations and of int8 weights: an even number, or one in all
   int stage_bytes, raw_bytes;
+  int ring_bytes;          // both rings, or the output tile that lies over them at the end
   int a_stages;            // ring of chunks of expanded weights in TMEM (likewise)
   int a_col0;              // its first TMEM column
   int tmem_cols;
@@ -65,19 +71,6 @@ struct MidParams {
 };
 
 template <typename T>
-__device__ __forceinline__ uint16_t bits16(T v) {
-  return *reinterpret_cast<const uint16_t*>(&v);
-}
-
-// One sum -> one scaled value.
-template <typename T>
-__device__ __forceinline__ T finish(uint32_t acc, float w_s, const T* bias, int n) {
-  float v = __fmul_rn(__uint_as_float(acc), w_s);
-  if (bias != nullptr) v = __fadd_rn(v, to_float<T>(bias[n]));
-  return from_float<T>(v);
-}
-
-template <typename T>
 __global__ void __launch_bounds__(kMidThreads, 2)
 w8a16_mid_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
                  const __grid_constant__ CUtensorMap tmap_x3, const __grid_constant__ CUtensorMap tmap_w3,
@@ -85,7 +78,7 @@ w8a16_mid_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
   extern __shared__ __align__(1024) uint8_t smem[];
   const int rows_own = (p.bt + p.splits - 1) / p.splits;       // tokens a CTA owns
   const uint32_t raw_base = static_cast<uint32_t>(p.stages * p.stage_bytes);
-  uint8_t* red = smem + raw_base + p.stages * p.raw_bytes; // [S][rows_own][128] 32-bit sums (S > 1)
+  uint8_t* red = smem + p.ring_bytes;                          // [S][rows_own][128] 32-bit sums (S > 1)
   float* s_ws = reinterpret_cast<float*>(red + (p.splits > 1 ? p.splits * rows_own * kMidCh * 4 : 0));   // [128]
   uint8_t* ctrl = reinterpret_cast<uint8_t*>(s_ws + kMidCh);
   uint64_t* xfull = reinterpret_cast<uint64_t*>(ctrl);         // activations of a stage have landed
@@ -283,20 +276,45 @@ w8a16_mid_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
                   v[j]);
           }
         } else {
-          // no split: straight from the registers.  Neighbouring lanes exchange halves, so that each
-          // stores two channels of one token: even lanes token j, odd lanes token j + 1.
+          // no split: scaled, rounded and two tokens to a word into shared memory as [token / 2][channel] (the rings
+          // are done with: the MMAs that read the last of them have completed)
+          uint32_t* slab = reinterpret_cast<uint32_t*>(smem + (c >> 1) * kOutPitch) + ch;
           const float w_s = s_ws[ch];
-          const bool odd = (lane & 1) != 0;
-          T* out = static_cast<T*>(p.out) + static_cast<size_t>(tile_t * p.bt + c + (odd ? 1 : 0)) * p.N + (odd ? n - 1 : n);
+          const float b = bias != nullptr && mine_n ? to_float<T>(bias[n]) : 0.f;
 #pragma unroll
           for (int j = 0; j < 32; j += 2) {
-            const T* b = mine_n ? bias : nullptr;
-            const uint32_t lo = bits16(finish<T>(v[j], w_s, b, n));
-            const uint32_t hi = bits16(finish<T>(v[j + 1], w_s, b, n));
-            const uint32_t got = __shfl_xor_sync(0xFFFFFFFFu, odd ? lo : hi, 1);
-            const uint32_t word = odd ? (got | (hi << 16)) : (lo | (got << 16));
-            if (c + j + (odd ? 1 : 0) < live && mine_n) *reinterpret_cast<uint32_t*>(out) = word;   // N is even
-            out += 2 * static_cast<size_t>(p.N);
+            float2 o = make_float2(__fmul_rn(__uint_as_float(v[j]), w_s), __fmul_rn(__uint_as_float(v[j + 1]), w_s));
+            if (bias != nullptr) o = make_float2(__fadd_rn(o.x, b), __fadd_rn(o.y, b));
+            slab[(j >> 1) * (kOutPitch / 4)] = pack2_rn<T>(o);
+          }
+        }
+      }
+    }
+    if (p.splits == 1) {
+      // whole rows of the tile, 16 bytes a thread (N % 8 == 0, rows % 8 == 0: a piece is inside or outside)
+      ptx::named_bar_sync(1, 256);
+      const int sub = tid & 15, n0 = tile_c * p.rows + sub * 8;
+      if (done && sub < (p.rows >> 3) && n0 < p.N) {
+        const int live = min(p.bt, p.M - tile_t * p.bt);
+        T* out = static_cast<T*>(p.out) + static_cast<size_t>(tile_t * p.bt) * p.N + n0;
+        for (int t0 = (tid >> 4) * 2; t0 < live; t0 += 64) {
+          uint4 v[4];     // of token pairs t0 and t0 + 32: channels 0-3 and 4-7 of the piece
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (t0 + 32 * (j >> 1) < live)
+              v[j] = *reinterpret_cast<const uint4*>(smem + (t0 / 2 + 16 * (j >> 1)) * kOutPitch + sub * 32 + 16 * (j & 1));
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            const int t = t0 + 32 * j;
+            const uint4 a = v[2 * j], b = v[2 * j + 1];
+            if (t < live)
+              *reinterpret_cast<uint4*>(out + static_cast<size_t>(t) * p.N) =
+                  make_uint4(__byte_perm(a.x, a.y, 0x5410), __byte_perm(a.z, a.w, 0x5410), __byte_perm(b.x, b.y, 0x5410),
+                             __byte_perm(b.z, b.w, 0x5410));
+            if (t + 1 < live)
+              *reinterpret_cast<uint4*>(out + static_cast<size_t>(t + 1) * p.N) =
+                  make_uint4(__byte_perm(a.x, a.y, 0x7632), __byte_perm(a.z, a.w, 0x7632), __byte_perm(b.x, b.y, 0x7632),
+                             __byte_perm(b.z, b.w, 0x7632));
           }
         }
       }
@@ -327,21 +345,27 @@ w8a16_mid_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
       const int tok = tl * p.splits + rank;
       const int row = tile_t * p.bt + tok, col = tile_c * p.rows + cg * 8;
       if (tok >= p.bt || cg * 8 >= p.rows || row >= p.M || col >= p.N) continue;   // N % 8 == 0
-      uint32_t w[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
+      float2 w[4];
       for (int s = 0; s < p.splits; ++s) {       // rank order: results do not depend on the run
-        const uint4* src = reinterpret_cast<const uint4*>(red) + ((s * rows_own + tl) * kMidCh + cg * 8) / 4;
-        const uint4 a = src[0], b = src[1];
-        const uint32_t in[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+        const float4* src = reinterpret_cast<const float4*>(red) + ((s * rows_own + tl) * kMidCh + cg * 8) / 4;
+        const float4 a = src[0], b = src[1];
+        const float2 in[4] = {{a.x, a.y}, {a.z, a.w}, {b.x, b.y}, {b.z, b.w}};
 #pragma unroll
-        for (int j = 0; j < 8; ++j)
-          w[j] = s == 0 ? in[j] : __float_as_uint(__fadd_rn(__uint_as_float(w[j]), __uint_as_float(in[j])));
+        for (int j = 0; j < 4; ++j)
+          w[j] = s == 0 ? in[j] : make_float2(__fadd_rn(w[j].x, in[j].x), __fadd_rn(w[j].y, in[j].y));
+      }
+      const float4 s0 = *reinterpret_cast<const float4*>(s_ws + cg * 8), s1 = *reinterpret_cast<const float4*>(s_ws + cg * 8 + 4);
+      const float2 sc[4] = {{s0.x, s0.y}, {s0.z, s0.w}, {s1.x, s1.y}, {s1.z, s1.w}};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) w[j] = make_float2(__fmul_rn(w[j].x, sc[j].x), __fmul_rn(w[j].y, sc[j].y));
+      if (bias != nullptr) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          w[j] = make_float2(__fadd_rn(w[j].x, to_float<T>(bias[col + 2 * j])), __fadd_rn(w[j].y, to_float<T>(bias[col + 2 * j + 1])));
       }
       uint32_t packed[4];
 #pragma unroll
-      for (int j = 0; j < 8; j += 2)
-        packed[j / 2] =
-            bits16(finish<T>(w[j], s_ws[cg * 8 + j], bias, col + j)) |
-            (static_cast<uint32_t>(bits16(finish<T>(w[j + 1], s_ws[cg * 8 + j + 1], bias, col + j + 1))) << 16);
+      for (int j = 0; j < 4; ++j) packed[j] = pack2_rn<T>(w[j]);
       *reinterpret_cast<uint4*>(static_cast<T*>(p.out) + static_cast<size_t>(row) * p.N + col) =
           make_uint4(packed[0], packed[1], packed[2], packed[3]);
     }
@@ -357,7 +381,7 @@ namespace {
 
 struct MidPlan {
   int bt, rows, splits, kc, chunks, chunks_per_split, tiles_t, tiles_c;
-  int stages, stage_bytes, raw_bytes, a_stages, a_col0, tmem_cols;
+  int stages, stage_bytes, raw_bytes, ring_bytes, a_stages, a_col0, tmem_cols;
   size_t smem;
 };
 
@@ -391,7 +415,10 @@ bool mid_plan_for(int M, int N, int k_blocks, int bt, int rows, int splits, int 
   pl->stages = stages;
   pl->tmem_cols = 32;
   while (pl->tmem_cols < cols) pl->tmem_cols *= 2;
-  pl->smem = static_cast<size_t>(stages) * ring_bytes + fixed;
+  pl->ring_bytes = stages * ring_bytes;
+  if (splits == 1) pl->ring_bytes = std::max(pl->ring_bytes, (bt + 31) / 32 * 16 * kOutPitch);
+  pl->smem = static_cast<size_t>(pl->ring_bytes) + fixed;
+  if (pl->smem > static_cast<size_t>(smem_cap)) return false;
   // no other CTA of a cluster fits beside it (see the residency rule in umma_mid_common.cuh)
   if (splits > 1 && pl->tmem_cols > 256) pl->smem = kMidSmemOne;
   return true;
@@ -508,6 +535,7 @@ int launch_umma16_mid(const GemmArgs& a) {
   mp.stages = pl.stages;
   mp.stage_bytes = pl.stage_bytes;
   mp.raw_bytes = pl.raw_bytes;
+  mp.ring_bytes = pl.ring_bytes;
   mp.a_stages = pl.a_stages;
   mp.a_col0 = pl.a_col0;
   mp.tmem_cols = pl.tmem_cols;
