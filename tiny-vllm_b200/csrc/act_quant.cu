@@ -117,10 +117,10 @@ act_quant_long_rows_kernel(const T* x, int64_t ldx, int8_t* xq, float* a_scales,
 
 template <typename T>
 cudaError_t launch_typed(const T* x, int64_t ldx, int8_t* xq, float* a_scales, int M, int K,
-                         bool early, cudaStream_t st) {
+                         bool early, Carveout carve, cudaStream_t st) {
   cudaError_t e;
   if (act_quant_long_row(K))
-    return launch_overlapped(act_quant_long_rows_kernel<T>, M, 256, 0, st, x, ldx, xq, a_scales, M, K,
+    return launch_overlapped(carve, act_quant_long_rows_kernel<T>, M, 256, 0, st, x, ldx, xq, a_scales, M, K,
                              early);
   B200Q_ROWS_DISPATCH(act_quant_rows_kernel, K >> 3, x, ldx, xq, a_scales, M, K, early);
   return e;
@@ -129,12 +129,12 @@ cudaError_t launch_typed(const T* x, int64_t ldx, int8_t* xq, float* a_scales, i
 }  // namespace
 
 cudaError_t launch_act_quant(const void* x, int64_t ldx, int x_dtype, int8_t* xq, float* a_scales,
-                             int M, int K, bool early, cudaStream_t stream) {
+                             int M, int K, bool early, Carveout carve, cudaStream_t stream) {
   cudaError_t e;
   if (x_dtype == B200Q_DTYPE_BF16) {
-    e = launch_typed(reinterpret_cast<const __nv_bfloat16*>(x), ldx, xq, a_scales, M, K, early, stream);
+    e = launch_typed(reinterpret_cast<const __nv_bfloat16*>(x), ldx, xq, a_scales, M, K, early, carve, stream);
   } else {
-    e = launch_typed(reinterpret_cast<const __half*>(x), ldx, xq, a_scales, M, K, early, stream);
+    e = launch_typed(reinterpret_cast<const __half*>(x), ldx, xq, a_scales, M, K, early, carve, stream);
   }
   if (e == cudaSuccess) count_launch();
   return e;

@@ -228,10 +228,10 @@ __device__ __forceinline__ void quantise_row(const uint4 (&y)[CHUNKS], bool acti
   }
 }
 
-// Launches KERNEL<T, threads per row, chunks per thread> (`e = launch_overlapped(...)` on stream st) for M rows of
+// Launches KERNEL<T, threads per row, chunks per thread> (`e = launch_overlapped(carve, ...)` on stream st) for M rows of
 // NCHUNK 16-byte chunks (at most 2048).
 #define B200Q_ROWS(KERNEL, G, C, ...) \
-  e = launch_overlapped(KERNEL<T, G, C>, (M + 256 / G - 1) / (256 / G), 256, 0, st, __VA_ARGS__)
+  e = launch_overlapped(carve, KERNEL<T, G, C>, (M + 256 / G - 1) / (256 / G), 256, 0, st, __VA_ARGS__)
 #define B200Q_ROWS_C(KERNEL, G, C_, ...)                        \
   do {                                                          \
     if ((C_) == 1) B200Q_ROWS(KERNEL, G, 1, __VA_ARGS__);       \

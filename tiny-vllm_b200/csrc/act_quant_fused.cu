@@ -151,11 +151,15 @@ silu_mul_quant_kernel(const T* gate_up, int64_t ld, T* y_out, int8_t* xq, float*
   quantise_row<T, G, CHUNKS>(y, active, row, t, g, nchunk, I, y_out, xq, a_scales, red);
 }
 
+// from 17 tokens on the next kernel is one of the tcgen05 ones, but for odd channel counts
+Carveout producer_carveout(int M) { return M > 16 ? MAX_SHARED : DEFAULT_SPLIT; }
+
 template <typename T>
 cudaError_t launch_rmsnorm(const void* x, const void* res_in, const void* weight, float eps,
                            void* res_out, void* y, int8_t* xq, float* a_s, int M, int K,
                            cudaStream_t st) {
   cudaError_t e;
+  const Carveout carve = producer_carveout(M);
   B200Q_ROWS_DISPATCH(add_rmsnorm_quant_kernel, K >> 3, static_cast<const T*>(x),
                        static_cast<const T*>(res_in), static_cast<const T*>(weight), eps,
                        static_cast<T*>(res_out), static_cast<T*>(y), xq, a_s, M, K);
@@ -166,6 +170,7 @@ template <typename T>
 cudaError_t launch_silu(const void* gate_up, int64_t ld, void* y, int8_t* xq, float* a_s, int M,
                         int I, cudaStream_t st) {
   cudaError_t e;
+  const Carveout carve = producer_carveout(M);
   B200Q_ROWS_DISPATCH(silu_mul_quant_kernel, I >> 3, static_cast<const T*>(gate_up), ld,
                        static_cast<T*>(y), xq, a_s, M, I);
   return e;

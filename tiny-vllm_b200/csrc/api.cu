@@ -144,9 +144,9 @@ bool dynamic_is_fused(int M, int N, int K) {
          !bulk_decode_applicable(M, N, K, false) && reg_decode_dynamic_applicable(M, N, K);
 }
 
-// b200q_act_quant_i8 with the choice of `early` (common.h)
+// b200q_act_quant_i8 with the choice of `carve` and `early` (common.h)
 int run_act_quant(const void* x, int64_t ldx, int x_dtype, int8_t* xq, float* a_scales, int M, int K,
-                  bool early, void* stream) {
+                  Carveout carve, bool early, void* stream) {
   if (x == nullptr || xq == nullptr || a_scales == nullptr) return B200Q_ERR_NULL_POINTER;
   if (M <= 0 || K <= 0 || static_cast<long long>(M) * K > INT_MAX) return B200Q_ERR_BAD_SHAPE;
   if (x_dtype != B200Q_DTYPE_F16 && x_dtype != B200Q_DTYPE_BF16) return B200Q_ERR_BAD_ARGUMENT;
@@ -157,7 +157,7 @@ int run_act_quant(const void* x, int64_t ldx, int x_dtype, int8_t* xq, float* a_
   if (d == nullptr) return B200Q_ERR_LAUNCH;
   if (d->cc_major != 10) return B200Q_ERR_UNSUPPORTED_ARCH;
   cudaError_t e =
-      launch_act_quant(x, ldx, x_dtype, xq, a_scales, M, K, early, static_cast<cudaStream_t>(stream));
+      launch_act_quant(x, ldx, x_dtype, xq, a_scales, M, K, early, carve, static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) {
     note_cuda_error(e);
     return B200Q_ERR_LAUNCH;
@@ -202,7 +202,7 @@ extern "C" {
 
 int b200q_act_quant_i8(const void* x, int64_t ldx, int x_dtype, int8_t* xq, float* a_scales, int M,
                        int K, void* stream) {
-  return run_act_quant(x, ldx, x_dtype, xq, a_scales, M, K, false, stream);
+  return run_act_quant(x, ldx, x_dtype, xq, a_scales, M, K, DEFAULT_SPLIT, false, stream);
 }
 
 int b200q_w8a8_gemm(const int8_t* xq, const float* a_scales, const int8_t* qweight,
@@ -454,7 +454,9 @@ int b200q_w8a8_dynamic_gemm(const void* x, const int8_t* qweight, const float* w
     // scales first, codes behind them
     float* a_s = static_cast<float*>(scratch);
     int8_t* xq = static_cast<int8_t*>(scratch) + dynamic_code_offset(M);
-    if (int rc = run_act_quant(x, K, x_dtype, xq, a_s, M, K, true, stream)) return rc;
+    const Carveout carve = resolve_path(B200Q_OP_W8A8, M, N, K) != B200Q_PATH_MMA_STREAM || bulk_decode_applicable(M, N, K, false)
+                               ? MAX_SHARED : DEFAULT_SPLIT;
+    if (int rc = run_act_quant(x, K, x_dtype, xq, a_s, M, K, carve, true, stream)) return rc;
     return b200q_w8a8_gemm(xq, a_s, qweight, w_scales, bias, y, M, N, K, x_dtype, workspace,
                            workspace_bytes, stream);
   }

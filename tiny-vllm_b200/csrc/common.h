@@ -75,11 +75,18 @@ inline RowShape row_shape(int M, int nchunk) {
 int device_cc_major();
 int* device_status_ptr();
 
+// An SM divides its memory between L1 and shared memory by the kernel that starts on it and cannot change that while
+// CTAs run.  A kernel that would leave most of it to L1, and stands between two that need nearly all of it as shared memory,
+// keeps the second one off its SMs until it has ended; so does one with less of its own.  MAX_SHARED asks for the division
+// that those need: for the tcgen05 and ring kernels and for what quantises their activations (256 tokens of the 0.6B
+// model, W8A8, 376 -> 359 us), not for the kernels that live on L1 (16 tokens, weights in registers, 129 -> 157 us).
+enum Carveout { DEFAULT_SPLIT = 0, MAX_SHARED = 1 };
+
 // act_quant.cu: rows too long for a thread group's registers are read twice
 inline bool act_quant_long_row(int K) { return K > 256 * 8 * 8; }
-// early: the next kernel takes the codes as activations and may start at once
+// early: the next kernel takes the codes as activations and may start at once; carve: what suits that kernel
 cudaError_t launch_act_quant(const void* x, int64_t ldx, int x_dtype, int8_t* xq, float* a_scales,
-                             int M, int K, bool early, cudaStream_t stream);
+                             int M, int K, bool early, Carveout carve, cudaStream_t stream);
 
 // gemm_simt.cu
 cudaError_t launch_w8a8_simt(const GemmArgs& a);
@@ -187,38 +194,42 @@ int launch_w8a16_umma_ts(const GemmArgs& a);
 // (act_quant.cu).  B200Q_KNOB_NO_PDL turns the overlap off.
 bool pdl_enabled();
 template <typename... KArgs, typename... Args>
-cudaError_t launch_clustered(int cluster, bool overlap, void (*kernel)(KArgs...), dim3 grid,
+cudaError_t launch_clustered(Carveout carve, int cluster, bool overlap, void (*kernel)(KArgs...), dim3 grid,
                              dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[2];
+  cudaLaunchAttribute attr[3];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = (overlap && pdl_enabled()) ? 1 : 0;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
+  if (carve == MAX_SHARED) {
+    cudaLaunchAttribute& c = attr[cfg.numAttrs++];
+    c.id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    c.val.sharedMemCarveout = cudaSharedmemCarveoutMaxShared;
+  }
   if (cluster > 1) {  // grid.x must be a multiple of the cluster size
-    attr[1].id = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.x = static_cast<unsigned int>(cluster);
-    attr[1].val.clusterDim.y = 1;
-    attr[1].val.clusterDim.z = 1;
-    cfg.numAttrs = 2;
+    cudaLaunchAttribute& c = attr[cfg.numAttrs++];
+    c.id = cudaLaunchAttributeClusterDimension;
+    c.val.clusterDim.x = static_cast<unsigned int>(cluster);
+    c.val.clusterDim.y = 1;
+    c.val.clusterDim.z = 1;
   }
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 template <typename... KArgs, typename... Args>
 cudaError_t launch_maybe_overlapped(bool overlap, void (*kernel)(KArgs...), dim3 grid, dim3 block,
                                     size_t smem, cudaStream_t stream, Args&&... args) {
-  return launch_clustered(1, overlap, kernel, grid, block, smem, stream,
+  return launch_clustered(DEFAULT_SPLIT, 1, overlap, kernel, grid, block, smem, stream,
                           static_cast<Args&&>(args)...);
 }
 template <typename... KArgs, typename... Args>
-cudaError_t launch_overlapped(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
+cudaError_t launch_overlapped(Carveout carve, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
                               cudaStream_t stream, Args&&... args) {
-  return launch_maybe_overlapped(true, kernel, grid, block, smem, stream,
-                                 static_cast<Args&&>(args)...);
+  return launch_clustered(carve, 1, true, kernel, grid, block, smem, stream, static_cast<Args&&>(args)...);
 }
 
 void note_cuda_error(cudaError_t e);

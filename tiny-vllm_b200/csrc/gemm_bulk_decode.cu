@@ -716,7 +716,7 @@ cudaError_t launch_stream(int grid, int threads, size_t smem, cudaStream_t strea
     if (e != cudaSuccess) return e;
     if (dev < 64) raised[dev] = true;
   }
-  return launch_overlapped(kernel, dim3(grid), dim3(threads), smem, stream, args...);
+  return launch_overlapped(MAX_SHARED, kernel, dim3(grid), dim3(threads), smem, stream, args...);
 }
 
 // knob BULK_WPP = 1: the 16-token kernels also for M <= 8 (tests compare the two forms)

@@ -278,8 +278,8 @@ template <int KIND, typename T, int NT, int BLK>
 cudaError_t launch_hi(const RegParams& p, cudaStream_t stream) {
   const dim3 grid((p.N + 8 * NT - 1) / (8 * NT));
   const size_t smem = KIND == REG_A8_DYN ? static_cast<size_t>(p.M) * (p.K + kCodePad) : 0;
-  return p.M > 8 ? launch_overlapped(reg_decode_kernel<KIND, T, NT, BLK, true>, grid, dim3(kThreads), smem, stream, p)
-                 : launch_overlapped(reg_decode_kernel<KIND, T, NT, BLK, false>, grid, dim3(kThreads), smem, stream, p);
+  return p.M > 8 ? launch_overlapped(DEFAULT_SPLIT, reg_decode_kernel<KIND, T, NT, BLK, true>, grid, dim3(kThreads), smem, stream, p)
+                 : launch_overlapped(DEFAULT_SPLIT, reg_decode_kernel<KIND, T, NT, BLK, false>, grid, dim3(kThreads), smem, stream, p);
 }
 
 template <int KIND, typename T>

@@ -480,7 +480,7 @@ cudaError_t launch_variant(const CUtensorMap& ta, const CUtensorMap& tb, const K
     if (e != cudaSuccess) return e;
     attr_set[dev] = true;
   }
-  return launch_clustered(plan.cluster, true, kern, plan.grid, kThreads, plan.smem_bytes, stream, ta,
+  return launch_clustered(MAX_SHARED, plan.cluster, true, kern, plan.grid, kThreads, plan.smem_bytes, stream, ta,
                           tb, kp);
 }
 

@@ -41,6 +41,9 @@ namespace {
 
 constexpr int kMidTok = 128;                     // UMMA M: token rows of a tile
 constexpr int kMidXTile = kMidTok * 128;         // bytes the UMMA reads per K block of activations
+// One CTA per SM, and room beside it for those of the quantiser that runs between two such kernels (1 KB each): with all
+// of the shared memory taken, a CTA waits for the quantiser to leave its SM (0.6B layer, 200 to 512 tokens, 1.5-2 %).
+constexpr int kMidSmemQuant = 218 * 1024;
 
 struct MidParams {
   int M, N;
@@ -351,7 +354,10 @@ double mid_cost(const MidPlan& pl, int M) {
   // both fit the GPU
   const double slots = static_cast<double>(sm_count()) * per_sm;
   us += 1.4 * std::min(1.0, std::max(0.0, (2.0 * ctas - slots) / slots));
-  return us + (per_sm == 1 ? 2.6 : 2.15) * (waves - 1);
+  us += (per_sm == 1 ? 2.6 : 2.15) * (waves - 1);
+  // Clusters that need several SMs at once, two CTAs on each, start late where the quantiser of the activations still
+  // has CTAs of its own (whole layers of the 8B model at 32 tokens 59.0 -> 55.5 us, at 20 56.7 -> 54.7, nothing else moved)
+  return pl.splits > 1 && ctas > sm_count() ? 1.15 * us : us;
 }
 
 bool search_plan(int M, int N, int K, MidPlan* best) {
@@ -363,7 +369,7 @@ bool search_plan(int M, int N, int K, MidPlan* best) {
     for (int s : {1, 2, 4, 8}) {
       if (want_s != 0 && s != want_s) continue;
       for (int kc : {4, 2, 1}) {
-        for (int cap : {kMidSmemOne, kMidSmemTwo}) {
+        for (int cap : {kMidSmemQuant, kMidSmemTwo}) {
           MidPlan pl;
           if (!mid_plan_for(M, N, k_blocks, bn, s, kc, cap, &pl)) continue;
           const double cost = mid_cost(pl, M);

@@ -538,7 +538,7 @@ cudaError_t launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUte
     if (e != cudaSuccess) return e;
     attr_set[dev] = true;
   }
-  return launch_overlapped(kern, grid, kThreads, smem, stream, ta, tb, ty, pp, sp);
+  return launch_overlapped(MAX_SHARED, kern, grid, kThreads, smem, stream, ta, tb, ty, pp, sp);
 }
 
 template <int KIND, typename OutT>

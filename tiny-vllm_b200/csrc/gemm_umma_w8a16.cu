@@ -375,7 +375,7 @@ cudaError_t launch_kernel(const CUtensorMap& tx, const CUtensorMap& tw, const Ke
     if (e != cudaSuccess) return e;
     attr_set[dev] = true;
   }
-  return launch_overlapped(kern, plan.grid, kThreads, plan.smem_bytes, stream, tx, tw, kp);
+  return launch_overlapped(MAX_SHARED, kern, plan.grid, kThreads, plan.smem_bytes, stream, tx, tw, kp);
 }
 
 }  // namespace

@@ -319,7 +319,7 @@ cudaError_t launch_ts(const CUtensorMap& tx, const CUtensorMap& tw, const TsPara
     if (e != cudaSuccess) return e;
     attr_set[dev] = true;
   }
-  return launch_overlapped(kern, grid, kTsThreads, kTsSmem, stream, tx, tw, tp);
+  return launch_overlapped(MAX_SHARED, kern, grid, kTsThreads, kTsSmem, stream, tx, tw, tp);
 }
 
 }  // namespace

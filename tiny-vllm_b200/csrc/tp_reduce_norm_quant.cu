@@ -249,7 +249,7 @@ cudaError_t launch_exchange_g(const ExchangeParams& p, cudaStream_t st) {
   const int resident = sm_count() * (dev < 64 ? per_sm[dev] : 1);
   const int row_blocks = (p.rows_per_rank + (256 / G) - 1) / (256 / G);
   const int grid = row_blocks < resident ? row_blocks : resident;
-  return launch_overlapped(kern, grid, 256, 0, st, p);
+  return launch_overlapped(DEFAULT_SPLIT, kern, grid, 256, 0, st, p);
 }
 
 template <typename T, int W>

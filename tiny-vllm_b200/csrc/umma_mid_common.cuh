@@ -149,7 +149,7 @@ cudaError_t launch_mid_kernel(int ctas, int splits, size_t smem, cudaStream_t st
     if (per_sm > 2) return cudaErrorInvalidConfiguration;
     if (dev < 64) attr_set[dev] = true;
   }
-  return launch_clustered(splits, true, kernel, dim3(ctas), dim3(kMidThreads), smem, stream, maps.x, maps.w,
+  return launch_clustered(MAX_SHARED, splits, true, kernel, dim3(ctas), dim3(kMidThreads), smem, stream, maps.x, maps.w,
                           maps.x3, maps.w3, mp);
 }
 
