@@ -24,13 +24,15 @@
 // Every mbarrier wait is bounded; the two cluster-wide hardware barriers (after set-up,
 // before tear-down) are reached by every thread on every path.
 //
-// The epilogue: sixteen warps, each 32 rows x 64 columns of a tile.  A warp takes its share of the accumulators
-// into registers at once and hands the TMEM buffer back before it converts anything, so the
-// MMAs of the tile after next never wait for stores.  Against eight warps with two column groups each
-// this gains where a pair has many short tiles and loses where it has two (8192 tokens, us before / now: 1024 -> 4096
-// 34.0 / 32.9, 1024 -> 6144 48.1 / 48.0, 4096 -> 4096 90.2 / 89.7, 4096 -> 6144 136.5 / 134.7, but 2048 -> 1024 17.9 / 18.4,
-// 3072 -> 1024 22.8 / 23.2): level over the projections of a layer.  Eighteen warps leave 96 registers a thread, and the
-// int8 instances spill (40 bytes stored, 68 loaded per thread with EPI_TMA).  Its output routes:
+// The epilogue: eight warps, each 32 rows x 128 columns of a tile, 32 at a time: the next 32 accumulators are on their
+// way while these are converted, and the TMEM buffer goes back to the issuer before the last 32 are.  The scales are
+// fetched a tile ahead.  (Sixteen warps that took 64 columns at once were no faster: 8192 x 4096 x 1024 34 us either way.)
+// What counts for the calls as a user makes them is what stands beside the kernel: ten warps of 128 registers and 194 KB
+// leave room on every SM for the CTAs of the kernel that quantises the activations, so that this one is set up, with its first
+// weights in the ring, when they are ready, and the next quantiser's CTAs are there when this one ends.  Quantiser and
+// GEMM, us before / now: 1999 tokens 1024 -> 4096 15.6 / 14.2, 1024 -> 6144 19.1 / 17.9; 1500 tokens 4096 -> 6144 33.5 / 31.8;
+// 700 tokens 4096 -> 24576 58.5 / 56.8; the 8192 tokens of the 0.6B layer 173 / 169.  Two slabs a warp and four stages: 14.4,
+// 18.0, 33.5, 61.0.  Its output routes:
 //   EPI_TMA     convert -> swizzled shared-memory slab -> one thread issues a TMA tensor store
 //               of the 32 x 64 box (this GPU's memory only); the epilogue warps never read the
 //               slab back and never issue a global store, and the stores drain while the warp waits for
@@ -60,9 +62,10 @@ constexpr int kBlockBytes = 128;              // bytes of K per pipeline stage =
 constexpr int kUmmaBytes = 32;                // bytes of K per tcgen05.mma (32 int8 / 16 halves)
 constexpr int kPairBN = 256;                  // N of the pair's UMMA
 constexpr int kStageBytes = 2 * kTileRows * kBlockBytes;  // 32 KB per CTA
-constexpr int kEpiWarps = 16;
+constexpr int kEpiWarps = 8;
 constexpr int kEpiThreads = kEpiWarps * 32;
 constexpr int kThreads = 64 + kEpiThreads;    // + warp 0 (TMA) + warp 1 (UMMA)
+constexpr int kRegThreads = 512;              // launch bound: 128 registers a thread
 constexpr int kSlabBytes = 32 * 128;          // 32 rows x 64 columns x 2 bytes
 constexpr int kScaleBytes = 2 * 256 * 4;      // channel scales of two tiles in flight
 constexpr int kCtrlBytes = 256;
@@ -258,7 +261,7 @@ __device__ __forceinline__ void store_row_i32(int32_t* out, int M, int N, int ro
 }
 
 template <int KIND, typename OutT, int EPI, bool SCATTER>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kRegThreads, 1)
 umma_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
                  const __grid_constant__ CUtensorMap tmap_b,
                  const __grid_constant__ CUtensorMap tmap_y, const PairParams pp,
@@ -409,13 +412,29 @@ umma_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
     // ------------------------------------------------------------ epilogue (both CTAs)
     const int epi_warp = warp - 2;
     const int quarter = warp & 3;      // the TMEM lane quarter this warp may read
-    const int c0 = (epi_warp >> 2) * 64;   // this warp's 64 columns of the tile
+    const int c0 = (epi_warp >> 2) * 128;  // this warp's 128 columns of the tile
     const int row_in_tile = quarter * 32 + lane;
     const int epi_tid = threadIdx.x - 64;
     uint8_t* slab = staging + epi_warp * (S::kSlabs * kSlabBytes);
     const uint32_t leader_tempty0 = ptx::map_to_cta(ptx::smem_u32(tempty_bar), 0);
     const OutT* bias = reinterpret_cast<const OutT*>(pp.bias);
+    // scales of a tile: the channels' in shared memory, this row's in a register; fetched a tile ahead
+    auto channel_scale = [&](int item) {
+      int tile_n, tile_m2;
+      item_to_tile<SCATTER>(item, pp, sp, &tile_n, &tile_m2);
+      const int col = tile_n * kPairBN + epi_tid;
+      return KIND != KIND_I8_RAW && col < pp.N ? __ldg(pp.w_scales + col) : 0.f;
+    };
+    auto row_scale = [&](int item) {
+      int tile_n, tile_m2;
+      item_to_tile<SCATTER>(item, pp, sp, &tile_n, &tile_m2);
+      const int row = (tile_m2 * 2 + static_cast<int>(rank)) * kTileRows + row_in_tile;
+      return KIND == KIND_I8 && row < pp.M ? ld_plain(pp.a_scales + row) : 0.f;
+    };
+    if (pair < total_items) s_ws[epi_tid] = channel_scale(pair);
     ptx::grid_dependency_wait();       // a_scales come from the previous kernel, out may be in use by it
+    float a_next = pair < total_items ? row_scale(pair) : 0.f;
+    ptx::named_bar_sync(2, kEpiThreads);
     int it = 0;
     for (int item = pair; item < total_items; item += num_pairs, ++it) {
       int tile_n, tile_m2;
@@ -423,13 +442,12 @@ umma_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
       const int tile_m = tile_m2 * 2 + static_cast<int>(rank);
       const int buf = it & 1;
       const uint32_t tphase = static_cast<uint32_t>(it >> 1) & 1u;
-      float* ws_tile = s_ws + buf * 256;
-      if (KIND != KIND_I8_RAW && epi_tid < kPairBN) {
-        const int col = tile_n * kPairBN + epi_tid;
-        ws_tile[epi_tid] = col < pp.N ? __ldg(pp.w_scales + col) : 0.f;
-      }
+      const float* ws_tile = s_ws + buf * 256;
       const int row = tile_m * kTileRows + row_in_tile;
-      const float a_s = (KIND == KIND_I8 && row < pp.M) ? ld_plain(pp.a_scales + row) : 0.f;
+      const float a_s = a_next;
+      const bool more = item + num_pairs < total_items;
+      const float ws_next = more ? channel_scale(item + num_pairs) : 0.f;
+      if (more) a_next = row_scale(item + num_pairs);
       OutT* out = reinterpret_cast<OutT*>(pp.out);
       if (SCATTER) {
         // this tile's rows belong to one owner: redirect the output there
@@ -437,57 +455,59 @@ umma_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
         out = reinterpret_cast<OutT*>(sp.stage[owner]) +
               static_cast<ptrdiff_t>(sp.rank - owner) * sp.rows_per_owner * pp.N;
       }
-      ptx::named_bar_sync(2, kEpiThreads);
       if (!ptx::mbar_wait(ptx::smem_u32(tfull_bar + buf), tphase, abort_flag)) break;
       ptx::tc_fence_after_sync();
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) +
-                             static_cast<uint32_t>(buf * kPairBN);
-      uint32_t va[32], vb[32];
-      ptx::tmem_ld_32x32b_x32(taddr + c0, va);
-      ptx::tmem_ld_32x32b_x32(taddr + c0 + 32, vb);
-      ptx::tmem_ld_wait();
-      // the accumulators are in registers: tell the leader's UMMA issuer (local or remote arrive)
-      ptx::tc_fence_before_sync();
-      ptx::mbar_arrive_cluster(leader_tempty0 + static_cast<uint32_t>(buf) * 8u);
+                             static_cast<uint32_t>(buf * kPairBN + c0);
       const int row0 = tile_m * kTileRows + quarter * 32;
-      const int col0 = tile_n * kPairBN + c0;
-      if (KIND == KIND_I8_RAW) {
-        if (!(pp.debug_flags & 4)) {
-          store_row_i32(reinterpret_cast<int32_t*>(pp.out), pp.M, pp.N, row, col0, va);
-          store_row_i32(reinterpret_cast<int32_t*>(pp.out), pp.M, pp.N, row, col0 + 32, vb);
+      uint32_t v[2][32];
+      ptx::tmem_ld_32x32b_x32(taddr, v[0]);
+      ptx::tmem_ld_wait();
+#pragma unroll
+      for (int g = 0; g < 4; ++g) {
+        // the next 32 accumulators are on their way while these are converted
+        if (g < 3) ptx::tmem_ld_32x32b_x32(taddr + 32 * (g + 1), v[(g + 1) & 1]);
+        const int col0 = tile_n * kPairBN + c0 + 32 * g;
+        if (KIND == KIND_I8_RAW) {
+          if (!(pp.debug_flags & 4)) store_row_i32(reinterpret_cast<int32_t*>(pp.out), pp.M, pp.N, row, col0, v[g & 1]);
+        } else if (!(pp.debug_flags & 1)) {
+          uint32_t packed[16];
+          if (bias != nullptr)
+            convert32<KIND, OutT, true>(ws_tile + c0 + 32 * g, a_s, bias, col0, pp.N, v[g & 1], packed);
+          else
+            convert32<KIND, OutT, false>(ws_tile + c0 + 32 * g, a_s, bias, col0, pp.N, v[g & 1], packed);
+          if (EPI == EPI_TMA && (g & 1) == 0) {
+            // the store issued from this slab before must have finished reading it
+            if (lane == 0) ptx::bulk_wait_group_read<0>();
+            __syncwarp();
+          }
+          park32(slab, lane, g & 1, packed);
+          if ((g & 1) != 0) {
+            if (EPI == EPI_TMA) {
+              ptx::fence_proxy_async_smem();
+              __syncwarp();
+              if (lane == 0) {
+                if (!(pp.debug_flags & 4) && row0 < pp.M && col0 - 32 < pp.N)
+                  ptx::tma_store_2d(&tmap_y, ptx::smem_u32(slab), (col0 - 32) * 2, row0);
+                ptx::bulk_commit_group();
+              }
+            } else {
+              __syncwarp();
+              if (!(pp.debug_flags & 4)) store_slab_rows<OutT>(out, pp.M, pp.N, slab, lane, row0, col0 - 32);
+              __syncwarp();
+            }
+          }
         }
-        continue;
-      }
-      if (pp.debug_flags & 1) continue;
-      uint32_t packed[16];
-      if (bias != nullptr)
-        convert32<KIND, OutT, true>(ws_tile + c0, a_s, bias, col0, pp.N, va, packed);
-      else
-        convert32<KIND, OutT, false>(ws_tile + c0, a_s, bias, col0, pp.N, va, packed);
-      if (EPI == EPI_TMA) {
-        // the store issued from the slab one tile ago must have finished reading it
-        if (lane == 0) ptx::bulk_wait_group_read<0>();
-        __syncwarp();
-      }
-      park32(slab, lane, 0, packed);
-      if (bias != nullptr)
-        convert32<KIND, OutT, true>(ws_tile + c0 + 32, a_s, bias, col0 + 32, pp.N, vb, packed);
-      else
-        convert32<KIND, OutT, false>(ws_tile + c0 + 32, a_s, bias, col0 + 32, pp.N, vb, packed);
-      park32(slab, lane, 1, packed);
-      if (EPI == EPI_TMA) {
-        ptx::fence_proxy_async_smem();
-        __syncwarp();
-        if (lane == 0) {
-          if (!(pp.debug_flags & 4) && row0 < pp.M && col0 < pp.N)
-            ptx::tma_store_2d(&tmap_y, ptx::smem_u32(slab), col0 * 2, row0);
-          ptx::bulk_commit_group();
+        if (g < 3) ptx::tmem_ld_wait();
+        if (g == 2) {
+          // the accumulators are in registers: tell the leader's UMMA issuer (local or remote arrive)
+          ptx::tc_fence_before_sync();
+          ptx::mbar_arrive_cluster(leader_tempty0 + static_cast<uint32_t>(buf) * 8u);
         }
-      } else {
-        __syncwarp();
-        if (!(pp.debug_flags & 4)) store_slab_rows<OutT>(out, pp.M, pp.N, slab, lane, row0, col0);
-        __syncwarp();
       }
+      // the other half of s_ws was last read a tile ago, before the barrier of that tile
+      s_ws[(buf ^ 1) * 256 + epi_tid] = ws_next;
+      ptx::named_bar_sync(2, kEpiThreads);
     }
     // shared memory must stay valid until the last TMA store has read it, and the output
     // must be complete when the kernel ends
