@@ -55,6 +55,8 @@ struct MidParams {
   int chunks_3d;           // chunks below this one come through the 3-D maps: one TMA instruction
   int splits;              // cluster size
   int stages, stage_bytes; // ring of chunks: activations and weights
+  int ring_bytes;          // the ring, or the output tile that lies over it at the end
+  int out_pitch;           // bytes of a token's row of that tile, 0: not through shared memory
   int tmem_cols;
   const float* a_scales;   // per token
   const float* w_scales;   // per channel
@@ -63,31 +65,30 @@ struct MidParams {
   int* status;
 };
 
-// Eight sums of one token row -> eight outputs, one 16-byte store (two for raw int32).
-template <bool RAW, typename T>
-__device__ __forceinline__ void store8(const MidParams& p, const uint32_t (&w)[8], float a_s,
-                                       const float* s_ws, const T* bias, int row, int col) {
-  const size_t at = static_cast<size_t>(row) * p.N + col;
-  if (RAW) {
-    uint4* dst = reinterpret_cast<uint4*>(static_cast<int32_t*>(p.out) + at);
-    dst[0] = make_uint4(w[0], w[1], w[2], w[3]);
-    dst[1] = make_uint4(w[4], w[5], w[6], w[7]);
-    return;
-  }
-  uint32_t packed[4];
+// Eight sums of one token row -> eight outputs.  Packed products round each half like the scalar instruction; the sums
+// with the bias are scalar, so that they are not contracted with them.
+template <typename T>
+__device__ __forceinline__ uint4 scale8(const uint32_t (&w)[8], float a_s, const float* s_ws, const T* bias, int col) {
+  const float4 c0 = *reinterpret_cast<const float4*>(s_ws), c1 = *reinterpret_cast<const float4*>(s_ws + 4);
+  const float2 c[4] = {{c0.x, c0.y}, {c0.z, c0.w}, {c1.x, c1.y}, {c1.z, c1.w}}, a2 = make_float2(a_s, a_s);
+  float2 v[4];
 #pragma unroll
-  for (int j = 0; j < 8; j += 2) {
-    float v[2];
+  for (int j = 0; j < 4; ++j)
+    v[j] = __fmul2_rn(__fmul2_rn(make_float2(static_cast<float>(static_cast<int>(w[2 * j])),
+                                             static_cast<float>(static_cast<int>(w[2 * j + 1]))), a2), c[j]);
+  if (bias != nullptr) {
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      v[h] = __fmul_rn(static_cast<float>(static_cast<int>(w[j + h])), a_s);
-      v[h] = __fmul_rn(v[h], s_ws[j + h]);
-      if (bias != nullptr) v[h] = __fadd_rn(v[h], to_float<T>(bias[col + j + h]));
-    }
-    packed[j / 2] = pack2_rn<T>(make_float2(v[0], v[1]));
+    for (int j = 0; j < 4; ++j)
+      v[j] = make_float2(__fadd_rn(v[j].x, to_float<T>(bias[col + 2 * j])), __fadd_rn(v[j].y, to_float<T>(bias[col + 2 * j + 1])));
   }
-  *reinterpret_cast<uint4*>(static_cast<T*>(p.out) + at) =
-      make_uint4(packed[0], packed[1], packed[2], packed[3]);
+  return make_uint4(pack2_rn<T>(v[0]), pack2_rn<T>(v[1]), pack2_rn<T>(v[2]), pack2_rn<T>(v[3]));
+}
+
+// Eight raw sums of a row.
+__device__ __forceinline__ void store8_raw(const MidParams& p, const uint32_t (&w)[8], int row, int col) {
+  uint4* dst = reinterpret_cast<uint4*>(static_cast<int32_t*>(p.out) + static_cast<size_t>(row) * p.N + col);
+  dst[0] = make_uint4(w[0], w[1], w[2], w[3]);
+  dst[1] = make_uint4(w[4], w[5], w[6], w[7]);
 }
 
 template <bool RAW, typename T>
@@ -96,7 +97,7 @@ w8a8_mid_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
                 const __grid_constant__ CUtensorMap tmap_x3, const __grid_constant__ CUtensorMap tmap_w3,
                 const MidParams p) {
   extern __shared__ __align__(1024) uint8_t smem[];
-  uint8_t* red = smem + p.stages * p.stage_bytes;     // [S][rows_own][bn] 32-bit sums (S > 1)
+  uint8_t* red = smem + p.ring_bytes;                 // [S][rows_own][bn] 32-bit sums (S > 1)
   const int rows_own = (min(kMidTok, p.x_rows) + p.splits - 1) / p.splits;   // token rows a CTA owns
   const int x_blk = p.x_rows * 128;                            // bytes of one K block of activations
   float* s_ws = reinterpret_cast<float*>(red + (p.splits > 1 ? p.splits * rows_own * p.bn * 4 : 0));
@@ -238,13 +239,41 @@ w8a8_mid_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
                           v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
           continue;
         }
-        // no split: straight from the registers, 8 channels (16 bytes) at a time
+        // no split.  Wide tiles go through shared memory (over the ring, which is done with: the MMAs that read the
+        // last of it have completed); of a narrow one, and of raw sums, a thread stores its pieces of a row itself
 #pragma unroll
         for (int j = 0; j < 32; j += 8) {
           const int col = tile_n * p.bn + c * 32 + j;
           if (col >= p.N) break;         // N % 8 == 0
           const uint32_t w[8] = {v[j], v[j + 1], v[j + 2], v[j + 3], v[j + 4], v[j + 5], v[j + 6], v[j + 7]};
-          store8<RAW, T>(p, w, a_s, s_ws + c * 32 + j, bias, grow, col);
+          if (RAW) {
+            store8_raw(p, w, grow, col);
+          } else {
+            const uint4 o = scale8<T>(w, a_s, s_ws + c * 32 + j, bias, col);
+            if (p.out_pitch > 0)
+              *reinterpret_cast<uint4*>(smem + row * p.out_pitch + (c * 32 + j) * 2) = o;
+            else
+              *reinterpret_cast<uint4*>(static_cast<T*>(p.out) + static_cast<size_t>(grow) * p.N + col) = o;
+          }
+        }
+      }
+    }
+    if (!RAW && p.out_pitch > 0) {
+      // out in whole rows, 16 bytes a thread
+      ptx::named_bar_sync(1, 256);
+      const int shift = __ffs(p.bn) - 4, pieces = 1 << shift;     // 16-byte pieces of a row
+      const int sub = tid & (pieces - 1), n0 = tile_n * p.bn + sub * 8, step = 256 >> shift;
+      const int rows = min(kMidTok, p.M - tile_m * kMidTok);
+      if (done && n0 < p.N) {
+        T* out = static_cast<T*>(p.out) + static_cast<size_t>(tile_m * kMidTok) * p.N + n0;
+        for (int r0 = tid >> shift; r0 < rows; r0 += 4 * step) {
+          uint4 v[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (r0 + j * step < rows) v[j] = *reinterpret_cast<const uint4*>(smem + (r0 + j * step) * p.out_pitch + sub * 16);
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (r0 + j * step < rows) *reinterpret_cast<uint4*>(out + static_cast<size_t>(r0 + j * step) * p.N) = v[j];
         }
       }
     }
@@ -287,7 +316,11 @@ w8a8_mid_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
         for (int j = 0; j < 8; ++j)
           w[j] += in[j];
       }
-      store8<RAW, T>(p, w, s_as[row], s_ws + cg * 8, bias, grow, col);
+      if (RAW)
+        store8_raw(p, w, grow, col);
+      else
+        *reinterpret_cast<uint4*>(static_cast<T*>(p.out) + static_cast<size_t>(grow) * p.N + col) =
+            scale8<T>(w, s_as[row], s_ws + cg * 8, bias, col);
     }
   }
   if (threadIdx.x == 0 && *abort_flag != 0)
@@ -300,7 +333,7 @@ w8a8_mid_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
 namespace {
 
 struct MidPlan {
-  int bn, x_rows, splits, kc, chunks, chunks_per_split, tiles_m, tiles_n, stages, stage_bytes;
+  int bn, x_rows, splits, kc, chunks, chunks_per_split, tiles_m, tiles_n, stages, stage_bytes, ring_bytes, out_pitch;
   size_t smem;
 };
 
@@ -323,8 +356,15 @@ bool mid_plan_for(int M, int N, int k_blocks, int bn, int splits, int kc,
   fixed = std::max(fixed, (kc - 1) * pl->x_rows * 128 + kMidXTile - pl->stage_bytes);
   pl->stages = std::min({(smem_cap - fixed) / pl->stage_bytes, kMidMaxStages, pl->chunks_per_split});
   if (pl->stages < 1 || (pl->stages < 2 && pl->chunks_per_split > 1)) return false;
-  pl->smem = static_cast<size_t>(pl->stages) * pl->stage_bytes + fixed;
-  return true;
+  // A thread's pieces of a row fill whole lines where the tile is narrow, and few rows are soon stored (64 tokens, 4096 x
+  // 1024 in tiles of 32 channels 3.7 us, 4.0 through shared memory); larger tiles are stored by rows (256 tokens, 6144 x
+  // 1024 in tiles of 128 5.9 -> 5.4 us, 128 tokens, 24576 x 4096 25.2 -> 23.8, one eighth of the 8B model at 256 tokens, in tiles of
+  // 64, 37.5 -> 36.8 a layer)
+  const bool by_rows = splits == 1 && (bn >= 128 || (bn == 64 && 4 * M >= 3 * kMidTok));
+  pl->out_pitch = by_rows ? bn * 2 + 16 : 0;   // + 16: rows on different banks
+  pl->ring_bytes = std::max(pl->stages * pl->stage_bytes, pl->x_rows * pl->out_pitch);
+  pl->smem = static_cast<size_t>(pl->ring_bytes) + fixed;
+  return pl->smem <= static_cast<size_t>(smem_cap);
 }
 
 // Predicted time of one call in a stream of such calls, in microseconds.  The form follows what the
@@ -428,6 +468,8 @@ int launch_umma_mid(const GemmArgs& a) {
   mp.splits = pl.splits;
   mp.stages = pl.stages;
   mp.stage_bytes = pl.stage_bytes;
+  mp.ring_bytes = pl.ring_bytes;
+  mp.out_pitch = pl.out_pitch;
   mp.tmem_cols = pl.bn;
   mp.a_scales = a.a_scales;
   mp.w_scales = a.w_scales;
