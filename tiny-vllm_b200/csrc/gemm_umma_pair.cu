@@ -529,19 +529,39 @@ umma_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
   }
 }
 
-// int8 [n] -> T [n], exact (|q| <= 128 has at most 8 significant bits).  16 codes per thread.
-template <typename T>
-__global__ void __launch_bounds__(256) w8a16_expand_kernel(const int8_t* __restrict__ q,
-                                                           T* __restrict__ out, size_t n16) {
-  const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
-  for (size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n16; i += stride) {
-    const uint4 w = __ldg(reinterpret_cast<const uint4*>(q) + i);
-    const uint2 e0 = expand4<T>(w.x), e1 = expand4<T>(w.y), e2 = expand4<T>(w.z),
-                e3 = expand4<T>(w.w);
-    uint4* dst = reinterpret_cast<uint4*>(out) + 2 * i;
+// int8 [n] -> T [n], exact (|q| <= 128 has at most 8 significant bits).  HBM-bound: 3 bytes of traffic a weight.  Sixteen codes
+// a thread, one load and one 32-byte store (two of 16 where the workspace is not on a 32-byte boundary), as many CTAs as
+// that takes: 24576 x 4096 47.5 us = 0.99 of the copy rate, 4096 x 4096 8.5, 6144 x 1024 4.5.  (A grid of 8 CTAs per SM that
+// went over the matrix with two 16-byte stores, which leave every 32-byte sector to the second: 65.9, 13.1, 6.5.)
+// The codes are constants and loaded ahead of the wait for the kernel that may still read the previous call's expansion;
+// the GEMM behind it may set itself up at once, it waits before it touches the weights.
+template <typename T, bool WIDE>
+__global__ void __launch_bounds__(256) w8a16_expand_kernel(const int8_t* __restrict__ q, T* out, size_t n16) {
+  const size_t i = static_cast<size_t>(blockIdx.x) * 256 + threadIdx.x;
+  uint4 w = make_uint4(0u, 0u, 0u, 0u);
+  if (i < n16) w = __ldcs(reinterpret_cast<const uint4*>(q) + i);
+  ptx::grid_launch_dependents();
+  ptx::grid_dependency_wait();
+  if (i >= n16) return;
+  const uint2 e0 = expand4<T>(w.x), e1 = expand4<T>(w.y), e2 = expand4<T>(w.z), e3 = expand4<T>(w.w);
+  uint4* dst = reinterpret_cast<uint4*>(out) + 2 * i;
+  if (WIDE) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(e0.x), "r"(e0.y), "r"(e1.x),
+                 "r"(e1.y), "r"(e2.x), "r"(e2.y), "r"(e3.x), "r"(e3.y)
+                 : "memory");
+  } else {
     dst[0] = make_uint4(e0.x, e0.y, e1.x, e1.y);
     dst[1] = make_uint4(e2.x, e2.y, e3.x, e3.y);
   }
+}
+
+template <typename T>
+cudaError_t launch_expand(const int8_t* q, void* out, size_t n16, cudaStream_t stream) {
+  const unsigned blocks = static_cast<unsigned>((n16 + 255) / 256);
+  T* dst = static_cast<T*>(out);
+  return reinterpret_cast<uintptr_t>(out) % 32 == 0
+             ? launch_overlapped(MAX_SHARED, w8a16_expand_kernel<T, true>, dim3(blocks), dim3(256), 0, stream, q, dst, n16)
+             : launch_overlapped(MAX_SHARED, w8a16_expand_kernel<T, false>, dim3(blocks), dim3(256), 0, stream, q, dst, n16);
 }
 
 template <int KIND, typename OutT, int EPI, bool SCATTER = false>
@@ -709,13 +729,8 @@ int launch_w8a16_umma_pair(const GemmArgs& a) {
   const bool bf16 = a.dtype == B200Q_DTYPE_BF16;
   void* expanded = static_cast<uint8_t*>(a.workspace) + kCounterBytes;
   const size_t n16 = static_cast<size_t>(a.N) * a.K / 16;
-  const int blocks = static_cast<int>(std::min<size_t>((n16 + 255) / 256, static_cast<size_t>(sm_count()) * 8));
-  if (bf16)
-    w8a16_expand_kernel<__nv_bfloat16><<<blocks, 256, 0, a.stream>>>(
-        a.w, static_cast<__nv_bfloat16*>(expanded), n16);
-  else
-    w8a16_expand_kernel<__half><<<blocks, 256, 0, a.stream>>>(a.w, static_cast<__half*>(expanded), n16);
-  cudaError_t e = cudaGetLastError();
+  const cudaError_t e = bf16 ? launch_expand<__nv_bfloat16>(a.w, expanded, n16, a.stream)
+                             : launch_expand<__half>(a.w, expanded, n16, a.stream);
   if (e != cudaSuccess) return finish(e);
 
   CUtensorMap ta, tb, ty;
