@@ -99,3 +99,21 @@ def test_w8a16_beyond_the_mid_sizes_takes_the_tensor_memory_kernel(M, N, K):
     m = O.tensor_metrics(O.w8a16_native_reference(x, q, s, None), y)
     assert m["relative_l2"] <= 4e-3 and m["cosine_similarity"] >= 0.9999, m
     assert device_status_ok()
+
+
+@pytest.mark.parametrize("M,N,K,pair", [(513, 16384, 1040, True), (700, 12296, 2064, True), (1023, 9728, 2560, True),
+                                        (513, 22016, 1024, False), (830, 9728, 2560, False), (512, 16384, 1040, False)])
+def test_w8a16_513_to_1023_tokens_expand_once_where_that_costs_no_round(M, N, K, pair):
+    expect = "umma_f16_pair_expand_once_tokens256" if pair else "umma_f16_tmem_weights_channels256"
+    assert select_path(_lib.OP_W8A16, M, N, K) == expect
+    q, s = O.make_weight(N, K, seed=N + K)
+    x = O.make_activation(M, K, seed=M, dtype=torch.bfloat16)
+    b = (torch.randn(N, generator=torch.Generator().manual_seed(M)) * 0.1).to(torch.bfloat16)
+    dev = [t.cuda() for t in (x, q, s, b)]
+    y = apply_int8_weight_only_linear(*dev)
+    m = O.tensor_metrics(O.w8a16_native_reference(x, q, s, b), y)
+    assert m["relative_l2"] <= 4e-3 and m["cosine_similarity"] >= 0.9999, m
+    with knobs(W8A16_PAIR_MIN_M=1024):          # the route of a call without a workspace: sums in another order
+        y_ts = apply_int8_weight_only_linear(*dev)
+    assert O.tensor_metrics(y_ts, y)["relative_l2"] <= 2e-3
+    assert device_status_ok()

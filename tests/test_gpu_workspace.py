@@ -72,7 +72,31 @@ assert torch.equal(y, expect)
 """
 
 
-@pytest.mark.parametrize("body", [NEEDS_NONE, NEEDS_SOME, OUTGROWN], ids=["needs-none", "needs-some", "outgrown"])
+ITS_OWN = """
+x, q, s = problem(700, 24576, 2048)        # W8A16 at 513 to 1023 tokens: a buffer of each call's own
+fn = lambda: apply_int8_weight_only_linear(x, q, s)
+torch.cuda.synchronize()
+graph, y = captured(fn)                    # from the capture's pool, without a call before it
+graph.replay()
+torch.cuda.synchronize()
+expect = fn()
+assert torch.equal(y, expect)
+x2, q2, s2 = problem(700, 24576, 2064)
+expect2 = apply_int8_weight_only_linear(x2, q2, s2)
+a, b = torch.cuda.Stream(), torch.cuda.Stream()
+torch.cuda.synchronize()
+for _ in range(20):                        # two streams at once do not share it
+    with torch.cuda.stream(a):
+        ya = fn()
+    with torch.cuda.stream(b):
+        yb = apply_int8_weight_only_linear(x2, q2, s2)
+    torch.cuda.synchronize()
+    assert torch.equal(ya, expect) and torch.equal(yb, expect2)
+"""
+
+
+@pytest.mark.parametrize("body", [NEEDS_NONE, NEEDS_SOME, OUTGROWN, ITS_OWN],
+                         ids=["needs-none", "needs-some", "outgrown", "its-own"])
 def test_capture_in_a_fresh_process(body):
     r = subprocess.run([sys.executable, "-c", HEAD + body], cwd=ROOT, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout + r.stderr
