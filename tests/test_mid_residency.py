@@ -1,5 +1,8 @@
 """Plans of the tcgen05 kernels for tens to hundreds of tokens (host code, no GPU).  A CTA of a cluster that waits for
 tensor memory held by another such CTA never ends, so the ones that fit an SM together may not need more than it has."""
+import re
+from pathlib import Path
+
 import pytest
 
 from tests.gpu_util import knobs, mid_plan
@@ -9,6 +12,9 @@ from tiny_vllm_b200 import _lib, build as b200_build
 SM_SHARED, CTA_RESERVED = 228 * 1024, 1024    # bytes per SM; bytes the runtime adds to every CTA
 SM_COLUMNS = 512                              # of tensor memory
 MAX_CTAS = 2                                  # of these kernels on an SM, by registers
+
+COMMON = (Path(__file__).resolve().parent.parent / "tiny-vllm_b200" / "csrc" / "common.h").read_text()
+PAIR_SHARED = int(re.search(r"kPairSmem = (\d+) \* 1024", COMMON).group(1)) * 1024    # the CTA-pair kernel, all 512 columns
 
 TOKENS = [1, 8, 16, 17, 24, 33, 40, 48, 64, 77, 96, 128, 129, 200, 256, 384, 512, 700, 1024, 1500, 2048]
 CHANNELS = [8, 72, 128, 264, 440, 512, 640, 768, 1024, 1536, 2048, 3072, 3968, 4096, 6144, 9728, 12288, 24576]
@@ -35,4 +41,5 @@ def test_clusters_never_wait_for_tensor_memory(op, forced):
                     assert fit >= 1 and fit * p["columns"] <= SM_COLUMNS, (M, N, K, p)
                     left = SM_SHARED - p["shared"] - CTA_RESERVED
                     assert p["columns"] <= SM_COLUMNS // 2 or left <= CTA_RESERVED, (M, N, K, p)
+                    assert p["shared"] + PAIR_SHARED + 2 * CTA_RESERVED > SM_SHARED, (M, N, K, p)
     assert seen > 50

@@ -50,6 +50,14 @@ struct UmmaPlan {
 
 constexpr size_t kCounterBytes = 16384;  // zero-initialised tile counters at workspace start
 
+// Shared memory of an SM, and what a CTA takes beyond its own.  The CTA-pair kernel allocates all of an SM's tensor memory
+// for a cluster, so no CTA of another cluster that allocates some may be beside it (the residency rule of
+// umma_mid_common.cuh): it asks for kPairSmem, and such a CTA for kClusterSmemMin at least.  The 9 KB that are left hold the
+// CTAs of the kernels that quantise activations.
+constexpr int kSmSharedBytes = 228 * 1024, kCtaSharedExtra = 1024;
+constexpr int kPairSmem = 218 * 1024, kClusterSmemMin = 12 * 1024;
+static_assert(kPairSmem + kClusterSmemMin + 2 * kCtaSharedExtra > kSmSharedBytes, "a cluster beside the CTA-pair kernel");
+
 // Number of SMs of the current device (cached).
 int sm_count();
 

@@ -364,6 +364,7 @@ bool mid_plan_for(int M, int N, int k_blocks, int bn, int splits, int kc,
   pl->out_pitch = by_rows ? bn * 2 + 16 : 0;   // + 16: rows on different banks
   pl->ring_bytes = std::max(pl->stages * pl->stage_bytes, pl->x_rows * pl->out_pitch);
   pl->smem = static_cast<size_t>(pl->ring_bytes) + fixed;
+  if (splits > 1) pl->smem = std::max<size_t>(pl->smem, kClusterSmemMin);
   return pl->smem <= static_cast<size_t>(smem_cap);
 }
 

@@ -420,7 +420,7 @@ bool mid_plan_for(int M, int N, int k_blocks, int bt, int rows, int splits, int 
   pl->smem = static_cast<size_t>(pl->ring_bytes) + fixed;
   if (pl->smem > static_cast<size_t>(smem_cap)) return false;
   // no other CTA of a cluster fits beside it (see the residency rule in umma_mid_common.cuh)
-  if (splits > 1 && pl->tmem_cols > 256) pl->smem = kMidSmemOne;
+  if (splits > 1) pl->smem = pl->tmem_cols > 256 ? kMidSmemOne : std::max<size_t>(pl->smem, kClusterSmemMin);
   return true;
 }
 

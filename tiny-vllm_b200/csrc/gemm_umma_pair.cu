@@ -27,8 +27,8 @@
 // The epilogue: eight warps, each 32 rows x 128 columns of a tile, 32 at a time: the next 32 accumulators are on their
 // way while these are converted, and the TMEM buffer goes back to the issuer before the last 32 are.  The scales are
 // fetched a tile ahead.  (Sixteen warps that took 64 columns at once were no faster: 8192 x 4096 x 1024 34 us either way.)
-// What counts for the calls as a user makes them is what stands beside the kernel: ten warps of 128 registers and 194 KB
-// leave room on every SM for the CTAs of the kernel that quantises the activations, so that this one is set up, with its first
+// What counts for the calls as a user makes them is what stands beside the kernel: ten warps of 128 registers and 218 KB (of
+// which it needs 194: kPairSmem) leave room on every SM for the CTAs of the kernel that quantises the activations, so that this one is set up, with its first
 // weights in the ring, when they are ready, and the next quantiser's CTAs are there when this one ends.  Quantiser and
 // GEMM, us before / now: 1999 tokens 1024 -> 4096 15.6 / 14.2, 1024 -> 6144 19.1 / 17.9; 1500 tokens 4096 -> 6144 33.5 / 31.8;
 // 700 tokens 4096 -> 24576 58.5 / 56.8; the 8192 tokens of the 0.6B layer 173 / 169.  Two slabs a warp and four stages: 14.4,
@@ -80,7 +80,8 @@ struct Shape {
   static constexpr int kSlabs = EPI == EPI_DIRECT ? 0 : 1;  // per warp
   static constexpr int kStages = EPI == EPI_DIRECT ? 7 : 5;
   static constexpr int kStagingBytes = kEpiWarps * kSlabs * kSlabBytes;
-  static constexpr int kSmem = kStages * kStageBytes + kStagingBytes + kScaleBytes + kCtrlBytes;
+  static constexpr int kUsed = kStages * kStageBytes + kStagingBytes + kScaleBytes + kCtrlBytes;
+  static constexpr int kSmem = kUsed > kPairSmem ? kUsed : kPairSmem;   // (the residency rule, see kPairSmem)
   static_assert(kSmem <= 227 * 1024, "shared memory budget");
 };
 

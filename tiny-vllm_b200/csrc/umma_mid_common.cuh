@@ -17,8 +17,8 @@ namespace b200q {
 //   * a CTA of a cluster has at most 256 columns, or it takes the shared memory of a whole SM (kMidSmemOne: beside it there
 //     is room for no kernel with dynamic shared memory).
 // A CTA without a cluster may wait for columns: who holds them ends without it.  The other kernels that allocate
-// tensor memory for clusters are alone on their SM: umma_pair_kernel by its shared memory, the clustered
-// w8a8_umma_kernel by its registers.
+// tensor memory for clusters are alone on their SM: umma_pair_kernel by its shared memory (kPairSmem and kClusterSmemMin
+// in common.h), the clustered w8a8_umma_kernel by its registers and its shared memory.
 constexpr int kMidThreads = 352;
 constexpr int kMidMaxStages = 12;
 constexpr int kMidCtrlBytes = 768;
