@@ -14,7 +14,8 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("writer", ["quantiser", "copy", "torch"])
 @pytest.mark.parametrize("scheme", ["w8a8", "w8a16"])
 @pytest.mark.parametrize("M,N,K", [(1, 1024, 1024), (8, 4096, 1024), (16, 6144, 4096), (40, 1024, 3072),
-                                   (300, 4096, 1024), (700, 6144, 4096), (8, 24576, 4096)])
+                                   (300, 4096, 1024), (700, 6144, 4096), (8, 24576, 4096),
+                                   (1100, 2048, 2048), (1, 6144, 4096)])
 def test_weights_written_by_the_work_ahead(M, N, K, scheme, writer):
     gen = torch.Generator(device="cuda").manual_seed(M + N + K)
     x = torch.randn(M, K, device="cuda", generator=gen).to(torch.bfloat16)

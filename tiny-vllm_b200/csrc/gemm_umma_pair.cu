@@ -436,6 +436,7 @@ umma_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
     ptx::grid_dependency_wait();       // a_scales come from the previous kernel, out may be in use by it
     float a_next = pair < total_items ? row_scale(pair) : 0.f;
     ptx::named_bar_sync(2, kEpiThreads);
+    bool alive = true;
     int it = 0;
     for (int item = pair; item < total_items; item += num_pairs, ++it) {
       int tile_n, tile_m2;
@@ -456,16 +457,21 @@ umma_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
         out = reinterpret_cast<OutT*>(sp.stage[owner]) +
               static_cast<ptrdiff_t>(sp.rank - owner) * sp.rows_per_owner * pp.N;
       }
-      if (!ptx::mbar_wait(ptx::smem_u32(tfull_bar + buf), tphase, abort_flag)) break;
+      // a warp whose wait ran out goes on to meet the others at the barrier of each tile
+      if (alive) alive = ptx::mbar_wait(ptx::smem_u32(tfull_bar + buf), tphase, abort_flag);
+      alive = __all_sync(0xFFFFFFFFu, alive);
       ptx::tc_fence_after_sync();
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) +
                              static_cast<uint32_t>(buf * kPairBN + c0);
       const int row0 = tile_m * kTileRows + quarter * 32;
       uint32_t v[2][32];
-      ptx::tmem_ld_32x32b_x32(taddr, v[0]);
-      ptx::tmem_ld_wait();
+      if (alive) {
+        ptx::tmem_ld_32x32b_x32(taddr, v[0]);
+        ptx::tmem_ld_wait();
+      }
 #pragma unroll
       for (int g = 0; g < 4; ++g) {
+        if (!alive) break;
         // the next 32 accumulators are on their way while these are converted
         if (g < 3) ptx::tmem_ld_32x32b_x32(taddr + 32 * (g + 1), v[(g + 1) & 1]);
         const int col0 = tile_n * kPairBN + c0 + 32 * g;
