@@ -200,7 +200,7 @@ w8a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_a,
       if (clustered && split > 0) {
         // K split over the cluster: hand this CTA's partial tile (exact int32 sums) to the
         // leader (cluster rank 0 = split 0) through its shared memory, [split - 1][column][row]
-        if (!ptx::mbar_wait(ptx::smem_u32(tfull_bar + buf), tphase, abort_flag)) break;
+        if (!ptx::warp_all(ptx::mbar_wait(ptx::smem_u32(tfull_bar + buf), tphase, abort_flag))) break;
         ptx::tc_fence_after_sync();
         const uint32_t taddr_p = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) +
                                  static_cast<uint32_t>(buf * p.bn);
@@ -230,8 +230,8 @@ w8a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_a,
         if (row < p.rows_a) a_s = p.a_scales[row];   // (not __ldg: the previous kernel writes it)
         ptx::named_bar_sync(2, kEpiThreads);
       }
-      if (!ptx::mbar_wait(ptx::smem_u32(tfull_bar + buf), tphase, abort_flag)) break;
-      if (clustered && !ptx::mbar_wait_cluster(ptx::smem_u32(pfull_bar), 0u, abort_flag)) break;
+      if (!ptx::warp_all(ptx::mbar_wait(ptx::smem_u32(tfull_bar + buf), tphase, abort_flag))) break;
+      if (clustered && !ptx::warp_all(ptx::mbar_wait_cluster(ptx::smem_u32(pfull_bar), 0u, abort_flag))) break;
       ptx::tc_fence_after_sync();
       const uint32_t taddr =
           tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(buf * p.bn);

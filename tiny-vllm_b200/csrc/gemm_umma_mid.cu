@@ -170,8 +170,8 @@ w8a8_mid_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
       uint32_t phase = 0;
       bool ok = true;
       for (int i = 0; i < n_ch; ++i) {
-        if (!ptx::mbar_wait(ptx::smem_u32(wfull + stage), phase, abort_flag) ||
-            !ptx::mbar_wait(ptx::smem_u32(xfull + stage), phase, abort_flag)) {
+        if (!ptx::warp_all(ptx::mbar_wait(ptx::smem_u32(wfull + stage), phase, abort_flag) &&
+                           ptx::mbar_wait(ptx::smem_u32(xfull + stage), phase, abort_flag))) {
           ok = false;
           break;
         }
@@ -219,8 +219,7 @@ w8a8_mid_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
     // ------------------------------------------------ partial sums -> the rows' owners
     if (p.splits > 1) cluster_wait();    // every CTA of the cluster runs: its memory may be written
     else ptx::named_bar_sync(1, 256);             // s_ws complete
-    bool done = run && ptx::mbar_wait(ptx::smem_u32(tfull), 0u, abort_flag);
-    done = __all_sync(0xFFFFFFFFu, done);
+    const bool done = run && ptx::warp_all(ptx::mbar_wait(ptx::smem_u32(tfull), 0u, abort_flag));
     if (done) {
       ptx::tc_fence_after_sync();
       const int shift = __ffs(p.splits) - 1;

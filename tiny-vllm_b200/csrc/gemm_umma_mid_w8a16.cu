@@ -154,8 +154,8 @@ w8a16_mid_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
       uint32_t phase = 0, aphase = 0;
       bool ok = true;
       for (int i = 0; i < n_ch; ++i) {
-        if (!ptx::mbar_wait(ptx::smem_u32(cfull + as), aphase, abort_flag) ||
-            !ptx::mbar_wait(ptx::smem_u32(xfull + stage), phase, abort_flag)) {
+        if (!ptx::warp_all(ptx::mbar_wait(ptx::smem_u32(cfull + as), aphase, abort_flag) &&
+                           ptx::mbar_wait(ptx::smem_u32(xfull + stage), phase, abort_flag))) {
           ok = false;
           break;
         }
@@ -205,9 +205,10 @@ w8a16_mid_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
       const int sw8 = (min(ch, p.rows - 1) >> 1) & 3;          // rows % 8 == 0: the same in every block
       int rs = group, as = group;
       uint32_t rphase = 0, aphase = 1;
+      bool ok = true;
       for (int i = group; i < n_ch; i += 2) {
-        if (!ptx::mbar_wait(ptx::smem_u32(wfull + rs), rphase, abort_flag)) break;
-        if (i >= p.a_stages && !ptx::mbar_wait(ptx::smem_u32(aempty + as), aphase, abort_flag)) break;
+        if (!ptx::mbar_wait(ptx::smem_u32(wfull + rs), rphase, abort_flag)) ok = false;
+        if (i >= p.a_stages && !ptx::mbar_wait(ptx::smem_u32(aempty + as), aphase, abort_flag)) ok = false;
         ptx::tc_fence_after_sync();
         // rows beyond the tile's last: what they hold only reaches accumulator lanes nobody reads
         const uint8_t* src = smem + raw_base + rs * p.raw_bytes + min(ch, p.rows - 1) * kRow8;
@@ -231,7 +232,7 @@ w8a16_mid_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
         ptx::tmem_st_wait();
         ptx::tc_fence_before_sync();
         __syncwarp();
-        if (lane == 0) {
+        if (lane == 0 && ok) {
           ptx::mbar_arrive(ptx::smem_u32(cfull + as));
           ptx::mbar_arrive(ptx::smem_u32(rempty + rs));
         }
@@ -250,8 +251,7 @@ w8a16_mid_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
     // every CTA of the cluster runs: its memory may be written / scales of this CTA complete
     if (p.splits > 1) cluster_wait();
     else ptx::named_bar_sync(1, 256);
-    bool done = run && ptx::mbar_wait(ptx::smem_u32(tfull), 0u, abort_flag);
-    done = __all_sync(0xFFFFFFFFu, done);
+    const bool done = run && ptx::warp_all(ptx::mbar_wait(ptx::smem_u32(tfull), 0u, abort_flag));
     if (done) {
       ptx::tc_fence_after_sync();
       const T* bias = reinterpret_cast<const T*>(p.bias);

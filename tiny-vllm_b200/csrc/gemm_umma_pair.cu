@@ -458,8 +458,7 @@ umma_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
               static_cast<ptrdiff_t>(sp.rank - owner) * sp.rows_per_owner * pp.N;
       }
       // a warp whose wait ran out goes on to meet the others at the barrier of each tile
-      if (alive) alive = ptx::mbar_wait(ptx::smem_u32(tfull_bar + buf), tphase, abort_flag);
-      alive = __all_sync(0xFFFFFFFFu, alive);
+      if (alive) alive = ptx::warp_all(ptx::mbar_wait(ptx::smem_u32(tfull_bar + buf), tphase, abort_flag));
       ptx::tc_fence_after_sync();
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) +
                              static_cast<uint32_t>(buf * kPairBN + c0);

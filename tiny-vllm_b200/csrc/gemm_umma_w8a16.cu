@@ -204,8 +204,8 @@ w8a16_umma_kernel(const __grid_constant__ CUtensorMap tmap_x,
       const int kb0 = split * p.kb_per_split;
       const int kb1 = min(p.k_blocks, kb0 + p.kb_per_split);
       for (int kb = kb0; kb < kb1; ++kb) {
-        if (!ptx::mbar_wait(ptx::smem_u32(full_bar + stage), phase, abort_flag) ||
-            !ptx::mbar_wait(ptx::smem_u32(cempty_bar + cb), cphase ^ 1u, abort_flag)) {
+        if (!ptx::warp_all(ptx::mbar_wait(ptx::smem_u32(full_bar + stage), phase, abort_flag) &&
+                           ptx::mbar_wait(ptx::smem_u32(cempty_bar + cb), cphase ^ 1u, abort_flag))) {
           ok = false;
           break;
         }
@@ -257,7 +257,7 @@ w8a16_umma_kernel(const __grid_constant__ CUtensorMap tmap_x,
         }
         ptx::named_bar_sync(2, kEpiThreads);
       }
-      if (!ptx::mbar_wait(ptx::smem_u32(tfull_bar + buf), tphase, abort_flag)) break;
+      if (!ptx::warp_all(ptx::mbar_wait(ptx::smem_u32(tfull_bar + buf), tphase, abort_flag))) break;
       ptx::tc_fence_after_sync();
       const uint32_t taddr =
           tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(buf * p.bn);

@@ -209,8 +209,8 @@ w8a16_umma_ts_kernel(const __grid_constant__ CUtensorMap tmap_x,
         if (static_cast<int>(blk & 1u) != group) continue;
         const uint32_t stage = blk % kTsStages, phase = (blk / kTsStages) & 1u;
         const uint32_t as = blk % kTsAStages, aphase = (blk / kTsAStages) & 1u;
-        if (!ptx::mbar_wait(ptx::smem_u32(full_bar + stage), phase, abort_flag) ||
-            !ptx::mbar_wait(ptx::smem_u32(aempty_bar + as), aphase ^ 1u, abort_flag)) {
+        if (!ptx::warp_all(ptx::mbar_wait(ptx::smem_u32(full_bar + stage), phase, abort_flag) &&
+                           ptx::mbar_wait(ptx::smem_u32(aempty_bar + as), aphase ^ 1u, abort_flag))) {
           ok = false;
           break;
         }
@@ -256,7 +256,7 @@ w8a16_umma_ts_kernel(const __grid_constant__ CUtensorMap tmap_x,
     for (int item = blockIdx.x; item < total_items; item += gridDim.x, ++it) {
       const int tile_ch = item % p.tiles_ch;
       const int tile_tok = item / p.tiles_ch;
-      if (!ptx::mbar_wait(ptx::smem_u32(tfull_bar), static_cast<uint32_t>(it) & 1u, abort_flag)) break;
+      if (!ptx::warp_all(ptx::mbar_wait(ptx::smem_u32(tfull_bar), static_cast<uint32_t>(it) & 1u, abort_flag))) break;
       ptx::tc_fence_after_sync();
       const int ch0 = tile_ch * kTsChannels + t * kTileA;       // first channel of this A tile
       const int ch = ch0 + quarter * 32 + lane;

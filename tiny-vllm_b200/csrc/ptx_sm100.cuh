@@ -72,6 +72,11 @@ constexpr long long kWaitLimitCycles = 2000000000LL;
 
 // Waits for the phase with the given parity.  Returns false when the limit ran
 // out or when another thread of the CTA has already raised *abort_flag.
+// The lanes of a warp may get different answers: the limit runs out for one while the phase completes for another.  So a
+// warp that waits together votes (warp_all), or its lanes go on together whatever the answer, with no branch around an
+// instruction of the warp (elect, votes, mma.sync, tcgen05.ld / st, barriers), and one whose wait ran out no longer waits,
+// signals or issues.  Votes cost nothing in an issuer that takes one for all waits of a step; a vote for every wait of
+// issuers, producers and converters cost 1.5-2 % of a decode step of 256 or 512 tokens.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
   if (mbar_try_wait(bar, parity)) return true;
   const long long t0 = clock64();
@@ -87,6 +92,9 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     }
   }
 }
+
+// The same answer for the whole, converged warp.
+__device__ __forceinline__ bool warp_all(bool mine) { return __all_sync(0xFFFFFFFFu, mine) != 0; }
 
 // --------------------------------------------------------------------- TMA
 // 2-D tiled load global -> shared of this CTA, completion counted on an mbarrier.

@@ -55,9 +55,10 @@ struct MidStream {
 __device__ __forceinline__ void mid_produce(const MidStream& s, volatile int* abort_flag) {
   int stage = 0, issued = 0;
   uint32_t phase = 1;                                      // the first round waits for nobody
-  for (; issued < s.chunks; ++issued) {
-    if (issued >= s.ring && !ptx::mbar_wait(ptx::smem_u32(s.free_bar + stage), phase, abort_flag)) break;
-    if (ptx::elect_one()) {
+  bool ok = true;
+  for (int i = 0; i < s.chunks; ++i) {
+    if (ok && issued >= s.ring) ok = ptx::mbar_wait(ptx::smem_u32(s.free_bar + stage), phase, abort_flag);
+    if (ptx::elect_one() && ok) {
       const uint32_t bar = ptx::smem_u32(s.full + stage), dst = s.dst + stage * s.dst_step;
       const int c = (s.c0 + issued) * s.kc;
       ptx::mbar_arrive_expect_tx(bar, static_cast<uint32_t>(s.kc * s.blk));
@@ -68,12 +69,13 @@ __device__ __forceinline__ void mid_produce(const MidStream& s, volatile int* ab
       }
     }
     __syncwarp();
-    if (++stage == s.ring) {
+    issued += ok ? 1 : 0;
+    if (ok && ++stage == s.ring) {
       stage = 0;
       phase ^= 1u;
     }
   }
-  if (*abort_flag != 0) {
+  if (ptx::elect_one() && *abort_flag != 0) {
     // a wait ran out: give the copies in flight a bounded time to land before the CTA ends
     for (int j = max(0, issued - s.ring); j < issued; ++j) {
       const uint32_t parity = static_cast<uint32_t>((j / s.ring) & 1);
