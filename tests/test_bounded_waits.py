@@ -1,8 +1,9 @@
 """How the kernels give up a wait that ran out, read from their sources (nothing here runs on a GPU).
 
-A bounded mbarrier wait can end differently for the lanes of one warp.  So
+A bounded mbarrier wait can end differently for the lanes of one warp, and differently for the warps of a CTA.  So
 * a warp that waits together votes, or its lanes keep the answer in a flag of their own and go on together: the flag
-  stands in no condition around an instruction of the warp, only beside the one lane that signals or issues.
+  stands in no condition around an instruction of the warp, only beside the one lane that signals or issues;
+* a loop that meets a barrier of several warps is not left when a wait runs out: the others would wait for good.
 """
 import re
 from pathlib import Path
@@ -12,6 +13,7 @@ import pytest
 CSRC = Path(__file__).resolve().parent.parent / "tiny-vllm_b200" / "csrc"
 SOURCES = [p for p in sorted(CSRC.glob("*.cu*")) if p.name != "ptx_sm100.cuh" and "mbar_wait" in p.read_text()]
 ONE_LANE = re.compile(r"\blane == 0\b|\bproduce\(")       # produce(): under `lane < kPipes`, a ring per lane
+BARRIER = re.compile(r"named_bar_sync|consumer_barrier|__syncthreads|cluster_wait|cluster_sync_all")
 WAIT = r"ptx::mbar_wait\([^;]*\)"
 
 
@@ -77,3 +79,19 @@ def test_a_warp_goes_on_or_gives_up_as_one(path):
             assert waits_only or one_lane or own_count, cond
     for m in re.finditer(r"(?<!void )\bproduce\(&", code):
         assert re.search(r"if \(lane < kPipes\)\s*$", code[:m.start()])
+
+
+@pytest.mark.parametrize("path", SOURCES, ids=lambda p: p.name)
+def test_no_warp_leaves_the_others_at_a_barrier(path):
+    code = code_of(path)
+    loops = [b for b in blocks(code) if b[0].startswith("for")]
+    for _, start, end in loops:
+        if not BARRIER.search(code[start:end]):
+            continue
+        inner = [b for b in loops if start < b[1] and b[2] < end and not BARRIER.search(code[b[1]:b[2]])]
+        for m in re.finditer(r"mbar_wait\w*\(", code[start:end]):
+            at = start + m.start()
+            if any(b[1] < at < b[2] for b in inner):
+                continue
+            statement = code[code.rfind(";", 0, at):code.find(";", at)]
+            assert "break" not in statement and "return" not in statement, statement

@@ -186,6 +186,7 @@ w8a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_a,
     const int n_groups_tile = (n_chunks_tile + 1) >> 1;  // 64-column groups (last may be half)
     const int my_groups = (n_groups_tile - half + 1) >> 1;
     uint8_t* slab = staging + epi_warp * kSlabBytes;
+    bool alive = true;
     int it = 0;
     for (int item = blockIdx.x; item < total_items; item += gridDim.x, ++it) {
       const int split = item % p.splits;
@@ -200,7 +201,8 @@ w8a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_a,
       if (clustered && split > 0) {
         // K split over the cluster: hand this CTA's partial tile (exact int32 sums) to the
         // leader (cluster rank 0 = split 0) through its shared memory, [split - 1][column][row]
-        if (!ptx::warp_all(ptx::mbar_wait(ptx::smem_u32(tfull_bar + buf), tphase, abort_flag))) break;
+        if (alive) alive = ptx::warp_all(ptx::mbar_wait(ptx::smem_u32(tfull_bar + buf), tphase, abort_flag));
+        if (!alive) continue;   // (no barrier of the CTA on this path)
         ptx::tc_fence_after_sync();
         const uint32_t taddr_p = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) +
                                  static_cast<uint32_t>(buf * p.bn);
@@ -230,8 +232,26 @@ w8a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_a,
         if (row < p.rows_a) a_s = p.a_scales[row];   // (not __ldg: the previous kernel writes it)
         ptx::named_bar_sync(2, kEpiThreads);
       }
-      if (!ptx::warp_all(ptx::mbar_wait(ptx::smem_u32(tfull_bar + buf), tphase, abort_flag))) break;
-      if (clustered && !ptx::warp_all(ptx::mbar_wait_cluster(ptx::smem_u32(pfull_bar), 0u, abort_flag))) break;
+      // K split through memory: true in the last CTA to arrive for this tile
+      auto last_of_tile = [&] {
+        __threadfence();
+        ptx::named_bar_sync(1, kEpiThreads);
+        if (epi_tid == 0) {
+          const unsigned int old = atomicAdd(p.counters + t, 1u);
+          const int last = (old == static_cast<unsigned int>(p.splits - 1));
+          if (last) p.counters[t] = 0u;  // every split has arrived: leave the counter clean
+          last_flag[it & 1] = last;
+        }
+        ptx::named_bar_sync(1, kEpiThreads);
+        return last_flag[it & 1] != 0;
+      };
+      if (alive)
+        alive = ptx::warp_all(ptx::mbar_wait(ptx::smem_u32(tfull_bar + buf), tphase, abort_flag)) &&
+                (!clustered || ptx::warp_all(ptx::mbar_wait_cluster(ptx::smem_u32(pfull_bar), 0u, abort_flag)));
+      if (!alive) {   // a warp whose wait ran out goes on to meet the others at the barriers of each tile
+        if (p.splits > 1 && !clustered) last_of_tile();
+        continue;
+      }
       ptx::tc_fence_after_sync();
       const uint32_t taddr =
           tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(buf * p.bn);
@@ -311,16 +331,7 @@ w8a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_a,
 
       if (p.splits > 1 && !clustered) {
         // split-K: the last CTA to arrive for this tile sums all partial tiles.
-        __threadfence();
-        ptx::named_bar_sync(1, kEpiThreads);
-        if (epi_tid == 0) {
-          const unsigned int old = atomicAdd(p.counters + t, 1u);
-          const int last = (old == static_cast<unsigned int>(p.splits - 1));
-          if (last) p.counters[t] = 0u;  // every split has arrived: leave the counter clean
-          last_flag[it & 1] = last;
-        }
-        ptx::named_bar_sync(1, kEpiThreads);
-        if (last_flag[it & 1]) {
+        if (last_of_tile()) {
           __threadfence();
           const int32_t* base =
               p.partials + static_cast<size_t>(t) * p.splits * p.bn * kTileA + row_in_tile;

@@ -240,6 +240,7 @@ w8a16_umma_kernel(const __grid_constant__ CUtensorMap tmap_x,
     const int n_chunks_tile = p.bn >> 5;
     const int n_groups = (n_chunks_tile + 1) >> 1;
     uint8_t* slab = staging + epi_warp * kSlabBytes;
+    bool alive = true;
     int it = 0;
     for (int item = blockIdx.x; item < total_items; item += gridDim.x, ++it) {
       const int split = item % p.splits;
@@ -257,7 +258,24 @@ w8a16_umma_kernel(const __grid_constant__ CUtensorMap tmap_x,
         }
         ptx::named_bar_sync(2, kEpiThreads);
       }
-      if (!ptx::warp_all(ptx::mbar_wait(ptx::smem_u32(tfull_bar + buf), tphase, abort_flag))) break;
+      // K split through memory: true in the last CTA to arrive for this tile
+      auto last_of_tile = [&] {
+        __threadfence();
+        ptx::named_bar_sync(1, kEpiThreads);
+        if (epi_tid == 0) {
+          const unsigned int old = atomicAdd(p.counters + t, 1u);
+          const int last = (old == static_cast<unsigned int>(p.splits - 1));
+          if (last) p.counters[t] = 0u;  // every split has arrived: leave the counter clean
+          last_flag[it & 1] = last;
+        }
+        ptx::named_bar_sync(1, kEpiThreads);
+        return last_flag[it & 1] != 0;
+      };
+      if (alive) alive = ptx::warp_all(ptx::mbar_wait(ptx::smem_u32(tfull_bar + buf), tphase, abort_flag));
+      if (!alive) {   // a warp whose wait ran out goes on to meet the others at the barriers of each tile
+        if (p.splits > 1) last_of_tile();
+        continue;
+      }
       ptx::tc_fence_after_sync();
       const uint32_t taddr =
           tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(buf * p.bn);
@@ -314,16 +332,7 @@ w8a16_umma_kernel(const __grid_constant__ CUtensorMap tmap_x,
       ptx::mbar_arrive(ptx::smem_u32(tempty_bar + buf));
 
       if (p.splits > 1) {
-        __threadfence();
-        ptx::named_bar_sync(1, kEpiThreads);
-        if (epi_tid == 0) {
-          const unsigned int old = atomicAdd(p.counters + t, 1u);
-          const int last = (old == static_cast<unsigned int>(p.splits - 1));
-          if (last) p.counters[t] = 0u;
-          last_flag[it & 1] = last;
-        }
-        ptx::named_bar_sync(1, kEpiThreads);
-        if (last_flag[it & 1]) {
+        if (last_of_tile()) {
           __threadfence();
           const float* base =
               p.partials + static_cast<size_t>(t) * p.splits * p.bn * kTileA + row_in_tile;

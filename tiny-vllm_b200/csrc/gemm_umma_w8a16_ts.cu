@@ -252,11 +252,16 @@ w8a16_umma_ts_kernel(const __grid_constant__ CUtensorMap tmap_x,
     const T* bias = reinterpret_cast<const T*>(p.bias);
     T* out = reinterpret_cast<T*>(p.out);
     uint8_t* my_stage = out_stage + t * 2 * kTsStageOutBytes;
+    bool alive = true;
     int it = 0, round = 0;
     for (int item = blockIdx.x; item < total_items; item += gridDim.x, ++it) {
       const int tile_ch = item % p.tiles_ch;
       const int tile_tok = item / p.tiles_ch;
-      if (!ptx::warp_all(ptx::mbar_wait(ptx::smem_u32(tfull_bar), static_cast<uint32_t>(it) & 1u, abort_flag))) break;
+      if (alive) alive = ptx::warp_all(ptx::mbar_wait(ptx::smem_u32(tfull_bar), static_cast<uint32_t>(it) & 1u, abort_flag));
+      if (!alive) {   // a warp whose wait ran out goes on to meet the others of its group at their barriers
+        for (int c = 0; c < kTsTokens / 32 && !(p.debug_flags & 1); ++c) ptx::named_bar_sync(2 + t, kEpiThreads);
+        continue;
+      }
       ptx::tc_fence_after_sync();
       const int ch0 = tile_ch * kTsChannels + t * kTileA;       // first channel of this A tile
       const int ch = ch0 + quarter * 32 + lane;
