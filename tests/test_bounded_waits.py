@@ -3,7 +3,8 @@
 A bounded mbarrier wait can end differently for the lanes of one warp, and differently for the warps of a CTA.  So
 * a warp that waits together votes, or its lanes keep the answer in a flag of their own and go on together: the flag
   stands in no condition around an instruction of the warp, only beside the one lane that signals or issues;
-* a loop that meets a barrier of several warps is not left when a wait runs out: the others would wait for good.
+* a loop that meets a barrier of several warps is not left when a wait runs out: the others would wait for good;
+* a TMA producer waits for its copies in flight before it ends.
 """
 import re
 from pathlib import Path
@@ -95,3 +96,8 @@ def test_no_warp_leaves_the_others_at_a_barrier(path):
                 continue
             statement = code[code.rfind(";", 0, at):code.find(";", at)]
             assert "break" not in statement and "return" not in statement, statement
+
+
+@pytest.mark.parametrize("path", [p for p in SOURCES if "tma_load" in p.read_text()], ids=lambda p: p.name)
+def test_a_producer_that_gives_up_waits_for_its_copies(path):
+    assert re.search(r"if \((rank == 0 && |ptx::elect_one\(\) && )?\*abort_flag != 0\) ptx::drain_ring\(", code_of(path))

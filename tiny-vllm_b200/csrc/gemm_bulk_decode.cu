@@ -127,16 +127,7 @@ __device__ __forceinline__ void produce(const CUtensorMap* tm_w, const StreamPla
       }
     }
   }
-  if (*abort_flag != 0) {
-    // a wait ran out somewhere in the CTA: give the tiles still in flight a bounded time to
-    // land before the CTA's shared memory is released
-    for (int j = max(0, it - p.slots); j < it; ++j) {
-      const uint32_t bar = ptx::smem_u32(full + j % p.slots);
-      const uint32_t parity = static_cast<uint32_t>((j / p.slots) & 1);
-      for (int tries = 0; tries < (1 << 16) && !ptx::mbar_try_wait(bar, parity); ++tries) {
-      }
-    }
-  }
+  if (*abort_flag != 0) ptx::drain_ring(full, p.slots, slot, phase ^ 1u);   // a wait ran out somewhere in the CTA
 }
 
 struct CtaSmem {

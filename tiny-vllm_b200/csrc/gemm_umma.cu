@@ -129,6 +129,7 @@ w8a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_a,
           }
         }
       }
+      if (*abort_flag != 0) ptx::drain_ring(full_bar, p.stages, stage, phase);
     }
   } else if (warp == 1) {
     if (lane == 0) {

@@ -366,6 +366,8 @@ umma_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
           }
         }
       }
+      // (the leader's barriers count the bytes of both CTAs, and neither leaves before the other)
+      if (rank == 0 && *abort_flag != 0) ptx::drain_ring(full_bar, kStages, stage, phase);
     }
   } else if (warp == 1) {
     if (lane == 0 && rank == 0 && run) {

@@ -139,6 +139,7 @@ w8a16_umma_kernel(const __grid_constant__ CUtensorMap tmap_x,
           }
         }
       }
+      if (*abort_flag != 0) ptx::drain_ring(full_bar, p.stages, stage, phase);
     }
   } else if (warp == 1) {
     if (lane == 0) {

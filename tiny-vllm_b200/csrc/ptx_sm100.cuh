@@ -96,6 +96,15 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
 // The same answer for the whole, converged warp.
 __device__ __forceinline__ bool warp_all(bool mine) { return __all_sync(0xFFFFFFFFu, mine) != 0; }
 
+// A TMA producer that gave up: its copies in flight get a bounded time to land before the CTA's shared memory is released.
+// `slot` is the next one of the ring to be filled and `turn` the parity of the fills of this turn; the others were
+// filled in the turn before (or never: the opposite parity of a fresh barrier passes at once).
+__device__ __forceinline__ void drain_ring(const uint64_t* full, int slots, int slot, uint32_t turn) {
+  for (int s = 0; s < slots; ++s)
+    for (int tries = 0; tries < (1 << 16) && !mbar_try_wait(smem_u32(full + s), s < slot ? turn : turn ^ 1u); ++tries) {
+    }
+}
+
 // --------------------------------------------------------------------- TMA
 // 2-D tiled load global -> shared of this CTA, completion counted on an mbarrier.
 // c0 is the innermost (contiguous) coordinate; c0 * element size must be a

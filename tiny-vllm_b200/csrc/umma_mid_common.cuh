@@ -53,10 +53,10 @@ struct MidStream {
 // One warp per operand: the weights run ahead as far as their ring allows, first of all ahead of
 // the kernel that produces the activations.
 __device__ __forceinline__ void mid_produce(const MidStream& s, volatile int* abort_flag) {
-  int stage = 0, issued = 0;
+  int stage = 0;
   uint32_t phase = 1;                                      // the first round waits for nobody
   bool ok = true;
-  for (int i = 0; i < s.chunks; ++i) {
+  for (int issued = 0; issued < s.chunks; ++issued) {
     if (ok && issued >= s.ring) ok = ptx::mbar_wait(ptx::smem_u32(s.free_bar + stage), phase, abort_flag);
     if (ptx::elect_one() && ok) {
       const uint32_t bar = ptx::smem_u32(s.full + stage), dst = s.dst + stage * s.dst_step;
@@ -69,21 +69,12 @@ __device__ __forceinline__ void mid_produce(const MidStream& s, volatile int* ab
       }
     }
     __syncwarp();
-    issued += ok ? 1 : 0;
     if (ok && ++stage == s.ring) {
       stage = 0;
       phase ^= 1u;
     }
   }
-  if (ptx::elect_one() && *abort_flag != 0) {
-    // a wait ran out: give the copies in flight a bounded time to land before the CTA ends
-    for (int j = max(0, issued - s.ring); j < issued; ++j) {
-      const uint32_t parity = static_cast<uint32_t>((j / s.ring) & 1);
-      for (int tries = 0;
-           tries < (1 << 16) && !ptx::mbar_try_wait(ptx::smem_u32(s.full + j % s.ring), parity); ++tries) {
-      }
-    }
-  }
+  if (ptx::elect_one() && *abort_flag != 0) ptx::drain_ring(s.full, s.ring, stage, phase ^ 1u);
 }
 
 // The search for a plan costs some 10 us of host time, more than the launch: its results are kept per
