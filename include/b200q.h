@@ -172,10 +172,6 @@ size_t b200q_w8a8_dynamic_scratch_bytes(int M, int N, int K);
  * size can be shared by all calls that are ordered on one stream.
  */
 size_t b200q_workspace_bytes(int op, int M, int N, int K);
-/* Sizes (513 to 1023 tokens of wide layers) at which b200q_w8a16_gemm needs no workspace, but is faster with one of at
- * least this many bytes: it then expands the weights into it, as it does from 1024 tokens on.  Any content; may be
- * this call's own.  0: no such workspace helps. */
-size_t b200q_w8a16_scratch_bytes(int M, int N, int K);
 
 /*
  * Name of the kernel family the library would run for this problem, e.g.

@@ -101,11 +101,12 @@ def test_w8a16_beyond_the_mid_sizes_takes_the_tensor_memory_kernel(M, N, K):
     assert device_status_ok()
 
 
-@pytest.mark.parametrize("M,N,K,pair", [(513, 16384, 1040, True), (700, 12296, 2064, True), (1023, 9728, 2560, True),
-                                        (513, 22016, 1024, False), (830, 9728, 2560, False), (512, 16384, 1040, False)])
-def test_w8a16_513_to_1023_tokens_expand_once_where_that_costs_no_round(M, N, K, pair):
-    expect = "umma_f16_pair_expand_once_tokens256" if pair else "umma_f16_tmem_weights_channels256"
-    assert select_path(_lib.OP_W8A16, M, N, K) == expect
+@pytest.mark.parametrize("M,N,K", [(513, 16384, 1040), (700, 12296, 2064), (1023, 9728, 2560), (513, 22016, 1024),
+                                   (830, 9728, 2560), (512, 16384, 1040)])
+def test_w8a16_to_1023_tokens_takes_one_route_whatever_the_workspace(M, N, K):
+    assert select_path(_lib.OP_W8A16, M, N, K) == "umma_f16_tmem_weights_channels256"
+    L = _lib.lib()
+    assert L.b200q_workspace_bytes(_lib.OP_W8A16, M, N, K) == 0
     q, s = O.make_weight(N, K, seed=N + K)
     x = O.make_activation(M, K, seed=M, dtype=torch.bfloat16)
     b = (torch.randn(N, generator=torch.Generator().manual_seed(M)) * 0.1).to(torch.bfloat16)
@@ -113,7 +114,12 @@ def test_w8a16_513_to_1023_tokens_expand_once_where_that_costs_no_round(M, N, K,
     y = apply_int8_weight_only_linear(*dev)
     m = O.tensor_metrics(O.w8a16_native_reference(x, q, s, b), y)
     assert m["relative_l2"] <= 4e-3 and m["cosine_similarity"] >= 0.9999, m
-    with knobs(W8A16_PAIR_MIN_M=1024):          # the route of a call without a workspace: sums in another order
-        y_ts = apply_int8_weight_only_linear(*dev)
-    assert O.tensor_metrics(y_ts, y)["relative_l2"] <= 2e-3
+    ws = torch.full((2 * N * K + 4096,), 0x5A, dtype=torch.uint8, device="cuda")
+    out = torch.empty_like(y)
+    rc = L.b200q_w8a16_gemm(*[t.data_ptr() for t in (*dev, out)], M, N, K, _lib.DTYPE_BF16, ws.data_ptr(), ws.numel(),
+                            torch.cuda.current_stream().cuda_stream)
+    assert rc == _lib.OK and torch.equal(bits(out), bits(y)) and bool((ws == 0x5A).all())
+    with knobs(W8A16_PAIR_MIN_M=512):           # the kernel of larger calls
+        y_pair = apply_int8_weight_only_linear(*dev)
+    assert O.tensor_metrics(y_pair, y)["relative_l2"] <= 2e-3
     assert device_status_ok()

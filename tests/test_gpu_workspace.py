@@ -72,11 +72,11 @@ assert torch.equal(y, expect)
 """
 
 
-ITS_OWN = """
-x, q, s = problem(700, 24576, 2048)        # W8A16 at 513 to 1023 tokens: a buffer of each call's own
+WIDE = """
+x, q, s = problem(700, 24576, 2048)        # W8A16 at 513 to 1023 tokens of wide layers: none either
 fn = lambda: apply_int8_weight_only_linear(x, q, s)
 torch.cuda.synchronize()
-graph, y = captured(fn)                    # from the capture's pool, without a call before it
+graph, y = captured(fn)                    # without a call before it
 graph.replay()
 torch.cuda.synchronize()
 expect = fn()
@@ -85,7 +85,7 @@ x2, q2, s2 = problem(700, 24576, 2064)
 expect2 = apply_int8_weight_only_linear(x2, q2, s2)
 a, b = torch.cuda.Stream(), torch.cuda.Stream()
 torch.cuda.synchronize()
-for _ in range(20):                        # two streams at once do not share it
+for _ in range(20):                        # two streams at once share nothing
     with torch.cuda.stream(a):
         ya = fn()
     with torch.cuda.stream(b):
@@ -95,8 +95,8 @@ for _ in range(20):                        # two streams at once do not share it
 """
 
 
-@pytest.mark.parametrize("body", [NEEDS_NONE, NEEDS_SOME, OUTGROWN, ITS_OWN],
-                         ids=["needs-none", "needs-some", "outgrown", "its-own"])
+@pytest.mark.parametrize("body", [NEEDS_NONE, NEEDS_SOME, OUTGROWN, WIDE],
+                         ids=["needs-none", "needs-some", "outgrown", "wide-layers"])
 def test_capture_in_a_fresh_process(body):
     r = subprocess.run([sys.executable, "-c", HEAD + body], cwd=ROOT, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout + r.stderr

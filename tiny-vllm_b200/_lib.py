@@ -82,7 +82,6 @@ SIGNATURES = {
                                            _c.c_int, _c.c_int, _c.c_int, _c.c_int, _c.c_void_p,
                                            _c.c_size_t, _c.c_void_p, _c.c_size_t, _c.c_void_p]),
     "b200q_w8a8_dynamic_scratch_bytes": (_c.c_size_t, [_c.c_int, _c.c_int, _c.c_int]),
-    "b200q_w8a16_scratch_bytes": (_c.c_size_t, [_c.c_int, _c.c_int, _c.c_int]),
     "b200q_workspace_bytes": (_c.c_size_t, [_c.c_int, _c.c_int, _c.c_int, _c.c_int]),
     "b200q_select_path": (_c.c_char_p, [_c.c_int, _c.c_int, _c.c_int, _c.c_int]),
     "b200q_strerror": (_c.c_char_p, [_c.c_int]),

@@ -418,10 +418,7 @@ int b200q_w8a16_gemm(const void* x, const int8_t* qweight, const float* scales, 
     return B200Q_OK;
   }
   if (path == B200Q_PATH_UMMA && umma16_mid_applicable(M, N, K)) return launch_umma16_mid(a);
-  if (path == B200Q_PATH_UMMA && umma16_pair_applicable(M, N, K) &&
-      (M >= kPairMinTokens || (workspace != nullptr && workspace_bytes >= umma16_pair_workspace_bytes(N, K)) ||
-       !umma16_ts_applicable(M, N, K)))
-    return launch_w8a16_umma_pair(a);
+  if (path == B200Q_PATH_UMMA && umma16_pair_applicable(M, N, K)) return launch_w8a16_umma_pair(a);
   if (path == B200Q_PATH_UMMA && umma16_ts_applicable(M, N, K)) return launch_w8a16_umma_ts(a);
   if (path == B200Q_PATH_UMMA || path == B200Q_PATH_UMMA_SWAP) {
     UmmaPlan plan;
@@ -485,18 +482,10 @@ int b200q_w8a8_dynamic_gemm(const void* x, const int8_t* qweight, const float* w
   return B200Q_OK;
 }
 
-size_t b200q_w8a16_scratch_bytes(int M, int N, int K) {
-  if (M <= 512 || M >= kPairMinTokens || check_dims(M, N, K) != B200Q_OK || resolve_path(B200Q_OP_W8A16, M, N, K) != B200Q_PATH_UMMA)
-    return 0;
-  return !umma16_mid_applicable(M, N, K) && umma16_pair_applicable(M, N, K) && umma16_ts_applicable(M, N, K)
-             ? umma16_pair_workspace_bytes(N, K) : 0;
-}
-
 size_t b200q_workspace_bytes(int op, int M, int N, int K) {
   if (op == B200Q_OP_W8A16 && check_dims(M, N, K) == B200Q_OK &&
       resolve_path(op, M, N, K) == B200Q_PATH_UMMA) {
-    if (!umma16_mid_applicable(M, N, K) && umma16_pair_applicable(M, N, K) && b200q_w8a16_scratch_bytes(M, N, K) == 0)
-      return umma16_pair_workspace_bytes(N, K);
+    if (!umma16_mid_applicable(M, N, K) && umma16_pair_applicable(M, N, K)) return umma16_pair_workspace_bytes(N, K);
   }
   if (op != B200Q_OP_W8A8 && op != B200Q_OP_W8A16) return 0;
   if (check_dims(M, N, K) != B200Q_OK) return 0;

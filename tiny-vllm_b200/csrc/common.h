@@ -166,7 +166,6 @@ int launch_tp_reduce_gather(const void* stage, void* const* peer_y,
 
 // gemm_umma_pair.cu: W8A16 prefill route — weights expanded once per call into the
 // workspace, then the 16-bit CTA-pair kernel
-constexpr int kPairMinTokens = 1024;   // below, a call without the workspace for it is taken by another kernel
 bool umma16_pair_applicable(int M, int N, int K);
 size_t umma16_pair_workspace_bytes(int N, int K);
 int launch_w8a16_umma_pair(const GemmArgs& a);

@@ -716,22 +716,14 @@ int launch_w8a8_umma_pair(const GemmArgs& a) {
 bool umma16_pair_applicable(int M, int N, int K) {
   if (debug_knob(B200Q_KNOB_NO_PAIR, 0) != 0) return false;
   if ((K % 16) != 0 || (N % 8) != 0) return false;
-  const int pairs = sm_count() / 2;
-  const int forced_min = debug_knob(B200Q_KNOB_W8A16_PAIR_MIN_M, 0);
-  if (M < (forced_min > 0 ? forced_min : kPairMinTokens)) {
-    // From 513 tokens on the rival is the kernel with the weights in tensor memory, whose 256 x 128 tiles cost an SM what
-    // a pair's 256 x 256 tile costs its two, and which does not overlap a tile's epilogue: this route wins, expansion
-    // included, unless rounding the tokens up to 256 costs it a round (us, that kernel / this: 4096 -> 24576 at 700 tokens
-    // 158 / 147, at 1000 251 / 192; 2048 -> 12288 at 600 43 / 37; 2560 -> 9728 at 700 54 / 41, but, with a round more, at 830 50 / 54
-    // and 4096 -> 22016 at 600 133 / 146).  At 512 and below it is even or behind (4096 -> 24576 115 / 123).
-    if (forced_min > 0 || M <= 512 || !umma16_ts_applicable(M, N, K)) return false;
-    const long long cols = (N + kPairBN - 1) / kPairBN, tiles = cols * ((M + 255) / 256), rival = cols * ((M + 127) / 128);
-    return (tiles + pairs - 1) / pairs <= (rival + sm_count() - 1) / sm_count();
-  }
+  // (Wide layers would gain from 513 tokens on, 4096 -> 24576 at 1000 tokens 251 -> 192 us; but there a call has always done
+  // without a workspace, under capture too, and a route that depends on whether 2 N K bytes are free is none.)
+  if (M < debug_knob(B200Q_KNOB_W8A16_PAIR_MIN_M, 1024)) return false;
   // The kernels that expand inside the main loop are so much slower at prefill size that this
   // route pays off well before every CTA pair has a tile: 2048 -> 1024 at 2048 tokens (32
   // tiles) 18.8 against 23.0 us; only short K loops on few tiles go the other way (512 -> 1024
   // at 2048 tokens: 10.6 against 9.9 us).
+  const int pairs = sm_count() / 2;
   return enough_pair_tiles(M, N, K >= 1024 ? (pairs * 2) / 5 : (pairs * 2) / 3);
 }
 

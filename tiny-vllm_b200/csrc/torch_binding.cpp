@@ -180,24 +180,11 @@ PyObject* w8a16(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   c10::cuda::CUDAGuard guard(device);
   const int m = static_cast<int>(M), n = static_cast<int>(p.N), k = static_cast<int>(p.K);
   at::Tensor y = empty_on(out_shape(*x, p.N), x->scalar_type(), device);
-  auto call = [&](void* ws, size_t bytes) {
+  const int rc = with_workspace(device, B200Q_OP_W8A16, m, n, k, [&](void* ws, size_t bytes) {
     return b200q_w8a16_gemm(x->data_ptr(), static_cast<const int8_t*>(ptr(p.w)),
                             static_cast<const float*>(ptr(p.s)), ptr(p.b), y.data_ptr(), m, n, k, dt, ws, bytes,
                             stream_of(device));
-  };
-  // sizes at which the library does without a workspace, but better with one: this call's own, so that calls on several
-  // streams stay independent
-  int rc;
-  if (const size_t wanted = b200q_w8a16_scratch_bytes(m, n, k)) {
-    at::Tensor scratch;
-    try {
-      scratch = empty_on({static_cast<int64_t>(wanted)}, at::kByte, device);
-    } catch (const c10::OutOfMemoryError&) {
-    }
-    rc = unlocked([&] { return call(scratch.defined() ? scratch.data_ptr() : nullptr, scratch.defined() ? wanted : 0); });
-  } else {
-    rc = with_workspace(device, B200Q_OP_W8A16, m, n, k, call);
-  }
+  });
   if (rc != B200Q_OK) return fail(rc, "b200q_w8a16_gemm", M, p.N, p.K);
   return THPVariable_Wrap(std::move(y));
   END_HANDLE_TH_ERRORS
