@@ -43,3 +43,12 @@ def test_clusters_never_wait_for_tensor_memory(op, forced):
                     assert p["columns"] <= SM_COLUMNS // 2 or left <= CTA_RESERVED, (M, N, K, p)
                     assert p["shared"] + PAIR_SHARED + 2 * CTA_RESERVED > SM_SHARED, (M, N, K, p)
     assert seen > 50
+
+
+@pytest.mark.parametrize("M,N,K,deep", [(129, 4096, 12288, True), (256, 2560, 9728, True), (200, 2048, 6144, True),
+                                        (128, 4096, 12288, False), (256, 4096, 4096, False), (256, 1024, 3072, False),
+                                        (256, 4096, 1024, False)])
+def test_w8a8_rings_leave_room_for_the_quantiser_unless_rows_are_long(M, N, K, deep):
+    b200_build.build()
+    plan = mid_plan(_lib.OP_W8A8, M, N, K)
+    assert (plan["shared"] > 218 * 1024) == deep, plan

@@ -42,8 +42,14 @@ namespace {
 constexpr int kMidTok = 128;                     // UMMA M: token rows of a tile
 constexpr int kMidXTile = kMidTok * 128;         // bytes the UMMA reads per K block of activations
 // One CTA per SM, and room beside it for those of the quantiser that runs between two such kernels (1 KB each): with all
-// of the shared memory taken, a CTA waits for the quantiser to leave its SM (0.6B layer, 200 to 512 tokens, 1.5-2 %).
+// of the shared memory taken, a CTA waits for the quantiser to leave its SM.  Plans that use it have fewer CTAs with wider
+// tiles, too, so the limit pays where no quantiser runs (layers of the 0.6B model at 129 to 512 tokens, 226 / 218 KB:
+// 1.018-1.025 with a quantiser, 1.005-1.047 on codes).
 constexpr int kMidSmemQuant = 218 * 1024;
+// But long rows of more than one token tile go round a ring of two or three chunks many times, and a chunk more is worth
+// more than the early start: at 129 to 256 tokens layers with down projections of K = 12288, 9728, 9472 and 6144 take
+// 0.960-0.985 of their time with 226 KB (0.936-0.975 on codes).  Up to one token tile, or K = 4096, it is either way.
+bool mid_wants_deep_ring(int M, int K) { return M > kMidTok && K > 4096; }
 
 struct MidParams {
   int M, N;
@@ -395,8 +401,9 @@ double mid_cost(const MidPlan& pl, int M) {
   const double slots = static_cast<double>(sm_count()) * per_sm;
   us += 1.4 * std::min(1.0, std::max(0.0, (2.0 * ctas - slots) / slots));
   us += (per_sm == 1 ? 2.6 : 2.15) * (waves - 1);
-  // Clusters that need several SMs at once, two CTAs on each, start late where the quantiser of the activations still
-  // has CTAs of its own (whole layers of the 8B model at 32 tokens 59.0 -> 55.5 us, at 20 56.7 -> 54.7, nothing else moved)
+  // Clusters that need several SMs at once, two CTAs on each, start late: behind a quantiser that still has CTAs of its own
+  // (layers of hidden 4096 and 2560 at 20 and 32 tokens without / with the factor 1.03-1.05) and behind another GEMM (1.02-1.045
+  // on codes).  Against it: layers of hidden 1024 on codes at 20 and 32 tokens, 0.987-0.992; elsewhere no difference.
   return pl.splits > 1 && ctas > sm_count() ? 1.15 * us : us;
 }
 
@@ -409,7 +416,7 @@ bool search_plan(int M, int N, int K, MidPlan* best) {
     for (int s : {1, 2, 4, 8}) {
       if (want_s != 0 && s != want_s) continue;
       for (int kc : {4, 2, 1}) {
-        for (int cap : {kMidSmemQuant, kMidSmemTwo}) {
+        for (int cap : {mid_wants_deep_ring(M, K) ? kMidSmemOne : kMidSmemQuant, kMidSmemTwo}) {
           MidPlan pl;
           if (!mid_plan_for(M, N, k_blocks, bn, s, kc, cap, &pl)) continue;
           const double cost = mid_cost(pl, M);
