@@ -38,13 +38,14 @@ def test_library_picks_the_staged_kernels_for_long_rows():
         assert select_path(_lib.OP_W8A8, 16, 6144, 1024) == "bulk_ring_s8_persistent"
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("M,N,K", SHAPES)
-def test_w8a8_bit_exact(M, N, K, oracle_c_lib):
+def test_w8a8_bit_exact(M, N, K, dtype, oracle_c_lib):
     g = torch.Generator().manual_seed(M + N + K)
     q, s = O.make_weight(N, K, seed=N)
-    x = O.make_activation(M, K, seed=M, dtype=torch.bfloat16)
+    x = O.make_activation(M, K, seed=M, dtype=dtype)
     xq, a_s = O.quantize_per_row_dynamic(x)
-    b = (torch.randn(N, generator=g) * 0.1).to(torch.bfloat16)
+    b = (torch.randn(N, generator=g) * 0.1).to(dtype)
     dev = [t.cuda() for t in (xq, a_s, q, s)]
     ref_acc = O.w8a8_int32_accumulators(xq, q)
     with forced_path("mma"), knobs(BULK_DECODE=2):
@@ -53,15 +54,15 @@ def test_w8a8_bit_exact(M, N, K, oracle_c_lib):
         else:
             assert select_path(_lib.OP_W8A8, M, N, K).startswith("bulk_ring")
         acc = w8a8_int32_accumulators(dev[0], dev[2])
-        y = apply_w8a8_linear(*dev, bias=b.cuda(), out_dtype=torch.bfloat16)
+        y = apply_w8a8_linear(*dev, bias=b.cuda(), out_dtype=dtype)
     with forced_path("mma"), knobs(BULK_DECODE=1):
         assert select_path(_lib.OP_W8A8, M, N, K).startswith("mma_stream")
-        y_regs = apply_w8a8_linear(*dev, bias=b.cuda(), out_dtype=torch.bfloat16)
+        y_regs = apply_w8a8_linear(*dev, bias=b.cuda(), out_dtype=dtype)
     assert torch.equal(bits(y), bits(y_regs))
     with forced_path("mma"), knobs(BULK_DECODE=2, BULK_WPP=1):   # one consumer warp per ring
-        assert torch.equal(bits(apply_w8a8_linear(*dev, bias=b.cuda(), out_dtype=torch.bfloat16)), bits(y))
+        assert torch.equal(bits(apply_w8a8_linear(*dev, bias=b.cuda(), out_dtype=dtype)), bits(y))
     assert torch.equal(acc.cpu(), ref_acc)
-    assert torch.equal(bits(y.cpu()), bits(O.w8a8_native_epilogue(ref_acc, a_s, s, b, torch.bfloat16)))
+    assert torch.equal(bits(y.cpu()), bits(O.w8a8_native_epilogue(ref_acc, a_s, s, b, dtype)))
     assert device_status_ok()
 
 

@@ -140,6 +140,45 @@ def test_expand_once_pair_kernel(M, N, K, dtype, bias, epilogue):
     assert device_status_ok()
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_expand_once_workspace_through_the_c_entry(dtype):
+    # the smallest token count of the route; a workspace on a 16-byte boundary takes narrower stores than torch's own
+    M, N, K = 1024, 6408, 1040
+    L = _lib.lib()
+    need = L.b200q_workspace_bytes(_lib.OP_W8A16, M, N, K)
+    assert need >= 2 * N * K and select_path(_lib.OP_W8A16, M, N, K) == "umma_f16_pair_expand_once_tokens256"
+    assert L.b200q_workspace_bytes(_lib.OP_W8A16, M - 1, N, K) == 0
+    q, s = O.make_weight(N, K, seed=N)
+    x = O.make_activation(M, K, seed=M, dtype=dtype, outliers=False)
+    dev = [t.cuda() for t in (x, q, s)]
+    buf = torch.zeros(need + 64, dtype=torch.uint8, device="cuda")
+    base = -buf.data_ptr() % 32
+
+    def call(offset, size):
+        y = torch.full((M, N), -1.0, dtype=dtype, device="cuda")
+        rc = L.b200q_w8a16_gemm(*[t.data_ptr() for t in dev], None, y.data_ptr(), M, N, K,
+                                _lib.DTYPE_BF16 if dtype == torch.bfloat16 else _lib.DTYPE_F16,
+                                None if offset is None else buf.data_ptr() + base + offset, size,
+                                torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+        return rc, y
+
+    for offset, size in ((None, 0), (0, need - 1), (16, need - 1)):
+        rc, y = call(offset, size)
+        assert rc == _lib.ERR_WORKSPACE and bool((y == -1).all())
+    outs = []
+    for offset in (0, 16):
+        buf.fill_(0)
+        buf[base + offset + need:] = 0x5A
+        rc, y = call(offset, need)
+        assert rc == _lib.OK and bool((buf[base + offset + need:] == 0x5A).all())
+        outs.append(y)
+    assert torch.equal(bits(outs[0]), bits(outs[1]))
+    m = O.tensor_metrics(O.w8a16_native_reference(x, q, s, None), outs[1])
+    assert m["relative_l2"] <= 4e-3 and m["cosine_similarity"] >= 0.9999, m
+    assert device_status_ok()
+
+
 def test_prefill_with_odd_channel_count_stays_on_the_shared_memory_kernel():
     # N % 8 != 0: no 16-byte output pieces, so neither the tensor-memory kernel nor the
     # full-line store path applies; element-wise stores of the shared-memory kernel
