@@ -28,15 +28,17 @@ import pytest
 import torch
 import torch.multiprocessing as mp
 
+from oracle import build_ref
+
 ROOT = Path(__file__).resolve().parent.parent
 HIDDEN, LAYERS, HEADS, KV_HEADS, HEAD_DIM, INTER, VOCAB = 64, 2, 4, 2, 16, 96, 128
 
 
 def reference_dir():
-    for cand in (os.environ.get("NANOVLLM_REFERENCE"), str(ROOT / "oracle" / "_ref"), "/root/reference"):
+    for cand in (os.environ.get("NANOVLLM_REFERENCE"), ROOT / "oracle" / "_ref", build_ref.reference_checkout()):
         if cand and (Path(cand) / "nanovllm" / "models" / "qwen3.py").is_file() \
                 and (Path(cand) / "scripts" / "quantize.py").is_file():
-            return cand
+            return str(cand)
     return None
 
 
