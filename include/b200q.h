@@ -211,10 +211,8 @@ int b200q_version(void);
 int b200q_debug_force_path(int path);
 
 /*
- * Test and tuning knobs.  A knob changes which kernel variant runs, how a problem is tiled,
- * or (B200Q_KNOB_FLAGS) switches parts of a kernel off so that their cost can be measured —
- * the last kind makes results WRONG on purpose.  All knobs are unset when the library is
- * loaded, nothing is read from the environment, and a setting is private to the thread
+ * Test and tuning knobs.  A knob changes which kernel variant runs or how a problem is tiled, never what is
+ * computed.  All knobs are unset when the library is loaded, nothing is read from the environment, and a setting is private to the thread
  * that made it: a serving process that never calls b200q_debug_set() cannot be affected.
  * b200q_debug_set returns 0, or -1 for an unknown knob; b200q_debug_reset unsets all knobs
  * of the calling thread.  (The reference's counterparts are environment variables read on
@@ -222,7 +220,6 @@ int b200q_debug_force_path(int path);
  */
 enum {
   B200Q_KNOB_FORCE_PATH = 0,       /* B200Q_PATH_* (same as b200q_debug_force_path) */
-  B200Q_KNOB_FLAGS = 1,            /* tcgen05 kernels: 1 skip epilogue arithmetic, 2 skip MMAs, 4 skip output stores */
   B200Q_KNOB_BN = 2,               /* single-CTA kernels: UMMA N */
   B200Q_KNOB_SPLITS = 3,           /* single-CTA kernels: split-K factor */
   B200Q_KNOB_CLUSTER = 4,          /* single-CTA kernels: cluster split-K size (1, 2, 4, 8) */

@@ -42,7 +42,6 @@ PATH_MMA_STREAM = 4
 
 # debug knobs (B200Q_KNOB_*): settings are private to the calling thread, unset at load
 KNOB_FORCE_PATH = 0
-KNOB_FLAGS = 1
 KNOB_BN = 2
 KNOB_SPLITS = 3
 KNOB_CLUSTER = 4

@@ -160,7 +160,6 @@ w8a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_a,
           const uint64_t b_desc = ptx::umma_desc_k_sw128(sb);
 #pragma unroll
           for (int k = 0; k < kBlockK / kUmmaK; ++k) {
-            if (p.debug_flags & 2) break;
             // advancing K by 32 bytes inside the swizzled row = +2 in 16-byte units
             ptx::umma_i8_ss(d_tmem, a_desc + 2u * k, b_desc + 2u * k, idesc,
                             (kb > kb0 || k > 0) ? 1u : 0u);
@@ -225,7 +224,7 @@ w8a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_a,
         ptx::mbar_arrive_cluster(ptx::map_to_cta(ptx::smem_u32(pfull_bar), 0));  // release: stores first
         continue;
       }
-      if (fast && !(p.debug_flags & 8)) {
+      if (fast) {
         // channel scales of this tile -> shared memory (while the main loop still runs)
         const int col = tile_b * p.bn + epi_tid;
         if (epi_tid < p.bn) ws_tile[epi_tid] = col < p.rows_b ? __ldg(p.w_scales + col) : 0.f;
@@ -283,13 +282,8 @@ w8a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_a,
       // issued as soon as the registers of group g have been converted, so they are in
       // flight while group g is written out.
       uint32_t va[32], vb[32];
-      if (p.debug_flags & 16) {
-#pragma unroll
-        for (int j = 0; j < 32; ++j) va[j] = vb[j] = j + lane;
-      }
       auto issue = [&](int g) {
         const int c = (half + 2 * g) * 2;  // first 32-column chunk of the group
-        if (p.debug_flags & 16) return;
         ptx::tmem_ld_32x32b_x32(taddr + c * 32, va);
         if (c + 1 < n_chunks_tile) ptx::tmem_ld_32x32b_x32(taddr + (c + 1) * 32, vb);
       };
@@ -298,10 +292,6 @@ w8a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_a,
         const int c = (half + 2 * g) * 2;
         const bool two = c + 1 < n_chunks_tile;
         ptx::tmem_ld_wait();
-        if (p.debug_flags & 1) {
-          if (g + 1 < my_groups) issue(g + 1);
-          continue;
-        }
         if (clustered) {
           add_partials(c * 32, va);
           if (two) add_partials(c * 32 + 32, vb);
@@ -318,7 +308,7 @@ w8a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_a,
           }
           if (g + 1 < my_groups) issue(g + 1);
           __syncwarp();
-          if (!(p.debug_flags & 4)) store_group<OutT>(p, slab, lane, row0, col0);
+          store_group<OutT>(p, slab, lane, row0, col0);
           __syncwarp();
         } else {
           consume(c * 32, va);
@@ -641,7 +631,6 @@ int launch_w8a8_umma(const GemmArgs& a, const UmmaPlan& plan) {
                     : nullptr;
   kp.status = a.status;
   kp.fast_store = fast_store ? 1 : 0;
-  kp.debug_flags = debug_knob(B200Q_KNOB_FLAGS, 0);
 
   cudaError_t e;
   if (a.acc_out != nullptr) {

@@ -97,7 +97,6 @@ struct PairParams {
   void* out;              // OutT [M, N] (int32 [M, N] for KIND_I8_RAW)
   int* status;
   uint32_t idesc;         // instruction descriptor (operand and accumulator formats)
-  int debug_flags;        // test hook: 1 = skip epilogue arithmetic, 4 = skip the output stores
 };
 
 // Row-parallel layers at prefill size: instead of its own output matrix, the SCATTER kernel
@@ -395,7 +394,6 @@ umma_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
 #pragma unroll
           for (int k = 0; k < kBlockBytes / kUmmaBytes; ++k) {
             const uint32_t acc = (kb > 0 || k > 0) ? 1u : 0u;
-            if (pp.debug_flags & 2) continue;  // test hook: time the pipeline without the MMAs
             if (KIND == KIND_F16)
               ptx::umma_f16_ss_pair(d_tmem, a_desc + 2u * k, b_desc + 2u * k, pp.idesc, acc);
             else
@@ -477,8 +475,8 @@ umma_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
         if (g < 3) ptx::tmem_ld_32x32b_x32(taddr + 32 * (g + 1), v[(g + 1) & 1]);
         const int col0 = tile_n * kPairBN + c0 + 32 * g;
         if (KIND == KIND_I8_RAW) {
-          if (!(pp.debug_flags & 4)) store_row_i32(reinterpret_cast<int32_t*>(pp.out), pp.M, pp.N, row, col0, v[g & 1]);
-        } else if (!(pp.debug_flags & 1)) {
+          store_row_i32(reinterpret_cast<int32_t*>(pp.out), pp.M, pp.N, row, col0, v[g & 1]);
+        } else {
           uint32_t packed[16];
           if (bias != nullptr)
             convert32<KIND, OutT, true>(ws_tile + c0 + 32 * g, a_s, bias, col0, pp.N, v[g & 1], packed);
@@ -495,13 +493,13 @@ umma_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
               ptx::fence_proxy_async_smem();
               __syncwarp();
               if (lane == 0) {
-                if (!(pp.debug_flags & 4) && row0 < pp.M && col0 - 32 < pp.N)
+                if (row0 < pp.M && col0 - 32 < pp.N)
                   ptx::tma_store_2d(&tmap_y, ptx::smem_u32(slab), (col0 - 32) * 2, row0);
                 ptx::bulk_commit_group();
               }
             } else {
               __syncwarp();
-              if (!(pp.debug_flags & 4)) store_slab_rows<OutT>(out, pp.M, pp.N, slab, lane, row0, col0 - 32);
+              store_slab_rows<OutT>(out, pp.M, pp.N, slab, lane, row0, col0 - 32);
               __syncwarp();
             }
           }
@@ -613,7 +611,6 @@ PairParams make_params(const GemmArgs& a, int k_bytes) {
   pp.bias = a.bias;
   pp.out = a.y;
   pp.status = a.status;
-  pp.debug_flags = debug_knob(B200Q_KNOB_FLAGS, 0);
   pp.m_fastest = a.N > a.M ? 1 : 0;
   return pp;
 }
@@ -677,7 +674,6 @@ int launch_w8a8_umma_pair_scatter(const GemmArgs& a, void* const* peer_stage, in
   PairParams pp = make_params(a, a.K);
   pp.out = nullptr;
   pp.idesc = ptx::umma_idesc(2u, 1u, 2 * kTileRows, kPairBN);
-  pp.debug_flags = 0;
   ScatterParams sp{};
   for (int r = 0; r < world; ++r) sp.stage[r] = peer_stage[r];
   sp.rank = rank;

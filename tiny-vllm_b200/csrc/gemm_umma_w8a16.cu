@@ -212,12 +212,10 @@ w8a16_umma_kernel(const __grid_constant__ CUtensorMap tmap_x,
         }
         const uint8_t* raw = smem + stage * stage_bytes + tile16_bytes;
         uint8_t* dst = conv_base + cb * conv_bytes;
-        if (!(p.debug_flags & 8)) {
-          if (rows8 * 4 <= kConvThreads) {
-            if (ctid < rows8 * 4) expand_quarter_row<T>(raw, dst, ctid >> 2, ctid & 3);
-          } else {
-            for (int r = ctid; r < rows8; r += kConvThreads) expand_row<T>(raw, dst, r);
-          }
+        if (rows8 * 4 <= kConvThreads) {
+          if (ctid < rows8 * 4) expand_quarter_row<T>(raw, dst, ctid >> 2, ctid & 3);
+        } else {
+          for (int r = ctid; r < rows8; r += kConvThreads) expand_row<T>(raw, dst, r);
         }
         ptx::fence_proxy_async_smem();  // generic-proxy writes -> visible to the UMMA reads
         __syncwarp();
@@ -305,10 +303,6 @@ w8a16_umma_kernel(const __grid_constant__ CUtensorMap tmap_x,
         const int c = 2 * g;
         const bool two = c + 1 < n_chunks_tile;
         ptx::tmem_ld_wait();
-        if (p.debug_flags & 1) {
-          if (g + 1 < n_groups) issue(g + 1);
-          continue;
-        }
         if (fast) {
           const int row0 = tile_a * kTileA + quarter * 32;
           const int col0 = tile_b * p.bn + c * 32;
@@ -498,7 +492,6 @@ int launch_w8a16_umma(const GemmArgs& a, const UmmaPlan& plan) {
                     : nullptr;
   kp.status = a.status;
   kp.fast_store = (!plan.swap && plan.splits == 1 && (a.N % 8) == 0 && (plan.bn % 64) == 0) ? 1 : 0;
-  kp.debug_flags = debug_knob(B200Q_KNOB_FLAGS, 0);
 
   cudaError_t e = a.dtype == B200Q_DTYPE_BF16
                       ? launch_kernel<__nv_bfloat16>(tx, tw, kp, plan, a.stream)

@@ -66,7 +66,6 @@ struct TsParams {
   const void* bias;
   void* out;
   int* status;
-  int debug_flags;             // test-only: 1 = skip epilogue work, 8 = skip the expansion
 };
 
 template <typename T>
@@ -221,8 +220,7 @@ w8a16_umma_ts_kernel(const __grid_constant__ CUtensorMap tmap_x,
         uint32_t v[32];
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-          uint4 w = make_uint4(0u, 0u, 0u, 0u);
-          if (!(p.debug_flags & 8)) w = *reinterpret_cast<const uint4*>(src_row + ((c ^ sw8) << 4));
+          const uint4 w = *reinterpret_cast<const uint4*>(src_row + ((c ^ sw8) << 4));
           const uint2 e0 = expand4_scaled<T>(w.x), e1 = expand4_scaled<T>(w.y), e2 = expand4_scaled<T>(w.z),
                       e3 = expand4_scaled<T>(w.w);
           v[8 * c + 0] = e0.x;
@@ -260,7 +258,7 @@ w8a16_umma_ts_kernel(const __grid_constant__ CUtensorMap tmap_x,
       const int tile_tok = item / p.tiles_ch;
       if (alive) alive = ptx::warp_all(ptx::mbar_wait(ptx::smem_u32(tfull_bar), static_cast<uint32_t>(it) & 1u, abort_flag));
       if (!alive) {   // a warp whose wait ran out goes on to meet the others of its group at their barriers
-        for (int c = 0; c < kTsTokens / 32 && !(p.debug_flags & 1); ++c) ptx::named_bar_sync(2 + t, kEpiThreads);
+        for (int c = 0; c < kTsTokens / 32; ++c) ptx::named_bar_sync(2 + t, kEpiThreads);
         continue;
       }
       ptx::tc_fence_after_sync();
@@ -276,7 +274,6 @@ w8a16_umma_ts_kernel(const __grid_constant__ CUtensorMap tmap_x,
         uint32_t v[32];
         ptx::tmem_ld_32x32b_x32(taddr + c * 32, v);
         ptx::tmem_ld_wait();
-        if (p.debug_flags & 1) continue;
         T* buf = reinterpret_cast<T*>(my_stage + (round & 1) * kTsStageOutBytes);
 #pragma unroll
         for (int j = 0; j < 32; ++j)
@@ -362,7 +359,6 @@ int launch_w8a16_umma_ts(const GemmArgs& a) {
   tp.bias = a.bias;
   tp.out = a.y;
   tp.status = a.status;
-  tp.debug_flags = debug_knob(B200Q_KNOB_FLAGS, 0);
   const long long items = static_cast<long long>(tp.tiles_ch) * tp.tiles_tok;
   const int grid = static_cast<int>(std::min<long long>(items, sm_count()));
   cudaError_t e = a.dtype == B200Q_DTYPE_BF16 ? launch_ts<__nv_bfloat16>(tx, tw, tp, grid, a.stream)

@@ -60,8 +60,6 @@ struct ExchangeParams {
   int M, K, rank, world, rows_per_rank;
   int* status;
   long long wait_limit;
-  int debug_flags;  // test hook (timing only, results wrong): 64 = codes to the own buffer only,
-                    // 128 = read the own partial in place of the peers'
 };
 
 template <typename T, int G, int CHUNKS, int W>
@@ -116,7 +114,7 @@ tp_reduce_norm_quant_kernel(const ExchangeParams p) {
       for (int r = 0; r < W; ++r) {
         part[c][r] = make_uint4(0u, 0u, 0u, 0u);
         if (r < p.world && live)
-          part[c][r] = ld_peer16(static_cast<const T*>(p.partial[(p.debug_flags & 128) ? p.rank : r]) +
+          part[c][r] = ld_peer16(static_cast<const T*>(p.partial[r]) +
                                  static_cast<size_t>(row) * p.K + idx * 8);
       }
       if (live && p.residual_in != nullptr)
@@ -191,7 +189,7 @@ tp_reduce_norm_quant_kernel(const ExchangeParams p) {
           const uint2 q = quant8<T>(y[c], scale, inv_scale);
 #pragma unroll
           for (int r = 0; r < W; ++r)
-            if (r < p.world && (!(p.debug_flags & 64) || r == p.rank))
+            if (r < p.world)
               *(reinterpret_cast<uint2*>(p.xq[r] + static_cast<size_t>(row) * p.K) + idx) = q;
           if (p.y_out != nullptr)
             *(reinterpret_cast<uint4*>(static_cast<T*>(p.y_out) + static_cast<size_t>(local_row) * p.K) + idx) = y[c];
@@ -317,7 +315,6 @@ extern "C" int b200q_tp_reduce_rmsnorm_quant(void* const* peer_partials, void* c
   p.rows_per_rank = M / world;
   p.status = device_status_ptr();
   p.wait_limit = peer_wait_limit_cycles();
-  p.debug_flags = debug_knob(B200Q_KNOB_FLAGS, 0);
   if (p.status == nullptr) return B200Q_ERR_LAUNCH;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   cudaError_t e = dtype == B200Q_DTYPE_BF16 ? launch_exchange_w<__nv_bfloat16>(p, st)

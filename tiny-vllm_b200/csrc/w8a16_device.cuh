@@ -49,7 +49,6 @@ struct KernelParams {
   unsigned int* counters;
   int* status;
   int fast_store;
-  int debug_flags;
 };
 
 template <typename T>

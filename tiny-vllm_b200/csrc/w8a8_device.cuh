@@ -45,7 +45,6 @@ struct KernelParams {
   int32_t* partials;
   unsigned int* counters;
   int* status;
-  int debug_flags;         // test-only: 1 = skip epilogue work, 2 = skip UMMA issue
   int fast_store;          // 1: 16-bit outputs are transposed through shared memory and stored as full 128-byte rows
 };
 
