@@ -86,7 +86,7 @@ int* device_status_ptr();
 // An SM divides its memory between L1 and shared memory by the kernel that starts on it and cannot change that while
 // CTAs run.  A kernel that would leave most of it to L1, and stands between two that need nearly all of it as shared memory,
 // keeps the second one off its SMs until it has ended; so does one with less of its own.  MAX_SHARED asks for the division
-// that those need: for the tcgen05 and ring kernels and for what quantises their activations (256 tokens of the 0.6B
+// that those need: for the tcgen05 (from 33 tokens on) and ring kernels and for what quantises their activations (256 tokens of the 0.6B
 // model, W8A8, 376 -> 359 us), not for the kernels that live on L1 (16 tokens, weights in registers, 129 -> 157 us).
 enum Carveout { DEFAULT_SPLIT = 0, MAX_SHARED = 1 };
 

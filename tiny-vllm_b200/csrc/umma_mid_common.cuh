@@ -142,8 +142,11 @@ cudaError_t launch_mid_kernel(int ctas, int splits, size_t smem, cudaStream_t st
     if (per_sm > 2) return cudaErrorInvalidConfiguration;
     if (dev < 64) attr_set[dev] = true;
   }
-  return launch_clustered(MAX_SHARED, splits, true, kernel, dim3(ctas), dim3(kMidThreads), smem, stream, maps.x, maps.w,
-                          maps.x3, maps.w3, mp);
+  // Up to 32 tokens the neighbours may be kernels that live on L1 (reg_decode_preferred), and these leave an SM's memory
+  // divided as it is: layers of 17 to 32 tokens with MAX_SHARED / without, W8A16 of hidden 1792 and 2048 1.03-1.045, W8A8 on codes of the 0.6B
+  // model and of an eighth of the 8B one 1.05-1.09, with a quantiser 1.00-1.025, elsewhere 0.985-1.01.
+  return launch_clustered(mp.M > 32 ? MAX_SHARED : DEFAULT_SPLIT, splits, true, kernel, dim3(ctas), dim3(kMidThreads), smem,
+                          stream, maps.x, maps.w, maps.x3, maps.w3, mp);
 }
 
 }  // namespace b200q
