@@ -77,7 +77,10 @@ def test_a_warp_goes_on_or_gives_up_as_one(path):
             waits_only = re.match(r"\s*%s = %s;" % (name, WAIT), then)
             one_lane = re.match(r"(?:ptx::elect_one\(\)|lane == \w+) && %s$" % name, cond)
             own_count = re.match(r"%s && \+\+\w+ == " % name, cond)      # the lane's own place in the ring
-            assert waits_only or one_lane or own_count, cond
+            # a template argument: true in the form without the vote, and the flag is the warp's in the other
+            no_branch = cond == "X_SMEM || alive" and re.search(r"if constexpr \(X_SMEM\) \{\s*if \(alive\) alive = %s;" % WAIT, code)
+            voted = re.match(r"\s*alive = ptx::warp_all\(", then)
+            assert waits_only or one_lane or own_count or no_branch or voted, cond
     for m in re.finditer(r"(?<!void )\bproduce\(&", code):
         assert re.search(r"if \(lane < kPipes\)\s*$", code[:m.start()])
 

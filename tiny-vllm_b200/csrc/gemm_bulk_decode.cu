@@ -36,9 +36,9 @@
 //         (nanovllm/quantization/csrc/int8_weight_only_gemm.cu:258-292)
 // At most 8 tokens have a kernel of their own (stream_decode_m8_kernel).
 // Rows and columns outside the matrices are zero-filled by TMA, so ragged K needs no masks.
-// Every mbarrier wait is bounded.  A lane whose wait ran out no longer waits or frees slots, but its warp goes through its
-// loops on whatever the ring holds and meets the others at their barriers; the status word reports it, and the
-// producer lanes stop and wait, again bounded, for the tiles they still have in flight.
+// Every mbarrier wait is bounded; a wait that runs out stops the CTA's loops (the consumer
+// warps still meet at their barriers), is reported through the status word, and the producer
+// lanes wait, again bounded, for the tiles they still have in flight.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -246,27 +246,29 @@ w8a8_stream_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const int8_t
     auto segment = [&](const uint4 (&xv)[MT][4]) {
       const int slot = it % p.slots;
       if (alive)
-        alive = ptx::mbar_wait(ptx::smem_u32(full + slot), static_cast<uint32_t>((it / p.slots) & 1),
-                               sm.abort_flag);
-      const uint8_t* ws = ring + slot * p.slot_bytes;
+        alive = ptx::warp_all(ptx::mbar_wait(ptx::smem_u32(full + slot), static_cast<uint32_t>((it / p.slots) & 1),
+                                             sm.abort_flag));
+      if (alive) {
+        const uint8_t* ws = ring + slot * p.slot_bytes;
 #pragma unroll
-      for (int j = 0; j < NTW; ++j) {
-        const int jj = part * NTW + j;  // tile of the unit
-        if (jj * 8 < rows) {
-          const uint4 w0 = *reinterpret_cast<const uint4*>(ws + jj * 1024 + o0);
-          const uint4 w1 = *reinterpret_cast<const uint4*>(ws + jj * 1024 + o1);
+        for (int j = 0; j < NTW; ++j) {
+          const int jj = part * NTW + j;  // tile of the unit
+          if (jj * 8 < rows) {
+            const uint4 w0 = *reinterpret_cast<const uint4*>(ws + jj * 1024 + o0);
+            const uint4 w1 = *reinterpret_cast<const uint4*>(ws + jj * 1024 + o1);
 #pragma unroll
-          for (int m = 0; m < MT; ++m) {
-            // each pair of words is one k32 step: slots 4t..4t+3 and 16+4t..16+4t+3
-            mma_s8(acc[m][j], xv[m][0].x, xv[m][2].x, xv[m][0].y, xv[m][2].y, w0.x, w0.y);
-            mma_s8(acc[m][j], xv[m][0].z, xv[m][2].z, xv[m][0].w, xv[m][2].w, w0.z, w0.w);
-            mma_s8(acc[m][j], xv[m][1].x, xv[m][3].x, xv[m][1].y, xv[m][3].y, w1.x, w1.y);
-            mma_s8(acc[m][j], xv[m][1].z, xv[m][3].z, xv[m][1].w, xv[m][3].w, w1.z, w1.w);
+            for (int m = 0; m < MT; ++m) {
+              // each pair of words is one k32 step: slots 4t..4t+3 and 16+4t..16+4t+3
+              mma_s8(acc[m][j], xv[m][0].x, xv[m][2].x, xv[m][0].y, xv[m][2].y, w0.x, w0.y);
+              mma_s8(acc[m][j], xv[m][0].z, xv[m][2].z, xv[m][0].w, xv[m][2].w, w0.z, w0.w);
+              mma_s8(acc[m][j], xv[m][1].x, xv[m][3].x, xv[m][1].y, xv[m][3].y, w1.x, w1.y);
+              mma_s8(acc[m][j], xv[m][1].z, xv[m][3].z, xv[m][1].w, xv[m][3].w, w1.z, w1.w);
+            }
           }
         }
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(empty + slot));
       }
-      __syncwarp();
-      if (lane == 0 && alive) ptx::mbar_arrive(ptx::smem_u32(empty + slot));
       ++it;
     };
     for (int c = 0; c < my_segs; ++c) {
@@ -385,33 +387,35 @@ w8a16_stream_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const T* x,
       if (c + 1 < my_segs || u + 1 < p.units) load_x(c + 1 < my_segs ? c + 1 : 0, na, nb);
       const int slot = it % p.slots;
       if (alive)
-        alive = ptx::mbar_wait(ptx::smem_u32(full + slot), static_cast<uint32_t>((it / p.slots) & 1),
-                               sm.abort_flag);
-      const uint8_t* ws = ring + slot * p.slot_bytes;
+        alive = ptx::warp_all(ptx::mbar_wait(ptx::smem_u32(full + slot), static_cast<uint32_t>((it / p.slots) & 1),
+                                             sm.abort_flag));
+      if (alive) {
+        const uint8_t* ws = ring + slot * p.slot_bytes;
 #pragma unroll
-      for (int j = 0; j < NTW; ++j) {
-        const int jj = part * NTW + j;  // tile of the unit
-        if (jj * 8 < rows) {
-          const uint4 w0 = *reinterpret_cast<const uint4*>(ws + jj * 1024 + o0);
-          const uint4 w1 = *reinterpret_cast<const uint4*>(ws + jj * 1024 + o1);
-          const uint2 e0 = expand4_scaled<T>(w0.x), e1 = expand4_scaled<T>(w0.y), e2 = expand4_scaled<T>(w0.z),
-                      e3 = expand4_scaled<T>(w0.w), e4 = expand4_scaled<T>(w1.x), e5 = expand4_scaled<T>(w1.y),
-                      e6 = expand4_scaled<T>(w1.z), e7 = expand4_scaled<T>(w1.w);
+        for (int j = 0; j < NTW; ++j) {
+          const int jj = part * NTW + j;  // tile of the unit
+          if (jj * 8 < rows) {
+            const uint4 w0 = *reinterpret_cast<const uint4*>(ws + jj * 1024 + o0);
+            const uint4 w1 = *reinterpret_cast<const uint4*>(ws + jj * 1024 + o1);
+            const uint2 e0 = expand4_scaled<T>(w0.x), e1 = expand4_scaled<T>(w0.y), e2 = expand4_scaled<T>(w0.z),
+                        e3 = expand4_scaled<T>(w0.w), e4 = expand4_scaled<T>(w1.x), e5 = expand4_scaled<T>(w1.y),
+                        e6 = expand4_scaled<T>(w1.z), e7 = expand4_scaled<T>(w1.w);
 #pragma unroll
-          for (int m = 0; m < MT; ++m) {
-            mma_16<T>(acc[m][j], ca[m][0].x, cb[m][0].x, ca[m][0].y, cb[m][0].y, e0.x, e0.y);
-            mma_16<T>(acc[m][j], ca[m][0].z, cb[m][0].z, ca[m][0].w, cb[m][0].w, e1.x, e1.y);
-            mma_16<T>(acc[m][j], ca[m][1].x, cb[m][1].x, ca[m][1].y, cb[m][1].y, e2.x, e2.y);
-            mma_16<T>(acc[m][j], ca[m][1].z, cb[m][1].z, ca[m][1].w, cb[m][1].w, e3.x, e3.y);
-            mma_16<T>(acc[m][j], ca[m][2].x, cb[m][2].x, ca[m][2].y, cb[m][2].y, e4.x, e4.y);
-            mma_16<T>(acc[m][j], ca[m][2].z, cb[m][2].z, ca[m][2].w, cb[m][2].w, e5.x, e5.y);
-            mma_16<T>(acc[m][j], ca[m][3].x, cb[m][3].x, ca[m][3].y, cb[m][3].y, e6.x, e6.y);
-            mma_16<T>(acc[m][j], ca[m][3].z, cb[m][3].z, ca[m][3].w, cb[m][3].w, e7.x, e7.y);
+            for (int m = 0; m < MT; ++m) {
+              mma_16<T>(acc[m][j], ca[m][0].x, cb[m][0].x, ca[m][0].y, cb[m][0].y, e0.x, e0.y);
+              mma_16<T>(acc[m][j], ca[m][0].z, cb[m][0].z, ca[m][0].w, cb[m][0].w, e1.x, e1.y);
+              mma_16<T>(acc[m][j], ca[m][1].x, cb[m][1].x, ca[m][1].y, cb[m][1].y, e2.x, e2.y);
+              mma_16<T>(acc[m][j], ca[m][1].z, cb[m][1].z, ca[m][1].w, cb[m][1].w, e3.x, e3.y);
+              mma_16<T>(acc[m][j], ca[m][2].x, cb[m][2].x, ca[m][2].y, cb[m][2].y, e4.x, e4.y);
+              mma_16<T>(acc[m][j], ca[m][2].z, cb[m][2].z, ca[m][2].w, cb[m][2].w, e5.x, e5.y);
+              mma_16<T>(acc[m][j], ca[m][3].x, cb[m][3].x, ca[m][3].y, cb[m][3].y, e6.x, e6.y);
+              mma_16<T>(acc[m][j], ca[m][3].z, cb[m][3].z, ca[m][3].w, cb[m][3].w, e7.x, e7.y);
+            }
           }
         }
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(empty + slot));
       }
-      __syncwarp();
-      if (lane == 0 && alive) ptx::mbar_arrive(ptx::smem_u32(empty + slot));
 #pragma unroll
       for (int m = 0; m < MT; ++m)
 #pragma unroll
@@ -564,39 +568,47 @@ stream_decode_m8_kernel(const __grid_constant__ CUtensorMap tm_w, const X* x, co
         for (int j = 0; j < kXP; ++j) xc[j] = xn[j];
         load_x(c + 1 < my_segs ? c + 1 : 0, xn);
       }
-      if (alive) alive = ptx::mbar_wait(full + slot * 8, phase, sm.abort_flag);
-      const uint8_t* ws = ring + slot * p.slot_bytes;
-      uint4 a[NQ], b[NQ];
-#pragma unroll
-      for (int q = 0; q < NQ; ++q) {
-        // channel 16 q + g (tile 2 q) and channel 16 q + 8 + g (tile 2 q + 1)
-        a[q] = *reinterpret_cast<const uint4*>(ws + (2 * q) * 1024);
-        b[q] = *reinterpret_cast<const uint4*>(ws + (2 * q + 1) * 1024);
+      // as a warp, by a vote where activations come from L2 on the way, else without (us, 1 token, staged: 8B, 16 linears
+      // 160.7 with votes, 159.4 without; 7 tokens, not staged, 8 linears 101.7 and 102.8)
+      if constexpr (X_SMEM) {
+        if (alive) alive = ptx::mbar_wait(full + slot * 8, phase, sm.abort_flag);
+      } else {
+        if (alive) alive = ptx::warp_all(ptx::mbar_wait(full + slot * 8, phase, sm.abort_flag));
       }
-      if (X_SMEM) load_x(c, xc);
-      // The slot may be overwritten once the loads have RETURNED: neither the barrier's release nor __syncwarp waits
-      // for a load in flight, and the refill does not come through the pipe of the loads.  So the arrival depends
-      // on a word of each of them (which lane arrives does not matter).
-      uint32_t seen = 0;
+      if (X_SMEM || alive) {
+        const uint8_t* ws = ring + slot * p.slot_bytes;
+        uint4 a[NQ], b[NQ];
 #pragma unroll
-      for (int q = 0; q < NQ; ++q) seen |= a[q].x | b[q].x;
-      const int who = __any_sync(0xFFFFFFFFu, seen == 0u) ? 1 : 0;
-      if (lane == who && alive) ptx::mbar_arrive(empty + slot * 8);
+        for (int q = 0; q < NQ; ++q) {
+          // channel 16 q + g (tile 2 q) and channel 16 q + 8 + g (tile 2 q + 1)
+          a[q] = *reinterpret_cast<const uint4*>(ws + (2 * q) * 1024);
+          b[q] = *reinterpret_cast<const uint4*>(ws + (2 * q + 1) * 1024);
+        }
+        if (X_SMEM) load_x(c, xc);
+        // The slot may be overwritten once the loads have RETURNED: neither the barrier's release nor __syncwarp waits
+        // for a load in flight, and the refill does not come through the pipe of the loads.  So the arrival depends
+        // on a word of each of them (which lane arrives does not matter).
+        uint32_t seen = 0;
 #pragma unroll
-      for (int q = 0; q < NQ; ++q) {
-        if constexpr (kA8) {
-          mma_s8(acc[q], a[q].x, b[q].x, a[q].y, b[q].y, xc[0].x, xc[0].y);
-          mma_s8(acc[q], a[q].z, b[q].z, a[q].w, b[q].w, xc[0].z, xc[0].w);
-        } else {
-          // weight word i of the piece meets activation words 2 i and 2 i + 1
-          uint2 ea = expand4_scaled<T>(a[q].x), eb = expand4_scaled<T>(b[q].x);
-          mma_16<T>(acc[q], ea.x, eb.x, ea.y, eb.y, xc[0].x, xc[0].y);
-          ea = expand4_scaled<T>(a[q].y); eb = expand4_scaled<T>(b[q].y);
-          mma_16<T>(acc[q], ea.x, eb.x, ea.y, eb.y, xc[0].z, xc[0].w);
-          ea = expand4_scaled<T>(a[q].z); eb = expand4_scaled<T>(b[q].z);
-          mma_16<T>(acc[q], ea.x, eb.x, ea.y, eb.y, xc[1].x, xc[1].y);
-          ea = expand4_scaled<T>(a[q].w); eb = expand4_scaled<T>(b[q].w);
-          mma_16<T>(acc[q], ea.x, eb.x, ea.y, eb.y, xc[1].z, xc[1].w);
+        for (int q = 0; q < NQ; ++q) seen |= a[q].x | b[q].x;
+        const int who = __any_sync(0xFFFFFFFFu, seen == 0u) ? 1 : 0;
+        if (lane == who && alive) ptx::mbar_arrive(empty + slot * 8);
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+          if constexpr (kA8) {
+            mma_s8(acc[q], a[q].x, b[q].x, a[q].y, b[q].y, xc[0].x, xc[0].y);
+            mma_s8(acc[q], a[q].z, b[q].z, a[q].w, b[q].w, xc[0].z, xc[0].w);
+          } else {
+            // weight word i of the piece meets activation words 2 i and 2 i + 1
+            uint2 ea = expand4_scaled<T>(a[q].x), eb = expand4_scaled<T>(b[q].x);
+            mma_16<T>(acc[q], ea.x, eb.x, ea.y, eb.y, xc[0].x, xc[0].y);
+            ea = expand4_scaled<T>(a[q].y); eb = expand4_scaled<T>(b[q].y);
+            mma_16<T>(acc[q], ea.x, eb.x, ea.y, eb.y, xc[0].z, xc[0].w);
+            ea = expand4_scaled<T>(a[q].z); eb = expand4_scaled<T>(b[q].z);
+            mma_16<T>(acc[q], ea.x, eb.x, ea.y, eb.y, xc[1].x, xc[1].y);
+            ea = expand4_scaled<T>(a[q].w); eb = expand4_scaled<T>(b[q].w);
+            mma_16<T>(acc[q], ea.x, eb.x, ea.y, eb.y, xc[1].z, xc[1].w);
+          }
         }
       }
       if (++slot == p.slots) {

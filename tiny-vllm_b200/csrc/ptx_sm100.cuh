@@ -75,8 +75,9 @@ constexpr long long kWaitLimitCycles = 2000000000LL;
 // The lanes of a warp may get different answers: the limit runs out for one while the phase completes for another.  So a
 // warp that waits together votes (warp_all), or its lanes go on together whatever the answer, with no branch around an
 // instruction of the warp (elect, votes, mma.sync, tcgen05.ld / st, barriers), and one whose wait ran out no longer waits,
-// signals or issues.  Votes cost nothing in an issuer that takes one for all waits of a step; a vote for every wait of
-// issuers, producers and converters cost 1.5-2 % of a decode step of 256 or 512 tokens.
+// signals or issues.  A vote costs nothing in an issuer that takes one for all waits of a step and, per tile of the rings, at
+// most what the second form does (W8A16, 2 to 8 tokens 0.3-1.5 against 0.6-3.7 %); a vote for every wait of issuers,
+// producers and converters cost 1.5-2 % of a decode step of 256 or 512 tokens, so producers and converters take the second.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
   if (mbar_try_wait(bar, parity)) return true;
   const long long t0 = clock64();
