@@ -26,7 +26,8 @@
 //
 // The epilogue: eight warps, each 32 rows x 128 columns of a tile, 32 at a time: the next 32 accumulators are on their
 // way while these are converted, and the TMEM buffer goes back to the issuer before the last 32 are.  The scales are
-// fetched a tile ahead.  (Sixteen warps that took 64 columns at once were no faster: 8192 x 4096 x 1024 34 us either way.)
+// fetched a tile ahead.  (Sixteen warps that took 64 columns at once and spilled: a round of 74 tiles
+// 3.9 us at K = 512, 4.1 at 1024, 6.7 at 2048; eight 3.3, 4.0, 6.7.)
 // What counts for the calls as a user makes them is what stands beside the kernel: ten warps of 128 registers and 218 KB (of
 // which it needs 194: kPairSmem) leave room on every SM for the CTAs of the kernel that quantises the activations, so that this one is set up, with its first
 // weights in the ring, when they are ready, and the next quantiser's CTAs are there when this one ends.  Quantiser and
