@@ -211,9 +211,10 @@ int b200q_version(void);
 int b200q_debug_force_path(int path);
 
 /*
- * Test and tuning knobs.  A knob changes which kernel variant runs or how a problem is tiled, never what is
- * computed.  All knobs are unset when the library is loaded, nothing is read from the environment, and a setting is private to the thread
- * that made it: a serving process that never calls b200q_debug_set() cannot be affected.
+ * Test and tuning knobs.  A knob changes which kernel variant runs or how a problem is tiled,
+ * never what is computed.  All knobs are unset when the library is loaded, nothing is read from
+ * the environment, and a setting is private to the thread that made it: a serving process that
+ * never calls b200q_debug_set() cannot be affected.
  * b200q_debug_set returns 0, or -1 for an unknown knob; b200q_debug_reset unsets all knobs
  * of the calling thread.  (The reference's counterparts are environment variables read on
  * every forward: nanovllm/quantization/cuda.py:46-53,249.)
